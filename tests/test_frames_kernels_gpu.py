@@ -1,0 +1,81 @@
+"""Frame kernels at the edges of their tiles: the rewind grid's product (64 rows of (path,
+axis) x 72 rewind rows, chunks of 8 frequencies), the warp-wide crossing search and the
+three-steps-a-pass refinement, against the same search in numpy."""
+
+import math
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+# float32 records: an offset is evaluated here at the recorded (rounded) z_emit, so it is
+# off by the offset's slope (below 100 on these windows) times half an ulp of z (6e-8 z)
+TOL = 2e-5
+
+
+def _dump(n, nw, bmax, seed):
+    r = np.random.default_rng(seed)
+    b = np.stack([np.stack([np.sort(r.choice(np.arange(2, bmax + 1), nw, replace=False))
+                            for _ in range(2)]) for _ in range(n)]).astype(float)
+    w = r.dirichlet(np.ones(nw), (n, 2))
+    a = w / b * r.choice([-1.0, 1.0], (n, 2, nw))
+    f = np.where(b % 2 == 0, r.uniform(0, math.pi, b.shape), 0.0)
+    return r.uniform(-1, 1, (n, 2)), a, b, f
+
+
+def _x(a2, a, b, f, z):
+    """Comoving positions [n][2] + shape of z."""
+    s = a2[..., None] * np.sin(z)
+    for j in range(a.shape[-1]):
+        s = s + a[..., j, None] * (np.sin(b[..., j, None] * z + f[..., j, None]) - np.sin(f[..., j, None]))
+    return s / np.sin(z)
+
+
+def _reach(z, z_obs, bmax):
+    b = np.arange(2, bmax + 1)[:, None]
+    da = (np.cos(b * z) - 1) / (b * np.sin(z)) - (np.cos(b * z_obs) - 1) / (b * np.sin(z_obs))
+    db = np.sin(b * z) / (b * np.sin(z)) - np.sin(b * z_obs) / (b * np.sin(z_obs))
+    return np.where(b % 2 == 0, np.hypot(da, db), np.abs(db)).max(0)
+
+
+@pytest.mark.parametrize("n,nw,bmax,front", [
+    (1, 1, 2, "fit"), (31, 6, 7, "speed"), (32, 7, 8, "fit"), (33, 8, 9, "fit"), (65, 23, 24, "fit"),
+    (7, 14, 15, "budget"),
+    (5, 255, 256, "budget"),   # 513 rewind rows: a last column tile of 9
+    (40, 1, 64, "fit"),        # few terms: summed directly
+])
+def test_hits_are_the_crossings_of_the_rewind_grid(ug, n, nw, bmax, front):
+    from ugb200.frames import bake
+
+    a2, a, b, f = _dump(n, nw, bmax, 100 * n + nw)
+    at, K, z_min, z_obs = (0.13, -0.29), 2, 0.05 * math.pi, 0.4 * math.pi
+    bk = bake(a2, a, b, f, observers=[("point", *at)], from_pi=0.4, to_pi=0.4, frames=1, zmin_pi=0.05,
+              front=front, metric="square", speed=0.33, wraps=K)
+    h = bk.hits[0][0]
+    top = int(max(2, b.max()))
+    i = np.arange(421 if front != "budget" else min(4000, max(420, 2 * top)) + 1)
+    eta = lambda z: np.log(np.tan(z / 2))  # noqa: E731
+    if front == "budget":
+        z = z_obs - (z_obs - z_min) * i / i[-1]
+        chi = _reach(z, z_obs, top)
+    else:
+        speed = 0.33 if front == "speed" else -1 / eta(z_min)
+        chi = speed * (eta(z_obs) - eta(z_min)) * i / i[-1]
+        z = 2 * np.arctan(np.exp(eta(z_obs) - chi / speed))
+    x = _x(a2, a, b, f, z)
+    want = np.zeros(n, int)
+    for nx in range(-K, K + 1):
+        for ny in range(-K, K + 1):
+            dmin = max(0.0, 2.0 * max(abs(nx), abs(ny)) - 4.0)
+            if dmin >= chi.max():
+                continue
+            i0 = 1 if front == "budget" else max(1, math.ceil(dmin * i[-1] / chi.max()))
+            g = np.abs(x + np.array([2 * nx - at[0], 2 * ny - at[1]])[:, None]).max(1) - chi
+            want += ((g[:, i0 - 1:-1] < 0) != (g[:, i0:] < 0)).sum(1)
+    assert np.array_equal(np.bincount(h["src"], minlength=n), want)
+    # each hit is an image of its source at its emission, on the front
+    d = _x(a2[h["src"]], a[h["src"]], b[h["src"]], f[h["src"]], h["z_emit"].astype(float)[:, None, None])[..., 0] - at
+    off = np.stack([h["dx"], h["dy"]], 1) - d
+    assert np.abs(off - 2 * np.round(off / 2)).max() < TOL
+    np.testing.assert_allclose(np.maximum(np.abs(h["dx"]), np.abs(h["dy"])), h["chi"], atol=TOL)

@@ -48,11 +48,13 @@ struct FPaths {
     const double* b;       // [n][2][nw]
     const double* f;       // [n][2][nw]
     const double2* coef;   // [n][2][bmax+1] a_b e^{i f_b} (Horner form)
+    const double* amp;     // [n] largest sum_j |a_j| of the axes
 };
 
 struct FFront {
     int budget, cheb, M, bMax;
     double spd, zObs, etaObs, chiMax;
+    const double2* reach;  // budget: terms of frequency b at z_obs (k_fb_reach)
 };
 
 __host__ __device__ inline double wiggle_direct(const double* a, const double* b, const double* f, int nw,
@@ -88,7 +90,7 @@ __device__ inline void comov(const FPaths& P, int p, double z, double* X, double
 }
 
 // Wiggle-budget reach of the front (frame_bake.cu:236-251).
-__host__ __device__ inline double reach_of(double z, double zObs, int bMax) {
+inline double reach_of(double z, double zObs, int bMax) {
     const double s = sin(z), sObs = sin(zObs);
     double best = 0.0;
     for (int b = 2; b <= bMax; b++) {
@@ -100,63 +102,170 @@ __host__ __device__ inline double reach_of(double z, double zObs, int bMax) {
     return best;
 }
 
+// reach_of with its z_obs terms (x: cosine, y: sine) tabulated once per frame.
+__device__ inline double reach_tab(const FFront& F, double z) {
+    const double s = sin(z);
+    double best = 0.0;
+    for (int b = 2; b <= F.bMax; b++) {
+        const double2 o = __ldg(F.reach + b);
+        double sb, cb;
+        sincos(b * z, &sb, &cb);
+        const double da = (cb - 1.0) / (b * s) - o.x;
+        const double db = sb / (b * s) - o.y;
+        const double d = (b % 2 == 0) ? sqrt(da * da + db * db) : fabs(db);
+        best = d > best ? d : best;
+    }
+    return best;
+}
+
+__global__ void k_fb_reach(int bMax, double zObs, double2* reach) {
+    const double sObs = sin(zObs);
+    for (int b = 2 + blockIdx.x * blockDim.x + threadIdx.x; b <= bMax; b += gridDim.x * blockDim.x)
+        reach[b] = make_double2((cos(b * zObs) - 1.0) / (b * sObs), sin(b * zObs) / (b * sObs));
+}
+
 __device__ inline double metric(double dx, double dy, int cheb) {
     return cheb ? fmax(fabs(dx), fabs(dy)) : sqrt(dx * dx + dy * dy);
 }
 
-// Rewind-grid positions, one thread per (path, 4 consecutive rows): four
-// independent Horner chains per thread (each row the same operations as comov).
+// Rewind-grid positions of few-term dumps, one thread per (path, row): a sine per term.
 __global__ void k_fb_grid(FPaths P, int M, const double* zg, double* px, double* py) {
-    const int R = M + 1, G = (R + 3) / 4;
-    const int64_t total = (int64_t)P.n * G;
+    const int R = M + 1;
+    const int64_t total = (int64_t)P.n * R;
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total;
          i += (int64_t)gridDim.x * blockDim.x) {
-        const int p = (int)(i / G), r0 = (int)(i % G) * 4;
-        double z[4], s[4], w[2][4];
-#pragma unroll
-        for (int q = 0; q < 4; q++) {
-            z[q] = zg[min(r0 + q, R - 1)];
-            s[q] = sin(z[q]);
+        comov(P, (int)(i / R), zg[i % R], px + i, py + i);
+    }
+}
+
+// The rewind grid as an FP64 product for full-band dumps: wiggle[row (p, ax)][i] =
+// sum_b re_b sin(b z_i) + im_b cos(b z_i), half the multiplications of evaluating the
+// polynomial at every (path, row).  The basis of a frame is laid out by k_fb_basis.
+constexpr int kGbRows = 64;    // (path, axis) rows of a tile, 16 per warp
+constexpr int kGbCols = 72;    // rewind rows of a tile: 421 rows are 6 tiles, 2.6 % padding
+constexpr int kGbB = 8;        // frequencies per chunk (16 terms)
+constexpr int kGbStages = 3;
+constexpr int kGbPitch = kGbCols + 2;  // two rows are 4 mod 16 apart: operand reads touch every bank once
+
+// basis[2 b][c], basis[2 b + 1][c] = sin, cos of b z_c, zero beyond the last row.  The
+// rounding of b z is carried into the result, so the phase is good to an ulp of z.
+__global__ void k_fb_basis(int bmax, int R, int Rp, const double* __restrict__ zg, double* __restrict__ basis) {
+    const int64_t total = (int64_t)(bmax + 1) * Rp;
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
+        const int b = (int)(i / Rp), c = (int)(i % Rp);
+        double s = 0.0, co = 0.0;
+        if (c < R) {
+            const double z = zg[c], x = b * z, e = fma((double)b, z, -x);
+            double s0, c0;
+            sincos(x, &s0, &c0);
+            s = fma(e, c0, s0);
+            co = fma(-e, s0, c0);
         }
-        for (int ax = 0; ax < 2; ax++) {
-            const size_t o = (size_t)p * 2 + ax;
-            if (P.horner) {
-                const double2* c = P.coef + o * (P.bmax + 1);
-                double sz[4], cz[4], pr[4], pi[4];
+        basis[(int64_t)(2 * b) * Rp + c] = s;
+        basis[(int64_t)(2 * b + 1) * Rp + c] = co;
+    }
+}
+
+// FP64 tensor product D += A B, 16 x 8 x 8.  Lane (g, t) = (lane / 4, lane % 4) holds
+// A(g, t), A(g + 8, t), A(g, t + 4), A(g + 8, t + 4); B(t, g), B(t + 4, g); and
+// D(g, 2t), D(g, 2t + 1), D(g + 8, 2t), D(g + 8, 2t + 1).
+__device__ __forceinline__ void dmma_16x8x8(double* d, const double* a, const double* b) {
+    asm volatile(
+        "mma.sync.aligned.m16n8k8.row.col.f64.f64.f64.f64 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+        : "+d"(d[0]), "+d"(d[1]), "+d"(d[2]), "+d"(d[3])
+        : "d"(a[0]), "d"(a[1]), "d"(a[2]), "d"(a[3]), "d"(b[0]), "d"(b[1]));
+}
+
+// One CTA per 64 x 72 tile, a warp per 16 rows (9 products of 16 x 8 a step of four
+// frequencies).  A step's terms are ordered sin of its four frequencies, then cos, so a
+// lane's A operands are the (re, im) pairs of its own frequency, read straight from
+// global memory two steps ahead; the basis chunks come in by cp.async, two in flight.
+// Bound by the FP64 tensor rate: 18 k paths x 421 rows at b_max 256 take 0.58 ms, 0.45 ms
+// at 37 TFLOP/s.  The same product on FP64 FMAs waited for its shared-memory operands
+// (0.90 ms); the polynomial at every (path, row) took 1.53 ms.
+__global__ void __launch_bounds__(128) k_fb_grid_mm(FPaths P, int R, int Rp, const double* __restrict__ zg,
+                                                    const double* __restrict__ basis, double* __restrict__ px,
+                                                    double* __restrict__ py) {
+    __shared__ __align__(16) double Bs[kGbStages][2 * kGbB][kGbPitch];
+    constexpr int kN = kGbCols / 8;
+    const int tid = threadIdx.x, lane = tid & 31, g = lane >> 2, t = lane & 3;
+    const int64_t nrows = (int64_t)P.n * 2;
+    // the column tiles of a row tile are neighbours: its coefficients are read from DRAM once
+    const int ct = Rp / kGbCols;
+    const int64_t row0 = (int64_t)(blockIdx.x / ct) * kGbRows + (tid >> 5) * 16;
+    const int col0 = (int)(blockIdx.x % ct) * kGbCols;
+    const int nb = P.bmax + 1;
+    const int nch = (nb + kGbB - 1) / kGbB;
+    auto stage = [&](int ch) {
+        const int terms = min(2 * kGbB, 2 * (nb - ch * kGbB));  // none past the last chunk
+        for (int e = tid; e < 2 * kGbB * (kGbCols / 2); e += 128) {
+            const int k = e / (kGbCols / 2), cc = (e % (kGbCols / 2)) * 2;
+            const uint32_t dst = (uint32_t)__cvta_generic_to_shared(&Bs[ch % kGbStages][k][cc]);
+            const double* src = basis + (k < terms ? (int64_t)(2 * ch * kGbB + k) * Rp : 0) + col0 + cc;
+            // terms beyond the last frequency: zeros
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(k < terms ? 16 : 0)
+                         : "memory");
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    const double2* ar[2] = {P.coef + min(row0 + g, nrows - 1) * nb, P.coef + min(row0 + g + 8, nrows - 1) * nb};
+    double2 a[3][2];  // this step's and the next two steps' (re, im) of rows g, g + 8
+    auto fetch = [&](int step, double2* v) {
+        const int b = 4 * step + t;
 #pragma unroll
-                for (int q = 0; q < 4; q++) {
-                    sincos(z[q], &sz[q], &cz[q]);
-                    pr[q] = c[P.bmax].x;
-                    pi[q] = c[P.bmax].y;
-                }
-                for (int k = P.bmax - 1; k >= 0; k--) {
-                    const double2 ck = c[k];
+        for (int q = 0; q < 2; q++) v[q] = b < nb ? __ldg(ar[q] + b) : make_double2(0.0, 0.0);
+    };
+    double acc[kN][4];
 #pragma unroll
-                    for (int q = 0; q < 4; q++) {
-                        const double nr = fma(pr[q], cz[q], fma(-pi[q], sz[q], ck.x));
-                        const double ni = fma(pr[q], sz[q], fma(pi[q], cz[q], ck.y));
-                        pr[q] = nr;
-                        pi[q] = ni;
-                    }
-                }
+    for (int j = 0; j < kN; j++)
 #pragma unroll
-                for (int q = 0; q < 4; q++) w[ax][q] = pi[q];
-            } else {
+        for (int q = 0; q < 4; q++) acc[j][q] = 0.0;
+    stage(0);
+    stage(1);
+    fetch(0, a[0]);
+    fetch(1, a[1]);
+    for (int ch = 0; ch < nch; ch++) {
+        asm volatile("cp.async.wait_group 1;" ::: "memory");
+        __syncthreads();  // chunk ch has landed, chunk ch - 1 has been read
+        stage(ch + 2);
 #pragma unroll
-                for (int q = 0; q < 4; q++)
-                    w[ax][q] = wiggle_direct(P.a + o * P.nw, P.b + o * P.nw, P.f + o * P.nw, P.nw, z[q]);
+        for (int h = 0; h < 2; h++) {
+            fetch(2 * ch + h + 2, a[2]);
+            const double av[4] = {a[0][0].x, a[0][1].x, a[0][0].y, a[0][1].y};
+            // basis row 2 b: sin, 2 b + 1: cos
+            const double* bs = &Bs[ch % kGbStages][8 * h + 2 * t][g];
+#pragma unroll
+            for (int j = 0; j < kN; j++) {
+                const double bv[2] = {bs[8 * j], bs[kGbPitch + 8 * j]};
+                dmma_16x8x8(acc[j], av, bv);
+            }
+#pragma unroll
+            for (int q = 0; q < 2; q++) {
+                a[0][q] = a[1][q];
+                a[1][q] = a[2][q];
             }
         }
-        const double a2x = P.a2[(size_t)p * 2], a2y = P.a2[(size_t)p * 2 + 1];
-        const double s0x = P.s0[(size_t)p * 2], s0y = P.s0[(size_t)p * 2 + 1];
-#pragma unroll
-        for (int q = 0; q < 4; q++) {
-            if (r0 + q >= R) break;
-            const int64_t at = (int64_t)p * R + r0 + q;
-            px[at] = (a2x * s[q] + w[0][q] - s0x) / s[q];
-            py[at] = (a2y * s[q] + w[1][q] - s0y) / s[q];
-        }
     }
+    double a2[2], s0[2];
+    double* out[2];
+#pragma unroll
+    for (int q = 0; q < 2; q++) {
+        const int64_t row = min(row0 + g + 8 * q, nrows - 1);
+        a2[q] = P.a2[row];
+        s0[q] = P.s0[row];
+        out[q] = row0 + g + 8 * q < nrows ? (row & 1 ? py : px) + (row >> 1) * R : nullptr;
+    }
+#pragma unroll
+    for (int j = 0; j < kN; j++)
+#pragma unroll
+        for (int e = 0; e < 2; e++) {
+            const int c = col0 + 8 * j + 2 * t + e;
+            if (c >= R) continue;
+            const double s = __ldg(basis + 2 * (int64_t)Rp + c);  // sin z
+#pragma unroll
+            for (int q = 0; q < 2; q++)
+                if (out[q]) out[q][c] = (a2[q] * s + acc[j][2 * q + e] - s0[q]) / s;
+        }
 }
 
 // A sign change of dist(image) - chi_front between rewind rows i-1 and i.
@@ -167,90 +276,318 @@ struct FCross {
     int32_t inside;  // the image was inside the front at row i-1
 };
 
-// One thread per (path, torus image): walks the rewind grid and records every
-// crossing; the bisections run in k_fb_refine, one thread per crossing, so no
-// warp waits for a single lane's refinement.
-__global__ void k_fb_cross(FPaths P, FFront F, double ox, double oy, int K, int obsIdx, const double* chig,
-                           const double* px, const double* py, FCross* cross, unsigned long long* count,
-                           unsigned long long cap) {
-    const int side = 2 * K + 1;
-    const int64_t total = (int64_t)P.n * side * side;
-    for (int64_t tid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; tid < total;
-         tid += (int64_t)gridDim.x * blockDim.x) {
-        const int p = (int)(tid / (side * side));
-        const int sh = (int)(tid % (side * side));
-        const int nx = sh % side - K, ny = sh / side - K;
-        const double bx = 2.0 * nx - ox, by = 2.0 * ny - oy;
-        // rows the front cannot reach for this image (comoving coords stay within +-2)
-        const double dmin = fmax(0.0, 2.0 * fmax(fabs((double)nx), fabs((double)ny)) - 4.0);
-        if (dmin >= F.chiMax) continue;
-        const int i0 = F.budget ? 1 : max(1, (int)ceil(dmin * F.M / F.chiMax));
-        if (i0 > F.M) continue;
-        const int64_t row = (int64_t)p * (F.M + 1);
-        double prev = metric(px[row + i0 - 1] + bx, py[row + i0 - 1] + by, F.cheb) - chig[i0 - 1];
-        // the observer sits on the front at chi = 0: keep its own image inside
-        if (p == obsIdx && nx == 0 && ny == 0 && i0 == 1 && fabs(prev) < 1e-9)
-            prev = -1e-12;
-        else if (prev == 0.0)
-            prev = 1e-12;
-        for (int i = i0; i <= F.M; i++) {
-            const double g = metric(px[row + i] + bx, py[row + i] + by, F.cheb) - chig[i];
-            if ((prev < 0.0) != (g < 0.0)) {
-                const unsigned long long slot = atomicAdd(count, 1ull);
-                if (slot < cap) cross[slot] = FCross{p, (int16_t)nx, (int16_t)ny, i, prev < 0.0 ? 1 : 0};
+// First rewind row the front can reach an image of ring s = max(|nx|, |ny|) at (comoving
+// coordinates stay within +-2), M + 1 when it never does.
+__device__ __forceinline__ int first_row(const FFront& F, int s) {
+    if (s <= 2) return F.chiMax > 0.0 ? 1 : F.M + 1;
+    const double dmin = 2.0 * s - 4.0;
+    if (dmin >= F.chiMax) return F.M + 1;
+    return F.budget ? 1 : max(1, (int)ceil(dmin * F.M / F.chiMax));
+}
+
+// One warp per path.  A lane holds a rewind row (chunks of 32 rows, the first of which is
+// the last of the chunk before), a ballot the signs of dist(image) - chi_front at all of
+// them; neighbouring bits that differ are the crossings, which k_fb_refine bisects.
+// The square metric is separable: max(|dx|, |dy|) < chi is |dx| < chi and |dy| < chi, so
+// 2 (2K + 1) ballots serve the (2K + 1)^2 images and the lanes combine one image each.
+// Bound by issue: 0.11 ms for 18 k paths (one thread per (path, image) walking the 421
+// rows: 0.36 ms).
+__global__ void __launch_bounds__(128) k_fb_cross(FPaths P, FFront F, double ox, double oy, int K, int obsIdx,
+                                                  const double* __restrict__ chig, const double* __restrict__ px,
+                                                  const double* __restrict__ py, FCross* cross,
+                                                  unsigned long long* count, unsigned long long cap) {
+    const int lane = threadIdx.x & 31;
+    const int warps = gridDim.x * (blockDim.x >> 5);
+    const int R = F.M + 1, side = 2 * K + 1;
+    const bool split = F.cheb && side <= 32;
+    for (int p = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); p < P.n; p += warps) {
+        const double* X = px + (int64_t)p * R;
+        const double* Y = py + (int64_t)p * R;
+        for (int c0 = 0; c0 + 1 < R; c0 += 31) {
+            const int i = c0 + lane;
+            const double x = i < R ? X[i] : 0.0, y = i < R ? Y[i] : 0.0, chi = i < R ? chig[i] : 0.0;
+            // rows that a crossing may end at: all of the chunk's but its first
+            const uint32_t rows = (R - c0 >= 32 ? 0xffffffffu : (1u << (R - c0)) - 1u) & ~1u;
+            // the observer sits on the front at chi = 0: keep its own image inside
+            const bool own = p == obsIdx && c0 == 0 && fabs(metric(x + (0.0 - ox), y + (0.0 - oy), F.cheb) - chi) < 1e-9;
+            const bool own0 = __shfl_sync(0xffffffffu, (int)own, 0) != 0;
+            uint32_t mx = 0, my = 0;
+            if (split)
+                for (int k = 0; k < side; k++) {
+                    const double b = 2.0 * (k - K);
+                    const uint32_t bx = __ballot_sync(0xffffffffu, i < R && fabs(x + (b - ox)) < chi);
+                    const uint32_t by = __ballot_sync(0xffffffffu, i < R && fabs(y + (b - oy)) < chi);
+                    if (lane == k) mx = bx, my = by;
+                }
+            for (int m0 = 0; m0 < side * side; m0 += 32) {
+                // this lane's image and the signs of its rows
+                const int m = m0 + lane;
+                const int nx = m % side - K, ny = m / side - K;
+                uint32_t sg = 0;
+                if (split) {
+                    sg = __shfl_sync(0xffffffffu, mx, (nx + K) & 31) & __shfl_sync(0xffffffffu, my, (ny + K) & 31);
+                } else {
+                    for (int q = 0; q < 32 && m0 + q < side * side; q++) {
+                        const int qx = (m0 + q) % side - K, qy = (m0 + q) / side - K;
+                        const uint32_t b = __ballot_sync(
+                            0xffffffffu,
+                            i < R && metric(x + (2.0 * qx - ox), y + (2.0 * qy - oy), F.cheb) - chi < 0.0);
+                        if (lane == q) sg = b;
+                    }
+                }
+                uint32_t cr = 0;
+                if (m < side * side) {
+                    if (own0 && nx == 0 && ny == 0 && first_row(F, 0) == 1) sg |= 1u;
+                    const int i0 = first_row(F, max(abs(nx), abs(ny)));
+                    cr = (sg ^ (sg << 1)) & rows;
+                    if (i0 > c0) cr &= i0 - c0 < 32 ? ~((1u << (i0 - c0)) - 1u) : 0u;  // rows from i0 on
+                }
+                const uint32_t any = __ballot_sync(0xffffffffu, cr != 0u);
+                if (!any) continue;
+                int incl = __popc(cr);
+                const int mine = incl;
+                for (int o = 1; o < 32; o <<= 1) {
+                    const int v = __shfl_up_sync(0xffffffffu, incl, o);
+                    if (lane >= o) incl += v;
+                }
+                unsigned long long base = 0;
+                if (lane == 31) base = atomicAdd(count, (unsigned long long)incl);
+                base = __shfl_sync(0xffffffffu, base, 31) + (unsigned long long)(incl - mine);
+                for (; cr; cr &= cr - 1, base++) {
+                    const int bit = __ffs(cr) - 1;
+                    if (base < cap)
+                        cross[base] = FCross{p, (int16_t)nx, (int16_t)ny, c0 + bit, (int32_t)((sg >> (bit - 1)) & 1u)};
+                }
             }
-            prev = g;
         }
     }
 }
 
-// One thread per crossing: 24 bisection steps with fresh evaluations
-// (frame_bake.cu:281-371), hit slot = crossing slot.
-__global__ void k_fb_refine(FPaths P, FFront F, double ox, double oy, const double* zg, const double* chig,
-                            const FCross* cross, const unsigned long long* count, unsigned long long cap,
-                            ug_hit* hits) {
+// Refinement of a crossing: 24 bisection steps over its row interval
+// (frame_bake.cu:281-371).
+//
+// Over one rewind row the wiggle of each axis is, to well below 1e-12, the polynomial
+// through its values at 16 Chebyshev nodes: sin(b z + f) on an interval of half-width h
+// is interpolated to 4 (b h / 2)^16 / 16! (Jacobi-Anger: its Chebyshev coefficients are
+// at most 2 J_k(b h)), and the rounding of the nodes' values (2 b_max ulps of the summed
+// amplitudes) grows at most threefold.  So the path's coefficients are read once, for the 16 nodes, and
+// the steps evaluate the interpolant.  A step whose distance to the front is below
+// kSure, where the interpolant might give the other sign, evaluates the path itself;
+// intervals too wide for the bound (kWide), and few-term dumps, always do.  Every step
+// therefore takes the side that a fresh evaluation gives, and the offsets of the hit
+// come from a fresh evaluation at the end.
+constexpr int kNodes = 16;
+constexpr double kSure = 1e-12;   // |g| above this: the interpolant's sign is the path's
+constexpr double kWide = 5e-13;   // largest error of an interpolated position
+
+// Wiggles of both axes at kQ instants: wiggle_horner's operations for each, as
+// independent chains that share every coefficient load.
+template <int kQ>
+__device__ __forceinline__ void wiggles(const FPaths& P, int p, const double* z, double (*w)[kQ]) {
+    const size_t o = (size_t)p * 2;
+    if (P.horner) {
+        const double2* c0 = P.coef + o * (P.bmax + 1);
+        const double2* c1 = c0 + (P.bmax + 1);
+        double sz[kQ], cz[kQ], pr[2][kQ], pi[2][kQ];
+#pragma unroll
+        for (int q = 0; q < kQ; q++) {
+            sincos(z[q], &sz[q], &cz[q]);
+            pr[0][q] = c0[P.bmax].x;
+            pi[0][q] = c0[P.bmax].y;
+            pr[1][q] = c1[P.bmax].x;
+            pi[1][q] = c1[P.bmax].y;
+        }
+#pragma unroll 4
+        for (int k = P.bmax - 1; k >= 0; k--) {
+            const double2 ck[2] = {__ldg(c0 + k), __ldg(c1 + k)};
+#pragma unroll
+            for (int ax = 0; ax < 2; ax++)
+#pragma unroll
+                for (int q = 0; q < kQ; q++) {
+                    const double nr = fma(pr[ax][q], cz[q], fma(-pi[ax][q], sz[q], ck[ax].x));
+                    const double ni = fma(pr[ax][q], sz[q], fma(pi[ax][q], cz[q], ck[ax].y));
+                    pr[ax][q] = nr;
+                    pi[ax][q] = ni;
+                }
+        }
+#pragma unroll
+        for (int q = 0; q < kQ; q++) {
+            w[0][q] = pi[0][q];
+            w[1][q] = pi[1][q];
+        }
+    } else {
+#pragma unroll
+        for (int ax = 0; ax < 2; ax++)
+#pragma unroll
+            for (int q = 0; q < kQ; q++)
+                w[ax][q] = wiggle_direct(P.a + (o + ax) * P.nw, P.b + (o + ax) * P.nw, P.f + (o + ax) * P.nw, P.nw, z[q]);
+    }
+}
+
+// Four lanes per crossing; a pass takes three bisection steps: the seven midpoints they
+// can reach (two per lane) are evaluated, then the steps follow from the signs -- the same
+// midpoints, from the same operations, as one step at a time.  Bound by FP64 issue: 0.24 ms
+// for 18 k crossings at b_max 256.  One thread per crossing, with 25 evaluations of its path
+// 8 KB from its neighbours', took 2.06 ms; four lanes with 9 of them 0.74 ms.
+__global__ void __launch_bounds__(128) k_fb_refine(FPaths P, FFront F, double ox, double oy, const double* zg,
+                                                   const double* chig, const FCross* cross,
+                                                   const unsigned long long* count, unsigned long long cap,
+                                                   ug_hit* hits) {
+    static_assert(kBisect % 3 == 0, "three bisection steps a pass");
+    __shared__ double s_cos[kNodes][kNodes];       // cos(k theta_i) / 8 (row 0: 1 / 16)
+    __shared__ double s_w[32][2][kNodes + 1];      // samples, then coefficients, of each crossing
     const unsigned long long c = *count;
     const int64_t n = (int64_t)(c < cap ? c : cap);
-    for (int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; k < n; k += (int64_t)gridDim.x * blockDim.x) {
+    for (int e = threadIdx.x; e < kNodes * kNodes; e += blockDim.x) {
+        const int k = e / kNodes, i = e % kNodes;
+        s_cos[k][i] = k == 0 ? 1.0 / kNodes : cospi((double)(k * (2 * i + 1)) / (2 * kNodes)) * (2.0 / kNodes);
+    }
+    __syncthreads();
+    const int j = threadIdx.x & 3;                       // lane of the crossing's four
+    const int sh = threadIdx.x & 28;                     // its first lane of the warp
+    double(*ws)[kNodes + 1] = s_w[threadIdx.x >> 2];
+    const uint32_t quad = 0xfu << sh;  // the four lanes share all of their crossing's branches
+    const int64_t stride = (int64_t)gridDim.x * blockDim.x >> 2;
+    for (int64_t k = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 2; k < n; k += stride) {
         const FCross x = cross[k];
         const int p = x.p, i = x.i;
         const bool inside = x.inside != 0;
+        const size_t o = (size_t)p * 2;
+        const double a2x = P.a2[o], a2y = P.a2[o + 1], s0x = P.s0[o], s0y = P.s0[o + 1];
         const double bx = 2.0 * x.nx - ox, by = 2.0 * x.ny - oy;
-        double chi, zEmit, qx, qy;
-        if (F.budget) {
-            double lo = zg[i - 1], hi = zg[i];
-            for (int it = 0; it < kBisect; it++) {
-                const double mid = (lo + hi) / 2.0;
-                comov(P, p, mid, &qx, &qy);
-                const double gm = metric(qx + bx, qy + by, F.cheb) - reach_of(mid, F.zObs, F.bMax);
-                if ((gm < 0.0) == inside)
-                    lo = mid;
-                else
-                    hi = mid;
-            }
-            zEmit = (lo + hi) / 2.0;
-            chi = reach_of(zEmit, F.zObs, F.bMax);
-        } else {
-            double lo = chig[i - 1], hi = chig[i];
-            for (int it = 0; it < kBisect; it++) {
-                const double mid = (lo + hi) / 2.0;
-                comov(P, p, 2.0 * atan(exp(F.etaObs - mid / F.spd)), &qx, &qy);
-                const double gm = metric(qx + bx, qy + by, F.cheb) - mid;
-                if ((gm < 0.0) == inside)
-                    lo = mid;
-                else
-                    hi = mid;
-            }
-            chi = (lo + hi) / 2.0;
-            zEmit = 2.0 * atan(exp(F.etaObs - chi / F.spd));
+        // the bracket in z (budget front) or chi (the others)
+        double lo = F.budget ? zg[i - 1] : chig[i - 1], hi = F.budget ? zg[i] : chig[i];
+        // emission times run down as the front grows
+        const double zc = 0.5 * (zg[i - 1] + zg[i]), zh = 0.5 * fabs(zg[i - 1] - zg[i]) * (1.0 + 1e-12) + 1e-15;
+        bool smooth = false;
+        if (P.horner) {
+            double u = 0.5 * P.bmax * zh;
+            u *= u;
+            u *= u;
+            u *= u;
+            u *= u;  // (b h / 2)^16, over 16!
+            smooth = P.amp[p] * (4.0 / 2.0922789888e13 * u + 1e-15 * P.bmax) < kWide * fmin(sin(zc - zh), sin(zc + zh));
         }
-        comov(P, p, zEmit, &qx, &qy);
+        if (smooth) {
+            double z[4], w[2][4];
+#pragma unroll
+            for (int q = 0; q < 4; q++) z[q] = fma(zh, cospi((2 * (4 * j + q) + 1) / (2.0 * kNodes)), zc);
+            wiggles<4>(P, p, z, w);
+#pragma unroll
+            for (int q = 0; q < 4; q++) {
+                ws[0][4 * j + q] = w[0][q];
+                ws[1][4 * j + q] = w[1][q];
+            }
+            __syncwarp(quad);
+#pragma unroll
+            for (int q = 0; q < 4; q++) w[0][q] = w[1][q] = 0.0;
+            for (int e = 0; e < kNodes; e++)
+#pragma unroll
+                for (int q = 0; q < 4; q++) {
+                    w[0][q] = fma(s_cos[4 * j + q][e], ws[0][e], w[0][q]);
+                    w[1][q] = fma(s_cos[4 * j + q][e], ws[1][e], w[1][q]);
+                }
+            __syncwarp(quad);
+#pragma unroll
+            for (int q = 0; q < 4; q++) {
+                ws[0][4 * j + q] = w[0][q];
+                ws[1][4 * j + q] = w[1][q];
+            }
+            __syncwarp(quad);
+        }
+        const double izh = 1.0 / zh;
+        for (int it = 0; it < kBisect; it += 3) {
+            // nodes of the pass's tree: 1 the midpoint, 2 and 3 those of its halves, 4..7
+            // of its quarters; lane j evaluates 4 + j and (j > 0) j
+            double m[2], z[2], w[2][2];
+#pragma unroll
+            for (int q = 0; q < 2; q++) {
+                const int node = q == 0 ? 4 + j : max(j, 1);
+                double l = lo, h = hi;
+                m[q] = (l + h) / 2.0;
+                for (int lev = node >= 4 ? 1 : (node >= 2 ? 0 : -1); lev >= 0; lev--) {
+                    if ((node >> lev) & 1)
+                        l = m[q];
+                    else
+                        h = m[q];
+                    m[q] = (l + h) / 2.0;
+                }
+                z[q] = F.budget ? m[q] : 2.0 * atan(exp(F.etaObs - m[q] / F.spd));
+            }
+            if (smooth) {  // Clenshaw, both axes and points together
+                double t2[2], b1[2][2] = {{0.0, 0.0}, {0.0, 0.0}}, b2[2][2] = {{0.0, 0.0}, {0.0, 0.0}};
+#pragma unroll
+                for (int q = 0; q < 2; q++) t2[q] = 2.0 * (z[q] - zc) * izh;
+                for (int e = kNodes - 1; e > 0; e--) {
+                    const double cc[2] = {ws[0][e], ws[1][e]};
+#pragma unroll
+                    for (int ax = 0; ax < 2; ax++)
+#pragma unroll
+                        for (int q = 0; q < 2; q++) {
+                            const double b0 = fma(t2[q], b1[ax][q], cc[ax] - b2[ax][q]);
+                            b2[ax][q] = b1[ax][q];
+                            b1[ax][q] = b0;
+                        }
+                }
+#pragma unroll
+                for (int ax = 0; ax < 2; ax++)
+#pragma unroll
+                    for (int q = 0; q < 2; q++) w[ax][q] = fma(0.5 * t2[q], b1[ax][q], ws[ax][0] - b2[ax][q]);
+            } else {
+                wiggles<2>(P, p, z, w);
+            }
+            uint32_t up = 0, sure = 0;  // bit of each node: the crossing lies above its midpoint
+            double front[2];
+#pragma unroll
+            for (int q = 0; q < 2; q++) {
+                const double s = sin(z[q]);
+                front[q] = F.budget ? reach_tab(F, m[q]) : m[q];
+                const double gm =
+                    metric((a2x * s + w[0][q] - s0x) / s + bx, (a2y * s + w[1][q] - s0y) / s + by, F.cheb) - front[q];
+                const uint32_t b = (__ballot_sync(quad, (gm < 0.0) == inside) >> sh) & 0xfu;
+                const uint32_t f = (__ballot_sync(quad, !smooth || fabs(gm) > kSure) >> sh) & 0xfu;
+                up |= q == 0 ? b << 4 : b & 0xeu;
+                sure |= q == 0 ? f << 4 : f & 0xeu;
+            }
+            int node = 1;
+#pragma unroll
+            for (int lev = 0; lev < 3; lev++) {
+                const double mid = (lo + hi) / 2.0;
+                int u = (up >> node) & 1;
+                if (!((sure >> node) & 1)) {  // the path itself
+                    double z1[1] = {F.budget ? mid : 2.0 * atan(exp(F.etaObs - mid / F.spd))}, w1[2][1];
+                    wiggles<1>(P, p, z1, w1);
+                    const double s = sin(z1[0]);
+                    const double gm =
+                        metric((a2x * s + w1[0][0] - s0x) / s + bx, (a2y * s + w1[1][0] - s0y) / s + by, F.cheb) -
+                        (F.budget ? reach_tab(F, mid) : mid);
+                    u = (gm < 0.0) == inside;
+                }
+                if (u)
+                    lo = mid;
+                else
+                    hi = mid;
+                node = 2 * node + u;
+            }
+        }
+        __syncwarp(quad);  // the next crossing's samples replace the coefficients
+        if (j != 0) continue;
+        double chi, z1[1], w1[2][1];
+        if (F.budget) {
+            z1[0] = (lo + hi) / 2.0;
+            chi = reach_tab(F, z1[0]);
+        } else {
+            chi = (lo + hi) / 2.0;
+            z1[0] = 2.0 * atan(exp(F.etaObs - chi / F.spd));
+        }
+        wiggles<1>(P, p, z1, w1);
+        const double s = sin(z1[0]);
         ug_hit h;
         h.src = (uint32_t)p;
-        h.dx = (float)(qx + bx);
-        h.dy = (float)(qy + by);
+        h.dx = (float)((a2x * s + w1[0][0] - s0x) / s + bx);
+        h.dy = (float)((a2y * s + w1[1][0] - s0y) / s + by);
         h.chi = (float)chi;
-        h.z_emit = (float)zEmit;
+        h.z_emit = (float)z1[0];
         hits[k] = h;
     }
 }
@@ -337,24 +674,41 @@ struct DevBuf {
     }
 };
 
-// Per (path, axis): s0 = sum_j a_j sin f_j and the Horner coefficients
-// a_b e^{i f_b} (coef zeroed by the caller; frequencies are unique per axis).
-__global__ void k_fb_prep(int n, int nw, int bmax, int horner, const double* a, const double* b,
-                          const double* f, double* s0, double2* coef) {
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < (int64_t)n * 2;
-         i += (int64_t)gridDim.x * blockDim.x) {
-        double acc = 0.0;
-        for (int j = 0; j < nw; j++) {
-            const int64_t o = i * nw + j;
-            const double sf = sin(f[o]);
-            acc += a[o] * sf;
-            if (horner) {
-                double2& c = coef[i * (bmax + 1) + (int)b[o]];
-                c.x += a[o] * cos(f[o]);
-                c.y += a[o] * sf;
+// Per (path, axis): s0 = sum_j a_j sin f_j, summed in term order, and the polynomial's
+// coefficients a_b e^{i f_b} (coef zeroed by the caller; a frequency listed twice adds up).
+// One warp per (path, axis): coalesced reads and the sines spread over the lanes (18 k
+// paths of 255 terms: 0.55 -> 0.14 ms against a thread each).
+__global__ void __launch_bounds__(128) k_fb_prep(int n, int nw, int bmax, int horner, const double* __restrict__ a,
+                                                 const double* __restrict__ b, const double* __restrict__ f,
+                                                 double* s0, double2* coef, double* amp) {
+    const int lane = threadIdx.x & 31;
+    const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
+    for (int64_t i = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); i < (int64_t)n * 2; i += warps) {
+        double acc = 0.0, aa = 0.0;
+        for (int j0 = 0; j0 < nw; j0 += 32) {
+            const int j = j0 + lane;
+            double term = 0.0;
+            if (j < nw) {
+                const int64_t o = i * nw + j;
+                double sf, cf;
+                sincos(f[o], &sf, &cf);
+                aa += fabs(a[o]);
+                term = __dmul_rn(a[o], sf);
+                if (horner) {
+                    double2* c = coef + i * (bmax + 1) + (int)b[o];
+                    atomicAdd(&c->x, a[o] * cf);
+                    atomicAdd(&c->y, term);
+                }
             }
+            const int m = min(32, nw - j0);
+            for (int q = 0; q < m; q++) acc += __shfl_sync(0xffffffffu, term, q);
         }
-        s0[i] = acc;
+        for (int q = 16; q > 0; q >>= 1) aa += __shfl_xor_sync(0xffffffffu, aa, q);
+        if (lane == 0) {
+            s0[i] = acc;
+            // non-negative doubles order as their bits (amp zeroed by the caller)
+            atomicMax((unsigned long long*)(amp + (i >> 1)), (unsigned long long)__double_as_longlong(aa));
+        }
     }
 }
 
@@ -397,6 +751,10 @@ int bake_device(const ug_frames_cfg* cfg, int n, int nw, int bMax, const double*
     const int NF = cfg->n_frames, NO = cfg->n_obs;
     double* dZg = buf.get<double>((size_t)NF * (Mmax + 1));
     double* dChig = buf.get<double>((size_t)NF * (Mmax + 1));
+    const int RpMax = (Mmax + 1 + kGbCols - 1) / kGbCols * kGbCols;
+    double* dAmp = buf.get<double>((size_t)n);
+    double2* dReach = buf.get<double2>((size_t)bMax + 1);
+    double* dBasis = buf.get<double>(horner ? (size_t)2 * (bMax + 1) * RpMax : 1);
     double* dPx = buf.get<double>((size_t)n * (Mmax + 1));
     double* dPy = buf.get<double>((size_t)n * (Mmax + 1));
     const bool want_hits = out->hits != nullptr;
@@ -409,13 +767,14 @@ int bake_device(const ug_frames_cfg* cfg, int n, int nw, int bMax, const double*
     ug_hit* dHits = buf.get<ug_hit>(hitCap);
     FCross* dCross = buf.get<FCross>(hitCap);
     unsigned long long* dCount = buf.get<unsigned long long>((size_t)NF * NO);
-    if (!dS0 || !dC || !dZg || !dChig || !dPx || !dPy || !dHits || !dCross || !dCount || (want_density && !dDen))
+    if (!dS0 || !dC || !dZg || !dChig || !dBasis || !dReach || !dAmp || !dPx || !dPy || !dHits || !dCross || !dCount || (want_density && !dDen))
         return set_error(UG_ENOMEM, "frame_bake: device allocation failed");
+    cudaMemsetAsync(dAmp, 0, (size_t)n * 8, st);
     if (horner) cudaMemsetAsync(dC, 0, (size_t)n * 2 * (bMax + 1) * sizeof(double2), st);
-    k_fb_prep<<<(int)std::min<int64_t>(((int64_t)n * 2 + 127) / 128, 65536), 128, 0, st>>>(n, nw, bMax, horner, dA,
-                                                                                           dB, dF, dS0, dC);
+    k_fb_prep<<<(int)std::min<int64_t>(((int64_t)n * 2 + 3) / 4, nsm * 64), 128, 0, st>>>(n, nw, bMax, horner, dA, dB,
+                                                                                        dF, dS0, dC, dAmp);
     cudaMemsetAsync(dCount, 0, (size_t)NF * NO * sizeof(unsigned long long), st);
-    FPaths P{n, nw, bMax, horner, dA2, dS0, dA, dB, dF, dC};
+    FPaths P{n, nw, bMax, horner, dA2, dS0, dA, dB, dF, dC, dAmp};
     const double zMin = std::max(2e-3, cfg->zmin_pi * kPiF);
     // fronts and rewind grids of every frame, uploaded once
     std::vector<FFront> fronts(NF);
@@ -428,6 +787,7 @@ int bake_device(const ug_frames_cfg* cfg, int n, int nw, int bMax, const double*
         FFront& F = fronts[fi];
         F = FFront{};
         F.budget = cfg->front == 2;
+        F.reach = dReach;
         F.cheb = F.budget || cfg->cheb;
         F.zObs = zObs;
         F.etaObs = h_eta(zObs);
@@ -467,8 +827,15 @@ int bake_device(const ug_frames_cfg* cfg, int n, int nw, int bMax, const double*
         const int K = Ks[fi];
         const double* zg = dZg + (size_t)fi * (Mmax + 1);
         const double* chig = dChig + (size_t)fi * (Mmax + 1);
-        {
-            const int64_t tot = (int64_t)n * ((F.M + 1 + 3) / 4);
+        if (F.budget) k_fb_reach<<<(bMax + 127) / 128, 128, 0, st>>>(bMax, F.zObs, dReach);
+        if (horner) {
+            const int R = F.M + 1, Rp = (R + kGbCols - 1) / kGbCols * kGbCols;
+            k_fb_basis<<<(int)std::min<int64_t>(((int64_t)(bMax + 1) * Rp + 127) / 128, nsm * 16), 128, 0, st>>>(
+                bMax, R, Rp, zg, dBasis);
+            const int64_t tiles = ((int64_t)n * 2 + kGbRows - 1) / kGbRows * (Rp / kGbCols);
+            k_fb_grid_mm<<<(unsigned)tiles, 128, 0, st>>>(P, R, Rp, zg, dBasis, dPx, dPy);
+        } else {
+            const int64_t tot = (int64_t)n * (F.M + 1);
             k_fb_grid<<<(int)std::min<int64_t>((tot + 127) / 128, 65536), 128, 0, st>>>(P, F.M, zg, dPx, dPy);
         }
         for (int o = 0; o < NO; o++) {
@@ -491,9 +858,7 @@ int bake_device(const ug_frames_cfg* cfg, int n, int nw, int bMax, const double*
                 m[3] = byv;
             }
             unsigned long long* cnt = dCount + (size_t)fi * NO + o;
-            const int side = 2 * K + 1;
-            const int64_t tot = (int64_t)n * side * side;
-            k_fb_cross<<<(int)std::min<int64_t>((tot + 127) / 128, 1 << 20), 128, 0, st>>>(
+            k_fb_cross<<<std::min((n + 3) / 4, nsm * 64), 128, 0, st>>>(
                 P, F, ox, oy, K, cfg->obs_type[o] == 0 ? cfg->obs_path[o] : -1, chig, dPx, dPy, dCross, cnt, hitCap);
             k_fb_refine<<<nsm * 8, 128, 0, st>>>(P, F, ox, oy, zg, chig, dCross, cnt, hitCap, dHits);
             if (!want_hits) {
