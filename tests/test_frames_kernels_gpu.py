@@ -79,3 +79,18 @@ def test_hits_are_the_crossings_of_the_rewind_grid(ug, n, nw, bmax, front):
     off = np.stack([h["dx"], h["dy"]], 1) - d
     assert np.abs(off - 2 * np.round(off / 2)).max() < TOL
     np.testing.assert_allclose(np.maximum(np.abs(h["dx"]), np.abs(h["dy"])), h["chi"], atol=TOL)
+
+
+@pytest.mark.parametrize("dim,T,pin", [(1, 4, 0), (2, 31, 1), (3, 33, 0), (2, 64, 0), (1, 255, 0), (2, 256, 0)])
+def test_dumped_parameters_equal_the_oracle(ug, oracle, dim, T, pin):
+    """The warp-per-axis parameter dump at odd and even bands, smallest and largest."""
+    u = ug.Universe(dim=dim, T=T, zgrid=1, excl=1, pin_sin1=pin, seed=T, attempts=2000, round_size=1024)
+    m = oracle.Model(dim=dim, T=T, zgrid=1, excl=1, pin=pin, seed=T)
+    with ug.Packer([u]) as p:
+        p.run()
+        idx, par = p.accepted(0)[0], p.params(0)
+    for k in range(0, len(idx), max(1, len(idx) // 9)):
+        c = oracle.candidate(m, int(idx[k]))
+        assert np.array_equal(par["b"][k], c["b"])
+        for q in ("a", "f", "a2"):  # an ulp of the two libms' logarithms
+            np.testing.assert_allclose(par[q][k], c[q], rtol=1e-14, atol=1e-300)

@@ -598,7 +598,7 @@ static bool all_done(const Batch& B) {
 // Internal accessor for ug_noalloc.cu: what a parameter dump of universe u
 // needs, without allocating anything.
 namespace ug {
-int batch_params_view(void* h, int u, const UniDev** dU, int64_t* n, int* dim, int* nw, int* dev,
+int batch_params_view(void* h, int u, const UniDev** dU, int64_t* n, int* rng, int* dim, int* nw, int* dev,
                       cudaStream_t* st) {
     Batch* B = (Batch*)h;
     if (!B || u < 0 || u >= B->n) return fail(UG_EINVAL, "bad arguments");
@@ -606,6 +606,7 @@ int batch_params_view(void* h, int u, const UniDev** dU, int64_t* n, int* dim, i
     if (rc) return rc;
     *dU = B->dU;
     *n = B->hCtl[u].n_slots;
+    *rng = B->U[u].d.rng;
     *dim = B->U[u].d.dim;
     *nw = B->U[u].d.nw;
     *dev = B->dev;
@@ -928,7 +929,7 @@ int ug_batch_params(void* h, int32_t u, double* a2, double* a, int32_t* b, doubl
     CKR(cudaMalloc(&da, (size_t)N * D * nw * 8));
     CKR(cudaMalloc(&df, (size_t)N * D * nw * 8));
     CKR(cudaMalloc(&db, (size_t)N * D * nw * 4));
-    launch_params(B->dU, u, N, da2, da, db, df, B->st);
+    launch_params(B->dU, u, B->U[u].d.rng, B->U[u].d.dim, N, da2, da, db, df, B->st);
     cudaError_t e = cudaStreamSynchronize(B->st);
     if (e == cudaSuccess && a2) e = cudaMemcpy(a2, da2, (size_t)N * D * 8, cudaMemcpyDeviceToHost);
     if (e == cudaSuccess && a) e = cudaMemcpy(a, da, (size_t)N * D * nw * 8, cudaMemcpyDeviceToHost);
@@ -965,7 +966,7 @@ int ug_batch_frames(void* h, int32_t u, const ug_frames_cfg* cfg, ug_frames_out*
         release();
         return fail(UG_ENOMEM, "frames: device allocation failed");
     }
-    launch_params(B->dU, u, N, da2, da, db, df, B->st);
+    launch_params(B->dU, u, B->U[u].d.rng, B->U[u].d.dim, N, da2, da, db, df, B->st);
     int bMax = 2;
     if (cudaStreamSynchronize(B->st) != cudaSuccess || (rc = max_b_device(db, N * 2 * nw, &bMax, B->st))) {
         release();

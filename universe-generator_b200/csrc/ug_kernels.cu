@@ -1478,97 +1478,119 @@ __global__ void k_rehash(const UniDev* __restrict__ U, UniCtl* ctl, int u, int64
 
 namespace ug {
 
-// Worldline parameters in term order (the --dump-params content): knot mode
-// replays the reference draw sequence (cuda/braid_knot.cu:111-166) keeping
-// each term; the Philox stream lists term j = frequency j + 2.
+// Worldline parameters in term order (the --dump-params content).  The knot stream
+// replays the reference draw sequence (cuda/braid_knot.cu:111-166) keeping each
+// term, one thread per path (the stream is sequential); the counter stream lists
+// term j = frequency j + 2 (k_params_philox).
 __global__ void k_params(const UniDev* __restrict__ U, int u, int64_t n, double* a2o, double* ao,
                          int32_t* bo, double* fo) {
     const UniDev& d = U[u];
-    const int D = d.dim, nw = d.nw, F = d.F;
+    const int D = d.dim, nw = d.nw;
     double wj[kMaxF];
     int32_t bj[kMaxF];
     for (int64_t s = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; s < n;
          s += (int64_t)gridDim.x * blockDim.x) {
         const uint64_t idx = (uint64_t)d.acc_idx[s];
-        if (d.rng == RNG_KNOT) {
-            Xo r;
-            r.seed(knot_seed(d.seed, idx));
-            for (int ax = 0; ax < D; ax++) {
-                const int64_t o = (s * D + ax) * nw;
-                if ((uint32_t)nw == d.modmax) {
-                    for (int j = 0; j < nw; j++) bj[j] = j + 2;
-                    for (int j = nw - 1; j > 0; j--) {
-                        const int k = (int)r.below((uint32_t)(j + 1));
-                        const int32_t tmp = bj[j];
-                        bj[j] = bj[k];
-                        bj[k] = tmp;
-                    }
-                } else {
-                    for (int j = 0; j < nw; j++) {
-                        int bnew = 0;
-                        bool dup = true;
-                        for (int guard = 0; dup && guard < 64; guard++) {
-                            bnew = (int)r.below(d.modmax) + 2;
-                            dup = false;
-                            for (int k = 0; k < j; k++)
-                                if (bj[k] == bnew) dup = true;
-                        }
-                        bj[j] = bnew;
-                    }
+        Xo r;
+        r.seed(knot_seed(d.seed, idx));
+        for (int ax = 0; ax < D; ax++) {
+            const int64_t o = (s * D + ax) * nw;
+            if ((uint32_t)nw == d.modmax) {
+                for (int j = 0; j < nw; j++) bj[j] = j + 2;
+                for (int j = nw - 1; j > 0; j--) {
+                    const int k = (int)r.below((uint32_t)(j + 1));
+                    const int32_t tmp = bj[j];
+                    bj[j] = bj[k];
+                    bj[k] = tmp;
                 }
-                double sum = 0.0;
+            } else {
                 for (int j = 0; j < nw; j++) {
-                    wj[j] = -log(1.0 - r.f64());
-                    sum += wj[j];
-                }
-                for (int j = 0; j < nw; j++) wj[j] /= sum;
-                for (int j = 0; j < nw; j++) {
-                    double amp = wj[j] / (double)bj[j];
-                    if (r.flip()) amp = -amp;
-                    ao[o + j] = amp;
-                    bo[o + j] = bj[j];
-                    fo[o + j] = (bj[j] % 2 == 0) ? r.f64() * kPi : 0.0;
-                }
-                a2o[s * D + ax] = d.pin ? 0.0 : (r.f64() * 2.0 - 1.0);
-            }
-        } else {
-            for (int ax = 0; ax < D; ax++) {
-                const int64_t o = (s * D + ax) * nw;
-                double sum = 0.0;
-                for (int p = 0; 2 * p <= F; p++) {
-                    const uint4 q = philox_block(d.seed, idx, ax, p);
-                    if (p == 0) {
-                        a2o[s * D + ax] = d.pin ? 0.0 : (double)q.x * (1.0 / 2147483648.0) - 1.0;
-                        continue;
+                    int bnew = 0;
+                    bool dup = true;
+                    for (int guard = 0; dup && guard < 64; guard++) {
+                        bnew = (int)r.below(d.modmax) + 2;
+                        dup = false;
+                        for (int k = 0; k < j; k++)
+                            if (bj[k] == bnew) dup = true;
                     }
-                    const int be = 2 * p, bo2 = 2 * p + 1;
-                    const double Ee = -log(((double)q.x + 0.5) * (1.0 / 4294967296.0));
-                    sum += Ee;
-                    ao[o + be - 2] = (q.z & 1u) ? -Ee : Ee;
-                    fo[o + be - 2] = (double)(q.z >> 1) * (1.0 / 2147483648.0) * kPi;
-                    bo[o + be - 2] = be;
-                    if (bo2 <= F) {
-                        const double Eo = -log(((double)q.y + 0.5) * (1.0 / 4294967296.0));
-                        sum += Eo;
-                        ao[o + bo2 - 2] = (q.w & 1u) ? -Eo : Eo;
-                        fo[o + bo2 - 2] = 0.0;
-                        bo[o + bo2 - 2] = bo2;
-                    }
-                }
-                for (int j = 0; j < nw; j++) {
-                    const double e = ao[o + j];
-                    double amp = fabs(e) / sum / (double)(j + 2);
-                    ao[o + j] = e < 0.0 ? -amp : amp;
+                    bj[j] = bnew;
                 }
             }
+            double sum = 0.0;
+            for (int j = 0; j < nw; j++) {
+                wj[j] = -log(1.0 - r.f64());
+                sum += wj[j];
+            }
+            for (int j = 0; j < nw; j++) wj[j] /= sum;
+            for (int j = 0; j < nw; j++) {
+                double amp = wj[j] / (double)bj[j];
+                if (r.flip()) amp = -amp;
+                ao[o + j] = amp;
+                bo[o + j] = bj[j];
+                fo[o + j] = (bj[j] % 2 == 0) ? r.f64() * kPi : 0.0;
+            }
+            a2o[s * D + ax] = d.pin ? 0.0 : (r.f64() * 2.0 - 1.0);
         }
     }
 }
 
-void launch_params(const UniDev* dU, int u, int64_t n, double* a2, double* a, int32_t* b, double* f,
-                   cudaStream_t st) {
-    const int blocks = (int)std::min<int64_t>((n + 127) / 128, 4096);
-    k_params<<<blocks, 128, 0, st>>>(dU, u, n, a2, a, b, f);
+// The counter stream's parameters: one warp per (path, axis), blocks spread over the
+// lanes, so every store is coalesced; the normalisation sums in ascending b as the
+// candidate test does.  Bound by the FP64 logarithms and the 20 bytes written per term:
+// 18 k paths x 2 axes x 255 terms in 0.11 ms (one thread per path, storing 5 KB apart from
+// its neighbours: 2.75 ms).
+__global__ void __launch_bounds__(128) k_params_philox(const UniDev* __restrict__ U, int u, int64_t n, double* a2o,
+                                                       double* ao, int32_t* bo, double* fo) {
+    __shared__ double s_e[4][kMaxF + 1];
+    const UniDev& d = U[u];
+    const int D = d.dim, nw = d.nw, F = d.F;
+    const int lane = threadIdx.x & 31;
+    double* e = s_e[threadIdx.x >> 5];
+    const int64_t warps = (int64_t)gridDim.x * 4;
+    for (int64_t i = (int64_t)blockIdx.x * 4 + (threadIdx.x >> 5); i < n * D; i += warps) {
+        const int64_t s = i / D;
+        const int ax = (int)(i - s * D);
+        const uint64_t idx = (uint64_t)d.acc_idx[s];
+        const int64_t o = i * nw - 2;  // term j = b - 2
+        for (int p = lane; 2 * p <= F; p += 32) {
+            const uint4 q = philox_block(d.seed, idx, ax, p);
+            if (p == 0) {
+                a2o[i] = d.pin ? 0.0 : (double)q.x * (1.0 / 2147483648.0) - 1.0;
+                continue;
+            }
+            const int be = 2 * p, bo2 = 2 * p + 1;
+            const double Ee = -log(((double)q.x + 0.5) * (1.0 / 4294967296.0));
+            e[be] = (q.z & 1u) ? -Ee : Ee;
+            fo[o + be] = (double)(q.z >> 1) * (1.0 / 2147483648.0) * kPi;
+            if (bo2 <= F) {
+                const double Eo = -log(((double)q.y + 0.5) * (1.0 / 4294967296.0));
+                e[bo2] = (q.w & 1u) ? -Eo : Eo;
+                fo[o + bo2] = 0.0;
+            }
+        }
+        __syncwarp();
+        double sum = 0.0;
+        if (lane == 0)
+            for (int b = 2; b <= F; b++) sum += fabs(e[b]);
+        sum = __shfl_sync(0xffffffffu, sum, 0);
+        for (int b = 2 + lane; b <= F; b += 32) {
+            const double amp = fabs(e[b]) / sum / (double)b;
+            ao[o + b] = e[b] < 0.0 ? -amp : amp;
+            bo[o + b] = b;
+        }
+        __syncwarp();
+    }
+}
+
+void launch_params(const UniDev* dU, int u, int rng, int dim, int64_t n, double* a2, double* a, int32_t* b,
+                   double* f, cudaStream_t st) {
+    if (rng == RNG_KNOT) {
+        const int blocks = (int)std::min<int64_t>((n + 127) / 128, 4096);
+        k_params<<<blocks, 128, 0, st>>>(dU, u, n, a2, a, b, f);
+        return;
+    }
+    const int blocks = (int)std::min<int64_t>((n * dim + 3) / 4, 148 * 64);
+    k_params_philox<<<blocks, 128, 0, st>>>(dU, u, n, a2, a, b, f);
 }
 
 // ------------------------------------------------------------- read-back

@@ -28,7 +28,7 @@
 
 namespace ug {
 
-int batch_params_view(void* h, int u, const UniDev** dU, int64_t* n, int* dim, int* nw, int* dev,
+int batch_params_view(void* h, int u, const UniDev** dU, int64_t* n, int* rng, int* dim, int* nw, int* dev,
                       cudaStream_t* st);
 int set_error(int code, const char* msg);
 
@@ -65,9 +65,9 @@ extern "C" int ug_batch_params_noalloc(void* h, int32_t u, double* a2, double* a
                                        int64_t cap_paths) {
     const UniDev* dU = nullptr;
     int64_t n = 0;
-    int dim = 0, nw = 0, dev = 0;
+    int rng = 0, dim = 0, nw = 0, dev = 0;
     cudaStream_t st = nullptr;
-    int rc = batch_params_view(h, u, &dU, &n, &dim, &nw, &dev, &st);
+    int rc = batch_params_view(h, u, &dU, &n, &rng, &dim, &nw, &dev, &st);
     if (rc) return rc;
     if (cap_paths < n) return set_error(UG_ECAP, "params buffer too small");
     if (n == 0) return UG_OK;
@@ -92,7 +92,7 @@ extern "C" int ug_batch_params_noalloc(void* h, int32_t u, double* a2, double* a
         double* da = (double*)(s + n_a2 * 8);
         double* df = (double*)(s + n_a2 * 8 + n_t * 8);
         int32_t* db = (int32_t*)(s + n_a2 * 8 + n_t * 16);
-        launch_params(dU, u, n, da2, da, db, df, st);
+        launch_params(dU, u, rng, dim, n, da2, da, db, df, st);
         cudaError_t e = cudaGetLastError();
         if (e == cudaSuccess && a2) e = cudaMemcpyAsync(a2, da2, n_a2 * 8, cudaMemcpyDeviceToHost, st);
         if (e == cudaSuccess && a) e = cudaMemcpyAsync(a, da, n_t * 8, cudaMemcpyDeviceToHost, st);
