@@ -699,48 +699,87 @@ __device__ __forceinline__ bool brick_cell_visit(const UniDev& U, int t, const N
 // cells fall into at most two bricks (a third only across the seam of a partial
 // last brick: then every coarse cell is tested on its own).  Each brick
 // combination costs one 64-bit word and a mask of the window's cells in it.
-template <class Visit>
-__device__ __forceinline__ bool nbhd_scan3(const UniDev& U, int t, const Nbhd<3>& nb, int64_t cpt,
-                                           Visit&& visit) {
+// The bricks (2^LB coarse cells long) of an axis window of n cells v[0..n): the first (bA)
+// with the mask of its coarse cells in the window, and the second (bB, -1 none).  True
+// when the window reaches a third, across the seam of a partial last brick.
+template <int LB>
+__device__ __forceinline__ bool window_bricks(const int (&v)[4], int n, int sh, int& bA, int& bB, uint32_t& mA,
+                                              uint32_t& mB) {
+    constexpr int W = 1 << LB;
+    const int last = n >= 4 ? v[3] : v[2];
+    const int oa = v[0] >> sh;
+    bA = oa >> LB;
+    if (last >= v[0]) {  // no wrap: a run of coarse cells, in at most two bricks
+        const uint32_t run = ((2u << ((last >> sh) - oa)) - 1u) << (oa & (W - 1));
+        mA = run & ((1u << W) - 1u);
+        mB = run >> W;
+        bB = mB ? bA + 1 : -1;
+        return false;
+    }
+    bB = -1;
+    mA = 1u << (oa & (W - 1));
+    mB = 0u;
+    bool three = false;
+#pragma unroll
+    for (int k = 1; k < 4; k++) {
+        if (k < n) {
+            const int o = v[k] >> sh, b = o >> LB;
+            const uint32_t bit = 1u << (o & (W - 1));
+            if (b == bA) {
+                mA |= bit;
+            } else if (bB < 0 || b == bB) {
+                bB = b;
+                mB |= bit;
+            } else {
+                three = true;
+            }
+        }
+    }
+    return three;
+}
+
+// p[i] when on, else 0: a predicated load, so that a caller's loads stay independent.
+__device__ __forceinline__ uint64_t ldg_if(const uint64_t* p, int64_t i, bool on) {
+    uint64_t v;
+    asm("{\n\t.reg .pred q;\n\t"
+        "setp.ne.b32 q, %2, 0;\n\t"
+        "mov.b64 %0, 0;\n\t"
+        "@q ld.global.nc.b64 %0, [%1];\n\t}"
+        : "=&l"(v)  // written before the address is read
+        : "l"(p + i), "r"((int)on));
+    return v;
+}
+
+// Calls cell(o0, o1, o2) for every occupied coarse cell of the window until it
+// returns true.
+template <class Cell>
+__device__ __forceinline__ bool nbhd_cells3(const UniDev& U, int t, const Nbhd<3>& nb, Cell&& cell) {
     const int sh = U.occ_shift, onb = U.occ_nb;
     int bA[3], bB[3];
     uint32_t mA[3], mB[3];
     bool three = false;
 #pragma unroll
-    for (int ax = 0; ax < 3; ax++) {
-        const int oa = nb.v[ax][0] >> sh;
-        bA[ax] = oa >> 2;
-        bB[ax] = -1;
-        mA[ax] = 1u << (oa & 3);
-        mB[ax] = 0u;
-#pragma unroll
-        for (int k = 1; k < 4; k++) {
-            if (k < nb.n[ax]) {
-                const int o = nb.v[ax][k] >> sh, b = o >> 2;
-                const uint32_t bit = 1u << (o & 3);
-                if (b == bA[ax]) {
-                    mA[ax] |= bit;
-                } else if (bB[ax] < 0 || b == bB[ax]) {
-                    bB[ax] = b;
-                    mB[ax] |= bit;
-                } else {
-                    three = true;
-                }
-            }
-        }
-    }
+    for (int ax = 0; ax < 3; ax++) three |= window_bricks<2>(nb.v[ax], nb.n[ax], sh, bA[ax], bB[ax], mA[ax], mB[ax]);
     const int64_t tb = (int64_t)t * U.occ_per_t;
     const uint64_t* W = reinterpret_cast<const uint64_t*>(U.occ);
     if (!three) {
+        // all loads first (predicated, no branch), then the masks: with the mask applied
+        // in the load's own branch the loads ran one after another
         uint64_t hits[8];
 #pragma unroll
         for (int c = 0; c < 8; c++) {
             const int B0 = (c & 4) ? bB[0] : bA[0], B1 = (c & 2) ? bB[1] : bA[1], B2 = (c & 1) ? bB[2] : bA[2];
-            hits[c] = 0;
-            if (B0 < 0 || B1 < 0 || B2 < 0) continue;
-            const uint32_t M0 = (c & 4) ? mB[0] : mA[0], M1 = (c & 2) ? mB[1] : mA[1], M2 = (c & 1) ? mB[2] : mA[2];
-            const uint64_t m = (uint64_t)(M2 * spread4(M1)) * spread16(M0);
-            hits[c] = __ldg(W + UG_IDX(tb + ((int64_t)B0 * onb + B1) * onb + B2, U.occ_words / 2)) & m;
+            const bool on = (B0 | B1 | B2) >= 0;  // -1: the window has no such brick
+            hits[c] = ldg_if(W, UG_IDX(on ? tb + ((int64_t)B0 * onb + B1) * onb + B2 : 0, U.occ_words / 2), on);
+        }
+        const uint32_t s1[2] = {spread4(mA[1]), spread4(mB[1])};
+        const uint64_t s0[2] = {spread16(mA[0]), spread16(mB[0])};
+#pragma unroll
+        for (int c = 0; c < 8; c++) {
+            // rows of 16 bits: the window's cells of axes 1 and 2, at the window's cells of axis 0
+            const uint32_t m12 = ((c & 1) ? mB[2] : mA[2]) * s1[(c >> 1) & 1];
+            const uint64_t z = s0[(c >> 2) & 1];
+            hits[c] &= (uint64_t)(m12 * (uint32_t)z) | (uint64_t)(m12 * (uint32_t)(z >> 32)) << 32;
         }
         uint32_t pend = 0;
 #pragma unroll
@@ -756,9 +795,7 @@ __device__ __forceinline__ bool nbhd_scan3(const UniDev& U, int t, const Nbhd<3>
             while (h) {
                 const int bit = __ffsll((long long)h) - 1;
                 h &= h - 1;
-                if (brick_cell_visit(U, t, nb, cpt, B0 * 4 + (bit >> 4), B1 * 4 + ((bit >> 2) & 3),
-                                     B2 * 4 + (bit & 3), visit))
-                    return true;
+                if (cell(B0 * 4 + (bit >> 4), B1 * 4 + ((bit >> 2) & 3), B2 * 4 + (bit & 3))) return true;
             }
         }
         return false;
@@ -776,11 +813,18 @@ __device__ __forceinline__ bool nbhd_scan3(const UniDev& U, int t, const Nbhd<3>
                 const int cc[3] = {f0, f1, f2};
                 const int64_t b = occ_bit(U, t, cc);
                 if (!((__ldg(U.occ + UG_IDX(b >> 5, U.occ_words)) >> (b & 31)) & 1u)) continue;
-                if (brick_cell_visit(U, t, nb, cpt, f0 >> sh, f1 >> sh, f2 >> sh, visit)) return true;
+                if (cell(f0 >> sh, f1 >> sh, f2 >> sh)) return true;
             }
         }
     }
     return false;
+}
+
+template <class Visit>
+__device__ __forceinline__ bool nbhd_scan3(const UniDev& U, int t, const Nbhd<3>& nb, int64_t cpt, Visit&& visit) {
+    return nbhd_cells3(U, t, nb, [&](int o0, int o1, int o2) {
+        return brick_cell_visit(U, t, nb, cpt, o0, o1, o2, visit);
+    });
 }
 
 // 1+1: coarse cells along the words.
@@ -896,47 +940,28 @@ __device__ __forceinline__ bool brick_cell_visit2(const UniDev& U, int t, const 
 
 // 2+1 neighbourhood scan over 8x8 bricks (as nbhd_scan3: at most two bricks per
 // axis, a third only across the seam of a partial last brick).
-template <class Visit>
-__device__ __forceinline__ bool nbhd_scan2(const UniDev& U, int t, const Nbhd<2>& nb, int64_t cpt,
-                                           Visit&& visit) {
+template <class Cell>
+__device__ __forceinline__ bool nbhd_cells2(const UniDev& U, int t, const Nbhd<2>& nb, Cell&& cell) {
     const int sh = U.occ_shift, onb = U.occ_nb;
     int bA[2], bB[2];
     uint32_t mA[2], mB[2];
     bool three = false;
 #pragma unroll
-    for (int ax = 0; ax < 2; ax++) {
-        const int oa = nb.v[ax][0] >> sh;
-        bA[ax] = oa >> 3;
-        bB[ax] = -1;
-        mA[ax] = 1u << (oa & 7);
-        mB[ax] = 0u;
-#pragma unroll
-        for (int k = 1; k < 4; k++) {
-            if (k < nb.n[ax]) {
-                const int o = nb.v[ax][k] >> sh, b = o >> 3;
-                const uint32_t bit = 1u << (o & 7);
-                if (b == bA[ax]) {
-                    mA[ax] |= bit;
-                } else if (bB[ax] < 0 || b == bB[ax]) {
-                    bB[ax] = b;
-                    mB[ax] |= bit;
-                } else {
-                    three = true;
-                }
-            }
-        }
-    }
+    for (int ax = 0; ax < 2; ax++) three |= window_bricks<3>(nb.v[ax], nb.n[ax], sh, bA[ax], bB[ax], mA[ax], mB[ax]);
     const int64_t tb = (int64_t)t * U.occ_per_t;
     const uint64_t* W = reinterpret_cast<const uint64_t*>(U.occ);
     if (!three) {
         uint64_t hits[4];
 #pragma unroll
-        for (int c = 0; c < 4; c++) {
+        for (int c = 0; c < 4; c++) {  // all loads first, as in nbhd_cells3
             const int B0 = (c & 2) ? bB[0] : bA[0], B1 = (c & 1) ? bB[1] : bA[1];
-            hits[c] = 0;
-            if (B0 < 0 || B1 < 0) continue;
+            const bool on = (B0 | B1) >= 0;
+            hits[c] = ldg_if(W, UG_IDX(on ? tb + (int64_t)B0 * onb + B1 : 0, U.occ_words / 2), on);
+        }
+#pragma unroll
+        for (int c = 0; c < 4; c++) {
             const uint32_t M0 = (c & 2) ? mB[0] : mA[0], M1 = (c & 1) ? mB[1] : mA[1];
-            hits[c] = __ldg(W + UG_IDX(tb + (int64_t)B0 * onb + B1, U.occ_words / 2)) & ((uint64_t)M1 * spread8(M0));
+            hits[c] &= (uint64_t)M1 * spread8(M0);
         }
         uint32_t pend = 0;
 #pragma unroll
@@ -952,7 +977,7 @@ __device__ __forceinline__ bool nbhd_scan2(const UniDev& U, int t, const Nbhd<2>
             while (h) {
                 const int bit = __ffsll((long long)h) - 1;
                 h &= h - 1;
-                if (brick_cell_visit2(U, t, nb, cpt, B0 * 8 + (bit >> 3), B1 * 8 + (bit & 7), visit)) return true;
+                if (cell(B0 * 8 + (bit >> 3), B1 * 8 + (bit & 7))) return true;
             }
         }
         return false;
@@ -966,10 +991,16 @@ __device__ __forceinline__ bool nbhd_scan2(const UniDev& U, int t, const Nbhd<2>
             const int cc[2] = {f0, f1};
             const int64_t b = occ_bit(U, t, cc);
             if (!((__ldg(U.occ + UG_IDX(b >> 5, U.occ_words)) >> (b & 31)) & 1u)) continue;
-            if (brick_cell_visit2(U, t, nb, cpt, f0 >> sh, f1 >> sh, visit)) return true;
+            if (cell(f0 >> sh, f1 >> sh)) return true;
         }
     }
     return false;
+}
+
+template <class Visit>
+__device__ __forceinline__ bool nbhd_scan2(const UniDev& U, int t, const Nbhd<2>& nb, int64_t cpt, Visit&& visit) {
+    return nbhd_cells2(U, t, nb,
+                       [&](int o0, int o1) { return brick_cell_visit2(U, t, nb, cpt, o0, o1, visit); });
 }
 
 // Visit the chains of the occupied cells of the neighbourhood at timestep t.

@@ -29,6 +29,7 @@
 #include <cmath>
 #include <cstdlib>
 #include <cstring>
+#include <type_traits>
 #include <vector>
 
 #include "ug_mixed.cuh"
@@ -76,6 +77,9 @@ __device__ __forceinline__ bool mbar_wait_ns(uint64_t* bar, uint32_t parity, uin
 // The prefilter's waits: ~1 s.
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity) {
     return mbar_wait_ns(bar, parity, 1000000000ull);
+}
+__device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
 __device__ __forceinline__ void mbar_expect_tx(uint64_t* bar, uint32_t bytes) {
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes)
@@ -133,6 +137,34 @@ __device__ __forceinline__ void tmem_ld8(uint32_t taddr, float* v) {
         : "memory");
 #pragma unroll
     for (int i = 0; i < 8; i++) v[i] = __uint_as_float(r[i]);
+}
+__device__ __forceinline__ void tmem_ld4(uint32_t taddr, float* v) {
+    uint32_t r[4];
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0, %1, %2, %3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+                 : "r"(taddr)
+                 : "memory");
+#pragma unroll
+    for (int i = 0; i < 4; i++) v[i] = __uint_as_float(r[i]);
+}
+__device__ __forceinline__ void tmem_ld2(uint32_t taddr, float* v) {
+    uint32_t r[2];
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x2.b32 {%0, %1}, [%2];"
+                 : "=r"(r[0]), "=r"(r[1])
+                 : "r"(taddr)
+                 : "memory");
+    v[0] = __uint_as_float(r[0]);
+    v[1] = __uint_as_float(r[1]);
+}
+template <int N>
+__device__ __forceinline__ void tmem_ldn(uint32_t taddr, float* v) {
+    static_assert(N == 2 || N == 4 || N == 8, "columns per load");
+    if constexpr (N == 8)
+        tmem_ld8(taddr, v);
+    else if constexpr (N == 4)
+        tmem_ld4(taddr, v);
+    else
+        tmem_ld2(taddr, v);
 }
 __device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 
@@ -230,57 +262,59 @@ __device__ __noinline__ bool group_contact(const UniDev& d, int32_t p, int t, in
     return cur != -1 && cur != gq;
 }
 
-// FP32 Chebyshev test of X (dim coords) at timestep t against the committed
-// packing.  Returns 1 when the candidate is certainly rejected; sets *gray when
-// a pair lies in the guard band.  The cell range covers every point within
-// r + m of X.  Group rounds (grp != nullptr): a certain contact joins the
-// candidate to the contact's group in *grp (shared by the row's threads); a
-// certain contact with a second group rejects.
-template <int D, bool kEuclid, bool kCheckL1 = true>
-__device__ __forceinline__ int test32_d(const UniDev& d, int t, const float* X, float r, float m,
-                                        float inv_cell, int64_t cpt, bool* gray, int* grp, int* nvis) {
-    // L2 ball: the FP32 distance vector is within sqrt(D) m of the exact one; r 1e-6
-    // more covers the FP32 rounding of the squared sums compared below (relative
-    // 3 2^-24 each).  The cell range covers the cube of half-width r + that bound.
-    const float mE = kEuclid ? m * (D == 3 ? 1.7320508f : (D == 2 ? 1.4142136f : 1.0f)) * 1.001f + r * 1e-6f : m;
-    const float band = mE * inv_cell + 1e-4f;
-    int c[D], elo[D], ehi[D];
-    float fr[D];
-#pragma unroll
-    for (int ax = 0; ax < D; ax++) {
-        const float u = (X[ax] + 1.0f) * inv_cell;
-        const float fl = floorf(u);
-        fr[ax] = u - fl;
-        int cc = (int)fl;
-        c[ax] = cc >= d.gw ? d.gw - 1 : (cc < 0 ? 0 : cc);
-    }
-    // the neighbourhood below lies within 2 cells of c on every axis
-    if (kCheckL1 && !occ1_hit<D>(d, t, c)) return 0;
-#pragma unroll
-    for (int ax = 0; ax < D; ax++) {
-        elo[ax] = fr[ax] < band ? 1 : 0;
-        ehi[ax] = fr[ax] > 1.0f - band ? 1 : 0;
-    }
+// FP32 Chebyshev (or L2-ball) test of X (dim coords) at timestep t against the committed
+// packing.  A certain contact rejects (hit returns true); a pair in the guard band sets
+// gray.  The cell range covers every point within r + m of X.  Group rounds (grp !=
+// nullptr): a certain contact joins the candidate to the contact's group in *grp (shared
+// by the row's threads); a certain contact with a second group rejects.
+template <int D, bool kEuclid>
+struct Test32 {
+    const UniDev& d;
+    int t;
+    const float* X;
+    float rin, rout, rin2, rout2;
+    bool gray = false;
+    int* grp;
+    int* nvis;
     Nbhd<D> nb;
-    nbhd_make<D>(d, c, elo, ehi, nb);
-    const float rin = r - mE, rout = r + mE;
-    const float rin2 = rin > 0.f ? rin * rin : -1.f, rout2 = rout * rout;
-    bool g = false;
-    const bool deep = nbhd_scan<D>(d, t, nb, cpt, [&](int32_t p, int32_t& nx) -> bool {
+
+    __device__ __forceinline__ Test32(const UniDev& d_, int t_, const float* X_, float r, float m, float inv_cell,
+                                      int* grp_, int* nvis_)
+        : d(d_), t(t_), X(X_), grp(grp_), nvis(nvis_) {
+        // L2 ball: the FP32 distance vector is within sqrt(D) m of the exact one; r 1e-6
+        // more covers the FP32 rounding of the squared sums compared below (relative
+        // 3 2^-24 each).  The cell range covers the cube of half-width r + that bound.
+        const float mE = kEuclid ? m * (D == 3 ? 1.7320508f : (D == 2 ? 1.4142136f : 1.0f)) * 1.001f + r * 1e-6f : m;
+        const float band = mE * inv_cell + 1e-4f;
+        int c[D], elo[D], ehi[D];
+#pragma unroll
+        for (int ax = 0; ax < D; ax++) {
+            const float u = (X[ax] + 1.0f) * inv_cell;
+            const float fl = floorf(u);
+            const float fr = u - fl;
+            const int cc = (int)fl;
+            c[ax] = cc >= d.gw ? d.gw - 1 : (cc < 0 ? 0 : cc);
+            elo[ax] = fr < band ? 1 : 0;
+            ehi[ax] = fr > 1.0f - band ? 1 : 0;
+        }
+        nbhd_make<D>(d, c, elo, ehi, nb);
+        rin = r - mE;
+        rout = r + mE;
+        rin2 = rin > 0.f ? rin * rin : -1.f;
+        rout2 = rout * rout;
+    }
+    // Accepted point p; nx gets the next of its chain.
+    __device__ __forceinline__ bool operator()(int32_t p, int32_t& nx) {
         const uint4 qr = __ldg(reinterpret_cast<const uint4*>(d.ptf) + UG_IDX((int64_t)p * d.T + t, d.slot_cap * d.T));
-        Pt32 q;
-        q.c[0] = __uint_as_float(qr.x);
-        q.c[1] = __uint_as_float(qr.y);
-        q.c[2] = __uint_as_float(qr.z);
-        q.next = (int32_t)qr.w;
-        nx = q.next;
+        const float c[3] = {__uint_as_float(qr.x), __uint_as_float(qr.y), __uint_as_float(qr.z)};
+        nx = (int32_t)qr.w;
         ++*nvis;
         bool miss = false, in = true;
         if (kEuclid) {
             float s2 = 0.f;
 #pragma unroll
             for (int ax = 0; ax < D; ax++) {
-                const float dd = torus_deltaf(X[ax] - q.c[ax]);
+                const float dd = torus_deltaf(X[ax] - c[ax]);
                 s2 = fmaf(dd, dd, s2);
             }
             miss = s2 > rout2;
@@ -288,27 +322,17 @@ __device__ __forceinline__ int test32_d(const UniDev& d, int t, const float* X, 
         } else {
 #pragma unroll
             for (int ax = 0; ax < D; ax++) {
-                const float dd = fabsf(torus_deltaf(X[ax] - q.c[ax]));
+                const float dd = fabsf(torus_deltaf(X[ax] - c[ax]));
                 miss |= dd > rout;
                 in &= dd < rin;
             }
         }
         if (miss) return false;
         if (in) return grp ? group_contact(d, p, t, grp) : true;
-        g = true;
+        gray = true;
         return false;
-    });
-    if (g) *gray = true;
-    return deep ? 1 : 0;
-}
-
-template <bool kEuclid, bool kCheckL1 = true>
-__device__ __forceinline__ int test32_at(const UniDev& d, int t, const float* X, float r, float m,
-                                         float inv_cell, int64_t cpt, bool* gray, int* grp, int* nvis) {
-    if (d.dim == 3) return test32_d<3, kEuclid, kCheckL1>(d, t, X, r, m, inv_cell, cpt, gray, grp, nvis);
-    if (d.dim == 2) return test32_d<2, kEuclid, kCheckL1>(d, t, X, r, m, inv_cell, cpt, gray, grp, nvis);
-    return test32_d<1, false, kCheckL1>(d, t, X, r, m, inv_cell, cpt, gray, grp, nvis);  // 1 axis: ball == cube
-}
+    }
+};
 
 // --------------------------------------------------------------- kernel
 
@@ -325,11 +349,16 @@ struct MixedLaunch {
 
 constexpr int kMxThreads = 512;  // 4 threads per candidate row
 constexpr int kMxParts = kMxThreads / kTile;
-constexpr int kXsFloats = 8 * 3 * 32 + 32 + 16;  // per-warp epilogue staging: positions, rho, columns
-constexpr int kMxCompact = 24;
-// the epilogue staging of all warps fits in the smallest pair of operand stages (T <= 16)
-static_assert((kMxThreads / 32) * kXsFloats * 4 <= 2 * (2 * kAImgBytes + 16 * kKC * 2 * 2),
-              "epilogue staging exceeds the operand stages");   // live rows of a warp at or below which their tests are spread (16, 24, 32 measured)
+constexpr int kQueue = 2048;  // tests of one epilogue stage: live rows x columns
+constexpr int kDense = 64;    // live rows of a stage of 32 columns or more (compacted), at most
+constexpr int kCells = 2560;  // occupied cells of their windows
+// the queues fit in the smallest pair of operand stages (T <= 16)
+static_assert(kQueue * 16 + kCells * 8 <= 2 * (2 * kAImgBytes + 16 * kKC * 2 * 2), "queues exceed the operand stages");
+// ... and so do the queue and a compacted stage's products (in the cells' place: kDense rows
+// of 16 columns at T <= 16, kQueue tests of 3 axes and a pad column per row above)
+static_assert(kQueue * 16 + kDense * 3 * 17 * 4 <= 2 * (2 * kAImgBytes + 16 * kKC * 2 * 2) &&
+                  kQueue * 16 + (kQueue + kDense) * 3 * 4 <= 2 * (2 * kAImgBytes + 32 * kKC * 2 * 2),
+              "compacted products exceed the operand stages");
 
 // kGroup: the batch holds group-mode universes (group rounds need the join /
 // two-group logic in the neighbour scans; batches without them run without it).
@@ -344,31 +373,45 @@ __global__ void __launch_bounds__(kMxThreads, 1) k_prefilter_mixed(const UniDev*
     const int part = warp >> 2;
     // carve: two stages of {A_hi, A_lo, B (hi then lo)}; per-row state; barriers
     const int stage_bytes = 2 * kAImgBytes + L.tpad_max * kKC * 2 * 2;
-    double* s_sum = reinterpret_cast<double*>(sm + 2 * stage_bytes);      // [kTile][kMxParts][2]
-    int* s_rej = reinterpret_cast<int*>(s_sum + kTile * kMxParts * 2);   // [kTile]
+    double* s_sum = reinterpret_cast<double*>(sm + 2 * stage_bytes);          // [3][kTile][kMxParts][2]
+    int* s_rej = reinterpret_cast<int*>(s_sum + 3 * kTile * kMxParts * 2);   // [kTile]
     int* s_gray = s_rej + kTile;                                          // [kTile]
     int* s_grp = s_gray + kTile;                                          // [kTile] group rounds
     uint64_t* bar = reinterpret_cast<uint64_t*>(s_grp + kTile);
     uint64_t* bar_b = bar;       // [2] B chunk landed
     uint64_t* bar_m = bar + 2;   // [2] MMAs reading the stage finished
-    uint64_t* bar_d = bar + 4;   // all MMAs of the pass finished
-    uint32_t* holder = reinterpret_cast<uint32_t*>(bar + 5);
+    uint64_t* bar_a = bar + 4;   // [2] A chunk written by the 16 warps
+    uint32_t* holder = reinterpret_cast<uint32_t*>(bar + 6);
+    __shared__ int s_to;  // a wait gave up
+    volatile int* vto = &s_to;
 
+    // epilogue: queued tests of the current and the next stage; the universe's timesteps
+    // in column order and 1 / sin z of each; each row's rho
+    __shared__ int s_qn[2], s_qc[2];
+    __shared__ int32_t s_t[kMaxF];
+    __shared__ float s_isz[kMaxF];
+    __shared__ float s_rho[kTile];
+    // compacted live rows of a stage: lanes per quarter, row, and 1 / sum E, a2 of each axis
+    __shared__ uint32_t s_live[4];
+    __shared__ int32_t s_row[kDense];
+    __shared__ float s_aff[kDense][6];
     // tile offsets of the universes, for the per-tile lookup of its universe
     __shared__ int32_t s_toff[kMaxUni + 1];
     if (L.dump == nullptr)
-        for (int i = tid; i <= info->n_uni; i += blockDim.x) s_toff[i] = info->tile_off[i];
+        for (int i = tid; i <= info->n_uni; i += kMxThreads) s_toff[i] = info->tile_off[i];
     if (warp == 0) tmem_alloc(holder, L.ncols);
     if (tid == 0) {
-        for (int i = 0; i < 5; i++) mbar_init(&bar[i], 1);
+        for (int i = 0; i < 6; i++) mbar_init(&bar[i], i < 4 ? 1 : kMxThreads / 32);
         fence_mbar_init();
+        s_to = 0;
     }
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = *holder;
 
-    uint32_t ph_b[2] = {0, 0}, ph_m[2] = {0, 0}, ph_d = 0;
+    // bit st: barrier phases of the stages, and whether its products are still to be waited for
+    uint32_t ph_b = 0, ph_m = 0, busy = 0;
     int seq = 0;
     bool timeout = false;
     const bool dump = L.dump != nullptr;
@@ -422,7 +465,6 @@ __global__ void __launch_bounds__(kMxThreads, 1) k_prefilter_mixed(const UniDev*
         }
         const int dim = d.dim, T = d.T, nch = d.mx_chunks, tpad = d.mx_tpad, nm = d.mx_nmma;
         const uint32_t bchunk = (uint32_t)tpad * kKC * 2 * 2;  // hi + lo images
-        const uint32_t idesc = idesc_bf16(128, nm);
         const float r = (float)d.cell, mrg = d.mx_margin, inv_cell = (float)(1.0 / d.cell);
         const int64_t cpt = cells_per_t(d);
         const uint32_t* __restrict__ occ1 = d.occ1;
@@ -438,10 +480,16 @@ __global__ void __launch_bounds__(kMxThreads, 1) k_prefilter_mixed(const UniDev*
             s_gray[row] = 0;
             s_grp[row] = -1;
         }
-        int nev = 0, nvis = 0;
+        for (int j = tid; j < T; j += kMxThreads) {
+            const int t = __ldg(d.order + j);
+            s_t[j] = t;
+            s_isz[j] = (float)__ldg(d.invsinz + t);
+        }
+        if (tid < 2) s_qn[tid] = s_qc[tid] = 0;
+        int nev = 0, nvis = 0, stage = 0;
         for (int pass = 0; pass < d.mx_npass && !timeout; pass++) {
-            if (pass > 0 && __syncthreads_and(vrej[row] != 0)) break;
-            for (int ax = 0; ax < dim && !timeout; ax++) {
+            if (pass > 0 && __syncthreads_count(vrej[row] == 0) == 0) break;
+            for (int ax = 0; ax < dim; ax++) {
                 double sumE = 0.0, sumEb = 0.0;
                 if (pass == 0 && valid) {
                     const uint4 o = philox_block(d.seed, idx, ax, 0);
@@ -452,74 +500,86 @@ __global__ void __launch_bounds__(kMxThreads, 1) k_prefilter_mixed(const UniDev*
                 }
                 for (int ch = 0; ch < nch; ch++, seq++) {
                     const int st = seq & 1;
-                    uint8_t* sbase = sm + st * stage_bytes;
-                    uint8_t* a_hi = sbase;
-                    uint8_t* a_lo = sbase + kAImgBytes;
-                    uint8_t* b_img = sbase + 2 * kAImgBytes;
-                    if (seq >= 2) {  // one thread polls; the CTA barrier releases the rest
-                        if (tid == 0 && !mbar_wait(&bar_m[st], ph_m[st])) timeout = true;
-                        ph_m[st] ^= 1;
-                    }
-                    if (__syncthreads_or(timeout)) {
-                        timeout = true;
-                        break;
+                    uint8_t* a_hi = sm + st * stage_bytes;
+                    uint8_t* a_lo = a_hi + kAImgBytes;
+                    if ((busy >> st) & 1) {  // one lane per warp polls for the stage
+                        if (lane == 0 && !mbar_wait(&bar_m[st], (ph_m >> st) & 1)) *vto = 1;
+                        ph_m ^= 1u << st;
+                        __syncwarp();
                     }
                     if (tid == 0) {
                         mbar_expect_tx(&bar_b[st], bchunk);
-                        bulk_g2s(b_img, d.mx_bimg + UG_IDX((int64_t)ch * bchunk + bchunk - 1, d.bimg_bytes) + 1 - bchunk,
-                                 bchunk, &bar_b[st]);
+                        bulk_g2s(a_hi + 2 * kAImgBytes,
+                                 d.mx_bimg + UG_IDX((int64_t)ch * bchunk + bchunk - 1, d.bimg_bytes) + 1 - bchunk, bchunk,
+                                 &bar_b[st]);
                     }
                     sumE += gen_quarter(d, idx, ax, ch, part, valid, a_hi, a_lo, row, &sumEb);
                     fence_proxy_async();
-                    __syncthreads();
-                    if (tid == 0) {
-                        if (!mbar_wait(&bar_b[st], ph_b[st])) timeout = true;
-                        tc_fence_after();
-                        if (!timeout) {
-                            const uint32_t ah = smem_u32(a_hi), al = smem_u32(a_lo);
-                            const uint32_t bh = smem_u32(b_img) + (uint32_t)(pass * nm * 16);
-                            const uint32_t bl = bh + (uint32_t)tpad * kKC * 2;
-                            const uint32_t dtm = tmem + (uint32_t)UG_IDX(ax * nm + nm - 1, L.ncols) + 1 - nm;
+                    __syncwarp();
+                    // The warps take turns at issuing a chunk's products (after those it issued
+                    // itself and, through the barrier, all earlier ones), committed to the
+                    // stage; the others go on to the next chunk.  No barrier of the CTA until
+                    // the end of the pass: with one, and thread 0 issuing, each chunk cost all
+                    // warps its wait and its issue.
+                    if (lane == 0) {
+                        tc_fence_before();
+                        mbar_arrive(&bar_a[st]);
+                        if (warp == (seq & (kMxThreads / 32 - 1))) {
+                            if (!mbar_wait(&bar_a[st], (ph_b >> st) & 1)) *vto = 1;
+                            tc_fence_after();
+                            if (!mbar_wait(&bar_b[st], (ph_b >> st) & 1)) *vto = 1;
+                            if (!*vto) {
+                                const uint32_t idesc = idesc_bf16(128, nm);
+                                const uint32_t ah = smem_u32(a_hi), al = ah + kAImgBytes;
+                                const uint32_t bh = ah + 2 * kAImgBytes + (uint32_t)(pass * nm * 16);
+                                const uint32_t bl = bh + (uint32_t)tpad * kKC * 2;
+                                const uint32_t dtm = tmem + (uint32_t)UG_IDX(ax * nm + nm - 1, L.ncols) + 1 - nm;
 #pragma unroll
-                            for (int j = 0; j < kKC / 16; j++) {
-                                const uint64_t dah = sdesc(ah + j * 2 * (kTile * 16), kTile * 16, 128);
-                                const uint64_t dal = sdesc(al + j * 2 * (kTile * 16), kTile * 16, 128);
-                                const uint64_t dbh = sdesc(bh + j * 2 * (tpad * 16), tpad * 16, 128);
-                                const uint64_t dbl = sdesc(bl + j * 2 * (tpad * 16), tpad * 16, 128);
-                                umma_bf16(dtm, dah, dbh, idesc, (ch > 0 || j > 0) ? 1u : 0u);
-                                umma_bf16(dtm, dah, dbl, idesc, 1u);
-                                umma_bf16(dtm, dal, dbh, idesc, 1u);
+                                for (int j = 0; j < kKC / 16; j++) {
+                                    const uint64_t dah = sdesc(ah + j * 2 * (kTile * 16), kTile * 16, 128);
+                                    const uint64_t dal = sdesc(al + j * 2 * (kTile * 16), kTile * 16, 128);
+                                    const uint64_t dbh = sdesc(bh + j * 2 * (tpad * 16), tpad * 16, 128);
+                                    const uint64_t dbl = sdesc(bl + j * 2 * (tpad * 16), tpad * 16, 128);
+                                    umma_bf16(dtm, dah, dbh, idesc, (ch > 0 || j > 0) ? 1u : 0u);
+                                    umma_bf16(dtm, dah, dbl, idesc, 1u);
+                                    umma_bf16(dtm, dal, dbh, idesc, 1u);
+                                }
                             }
+                            umma_commit(&bar_m[st]);
                         }
-                        umma_commit(&bar_m[st]);
                     }
-                    ph_b[st] ^= 1;
+                    __syncwarp();
+                    busy |= 1u << st;
+                    ph_b ^= 1u << st;
                 }
-                if (timeout) break;
-                if (pass == 0) {  // combine the four partial sums of the row in a fixed order
-                    double* ss = s_sum + row * kMxParts * 2;
-                    ss[2 * part] = sumE;
-                    ss[2 * part + 1] = sumEb;
-                    __syncthreads();
-                    const double tot = ss[0] + ss[2] + ss[4] + ss[6];
-                    const double teb = ss[1] + ss[3] + ss[5] + ss[7];
-                    const float iv = valid ? (float)(1.0 / tot) : 0.f;
+                if (pass == 0) {
+                    double* ss = s_sum + ((ax * kTile + row) * kMxParts + part) * 2;
+                    ss[0] = sumE;
+                    ss[1] = sumEb;
+                }
+            }
+            // the pass's products: earlier chunks of a stage were waited for at its next use
 #pragma unroll
-                    for (int k = 0; k < 3; k++)
-                        if (k == ax) inv_sum[k] = iv;
-                    if (valid) rho = fmaxf(rho, (float)(teb / tot));
-                    __syncthreads();
+            for (int st = 0; st < 2; st++)
+                if ((busy >> st) & 1) {
+                    if (tid == 0 && !mbar_wait(&bar_m[st], (ph_m >> st) & 1)) *vto = 1;
+                    ph_m ^= 1u << st;
                 }
-            }
-            if (timeout) break;
-            if (tid == 0) {
-                umma_commit(bar_d);
-                if (!mbar_wait(bar_d, ph_d)) timeout = true;
-            }
-            ph_d ^= 1;
-            if (__syncthreads_or(timeout)) {
+            busy = 0;
+            if (__syncthreads_or(*vto != 0)) {
                 timeout = true;
                 break;
+            }
+            if (pass == 0) {  // combine the four partial sums of the row in a fixed order
+#pragma unroll
+                for (int ax = 0; ax < 3; ax++)
+                    if (ax < dim && valid) {
+                        const double* ss = s_sum + (ax * kTile + row) * kMxParts * 2;
+                        const double tot = ss[0] + ss[2] + ss[4] + ss[6];
+                        const double teb = ss[1] + ss[3] + ss[5] + ss[7];
+                        inv_sum[ax] = (float)(1.0 / tot);
+                        rho = fmaxf(rho, (float)(teb / tot));
+                    }
             }
             tc_fence_after();
             if (dim == 1 && d.cross1d && !dump) {
@@ -629,20 +689,16 @@ __global__ void __launch_bounds__(kMxThreads, 1) k_prefilter_mixed(const UniDev*
                 __syncthreads();
                 continue;  // single pass for dim 1
             }
-            // epilogue: 8-column blocks part, part+4, ... of this pass (endpoint-first order)
             const uint32_t lane_base = tmem + ((uint32_t)((warp & 3) * 32) << 16);
-            for (int c0 = part * 8; c0 < nm; c0 += 8 * kMxParts) {
-                const int col0 = pass * nm + c0;
-                if (col0 >= T) break;
-                if (!dump && __all_sync(0xffffffffu, vrej[row] != 0)) break;
-                float x[3][8];
+            if (dump) {
+                for (int c0 = part * 8; c0 < nm && pass * nm + c0 < T; c0 += 8 * kMxParts) {
+                    float x[3][8];
 #pragma unroll
-                for (int ax = 0; ax < 3; ax++)
-                    if (ax < dim) tmem_ld8(lane_base + (uint32_t)UG_IDX(ax * nm + c0 + 7, L.ncols) - 7, x[ax]);
-                tmem_wait_ld();
-                if (dump) {
+                    for (int ax = 0; ax < 3; ax++)
+                        if (ax < dim) tmem_ld8(lane_base + (uint32_t)UG_IDX(ax * nm + c0 + 7, L.ncols) - 7, x[ax]);
+                    tmem_wait_ld();
                     for (int j = 0; j < 8; j++) {
-                        const int col = col0 + j;
+                        const int col = pass * nm + c0 + j;
                         if (col >= T) break;
                         // the crossing rule's B image (1+1D) holds the timesteps in natural order
                         const int t = (dim == 1 && d.cross1d) ? col : __ldg(d.order + col);
@@ -656,104 +712,266 @@ __global__ void __launch_bounds__(kMxThreads, 1) k_prefilter_mixed(const UniDev*
                             L.dump_m[(size_t)off * T + t] = mt;
                         }
                     }
-                    continue;
                 }
-                const uint32_t am = __ballot_sync(0xffffffffu, valid && !vrej[row]);
-                const int na = __popc(am);
-                if (na == 0) continue;
-                const int ncol = min(8, T - col0);
-                // The block's work is its (live row, column) tests.  Many live rows: each
-                // lane tests its own row's columns.  Few (<= kMxCompact): the tests are
-                // spread over all 32 lanes, column-major, so dead rows leave no lane idle.
-                // Either way a lane first issues the first-level loads of all its tests
-                // together (the dilated occupancy bit of each test point's own cell
-                // block; a clear bit proves the neighbourhood empty), then runs the
-                // exact test only where a bit is set.  The block's positions and column
-                // data are staged in this warp's slice of the (now idle) operand stages.
-                float* xs = reinterpret_cast<float*>(sm) + warp * kXsFloats;  // [8][3][32], rho[32], t[8], isz[8]
-                int* xt = reinterpret_cast<int*>(xs + 8 * 3 * 32 + 32);
-                float* xz = xs + 8 * 3 * 32 + 32 + 8;
-                if (lane < ncol) {
-                    const int t = __ldg(d.order + col0 + lane);
-                    xt[lane] = t;
-                    xz[lane] = (float)__ldg(d.invsinz + t);
-                }
-#pragma unroll
-                for (int j = 0; j < 8; j++)
+                tc_fence_before();
+                __syncthreads();
+                continue;
+            }
+            // Epilogue, in stages of columns (endpoint-first order: a step rejects 7 to 37 %
+            // of the live rows).  A stage is as wide as kQueue tests of the live rows allow:
+            // 8 columns while most rows live, 128 for the last few.  Its four parts of a row
+            // take a quarter of the columns each: positions from tensor memory, then the
+            // first-level loads of all of them together (the dilated occupancy bit of each
+            // position's own cell block; a clear bit proves the neighbourhood empty).  The
+            // positions with a set bit go to one queue of the CTA, from which all 512 threads
+            // take the exact guard-band tests, windows first, then chains.  These are chains of dependent loads: a lane
+            // that tested its own row's columns one after another (8 at a time, all parts at
+            // once) held its tile for up to 64 of them and tested 32 columns of every row.
+            float4* queue = reinterpret_cast<float4*>(sm);  // the operand stages are idle
+            uint2* cells = reinterpret_cast<uint2*>(queue + kQueue);
+            if (part == 0) s_rho[row] = rho;
+            const int pcols = min(nm, T - pass * nm);
+            for (int c0 = 0; c0 < pcols;) {
+                // (also the barrier between one stage's tests and the next stage's queue; the
+                // last tests may reject rows that are counted here: na is an upper bound)
+                const int na = __syncthreads_count(part == 0 && vrej[row] == 0);
+                if (na == 0) break;
+                const int na2 = dim == 3 ? na : 2 * na;
+                const int width = na2 > 128 ? 8 : (na2 > 64 ? 16 : (na2 > 32 ? 32 : (na2 > 16 ? 64 : 128)));
+                int* qn = &s_qn[stage & 1];
+                int* qc = &s_qc[stage & 1];
+                if (tid == 0) s_qn[(stage & 1) ^ 1] = s_qc[(stage & 1) ^ 1] = 0;  // read before the barrier above
+                stage++;
+                auto enqueue = [&](auto nc, int cb) {  // columns [cb, cb + nc) of the pass
+                    constexpr int N = decltype(nc)::value;
+                    float x[3][N];
 #pragma unroll
                     for (int ax = 0; ax < 3; ax++)
-                        if (j < ncol && ax < dim)
-                            xs[(j * 3 + ax) * 32 + lane] = torus_wrapf(fmaf(x[ax][j], inv_sum[ax], a2f[ax]));
-                xs[8 * 3 * 32 + lane] = rho;
-                __syncwarp();
-                const bool spread = na <= kMxCompact;
-                const int nitems = spread ? na * ncol : (((am >> lane) & 1u) ? ncol : 0);
-                const int rbase = (warp & 3) * 32;
-                uint32_t wv[8];
-                uint64_t bsh = 0;  // bit position of each test's block in its word, 5 bits each
+                        if (ax < dim) tmem_ldn<N>(lane_base + (uint32_t)UG_IDX(ax * nm + cb + N - 1, L.ncols) + 1 - N, x[ax]);
+                    tmem_wait_ld();
+                    const bool live = vrej[row] == 0;
+                    if (!__any_sync(0xffffffffu, live)) return;
+                    const int n = min(N, pcols - cb);
+                    uint32_t w[N], need = 0;
+                    uint64_t bsh = 0;  // bit position of each block in its word, 5 bits each
 #pragma unroll
-                for (int k = 0; k < 8; k++) {
-                    const int i = spread ? lane + 32 * k : k;
-                    wv[k] = 0u;
-                    if (i < nitems) {
-                        const int j = spread ? i / na : k;
-                        const int src = spread ? (int)__fns(am, 0, i - j * na + 1) : lane;
-                        const int t = xt[j];
+                    for (int j = 0; j < N; j++) {
+                        w[j] = 0u;
+                        if (!live || j >= n) continue;
                         int64_t lin = 0;
 #pragma unroll
                         for (int ax = 0; ax < 3; ax++) {
                             if (ax >= dim) break;
-                            int cc = (int)floorf((xs[(j * 3 + ax) * 32 + src] + 1.0f) * inv_cell);
+                            x[ax][j] = torus_wrapf(fmaf(x[ax][j], inv_sum[ax], a2f[ax]));
+                            int cc = (int)floorf((x[ax][j] + 1.0f) * inv_cell);
                             cc = cc >= gw ? gw - 1 : (cc < 0 ? 0 : cc);
                             lin = lin * occ1_gw + (cc >> occ1_sh);
                         }
-                        const int64_t b = (int64_t)t * occ1_pt + lin;
-                        bsh |= (uint64_t)(b & 31) << (5 * k);
-                        wv[k] = __ldg(occ1 + (b >> 5));
+                        const int64_t b = (int64_t)s_t[pass * nm + cb + j] * occ1_pt + lin;
+                        bsh |= (uint64_t)(b & 31) << (5 * j);
+                        w[j] = __ldg(occ1 + UG_IDX(b >> 5, d.occ1_words));
+                    }
+#pragma unroll
+                    for (int j = 0; j < N; j++) need |= ((w[j] >> ((bsh >> (5 * j)) & 31)) & 1u) << j;
+                    if (live) nev += n;
+                    // one claim of queue entries per warp
+                    int incl = __popc(need);
+                    const int mine = incl;
+#pragma unroll
+                    for (int o = 1; o < 32; o <<= 1) {
+                        const int v = __shfl_up_sync(0xffffffffu, incl, o);
+                        if (lane >= o) incl += v;
+                    }
+                    int at = 0;
+                    if (lane == 31 && incl) at = atomicAdd(qn, incl);
+                    at = __shfl_sync(0xffffffffu, at, 31) + incl - mine;
+#pragma unroll
+                    for (int j = 0; j < N; j++)
+                        if ((need >> j) & 1u) {
+                            queue[UG_IDX(at, kQueue)] = make_float4(x[0][j], dim > 1 ? x[1][j] : 0.f, dim > 2 ? x[2][j] : 0.f,
+                                                                    __int_as_float(row | (pass * nm + cb + j) << 8));
+                            at++;
+                        }
+                };
+                const int wp = width / kMxParts, cb = c0 + part * wp;
+                if (wp == 2) {  // cb even and below pcols: the load stays within the pass's nm columns
+                    if (cb < pcols) enqueue(std::integral_constant<int, 2>{}, cb);
+                } else if (wp == 4) {
+                    if (cb < pcols) enqueue(std::integral_constant<int, 4>{}, cb);
+                } else {  // wp a multiple of 8, cb too (nm is one of 16)
+                    // Few live rows: their products go to shared memory, and the tests are
+                    // spread evenly over the threads (a lane per row would leave most idle).
+                    if (part == 0) {  // live rows of this warp's quarter, in order
+                        const uint32_t lv = __ballot_sync(0xffffffffu, vrej[row] == 0);
+                        if (lane == 0) s_live[warp] = lv;
+                    }
+                    __syncthreads();
+                    const int q = warp & 3;
+                    const uint32_t lv = s_live[q];
+                    int slot = __popc(lv & ((1u << lane) - 1u)), nl = 0;
+#pragma unroll
+                    for (int k = 0; k < 4; k++) {
+                        if (k == q) slot += nl;
+                        nl += __popc(s_live[k]);
+                    }
+                    const bool live = (lv >> lane) & 1u;
+                    if (part == 0 && live) {
+                        s_row[slot] = row;
+#pragma unroll
+                        for (int ax = 0; ax < 3; ax++) {
+                            s_aff[slot][2 * ax] = inv_sum[ax];
+                            s_aff[slot][2 * ax + 1] = a2f[ax];
+                        }
+                    }
+                    float* raw = reinterpret_cast<float*>(cells);  // [slot][axis][column of the stage]
+                    const int nc = min(width, pcols - c0), nt = nl * nc, pitch = nc + 1;
+                    if (lv)
+                        for (int k = 0; k < wp && cb + k < pcols; k += 8) {
+                            float x[3][8];
+#pragma unroll
+                            for (int ax = 0; ax < 3; ax++)
+                                if (ax < dim) tmem_ld8(lane_base + (uint32_t)UG_IDX(ax * nm + cb + k + 7, L.ncols) - 7, x[ax]);
+                            tmem_wait_ld();
+                            if (live)
+#pragma unroll
+                                for (int ax = 0; ax < 3; ax++)
+                                    if (ax < dim)
+#pragma unroll
+                                        for (int j = 0; j < 8; j++)
+                                            if (cb - c0 + k + j < nc) raw[(slot * dim + ax) * pitch + cb - c0 + k + j] = x[ax][j];
+                        }
+                    __syncthreads();
+                    nev += nt > tid ? (nt - tid + kMxThreads - 1) / kMxThreads : 0;
+                    for (int i0 = 0; i0 < nt; i0 += 2 * kMxThreads) {  // two tests a thread at once
+                        float X[2][3];
+                        uint32_t w[2], sh[2];
+                        int rc[2];
+#pragma unroll
+                        for (int h = 0; h < 2; h++) {
+                            const int i = i0 + h * kMxThreads + tid;
+                            w[h] = sh[h] = 0u;
+                            if (i >= nt) continue;
+                            const int sl = i / nc, j = i - sl * nc;
+                            int64_t lin = 0;
+#pragma unroll
+                            for (int ax = 0; ax < 3; ax++) {
+                                X[h][ax] = 0.f;
+                                if (ax >= dim) continue;
+                                X[h][ax] = torus_wrapf(fmaf(raw[(sl * dim + ax) * pitch + j], s_aff[sl][2 * ax], s_aff[sl][2 * ax + 1]));
+                                int cc = (int)floorf((X[h][ax] + 1.0f) * inv_cell);
+                                cc = cc >= gw ? gw - 1 : (cc < 0 ? 0 : cc);
+                                lin = lin * occ1_gw + (cc >> occ1_sh);
+                            }
+                            const int col = pass * nm + c0 + j;
+                            const int64_t b = (int64_t)s_t[col] * occ1_pt + lin;
+                            rc[h] = s_row[sl] | col << 8;
+                            sh[h] = (uint32_t)(b & 31);
+                            w[h] = __ldg(occ1 + UG_IDX(b >> 5, d.occ1_words));
+                        }
+#pragma unroll
+                        for (int h = 0; h < 2; h++) {
+                            const bool need = (w[h] >> sh[h]) & 1u;
+                            const uint32_t m = __ballot_sync(0xffffffffu, need);
+                            if (!m) continue;
+                            int at = 0;
+                            if (lane == 0) at = atomicAdd(qn, __popc(m));
+                            at = __shfl_sync(0xffffffffu, at, 0) + __popc(m & ((1u << lane) - 1u));
+                            if (need) queue[UG_IDX(at, kQueue)] = make_float4(X[h][0], X[h][1], X[h][2], __int_as_float(rc[h]));
+                        }
                     }
                 }
-                uint32_t need = 0;
-#pragma unroll
-                for (int k = 0; k < 8; k++) need |= ((wv[k] >> ((bsh >> (5 * k)) & 31)) & 1u) << k;
-                // tests of this lane (main: the row's columns up to its first certain contact)
-                int tested = spread ? (nitems > lane ? (nitems - lane + 31) / 32 : 0) : nitems;
-                while (need) {
-                    const int k = __ffs(need) - 1;
-                    need &= need - 1;
-                    const int i = spread ? lane + 32 * k : k;
-                    const int j = spread ? i / na : k;
-                    const int src = spread ? (int)__fns(am, 0, i - j * na + 1) : lane;
-                    const int rrow = rbase + src;
-                    if (vrej[rrow]) {
-                        if (!spread) {
-                            tested = k;
-                            break;
-                        }
-                        continue;
-                    }
-                    const int t = xt[j];
-                    float X[3];
-#pragma unroll
-                    for (int ax = 0; ax < 3; ax++) X[ax] = ax < dim ? xs[(j * 3 + ax) * 32 + src] : 0.f;
-                    // guard band of this timestep (1% over the bound: FP32 evaluation of it)
-                    const float bnd = fminf(2.f, 2.f * xz[j] * xs[8 * 3 * 32 + src]);
-                    const float mt = (2.f * d.mx_mc1 * bnd + d.mx_mc0) * 1.01f;
-                    bool gr = false;
-                    int* gp = (kGroup && group) ? s_grp + rrow : nullptr;
-                    const int dead = (kEuclid && d.euclid)
-                                         ? test32_at<true, false>(d, t, X, r, mt, inv_cell, cpt, &gr, gp, &nvis)
-                                         : test32_at<false, false>(d, t, X, r, mt, inv_cell, cpt, &gr, gp, &nvis);
+                c0 += width;
+                __syncthreads();
+                const int nq = *qn;
+                // guard band of a test's timestep (1% over the bound: FP32 evaluation of it)
+                auto band = [&](int col, int rrow) {
+                    const float bnd = fminf(2.f, 2.f * s_isz[col] * s_rho[rrow]);
+                    return (2.f * d.mx_mc1 * bnd + d.mx_mc0) * 1.01f;
+                };
+                auto settle = [&](int rrow, bool dead, bool gr) {
                     if (gr) vgray[rrow] = 1;
-                    if (dead) {
-                        vrej[rrow] = 1;
-                        if (!spread) {
-                            tested = k + 1;
-                            break;
-                        }
+                    if (dead) vrej[rrow] = 1;
+                };
+                // The tests in two steps, so that no lane waits through another's chains: the
+                // occupied cells of each window (one set of independent bitmap loads), then
+                // the chain of each cell.
+                auto window = [&](auto dc, auto ec, int e) {
+                    constexpr int D = decltype(dc)::value;
+                    constexpr bool E = decltype(ec)::value;
+                    const float4 q = queue[e];
+                    const int rc = __float_as_int(q.w), rrow = rc & 255, col = rc >> 8, t = s_t[col];
+                    if (vrej[rrow]) return;
+                    const float X[3] = {q.x, q.y, q.z};
+                    int* gp = (kGroup && group) ? s_grp + rrow : nullptr;
+                    Test32<D, E> test(d, t, X, r, band(col, rrow), inv_cell, gp, &nvis);
+                    bool dead = false;
+                    if constexpr (D == 1) {
+                        dead = nbhd_scan<1>(d, t, test.nb, cpt, test);
+                    } else {
+                        auto put = [&](int o0, int o1, int o2) {
+                            const int at = atomicAdd(qc, 1);
+                            if (at < kCells) {
+                                cells[at] = make_uint2((uint32_t)e | (uint32_t)o0 << 16, (uint32_t)o1 | (uint32_t)o2 << 16);
+                                return false;
+                            }
+                            // no room: walk the chain here
+                            if constexpr (D == 3)
+                                return brick_cell_visit(d, t, test.nb, cpt, o0, o1, o2, test);
+                            else
+                                return brick_cell_visit2(d, t, test.nb, cpt, o0, o1, test);
+                        };
+                        if constexpr (D == 3)
+                            dead = nbhd_cells3(d, t, test.nb, put);
+                        else
+                            dead = nbhd_cells2(d, t, test.nb, [&](int o0, int o1) { return put(o0, o1, 0); });
                     }
-                }
-                nev += tested;
-                __syncwarp();
+                    settle(rrow, dead, test.gray);
+                };
+                auto chain = [&](auto dc, auto ec, int i) {
+                    constexpr int D = decltype(dc)::value;
+                    constexpr bool E = decltype(ec)::value;
+                    const uint2 cl = cells[i];
+                    const float4 q = queue[cl.x & 0xffffu];
+                    const int rc = __float_as_int(q.w), rrow = rc & 255, col = rc >> 8, t = s_t[col];
+                    if (vrej[rrow]) return;
+                    const float X[3] = {q.x, q.y, q.z};
+                    int* gp = (kGroup && group) ? s_grp + rrow : nullptr;
+                    Test32<D, E> test(d, t, X, r, band(col, rrow), inv_cell, gp, &nvis);
+                    bool dead = false;
+                    if constexpr (D == 3)
+                        dead = brick_cell_visit(d, t, test.nb, cpt, (int)(cl.x >> 16), (int)(cl.y & 0xffffu),
+                                                (int)(cl.y >> 16), test);
+                    else if constexpr (D == 2)
+                        dead = brick_cell_visit2(d, t, test.nb, cpt, (int)(cl.x >> 16), (int)(cl.y & 0xffffu), test);
+                    settle(rrow, dead, test.gray);
+                };
+                // calls f(dimension, ball) as compile-time constants
+                auto by_model = [&](auto&& f) {
+                    using std::bool_constant;
+                    using std::integral_constant;
+                    const bool ball = kEuclid && d.euclid;
+                    if (dim == 3) {
+                        if (ball)
+                            f(integral_constant<int, 3>{}, bool_constant<kEuclid>{});
+                        else
+                            f(integral_constant<int, 3>{}, bool_constant<false>{});
+                    } else if (dim == 2) {
+                        if (ball)
+                            f(integral_constant<int, 2>{}, bool_constant<kEuclid>{});
+                        else
+                            f(integral_constant<int, 2>{}, bool_constant<false>{});
+                    } else {  // 1 axis: ball == cube
+                        f(integral_constant<int, 1>{}, bool_constant<false>{});
+                    }
+                };
+                by_model([&](auto dc, auto ec) {
+                    for (int e = tid; e < nq; e += kMxThreads) window(dc, ec, e);
+                });
+                __syncthreads();
+                const int ncell = min(*qc, kCells);
+                by_model([&](auto dc, auto ec) {
+                    for (int i = tid; i < ncell; i += kMxThreads) chain(dc, ec, i);
+                });
             }
             tc_fence_before();
             __syncthreads();
@@ -777,6 +995,7 @@ __global__ void __launch_bounds__(kMxThreads, 1) k_prefilter_mixed(const UniDev*
                     if (ng) atomicAdd((unsigned long long*)&ctl[u].gray_total, (unsigned long long)ng);
                 }
             }
+            fence_proxy_async();  // the next tile's operand loads follow this tile's queue in shared memory
             if (tid == 0) {  // this tile's time orders the next round's tiles
                 const uint64_t dt = globaltimer() - tile_t0;
                 atomicMax(&ctl[u].tile_ns, (int)(dt < 0x7fffffffull ? dt : 0x7fffffffull));
@@ -790,12 +1009,10 @@ __global__ void __launch_bounds__(kMxThreads, 1) k_prefilter_mixed(const UniDev*
             ctl[v].state = ST_ERROR;
         }
     }
-    // drain: the last commits of this CTA must land before tensor memory is freed
-    if (tid == 0 && seq > 0) {
-        const int s1 = (seq - 1) & 1;
-        mbar_wait(&bar_m[s1], ph_m[s1]);
-        if (seq > 1) mbar_wait(&bar_m[s1 ^ 1], ph_m[s1 ^ 1]);
-    }
+    // after a timeout: products in flight must land before tensor memory is freed
+#pragma unroll
+    for (int st = 0; st < 2; st++)
+        if (((busy >> st) & 1) && tid == 0) mbar_wait(&bar_m[st], (ph_m >> st) & 1);
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
@@ -850,7 +1067,7 @@ static size_t g_smem = 0;
 static int g_ctas_per_sm = 1;
 
 static size_t smem_bytes() {
-    return (size_t)2 * (2 * kAImgBytes + g_tpad_max * kKC * 2 * 2) + (size_t)kTile * kMxParts * 16 +
+    return (size_t)2 * (2 * kAImgBytes + g_tpad_max * kKC * 2 * 2) + (size_t)3 * kTile * kMxParts * 16 +
            3 * kTile * 4 + 64;
 }
 
