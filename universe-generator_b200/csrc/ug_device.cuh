@@ -117,10 +117,9 @@ struct UniDev {
     int64_t slot_cap;
     // per-round buffers
     uint32_t* surv_bits;   // [B_max / 32]
-    uint32_t* gray_bits;   // [B_max / 32]
     int32_t* g0;           // [B_max]  group mode: single pre-round group touched (-1 none)
     int32_t* surv_off;     // [S_max]  candidate offset within the round
-    int32_t* gray_off;     // [B_max]  mixed: offsets of candidates sent to the FP64 retest
+    int32_t* gray_off;     // [B_max]  FP64 form: offsets of the round's candidates
     Pt64* spos;            // [S_max * T]
     uint64_t* rhead;       // round table [T * rblocks]: epoch<<32 | head survivor rank of
                            // each (timestep, block); entries of other epochs are empty
@@ -172,7 +171,7 @@ struct UniCtl {
     int32_t phase;         // 1 or 2
     int32_t state;         // ST_*
     int32_t epoch;         // round-table epoch
-    int32_t n_gray;        // mixed: candidates sent to the FP64 retest this round
+    int32_t n_gray;        // FP64 form: candidates tested this round
     int32_t accepted_round;
     int64_t gray_total;    // mixed: FP64 retests over the run
     int64_t rounds;

@@ -78,6 +78,7 @@ struct Batch {
     UniCtl* dCtl = nullptr;
     std::vector<UniCtl> hCtl;
     RoundInfo* dInfo = nullptr;
+    RetestQueue rq{};         // mixed form: undecided candidates of a round
     cudaGraphExec_t gexec = nullptr;
     int graph_rounds = 0;
     cudaEvent_t ev[2 * K_NK]{};
@@ -372,8 +373,7 @@ static int setup_universe(Batch& B, UniHost& h, int64_t dense_budget, int64_t* d
     if ((rc = alloc_points(h, cap))) return rc;
     // round buffers
     const int Bm = d.B_max, Sm = d.S_max;
-    if ((rc = dalloc(h, &d.surv_bits, Bm / 32, 0)) || (rc = dalloc(h, &d.gray_bits, Bm / 32, 0)) ||
-        (rc = dalloc(h, &d.gray_off, Bm, 0)) ||
+    if ((rc = dalloc(h, &d.surv_bits, Bm / 32, 0)) || (rc = dalloc(h, &d.gray_off, B.opts.precision == UG_PREC_MIXED ? 1 : Bm, 0)) ||
         (rc = dalloc(h, &d.g0, Bm, 0xff)) || (rc = dalloc(h, &d.surv_off, Sm + 1, 0)) ||
         (rc = dalloc(h, &d.spos, (size_t)Sm * T, 0)) || (rc = dalloc(h, &d.ccount, Sm, 0)) ||
         (rc = dalloc(h, &d.clist, (size_t)Sm * kConflictCap, 0)) ||
@@ -448,19 +448,17 @@ static int launch_round(Batch& B, bool timed) {
     te(K_PLAN);
     if (B.opts.precision == UG_PREC_MIXED && B.any_mixed) {
         tb(K_MIXED);
-        launch_prefilter_mixed(B.dU, B.dCtl, B.dInfo, B.nsm, B.any_group, B.any_euclid, B.st);
+        launch_prefilter_mixed(B.dU, B.dCtl, B.dInfo, B.rq, B.nsm, B.any_group, B.any_euclid, B.st);
         te(K_MIXED);
         tb(K_CONFIRM);
-        k_gray_compact<<<B.n, 256, 0, B.st>>>(B.dU, B.dCtl, B.dInfo, 0);
-        // the retest: few candidates per round, a block of warps per candidate
-        launch_confirm64w(0, B.nsm, B.dU, B.dCtl, B.dInfo, B.st);
+        k_retest<<<B.nsm * 4, 32 * kSurvWarps, kRetestSmem, B.st>>>(B.dU, B.dCtl, B.dInfo, B.rq);
         te(K_CONFIRM);
     } else {
         // the FP64 form: every candidate of the round, one warp per candidate
         // (coefficients in shared memory, lanes over timesteps in endpoint-first order)
         tb(K_PRE);
-        k_gray_compact<<<B.n, 256, 0, B.st>>>(B.dU, B.dCtl, B.dInfo, 1);
-        launch_confirm64w(1, B.nsm, B.dU, B.dCtl, B.dInfo, B.st);
+        k_all_list<<<B.n, 256, 0, B.st>>>(B.dU, B.dCtl, B.dInfo);
+        k_confirm64w<<<B.nsm * 4, 32 * kSurvWarps, kSurvWarps * kConfSmemPerWarp, B.st>>>(B.dU, B.dCtl, B.dInfo);
         te(K_PRE);
     }
     tb(K_COMPACT);
@@ -727,10 +725,20 @@ int ug_batch_create(const ug_universe_cfg* cfgs, int32_t n, const ug_run_opts* o
                              (int)(kSurvWarps * kSurvSmemPerWarp)) != cudaSuccess)
         return bail(fail(UG_ECUDA, "smem attribute failed"));
     if (B->any_mixed && (rc = mixed_init_kernels())) return bail(rc);
-    B->kernels_per_round = B->any_mixed ? 11 : 10;
-    // the warp FP64 test serves both forms (all candidates, or the undecided ones)
-    if (confirm64w_set_smem() != cudaSuccess)
+    B->kernels_per_round = 10;
+    if (cudaFuncSetAttribute(k_confirm64w, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)(kSurvWarps * kConfSmemPerWarp)) != cudaSuccess)
         return bail(fail(UG_ECUDA, "smem attribute failed"));
+    if (B->any_mixed) {
+        // every candidate of a round may be undecided; masks for an eighth of them
+        int64_t cap = 0;
+        for (const UniHost& u : B->U) cap += u.d.B_max;
+        B->rq.cap = (int32_t)std::min<int64_t>(cap, INT32_MAX);
+        B->rq.mask_cap = (int32_t)std::min<int64_t>(cap / 8 + 1, INT32_MAX);
+        if (cudaMalloc(&B->rq.item, sizeof(int2) * (size_t)B->rq.cap) != cudaSuccess ||
+            cudaMalloc(&B->rq.mask, 2 * sizeof(uint4) * (size_t)B->rq.mask_cap) != cudaSuccess)
+            return bail(fail(UG_ENOMEM, "retest queue allocation failed"));
+    }
     // one wave per SM, measured on c3 against 8 / 8 / 16 CTAs per SM: k_surv_gen 27.7 ->
     // 24.5 ms, k_surv_hash 33.5 -> 32.0 ms, k_conflicts 85.5 -> 80.2 ms per job.  k_commit
     // and k_confirm64w keep 8 and 4 per SM (more than resident): one wave measured slower
@@ -1215,6 +1223,8 @@ int ug_batch_destroy(void* h) {
         cudaFree(u.d.acc_idx);
         mixed_free(u.mt);
     }
+    cudaFree(B->rq.item);
+    cudaFree(B->rq.mask);
     cudaFree(B->dU);
     cudaFree(B->dCtl);
     cudaFree(B->d_gather_idx);

@@ -2,11 +2,12 @@
 //
 // One round of every active universe:
 //   k_plan         round sizes, phase transitions, tile decomposition
-//   k_gray_compact + k_confirm64w
+//   k_all_list + k_confirm64w
 //                  FP64 form: every candidate, warp per candidate (shared-memory
-//                  coefficients, lanes over timesteps) against the committed packing;
-//                  mixed form: k_prefilter_mixed (ug_mixed.cu), then the same warp
-//                  test for the candidates its guard band left undecided
+//                  coefficients, lanes over timesteps) against the committed packing
+//   k_prefilter_mixed (ug_mixed.cu) + k_retest
+//                  mixed form: the tensor-core test, then the FP64 test of the
+//                  timesteps that its guard band left undecided
 //   k_compact      survivors in candidate-index order (deterministic)
 //   k_surv_gen     FP64 coefficients of the survivors (term-ordered rows)
 //   k_surv_gemm    their FP64 trajectories as a register-tiled product
@@ -162,6 +163,7 @@ __global__ void k_plan(const UniDev* __restrict__ U, UniCtl* ctl, RoundInfo* inf
         info->total_tiles = acc;
         info->any_active = acc > 0;
         info->total_surv = 0;
+        info->total_gray = 0;
         info->compact_done = 0;
         info->tile_next = 0;
         info->confl_next = 0;
@@ -693,10 +695,10 @@ __global__ void __launch_bounds__(256) k_surv_hash(const UniDev* __restrict__ U,
     }
 }
 
-// Candidates the mixed prefilter could not decide (guard band, or universes
-// outside the tensor-core path), in index order, per universe.
-__global__ void __launch_bounds__(256) k_gray_compact(const UniDev* __restrict__ U, UniCtl* ctl,
-                                                      RoundInfo* info, int all) {
+// The FP64 form's work list: every candidate of the round, per universe, and cleared
+// survivor bits.
+__global__ void __launch_bounds__(256) k_all_list(const UniDev* __restrict__ U, UniCtl* ctl,
+                                                  RoundInfo* info) {
     __shared__ int32_t wsum[8];
     __shared__ int32_t s_running;
     __shared__ bool s_last;
@@ -710,9 +712,8 @@ __global__ void __launch_bounds__(256) k_gray_compact(const UniDev* __restrict__
     __syncthreads();
     for (int base = 0; base < nwords; base += 256) {
         const int w = base + tid;
-        // all: the FP64 form, every candidate of the round goes to the warp test
-        uint32_t bits = w < nwords ? (all ? 0xffffffffu : d.gray_bits[w]) : 0u;
-        if (all && w < nwords) d.surv_bits[UG_IDX(w, d.B_max / 32)] = 0u;
+        uint32_t bits = w < nwords ? 0xffffffffu : 0u;
+        if (w < nwords) d.surv_bits[UG_IDX(w, d.B_max / 32)] = 0u;
         if (w == nwords - 1 && (B & 31)) bits &= (1u << (B & 31)) - 1u;
         const int cnt = __popc(bits);
         int incl = cnt;
@@ -744,7 +745,7 @@ __global__ void __launch_bounds__(256) k_gray_compact(const UniDev* __restrict__
         s_last = atomicAdd(&info->gray_done, 1) == info->n_uni - 1;
     }
     __syncthreads();
-    if (s_last) {  // the last block: offsets of every universe's undecided candidates
+    if (s_last) {  // the last block: offsets of every universe's candidates
         __threadfence();
         const int n = info->n_uni;
         int acc = 0;
@@ -764,122 +765,104 @@ __global__ void __launch_bounds__(256) k_gray_compact(const UniDev* __restrict__
     }
 }
 
-// FP64 test of one candidate per group of WPI warps: FP64 regeneration and the
-// exact test against the committed packing, timesteps (1+1D: paths) spread
-// over the group's lanes.  WPI = 1 serves the FP64 form (every candidate of the
-// round: many items, throughput); WPI = kSurvWarps the guard-band retest of the
-// mixed form (few items per round, each of which would otherwise bound the
-// launch by one warp's latency): the axes are generated by separate warps and
-// four times the lanes share the timesteps.
-template <int WPI>
-__device__ __forceinline__ void group_sync() {
-    if (WPI == 1)
-        __syncwarp();
-    else
-        __syncthreads();
+// 1+1D crossing rule in FP64: trajectory P[0..T) against the accepted paths `first`,
+// first + step, ...; stops on *stop (another thread found a contact) outside group rounds.
+// True on rejection; group rounds keep the single touched group in *g.
+__device__ __forceinline__ bool cross64(const UniDev& d, const double* P, int64_t n_slots, int first, int step,
+                                        bool group, int32_t* g, volatile int32_t* stop) {
+    const int T = d.T;
+    for (int64_t s = first; s < n_slots; s += step) {
+        if (!group && *stop) return false;
+        const Pt64* q = d.pts + UG_IDX(s * T + T - 1, d.slot_cap * T) + 1 - T;
+        double d0 = torus_delta(P[0] - __ldcg(&q[0].c[0]));
+        bool hit = hit1(d0, d.cell, d.inclusive);
+        // the path's points 4 timesteps at a time (4 independent loads in flight)
+        for (int t0 = 1; t0 < T && !hit; t0 += 4) {
+            double qv[4];
+#pragma unroll
+            for (int k = 0; k < 4; k++) qv[k] = t0 + k < T ? __ldcg(&q[t0 + k].c[0]) : 0.0;
+#pragma unroll
+            for (int k = 0; k < 4; k++) {
+                if (hit || t0 + k >= T) break;
+                const double d1 = torus_delta(P[t0 + k] - qv[k]);
+                hit = hit1(d1, d.cell, d.inclusive) || crosses_step(d0, d1);
+                d0 = d1;
+            }
+        }
+        if (!hit) continue;
+        if (!group) return true;
+        const int32_t gq = __ldcg(&q[0].gid);
+        if (*g == -1)
+            *g = gq;
+        else if (*g != gq)
+            return true;
+    }
+    return false;
 }
 
-// (a register cap instead of launch bounds: with launch bounds alone ptxas keeps
-// the WPI = 1 form at 64 registers and spills)
-template <int WPI>
-__global__ void __maxnreg__(128) k_confirm64w(const UniDev* __restrict__ U,
-                                                                  UniCtl* ctl, RoundInfo* info, int all) {
-    static_assert(WPI == 1 || WPI == kSurvWarps, "a group is one warp or the whole block");
+__device__ __forceinline__ void eval64_at(const UniDev& d, const double* alpha, const double* beta, const double* a2,
+                                          int t, double* P) {
+    if (d.dim == 3)
+        eval64x<3>(d, alpha, beta, a2, t, P);
+    else if (d.dim == 2)
+        eval64x<2>(d, alpha, beta, a2, t, P);
+    else
+        eval64x<1>(d, alpha, beta, a2, t, P);
+}
+
+// The FP64 form's test, one warp per candidate: FP64 regeneration and the exact test
+// against the committed packing, timesteps (1+1D: paths) spread over the lanes.
+// (a register cap instead of launch bounds: with launch bounds alone ptxas keeps 64
+// registers and spills)
+__global__ void __maxnreg__(128) k_confirm64w(const UniDev* __restrict__ U, UniCtl* ctl, RoundInfo* info) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    constexpr int kG = kSurvWarps / WPI;  // groups per block
-    constexpr int kGT = 32 * WPI;         // threads per group
-    __shared__ int32_t s_hit[kG];
-    __shared__ int32_t s_first[kSurvWarps], s_rej[kSurvWarps];
+    __shared__ int32_t s_hit[kSurvWarps];
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-    const int grp = wib / WPI, wig = wib % WPI, gt = wig * 32 + lane;
-    unsigned char* my = smem_raw + (size_t)grp * kConfSmemPerWarp;
+    unsigned char* my = smem_raw + (size_t)wib * kConfSmemPerWarp;
     double* alpha = (double*)my;
     double* beta = alpha + 3 * (kMaxF + 1);
     double* a2 = beta + 3 * (kMaxF + 1);
     double* wj = a2 + 3;
     int32_t* bj = (int32_t*)(wj + kMaxF);
     double* P1 = (double*)(my + kSurvSmemPerWarpBase);
-    volatile int32_t* vhit = &s_hit[grp];
+    volatile int32_t* vhit = &s_hit[wib];
     const int n_uni = info->n_uni, total = info->total_gray;
-    const int ggrp = blockIdx.x * kG + grp, ngrp = gridDim.x * kG;
-    for (int item = ggrp; item < total; item += ngrp) {
+    const int gwarp = blockIdx.x * kSurvWarps + wib, nwarp = gridDim.x * kSurvWarps;
+    for (int item = gwarp; item < total; item += nwarp) {
         const int u = find_uni(info->gray_pref, n_uni, item);
         const UniDev& d = U[u];
         UniCtl& c = ctl[u];
         const int off = d.gray_off[UG_IDX(item - info->gray_pref[u], d.B_max)];
         const uint64_t idx = (uint64_t)(c.round_base + off);
         const int T = d.T;
-        if (d.rng == RNG_KNOT || WPI == 1) {
-            if (wig == 0) warp_gen64(d, idx, alpha, beta, a2, bj, wj, lane);
-        } else if (wig < d.dim) {
-            warp_gen64_axis(d, idx, wig, alpha, beta, a2, lane);
-        }
-        if (gt == 0) *vhit = 0;
-        group_sync<WPI>();
+        warp_gen64(d, idx, alpha, beta, a2, bj, wj, lane);
+        if (lane == 0) *vhit = 0;
+        __syncwarp();
         const bool group = group_phase(d, c);
         int32_t g = -1;
         bool hitl = false;
         int nev = 0, nvis = 0;
         if (d.dim == 1 && d.cross1d) {
-            for (int t = gt; t < T; t += kGT) P1[t] = eval64(d, alpha, beta, 1, a2[0], t);
-            group_sync<WPI>();
-            nev = gt == 0 ? T : 0;
-            for (int64_t s = gt; s < c.n_slots && !(hitl && !group); s += kGT) {
-                if (!group && *vhit) break;  // another lane of the group found a contact
-                const Pt64* q = d.pts + UG_IDX(s * T + T - 1, d.slot_cap * T) + 1 - T;
-                double d0 = torus_delta(P1[0] - __ldcg(&q[0].c[0]));
-                bool hit = hit1(d0, d.cell, d.inclusive);
-                // the path's points 4 timesteps at a time (4 independent loads in flight)
-                for (int t0 = 1; t0 < T && !hit; t0 += 4) {
-                    double qv[4];
-#pragma unroll
-                    for (int k = 0; k < 4; k++) qv[k] = t0 + k < T ? __ldcg(&q[t0 + k].c[0]) : 0.0;
-#pragma unroll
-                    for (int k = 0; k < 4; k++) {
-                        if (hit || t0 + k >= T) break;
-                        const double d1 = torus_delta(P1[t0 + k] - qv[k]);
-                        hit = hit1(d1, d.cell, d.inclusive) || crosses_step(d0, d1);
-                        d0 = d1;
-                    }
-                }
-                if (hit) {
-                    if (!group) {
-                        hitl = true;
-                        *vhit = 1;
-                    } else {
-                        const int32_t gq = __ldcg(&q[0].gid);
-                        if (g == -1)
-                            g = gq;
-                        else if (g != gq)
-                            hitl = true;
-                    }
-                }
-            }
+            for (int t = lane; t < T; t += 32) P1[t] = eval64(d, alpha, beta, 1, a2[0], t);
+            __syncwarp();
+            nev = lane == 0 ? T : 0;
+            hitl = cross64(d, P1, c.n_slots, lane, 32, group, &g, vhit);
+            if (hitl) *vhit = 1;
         } else {
             const int64_t cpt = cells_per_t(d);
-            for (int oi0 = 0; oi0 < T; oi0 += kGT) {
-                const int oi = oi0 + gt;
-                if (oi < T && !hitl) {
+            for (int oi0 = 0; oi0 < T; oi0 += 32) {
+                const int oi = oi0 + lane;
+                if (oi < T) {
                     const int t = __ldg(d.order + oi);
                     double P[3];
-                    if (d.dim == 3)
-                        eval64x<3>(d, alpha, beta, a2, t, P);
-                    else if (d.dim == 2)
-                        eval64x<2>(d, alpha, beta, a2, t, P);
-                    else
-                        eval64x<1>(d, alpha, beta, a2, t, P);
+                    eval64_at(d, alpha, beta, a2, t, P);
                     nev++;
-                    hitl = contacts64(d, t, P, group, &g, cpt, all ? &nvis : nullptr);
+                    hitl = contacts64(d, t, P, group, &g, cpt, &nvis);
                 }
-                if (__any_sync(0xffffffffu, hitl)) {
-                    if (lane == 0) *vhit = 1;
-                    break;
-                }
-                if (WPI > 1 && *vhit) break;
+                if (__any_sync(0xffffffffu, hitl)) break;
             }
         }
-        // merge the lanes of each warp, then the warps of the group: any rejection,
-        // or (group rounds) two distinct groups touched
+        // merge the lanes: any rejection, or (group rounds) two distinct groups touched
         bool rej = __any_sync(0xffffffffu, hitl);
         int32_t first = -1;
         for (int o = 0; o < 32; o++) {
@@ -891,45 +874,216 @@ __global__ void __maxnreg__(128) k_confirm64w(const UniDev* __restrict__ U,
         for (int o = 16; o > 0; o >>= 1) nvis += __shfl_xor_sync(0xffffffffu, nvis, o);
         if (lane == 0) {
             if (nev) atomicAdd((unsigned long long*)&c.evals_fp64, (unsigned long long)nev);
-            if (all && nev) atomicAdd((unsigned long long*)&c.evals, (unsigned long long)nev);
+            if (nev) atomicAdd((unsigned long long*)&c.evals, (unsigned long long)nev);
             if (nvis) atomicAdd((unsigned long long*)&c.visits, (unsigned long long)nvis);
-        }
-        if (WPI > 1) {
-            if (lane == 0) {
-                s_first[wib] = first;
-                s_rej[wib] = rej ? 1 : 0;
-            }
-            __syncthreads();
-            first = -1;
-            rej = false;
-            for (int w = 0; w < WPI; w++) {
-                const int32_t v = s_first[grp * WPI + w];
-                rej = rej || s_rej[grp * WPI + w] != 0 || (v != -1 && first != -1 && v != first);
-                if (first == -1) first = v;
-            }
-        }
-        if (gt == 0) {
             if (!rej) atomicOr(&d.surv_bits[UG_IDX(off >> 5, d.B_max / 32)], 1u << (off & 31));
             if (d.group_mode != GROUP_NONE) d.g0[UG_IDX(off, d.B_max)] = first;
         }
-        group_sync<WPI>();
+        __syncwarp();
     }
 }
 
-cudaError_t confirm64w_set_smem() {
-    cudaError_t e = cudaFuncSetAttribute(k_confirm64w<1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)(kSurvWarps * kConfSmemPerWarp));
-    if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(k_confirm64w<kSurvWarps>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)kConfSmemPerWarp);
-    return e;
+// FP64 tensor product D += A B, 8 x 8 x 4: lane (g, t) = (lane / 4, lane % 4) holds A(g, t),
+// B(t, g) and D(g, 2t), D(g, 2t + 1).  Each element accumulates its four products in
+// ascending order, one rounding each: the same bits as a chain of fused multiply-adds.
+__device__ __forceinline__ void dmma_8x8x4(double* d, double a, double b) {
+    asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};"
+                 : "+d"(d[0]), "+d"(d[1])
+                 : "d"(a), "d"(b));
 }
 
-void launch_confirm64w(int all, int nsm, const UniDev* U, UniCtl* ctl, RoundInfo* info, cudaStream_t st) {
-    if (all)
-        k_confirm64w<1><<<nsm * 4, 32 * kSurvWarps, kSurvWarps * kConfSmemPerWarp, st>>>(U, ctl, info, 1);
-    else
-        k_confirm64w<kSurvWarps><<<nsm * 4, 32 * kSurvWarps, kConfSmemPerWarp, st>>>(U, ctl, info, 0);
+// warp_gen64_axis of all axes by a whole block, as term-ordered rows (row pitch kRowK):
+// blocks, logarithms and sines spread over the threads, the normalisation
+// summed in ascending b by one lane per axis.
+__device__ __forceinline__ void block_gen64(const UniDev& d, uint64_t idx, double* rows, double* phase, double* a2,
+                                            double* sums) {
+    const int F = d.F, np = (F >> 1) + 1;
+    for (int e = threadIdx.x; e < d.dim * np; e += blockDim.x) {
+        const int ax = e / np, p = e - ax * np;
+        double* row = rows + ax * kRowK;
+        const uint4 o = philox_block(d.seed, idx, ax, p);
+        if (p == 0) {
+            a2[ax] = d.pin ? 0.0 : (double)o.x * (1.0 / 2147483648.0) - 1.0;
+            continue;
+        }
+        const int be = 2 * p, bo = 2 * p + 1;
+        const double Ee = -log(((double)o.x + 0.5) * (1.0 / 4294967296.0));
+        row[kseq_s(be)] = (o.z & 1u) ? -Ee : Ee;
+        phase[ax * kMaxF + be - 1] = (double)(o.z >> 1) * (1.0 / 2147483648.0) * kPi;
+        if (bo <= F) {
+            const double Eo = -log(((double)o.y + 0.5) * (1.0 / 4294967296.0));
+            row[kseq_s(bo)] = (o.w & 1u) ? -Eo : Eo;
+        }
+    }
+    __syncthreads();
+    if ((threadIdx.x & 31) == 0 && (int)(threadIdx.x >> 5) < d.dim) {
+        const double* row = rows + (threadIdx.x >> 5) * kRowK;
+        double sum = 0.0;
+#pragma unroll 4
+        for (int b = 2; b <= F; b++) sum += fabs(row[kseq_s(b)]);
+        sums[threadIdx.x >> 5] = sum;
+    }
+    __syncthreads();
+    for (int e = threadIdx.x; e < d.dim * (F - 1); e += blockDim.x) {
+        const int ax = e / (F - 1), b = e - ax * (F - 1) + 2;
+        double* row = rows + ax * kRowK + kseq_s(b);
+        const double v = row[0];
+        double amp = fabs(v) / sums[ax] / (double)b;
+        if (v < 0.0) amp = -amp;
+        if (b & 1) {
+            row[0] = amp;
+        } else {
+            double sf, cf;
+            sincos(phase[ax * kMaxF + b - 1], &sf, &cf);
+            row[0] = amp * cf;
+            row[1] = amp * sf;
+        }
+    }
+    __syncthreads();
+}
+
+// The mixed form's retest, one block of four warps per undecided candidate (few per round:
+// one candidate's latency bounds the launch).  Only the timesteps of its mask are
+// evaluated, 32 at a time, eight per warp as FP64 tensor products (the axes are rows), with
+// eval64's bits.  Candidates without a mask (no tensor-core test, the crossing rule, or
+// beyond the masks' room) are tested at all timesteps.  Per round, against a lane per
+// timestep of all T: 2+1 unique groups T = 256 (380 candidates, ~60 timesteps each)
+// 167 -> 108 us, 3+1 T = 128 (310) 50 -> 23 us.
+__global__ void __maxnreg__(128) k_retest(const UniDev* __restrict__ U, UniCtl* ctl, RoundInfo* info,
+                                          RetestQueue rq) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    __shared__ int32_t s_hit, s_g, s_nt;
+    __shared__ int32_t s_t[kMaxF];
+    __shared__ double s_P[32][3], s_sum[3], s_traj[kMaxF];
+    double* alpha = (double*)smem_raw;
+    double* beta = alpha + 3 * (kMaxF + 1);
+    double* a2 = beta + 3 * (kMaxF + 1);
+    double* wj = a2 + 3;
+    int32_t* bj = (int32_t*)(wj + kMaxF);
+    double* rows = (double*)(smem_raw + kSurvSmemPerWarpBase);
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int gl = lane >> 2, tl = lane & 3;
+    volatile int32_t* vhit = &s_hit;
+    const int total = min(info->total_gray, rq.cap);
+    for (int item = blockIdx.x; item < total; item += gridDim.x) {
+        const int2 it = rq.item[item];
+        const UniDev& d = U[it.x];
+        UniCtl& c = ctl[it.x];
+        const int off = it.y, T = d.T, F = d.F, K = d.K, dim = d.dim;
+        const uint64_t idx = (uint64_t)(c.round_base + off);
+        const bool group = group_phase(d, c), cross = dim == 1 && d.cross1d;
+        const bool masked = d.mx_ok && !cross && item < rq.mask_cap;
+        if (d.rng == RNG_KNOT) {
+            if (warp == 0) warp_gen64(d, idx, alpha, beta, a2, bj, wj, lane);
+            __syncthreads();
+            for (int e = tid; e < 3 * kRowK; e += blockDim.x) rows[e] = 0.0;
+            __syncthreads();
+            for (int e = tid; e < dim * (F - 1); e += blockDim.x) {
+                const int ax = e / (F - 1), b = e - ax * (F - 1) + 2;
+                double* row = rows + ax * kRowK + kseq_s(b);
+                row[0] = alpha[ax * (F + 1) + b];
+                if (!(b & 1)) row[1] = beta[ax * (F + 1) + b];
+            }
+        } else {
+            block_gen64(d, idx, rows, beta, a2, s_sum);
+        }
+        if (tid == 0) {
+            s_hit = 0;
+            // masked: the group that the decided timesteps touched
+            s_g = masked && group ? d.g0[UG_IDX(off, d.B_max)] : -1;
+        }
+        // the timesteps to evaluate
+        if (masked) {
+            if (warp == 0) {
+                const uint32_t* m = reinterpret_cast<const uint32_t*>(rq.mask + 2 * (int64_t)item);
+                uint32_t w = lane < kMaskWords ? m[lane] : 0u;
+                int incl = __popc(w);
+                const int mine = incl;
+                for (int o = 1; o < kMaskWords; o <<= 1) {
+                    const int v = __shfl_up_sync(0xffffffffu, incl, o);
+                    if (lane >= o) incl += v;
+                }
+                for (int at = incl - mine; w; w &= w - 1) s_t[at++] = lane * 32 + __ffs(w) - 1;
+                if (lane == kMaskWords - 1) s_nt = incl;
+            }
+        } else {
+            for (int t = tid; t < T; t += blockDim.x) s_t[t] = cross ? t : __ldg(d.order + t);
+            if (tid == 0) s_nt = T;
+        }
+        __syncthreads();
+        const int nt = s_nt;
+        const int64_t cpt = cells_per_t(d);
+        int32_t g = s_g;
+        bool hitl = false;
+        int nev = 0;
+        for (int t0 = 0; t0 < nt; t0 += 32) {
+            const int n = min(32, nt - t0);
+            if (8 * warp < n) {
+                const int q = 8 * warp + gl;  // this lane's timestep as a column of B
+                const double* B = d.KT + s_t[t0 + min(q, n - 1)];
+                const double* A = rows + (gl < dim ? gl * kRowK : 0);
+                double acc[2] = {0.0, 0.0};
+                double bv[2][8];  // two batches of eight steps' basis values
+                auto fetch = [&](int k0, double* v) {
+#pragma unroll
+                    for (int j = 0; j < 8; j++) {
+                        const int k = k0 + 4 * j + tl;
+                        v[j] = k < K ? __ldg(B + (int64_t)k * d.Tpad) : 0.0;
+                    }
+                };
+                fetch(0, bv[0]);
+                for (int k0 = 0; k0 < K; k0 += 64) {
+#pragma unroll
+                    for (int h = 0; h < 2; h++) {
+                        fetch(k0 + 32 * (h + 1), bv[h ^ 1]);
+#pragma unroll
+                        for (int j = 0; j < 8; j++) {
+                            const int k = k0 + 32 * h + 4 * j + tl;
+                            dmma_8x8x4(acc, gl < dim && k < K ? A[k] : 0.0, bv[h][j]);
+                        }
+                    }
+                }
+                if (gl < dim)
+#pragma unroll
+                    for (int j = 0; j < 2; j++) {
+                        const int col = 8 * warp + 2 * tl + j;
+                        if (col < n) s_P[col][gl] = torus_wrap(fma(acc[j], __ldg(d.invsinz + s_t[t0 + col]), a2[gl]));
+                    }
+            }
+            __syncthreads();
+            nev += n;
+            // a timestep's contacts on a lane of its own, spread over the warps
+            const int e = (lane >> 2) * 4 + warp;
+            if (cross) {
+                if (tid < n) s_traj[t0 + tid] = s_P[tid][0];
+            } else if ((lane & 3) == 0 && e < n) {
+                double P[3];
+                for (int ax = 0; ax < 3; ax++) P[ax] = ax < dim ? s_P[e][ax] : 0.0;
+                if (contacts64(d, s_t[t0 + e], P, group, &g, cpt, nullptr)) {
+                    hitl = true;
+                    *vhit = 1;
+                }
+            }
+            __syncthreads();
+            if (*vhit) break;
+        }
+        if (cross) {
+            hitl = cross64(d, s_traj, c.n_slots, tid, blockDim.x, group, &g, vhit);
+            if (hitl) *vhit = 1;
+        }
+        // any rejection, or (group rounds) two distinct groups touched
+        if (group && g != -1) {
+            const int32_t old = atomicCAS(&s_g, -1, g);
+            if (old != -1 && old != g) hitl = true;
+        }
+        const bool rej = __syncthreads_or(hitl);
+        if (tid == 0) {
+            if (nev) atomicAdd((unsigned long long*)&c.evals_fp64, (unsigned long long)nev);
+            if (!rej) atomicOr(&d.surv_bits[UG_IDX(off >> 5, d.B_max / 32)], 1u << (off & 31));
+            if (d.group_mode != GROUP_NONE) d.g0[UG_IDX(off, d.B_max)] = s_g;
+        }
+        __syncthreads();
+    }
 }
 
 // One warp per survivor r: the set of earlier survivors r' < r that it

@@ -38,6 +38,8 @@ struct RoundInfo {
 __host__ __device__ __forceinline__ int kseq_s(int b) { return (b - 2) + ((b - 1) >> 1); }
 __host__ __device__ __forceinline__ int kseq_len(int F) { return kseq_s(F) + 1 + ((F & 1) ? 0 : 1); }
 
+constexpr int kseq_len_max() { return kMaxF - 2 + (kMaxF - 1) / 2 + 2; }  // kMaxF is even
+
 __device__ __forceinline__ int find_uni(const int32_t* off, int n, int item) {
     int lo = 0, hi = n - 1;
     while (lo < hi) {
@@ -50,14 +52,24 @@ __device__ __forceinline__ int find_uni(const int32_t* off, int n, int item) {
     return lo;
 }
 
+// Candidates that the mixed prefilter leaves to the FP64 retest this round, in no order:
+// (universe, offset in the round), RoundInfo::total_gray of them.  The first mask_cap
+// carry a bit per timestep where a pair lies in the guard band: every pair of the other
+// timesteps is decided, so the retest evaluates those timesteps alone.
+struct RetestQueue {
+    int2* item;      // [sum of B_max]
+    uint4* mask;     // [mask_cap][2]
+    int32_t mask_cap;
+    int32_t cap;
+};
+constexpr int kMaskWords = kMaxF / 32;
+static_assert(kMaskWords == 8, "a mask is two uint4");
+
 // Kernels (ug_kernels.cu)
 __global__ void k_plan(const UniDev* __restrict__ U, UniCtl* ctl, RoundInfo* info);
-__global__ void k_gray_compact(const UniDev* __restrict__ U, UniCtl* ctl, RoundInfo* info, int all);
-// The FP64 test of undecided candidates (k_confirm64w, a template kept inside
-// ug_kernels.cu): every candidate of the round (all = 1, a warp per candidate) or
-// the mixed form's retest (all = 0, a block per candidate).
-cudaError_t confirm64w_set_smem();
-void launch_confirm64w(int all, int nsm, const UniDev* U, UniCtl* ctl, RoundInfo* info, cudaStream_t st);
+__global__ void k_all_list(const UniDev* __restrict__ U, UniCtl* ctl, RoundInfo* info);
+__global__ void k_confirm64w(const UniDev* __restrict__ U, UniCtl* ctl, RoundInfo* info);
+__global__ void k_retest(const UniDev* __restrict__ U, UniCtl* ctl, RoundInfo* info, RetestQueue rq);
 __global__ void k_compact(const UniDev* __restrict__ U, UniCtl* ctl, RoundInfo* info);
 __global__ void k_surv_gen(const UniDev* __restrict__ U, UniCtl* ctl, RoundInfo* info, int warp_bytes);
 __global__ void k_surv_gemm(const UniDev* __restrict__ U, UniCtl* ctl, RoundInfo* info);
@@ -85,5 +97,8 @@ constexpr size_t kSurvSmemPerWarp = kSurvSmemPerWarpBase;
 constexpr size_t kSurvSmemAxis = (size_t)2 * (kMaxF + 1) * sizeof(double);
 // k_confirm64w adds the FP64 trajectory of a 1+1D candidate
 constexpr size_t kConfSmemPerWarp = kSurvSmemPerWarpBase + (size_t)kMaxF * sizeof(double);
+// k_retest adds the candidate's term-ordered coefficient rows
+constexpr int kRowK = kseq_len_max();
+constexpr size_t kRetestSmem = kSurvSmemPerWarpBase + (size_t)3 * kRowK * sizeof(double);
 
 }  // namespace ug

@@ -13,7 +13,7 @@
 // epilogue reads D with tcgen05.ld and runs the Chebyshev test against the
 // FP32 copy of the collision grid with a guard band: a contact deeper than
 // the band rejects, a separation wider than the band clears, anything in
-// between marks the candidate for the FP64 retest (k_confirm64), so every
+// between marks the timestep for the FP64 retest (k_retest), so every
 // decision equals the FP64 one.
 //
 // Pipeline per CTA (128 threads, one candidate per thread, persistent over
@@ -365,7 +365,7 @@ static_assert(kQueue * 16 + kDense * 3 * 17 * 4 <= 2 * (2 * kAImgBytes + 16 * kK
 // kEuclid: the batch holds universes with the L2-ball exclusion.
 template <bool kGroup, bool kEuclid>
 __global__ void __launch_bounds__(kMxThreads, 1) k_prefilter_mixed(const UniDev* __restrict__ U, UniCtl* ctl,
-                                                                    RoundInfo* info, MixedLaunch L) {
+                                                                   RoundInfo* info, RetestQueue rq, MixedLaunch L) {
     extern __shared__ __align__(1024) uint8_t sm[];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     // thread (row, part): warps w and w+4k share the tensor-memory lane quarter w%4
@@ -395,6 +395,8 @@ __global__ void __launch_bounds__(kMxThreads, 1) k_prefilter_mixed(const UniDev*
     __shared__ uint32_t s_live[4];
     __shared__ int32_t s_row[kDense];
     __shared__ float s_aff[kDense][6];
+    // per row, a bit per timestep with a pair in the guard band
+    __shared__ uint32_t s_gm[kTile][kMaskWords];
     // tile offsets of the universes, for the per-tile lookup of its universe
     __shared__ int32_t s_toff[kMaxUni + 1];
     if (L.dump == nullptr)
@@ -454,12 +456,15 @@ __global__ void __launch_bounds__(kMxThreads, 1) k_prefilter_mixed(const UniDev*
         const bool valid = off < B;
         const uint64_t idx = (uint64_t)(base + off);
         if (!d.mx_ok) {  // not eligible for the tensor-core path: everything to the FP64 test
-            if (part == 0) {
+            if (part == 0 && !dump) {
                 const uint32_t g = __ballot_sync(0xffffffffu, valid);
-                if (lane == 0 && !dump) {
+                int at = 0;
+                if (lane == 0) {
                     d.surv_bits[UG_IDX(off >> 5, d.B_max / 32)] = 0u;
-                    d.gray_bits[UG_IDX(off >> 5, d.B_max / 32)] = g;
+                    at = atomicAdd(&info->total_gray, __popc(g));
                 }
+                at = __shfl_sync(0xffffffffu, at, 0) + __popc(g & ((1u << lane) - 1u));
+                if (valid) rq.item[UG_IDX(at, rq.cap)] = make_int2(u, off);
             }
             continue;
         }
@@ -480,6 +485,7 @@ __global__ void __launch_bounds__(kMxThreads, 1) k_prefilter_mixed(const UniDev*
             s_gray[row] = 0;
             s_grp[row] = -1;
         }
+        for (int j = tid; j < kTile * kMaskWords; j += kMxThreads) (&s_gm[0][0])[j] = 0u;
         for (int j = tid; j < T; j += kMxThreads) {
             const int t = __ldg(d.order + j);
             s_t[j] = t;
@@ -888,8 +894,11 @@ __global__ void __launch_bounds__(kMxThreads, 1) k_prefilter_mixed(const UniDev*
                     const float bnd = fminf(2.f, 2.f * s_isz[col] * s_rho[rrow]);
                     return (2.f * d.mx_mc1 * bnd + d.mx_mc0) * 1.01f;
                 };
-                auto settle = [&](int rrow, bool dead, bool gr) {
-                    if (gr) vgray[rrow] = 1;
+                auto settle = [&](int rrow, int t, bool dead, bool gr) {
+                    if (gr) {
+                        vgray[rrow] = 1;
+                        atomicOr(&s_gm[rrow][t >> 5], 1u << (t & 31));
+                    }
                     if (dead) vrej[rrow] = 1;
                 };
                 // The tests in two steps, so that no lane waits through another's chains: the
@@ -925,7 +934,7 @@ __global__ void __launch_bounds__(kMxThreads, 1) k_prefilter_mixed(const UniDev*
                         else
                             dead = nbhd_cells2(d, t, test.nb, [&](int o0, int o1) { return put(o0, o1, 0); });
                     }
-                    settle(rrow, dead, test.gray);
+                    settle(rrow, t, dead, test.gray);
                 };
                 auto chain = [&](auto dc, auto ec, int i) {
                     constexpr int D = decltype(dc)::value;
@@ -943,7 +952,7 @@ __global__ void __launch_bounds__(kMxThreads, 1) k_prefilter_mixed(const UniDev*
                                                 (int)(cl.y >> 16), test);
                     else if constexpr (D == 2)
                         dead = brick_cell_visit2(d, t, test.nb, cpt, (int)(cl.x >> 16), (int)(cl.y & 0xffffu), test);
-                    settle(rrow, dead, test.gray);
+                    settle(rrow, t, dead, test.gray);
                 };
                 // calls f(dimension, ball) as compile-time constants
                 auto by_model = [&](auto&& f) {
@@ -987,12 +996,24 @@ __global__ void __launch_bounds__(kMxThreads, 1) k_prefilter_mixed(const UniDev*
                 const bool gr = valid && !rej && (gry || timeout);
                 const uint32_t sb = __ballot_sync(0xffffffffu, surv);
                 const uint32_t gb = __ballot_sync(0xffffffffu, gr);
-                if (kGroup && surv && d.group_mode != GROUP_NONE) d.g0[UG_IDX(off, d.B_max)] = s_grp[row];
+                if (kGroup && (surv || gr) && d.group_mode != GROUP_NONE) d.g0[UG_IDX(off, d.B_max)] = s_grp[row];
+                const int ng = __popc(gb);
+                int at = 0;
                 if (lane == 0) {
                     d.surv_bits[UG_IDX(off >> 5, d.B_max / 32)] = sb;
-                    d.gray_bits[UG_IDX(off >> 5, d.B_max / 32)] = gb;
-                    const int ng = __popc(gb);
-                    if (ng) atomicAdd((unsigned long long*)&ctl[u].gray_total, (unsigned long long)ng);
+                    if (ng) {
+                        atomicAdd((unsigned long long*)&ctl[u].gray_total, (unsigned long long)ng);
+                        at = atomicAdd(&info->total_gray, ng);
+                    }
+                }
+                at = __shfl_sync(0xffffffffu, at, 0) + __popc(gb & ((1u << lane) - 1u));
+                if (gr) {
+                    rq.item[UG_IDX(at, rq.cap)] = make_int2(u, off);
+                    if (at < rq.mask_cap) {
+                        const uint32_t* m = s_gm[row];
+                        rq.mask[2 * (int64_t)at] = make_uint4(m[0], m[1], m[2], m[3]);
+                        rq.mask[2 * (int64_t)at + 1] = make_uint4(m[4], m[5], m[6], m[7]);
+                    }
                 }
             }
             fence_proxy_async();  // the next tile's operand loads follow this tile's queue in shared memory
@@ -1224,18 +1245,18 @@ int mixed_init_kernels() {
     return UG_OK;
 }
 
-void launch_prefilter_mixed(const UniDev* dU, UniCtl* dCtl, RoundInfo* dInfo, int nsm, bool any_group,
-                            bool any_euclid, cudaStream_t st) {
+void launch_prefilter_mixed(const UniDev* dU, UniCtl* dCtl, RoundInfo* dInfo, const RetestQueue& rq, int nsm,
+                            bool any_group, bool any_euclid, cudaStream_t st) {
     MixedLaunch L{(uint32_t)g_ncols, g_tpad_max, nullptr, nullptr, 0, 0, 0};
     const int g = nsm * g_ctas_per_sm;
     if (any_group && any_euclid)
-        k_prefilter_mixed<true, true><<<g, kMxThreads, g_smem, st>>>(dU, dCtl, dInfo, L);
+        k_prefilter_mixed<true, true><<<g, kMxThreads, g_smem, st>>>(dU, dCtl, dInfo, rq, L);
     else if (any_group)
-        k_prefilter_mixed<true, false><<<g, kMxThreads, g_smem, st>>>(dU, dCtl, dInfo, L);
+        k_prefilter_mixed<true, false><<<g, kMxThreads, g_smem, st>>>(dU, dCtl, dInfo, rq, L);
     else if (any_euclid)
-        k_prefilter_mixed<false, true><<<g, kMxThreads, g_smem, st>>>(dU, dCtl, dInfo, L);
+        k_prefilter_mixed<false, true><<<g, kMxThreads, g_smem, st>>>(dU, dCtl, dInfo, rq, L);
     else
-        k_prefilter_mixed<false, false><<<g, kMxThreads, g_smem, st>>>(dU, dCtl, dInfo, L);
+        k_prefilter_mixed<false, false><<<g, kMxThreads, g_smem, st>>>(dU, dCtl, dInfo, rq, L);
 }
 
 int mixed_error(const UniDev* dU, int u, const UniDev& d, const MixedTables& mt, int64_t first, int64_t count,
@@ -1256,7 +1277,7 @@ int mixed_error(const UniDev* dU, int u, const UniDev& d, const MixedTables& mt,
     MixedLaunch L{(uint32_t)g_ncols, g_tpad_max, d32, dm, u, first, count};
     int nsm = 148;
     cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, 0);
-    k_prefilter_mixed<false, false><<<nsm * g_ctas_per_sm, kMxThreads, g_smem, st>>>(dU, nullptr, nullptr, L);
+    k_prefilter_mixed<false, false><<<nsm * g_ctas_per_sm, kMxThreads, g_smem, st>>>(dU, nullptr, nullptr, RetestQueue{}, L);
     k_pos64<<<(int)std::min<int64_t>((count + 127) / 128, 2048), 128, 0, st>>>(dU, u, first, count, d64);
     std::vector<float> h32(n), hm(nm);
     std::vector<double> h64(n);
