@@ -471,7 +471,7 @@ static int launch_round(Batch& B, bool timed) {
     }
     te(K_SGEN);
     tb(K_SGEMM);
-    k_surv_gemm<<<B.nsm * 4, 128, kGemmSmem, B.st>>>(B.dU, B.dCtl, B.dInfo);
+    k_surv_gemm<<<B.nsm * 4, 128, 0, B.st>>>(B.dU, B.dCtl, B.dInfo);
     te(K_SGEMM);
     tb(K_SHASH);
     k_surv_hash<<<B.nsm * B.res_shash, 256, 0, B.st>>>(B.dU, B.dCtl, B.dInfo);
@@ -1122,7 +1122,7 @@ int ug_batch_restore(void* h, int32_t u, int64_t n, const int64_t* idx, const in
         k.round_base = 0;
         memset(ri, 0, sizeof(RoundInfo));
         ri->n_uni = B->n;
-        const int sev = ((m * d.dim + 31) >> 5) * ((T + 31) >> 5);
+        const int sev = gemm_tiles(m * d.dim, T);
         for (int v = 0; v <= B->n; v++) {
             const bool past = v > u;
             ri->surv_off[v] = past ? m : 0;
@@ -1143,7 +1143,7 @@ int ug_batch_restore(void* h, int32_t u, int64_t n, const int64_t* idx, const in
         if (e == cudaSuccess) e = cudaMemsetAsync(d.spos, 0, (size_t)m * T * sizeof(Pt64), B->st);  // unused axes
         if (e == cudaSuccess) {
             k_restore_gen<<<B->nsm * 4, 32 * kSurvWarps, kSurvWarps * kSurvSmemPerWarp, B->st>>>(B->dU, u, dIdx, m);
-            k_surv_gemm<<<B->nsm * 4, 128, kGemmSmem, B->st>>>(B->dU, B->dCtl, B->dInfo);
+            k_surv_gemm<<<B->nsm * 4, 128, 0, B->st>>>(B->dU, B->dCtl, B->dInfo);
             k_commit<<<B->nsm * 8, 256, 0, B->st>>>(B->dU, B->dCtl, B->dInfo);
             e = cudaGetLastError();
         }

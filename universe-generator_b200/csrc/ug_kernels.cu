@@ -317,12 +317,12 @@ __global__ void __launch_bounds__(256) k_compact(const UniDev* __restrict__ U, U
             int Sv = 0, sevv = 0, sptv = 0, So = 0, sevo = 0;
             if (v < n) {
                 Sv = *(volatile int32_t*)&ctl[v].S;
-                sevv = ((Sv * U[v].dim + 31) >> 5) * ((U[v].T + 31) >> 5);
+                sevv = gemm_tiles(Sv * U[v].dim, U[v].T);
                 sptv = Sv * U[v].T;
                 // the same survivors and product tiles, universes in tile order (costliest first)
                 const int uo = info->tile_uni[v];
                 So = *(volatile int32_t*)&ctl[uo].S;
-                sevo = ((So * U[uo].dim + 31) >> 5) * ((U[uo].T + 31) >> 5);
+                sevo = gemm_tiles(So * U[uo].dim, U[uo].T);
             }
             int t1, t2, t3, t4, t5;
             const int p1 = block_excl_scan256(Sv, wsum, &t1);
@@ -546,31 +546,35 @@ __global__ void __launch_bounds__(32 * kSurvWarps) k_restore_gen(const UniDev* _
     }
 }
 
-__device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(smem)),
-                 "l"(gmem)
-                 : "memory");
+// FP64 tensor products D += A B.  8 x 8 x 4: lane (g, t) = (lane / 4, lane % 4) holds A(g, t),
+// B(t, g) and D(g, 2t), D(g, 2t + 1).  16 x 8 x 8: A(g, t), A(g + 8, t), A(g, t + 4),
+// A(g + 8, t + 4); B(t, g), B(t + 4, g); D(g, 2t), D(g, 2t + 1), D(g + 8, 2t), D(g + 8, 2t + 1).
+// Each element accumulates its products in ascending order, one rounding each: the same
+// bits as a chain of fused multiply-adds.
+__device__ __forceinline__ void dmma_8x8x4(double* d, double a, double b) {
+    asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};"
+                 : "+d"(d[0]), "+d"(d[1])
+                 : "d"(a), "d"(b));
 }
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void cp_async_wait() {
-    asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
+__device__ __forceinline__ void dmma_16x8x8(double* d, const double* a, const double* b) {
+    asm volatile(
+        "mma.sync.aligned.m16n8k8.row.col.f64.f64.f64.f64 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+        : "+d"(d[0]), "+d"(d[1]), "+d"(d[2]), "+d"(d[3])
+        : "d"(a[0]), "d"(a[1]), "d"(a[2]), "d"(a[3]), "d"(b[0]), "d"(b[1]));
 }
 
-// k_surv_gemm: X[row][t] = wrap(a2 + invsinz_t * sum_k coef[k][row] KT[k][t]),
-// one warp per 32-row x 32-timestep tile.  Lane (rg, tg) owns rows
-// row0 + 0..3 and timesteps t0 + 8 jj + {0,1}; every (row, t) is a single FMA
-// chain in ascending k, i.e. eval64's operations in eval64's order.  Each warp
-// streams its tile's A rows and B columns through shared memory in chunks of
-// kGemmKC terms, two stages deep (cp.async), so the next chunk is in flight while
-// the current one is multiplied.
+// k_surv_gemm: X[row][t] = wrap(a2 + invsinz_t * sum_k coef[k][row] KT[k][t]), one warp per
+// tile of 16 rows x 32 timesteps (less at the last timesteps), as FP64 tensor products
+// over ascending k: eval64's operations in eval64's order.  The operands come straight
+// from L1/L2 two steps of eight terms ahead; the small tile keeps a round of few survivors
+// on many warps.  FP64 FMAs from shared memory waited for their operands (a lane's 4 x 8
+// outputs take 48 bytes of shared memory per 32 FMAs: two thirds of the FP64 rate at best).
+// Per round: 2+1 T = 256, 270 survivors 84 -> 42 us; 3+1 T = 128, 1800 52 -> 33 us; a
+// 32-universe batch 152 -> 120 us.
 __global__ void __launch_bounds__(128) k_surv_gemm(const UniDev* __restrict__ U, UniCtl* ctl,
                                                    RoundInfo* info) {
-    extern __shared__ __align__(16) double gemm_smem[];  // [warp][stage][A | B][kGemmKC][32]
-    const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-    double* wsm = gemm_smem + (size_t)wib * (2 * 2 * kGemmKC * 32);
+    const int lane = threadIdx.x & 31, gl = lane >> 2, tl = lane & 3;
     const int n_uni = info->n_uni, total = info->total_sev;
-    const int rg = lane >> 2, tg = lane & 3;
     // tiles handed out one at a time, costliest universes first (a tile's cost is
     // its universe's term count K, 24 to 384); the next claimed when one starts
     int item = 0, next = 0;
@@ -585,75 +589,58 @@ __global__ void __launch_bounds__(128) k_surv_gemm(const UniDev* __restrict__ U,
         const int T = d.T, dim = d.dim, K = d.K, R = d.Rpad, TP = d.Tpad;
         const int ntb = (T + 31) >> 5;
         const int rb = local / ntb, tb = local - rb * ntb;
-        const int row0 = rb * 32 + rg * 4;
-        const int t0 = tb * 32 + 2 * tg;
-        const double* Ag = d.coef + rb * 32;  // tile rows [rb*32, rb*32+32) < Rpad
-        const double* Bg = d.KT + tb * 32;    // tile timesteps [tb*32, tb*32+32) < Tpad
-        // chunk ch: terms [ch*KC, min(K, ch*KC+KC)), 16-byte pieces (16 per 32-double row)
-        auto issue = [&](int stage, int k0) {
-            double* As = wsm + stage * (2 * kGemmKC * 32);
-            double* Bs = As + kGemmKC * 32;
-            for (int i = lane; i < kGemmKC * 16; i += 32) {
-                const int kk = i >> 4, pc = (i & 15) * 2;
-                if (k0 + kk < K) {
-                    cp_async16(As + kk * 32 + pc, Ag + (size_t)(k0 + kk) * R + pc);
-                    cp_async16(Bs + kk * 32 + pc, Bg + (size_t)(k0 + kk) * TP + pc);
-                }
-            }
-            cp_async_commit();
+        const int t0 = tb * 32, nn = min(4, (T - t0 + 7) >> 3);  // timestep blocks of 8
+        const double* Ag = d.coef + rb * kGemmRows + gl;  // tile rows below Rpad
+        const double* Bg = d.KT + t0 + gl;                // tile timesteps below Tpad
+        struct Step {
+            double a[4], b[4][2];
         };
-        double acc[4][8];
+        auto fetch = [&](int k0, Step& s) {
 #pragma unroll
-        for (int i = 0; i < 4; i++)
+            for (int h = 0; h < 2; h++) {
+                const int k = k0 + 4 * h + tl;
+                const bool on = k < K;
+                s.a[2 * h] = on ? Ag[(size_t)k * R] : 0.0;
+                s.a[2 * h + 1] = on ? Ag[(size_t)k * R + 8] : 0.0;
 #pragma unroll
-            for (int j = 0; j < 8; j++) acc[i][j] = 0.0;
-        const int nch = (K + kGemmKC - 1) / kGemmKC;
-        issue(0, 0);
-        for (int ch = 0; ch < nch; ch++) {
-            if (ch + 1 < nch) {
-                issue((ch + 1) & 1, (ch + 1) * kGemmKC);
-                cp_async_wait<1>();
-            } else {
-                cp_async_wait<0>();
+                for (int j = 0; j < 4; j++) s.b[j][h] = on && j < nn ? __ldg(Bg + (size_t)k * TP + 8 * j) : 0.0;
             }
-            __syncwarp();
-            const double* As = wsm + (ch & 1) * (2 * kGemmKC * 32) + rg * 4;
-            const double* Bs = wsm + (ch & 1) * (2 * kGemmKC * 32) + kGemmKC * 32 + 2 * tg;
-            const int kn = min(kGemmKC, K - ch * kGemmKC);
-#pragma unroll 4
-            for (int kk = 0; kk < kn; kk++) {
-                const double2 a01 = *(const double2*)(As + kk * 32);
-                const double2 a23 = *(const double2*)(As + kk * 32 + 2);
-                const double av[4] = {a01.x, a01.y, a23.x, a23.y};
-                double bv[8];
+        };
+        double acc[4][4];
 #pragma unroll
-                for (int jj = 0; jj < 4; jj++) {
-                    const double2 b2 = *(const double2*)(Bs + kk * 32 + 8 * jj);
-                    bv[2 * jj] = b2.x;
-                    bv[2 * jj + 1] = b2.y;
-                }
+        for (int j = 0; j < 4; j++)
 #pragma unroll
-                for (int i = 0; i < 4; i++)
+            for (int q = 0; q < 4; q++) acc[j][q] = 0.0;
+        Step s[3];
+        fetch(0, s[0]);
+        fetch(8, s[1]);
+        for (int k0 = 0; k0 < K; k0 += 24) {
 #pragma unroll
-                    for (int j = 0; j < 8; j++) acc[i][j] = fma(av[i], bv[j], acc[i][j]);
+            for (int h = 0; h < 3; h++) {
+                if (k0 + 8 * h >= K) break;
+                fetch(k0 + 8 * (h + 2), s[(h + 2) % 3]);
+#pragma unroll
+                for (int j = 0; j < 4; j++)
+                    if (j < nn) dmma_16x8x8(acc[j], s[h].a, s[h].b[j]);
             }
-            __syncwarp();  // the stage is refilled by the issue of chunk ch + 2
         }
         const int nrows = ctl[u].S * dim;
         [[maybe_unused]] const int64_t nspos = (int64_t)d.S_max * T;
 #pragma unroll
-        for (int i = 0; i < 4; i++) {
-            const int row = row0 + i;
+        for (int q = 0; q < 2; q++) {
+            const int row = rb * kGemmRows + gl + 8 * q;
             if (row >= nrows) continue;
             const int r = row / dim, ax = row - r * dim;
             const double a2 = d.a2row[UG_IDX(row, R)];
 #pragma unroll
-            for (int j = 0; j < 8; j++) {
-                const int t = t0 + 8 * (j >> 1) + (j & 1);
-                if (t < T)
-                    d.spos[UG_IDX((int64_t)r * T + t, nspos)].c[ax] =
-                        torus_wrap(fma(acc[i][j], __ldg(d.invsinz + t), a2));
-            }
+            for (int j = 0; j < 4; j++)
+#pragma unroll
+                for (int e = 0; e < 2; e++) {
+                    const int t = t0 + 8 * j + 2 * tl + e;
+                    if (t < T)
+                        d.spos[UG_IDX((int64_t)r * T + t, nspos)].c[ax] =
+                            torus_wrap(fma(acc[j][2 * q + e], __ldg(d.invsinz + t), a2));
+                }
         }
     }
 }
@@ -881,15 +868,6 @@ __global__ void __maxnreg__(128) k_confirm64w(const UniDev* __restrict__ U, UniC
         }
         __syncwarp();
     }
-}
-
-// FP64 tensor product D += A B, 8 x 8 x 4: lane (g, t) = (lane / 4, lane % 4) holds A(g, t),
-// B(t, g) and D(g, 2t), D(g, 2t + 1).  Each element accumulates its four products in
-// ascending order, one rounding each: the same bits as a chain of fused multiply-adds.
-__device__ __forceinline__ void dmma_8x8x4(double* d, double a, double b) {
-    asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};"
-                 : "+d"(d[0]), "+d"(d[1])
-                 : "d"(a), "d"(b));
 }
 
 // warp_gen64_axis of all axes by a whole block, as term-ordered rows (row pitch kRowK):

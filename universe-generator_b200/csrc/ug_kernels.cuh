@@ -21,7 +21,7 @@ struct RoundInfo {
     int32_t gray_done;
     int32_t tile_next;     // mixed prefilter: tiles handed out beyond the first gridDim.x
     int32_t confl_next;    // k_conflicts: survivors handed out so far
-    int32_t total_sev;     // k_surv_gemm warp tiles (32 rows x 32 timesteps)
+    int32_t total_sev;     // k_surv_gemm warp tiles
     int32_t total_spt;     // survivor timesteps (k_surv_hash / k_commit items)
     int32_t tile_off[kMaxUni + 1];   // prefilter tiles: first tile of the i-th universe in tile order
     int32_t tile_uni[kMaxUni];       // the universe at position i of the tile order
@@ -84,9 +84,11 @@ __global__ void k_rehash(const UniDev* __restrict__ U, UniCtl* ctl, int u, int64
 __global__ void k_gather_accepted(const UniDev* __restrict__ U, const int64_t* __restrict__ off,
                                   int64_t* __restrict__ idx, int32_t* __restrict__ gid);
 
-// k_surv_gemm: terms per shared-memory chunk; two stages of A and B per warp.
-constexpr int kGemmKC = 8;
-constexpr size_t kGemmSmem = (size_t)4 * 2 * 2 * kGemmKC * 32 * sizeof(double);  // 4 warps per CTA
+// k_surv_gemm: warp tiles of kGemmRows rows x 32 timesteps.
+constexpr int kGemmRows = 16;
+__host__ __device__ __forceinline__ int gemm_tiles(int rows, int T) {
+    return (rows + kGemmRows - 1) / kGemmRows * ((T + 31) >> 5);
+}
 
 // Shared memory of k_surv_gen per warp (bytes), for F <= kMaxF.
 constexpr int kSurvWarps = 4;
