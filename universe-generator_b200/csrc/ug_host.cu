@@ -480,7 +480,7 @@ static int launch_round(Batch& B, bool timed) {
     k_conflicts<<<B.nsm * B.res_confl, 128, 0, B.st>>>(B.dU, B.dCtl, B.dInfo);
     te(K_CONFL);
     tb(K_GREEDY);
-    k_greedy<<<B.n, 32, 2 * kSmaxCap * sizeof(int32_t), B.st>>>(B.dU, B.dCtl, B.dInfo);
+    k_greedy<<<B.n, 32, kGreedySmem, B.st>>>(B.dU, B.dCtl, B.dInfo);
     te(K_GREEDY);
     tb(K_COMMIT);
     k_commit<<<B.nsm * 8, 256, 0, B.st>>>(B.dU, B.dCtl, B.dInfo);
@@ -716,8 +716,7 @@ int ug_batch_create(const ug_universe_cfg* cfgs, int32_t n, const ug_run_opts* o
         cudaMemcpy(B->dInfo, &ri, sizeof ri, cudaMemcpyHostToDevice) != cudaSuccess)
         return bail(fail(UG_ECUDA, "control block upload failed"));
     if ((rc = push_unidev(*B))) return bail(rc);
-    if (cudaFuncSetAttribute(k_greedy, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)(2 * kSmaxCap * sizeof(int32_t))) != cudaSuccess)
+    if (cudaFuncSetAttribute(k_greedy, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kGreedySmem) != cudaSuccess)
         return bail(fail(UG_ECUDA, "smem attribute failed"));
     if (cudaFuncSetAttribute(k_surv_gen, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              (int)(kSurvWarps * kSurvSmemPerWarp)) != cudaSuccess ||

@@ -1064,43 +1064,63 @@ __global__ void __maxnreg__(128) k_retest(const UniDev* __restrict__ U, UniCtl* 
     }
 }
 
-// One warp per survivor r: the set of earlier survivors r' < r that it
-// touches (Chebyshev contact at any timestep; plus crossings in 1+1D).
+// The set of earlier survivors r' < r that survivor r touches (Chebyshev contact at any
+// timestep; plus crossings in 1+1D).  A warp per survivor, lanes over timesteps; a block of
+// four warps where the round's survivors leave most of them idle.  A lane's chain of
+// dependent loads (its point, the round table's heads, the heads' points, the chains)
+// bounds it, so the loads of each link are issued together, four blocks of the window at
+// a time.  Against one probe after another and a warp per survivor, per round: 2+1
+// T = 256, 270 survivors 101 -> 30 us; 3+1 T = 128, 1800 65 -> 35 us; a 32-universe
+// batch 133 -> 119 us.  A block serves a survivor up to two per resident CTA: beyond that
+// the warps are all busy and short T leaves a block's lanes without a timestep.
 __global__ void __launch_bounds__(128) k_conflicts(const UniDev* __restrict__ U, UniCtl* ctl,
                                                     RoundInfo* info) {
-    __shared__ int32_t s_cnt[4];
+    __shared__ int32_t s_cnt[4], s_item;
     __shared__ int32_t s_list[4][kConflictCap];
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
     const int n_uni = info->n_uni, total = info->total_surv;
-    volatile int32_t* cnt = &s_cnt[wib];
-    volatile int32_t* lst = s_list[wib];
+    const bool wide = total <= 2 * (int)gridDim.x;
+    const int gt = wide ? threadIdx.x : lane, gn = wide ? 128 : 32;  // thread of the survivor's group
+    volatile int32_t* cnt = &s_cnt[wide ? 0 : wib];
+    volatile int32_t* lst = s_list[wide ? 0 : wib];
+    auto sync = [&]() {
+        if (wide)
+            __syncthreads();
+        else
+            __syncwarp();
+    };
     // Survivors are handed out one at a time, costliest universes first (their cost
     // differs by the timesteps and dimension); the next one is claimed when an item
     // starts so the atomic's latency hides behind the item.
-    int item = 0;
-    if (lane == 0) item = atomicAdd(&info->confl_next, 1);
-    item = __shfl_sync(0xffffffffu, item, 0);
+    int item = 0, next = 0;
+    auto settle = [&](int v) -> int {  // the value of the group's first thread
+        if (!wide) return __shfl_sync(0xffffffffu, v, 0);
+        if (threadIdx.x == 0) s_item = v;
+        __syncthreads();
+        return s_item;
+    };
+    if (gt == 0) item = atomicAdd(&info->confl_next, 1);
+    item = settle(item);
     while (item < total) {
-        int next = 0;
-        if (lane == 0) next = atomicAdd(&info->confl_next, 1);
+        if (gt == 0) next = atomicAdd(&info->confl_next, 1);
         const int pos = find_uni(info->surv_off_o, n_uni, item);
         const int u = info->tile_uni[pos];
         const int r = item - info->surv_off_o[pos];
         const UniDev& d = U[u];
         UniCtl& c = ctl[u];
         const int T = d.T;
-        if (lane == 0) *cnt = 0;
-        __syncwarp();
+        if (gt == 0) *cnt = 0;
+        sync();
         auto add = [&](int32_t r2) {
             const int n = *cnt < kConflictCap ? *cnt : kConflictCap;
             for (int i = 0; i < n; i++)
                 if (lst[i] == r2) return;
-            const int pos = atomicAdd((int32_t*)cnt, 1);
-            if (pos < kConflictCap) lst[pos] = r2;
+            const int at = atomicAdd((int32_t*)cnt, 1);
+            if (at < kConflictCap) lst[at] = r2;
         };
         if (d.dim == 1 && d.cross1d) {
             const Pt64* P = d.spos + UG_IDX((int64_t)r * T + T - 1, (int64_t)d.S_max * T) + 1 - T;
-            for (int r2 = lane; r2 < r; r2 += 32) {
+            for (int r2 = gt; r2 < r; r2 += gn) {
                 const Pt64* Q = d.spos + UG_IDX((int64_t)r2 * T + T - 1, (int64_t)d.S_max * T) + 1 - T;
                 double d0 = torus_delta(P[0].c[0] - Q[0].c[0]);
                 bool hit = hit1(d0, d.cell, d.inclusive);
@@ -1124,8 +1144,9 @@ __global__ void __launch_bounds__(128) k_conflicts(const UniDev* __restrict__ U,
             }
         } else {
             const int gw = d.gw, gwb = rblock_gw(d), rbs = d.rblock_shift;
-            for (int t = lane; t < T; t += 32) {
+            for (int t = gt; t < T; t += gn) {
                 const Pt64 P = d.spos[UG_IDX((int64_t)r * T + t, (int64_t)d.S_max * T)];
+                const Pt64* St = d.spos + t;
                 // distinct round-table blocks of the 3 neighbour cells per axis:
                 // bl[ax] packs up to three 10-bit block coordinates, nbk[ax] counts them
                 // (registers only: every index below is a compile-time constant)
@@ -1146,47 +1167,64 @@ __global__ void __launch_bounds__(128) k_conflicts(const UniDev* __restrict__ U,
                         nbk[ax] = n;
                     }
                 }
-                for (int i0 = 0; i0 < nbk[0]; i0++)
-                    for (int i1 = 0; i1 < nbk[1]; i1++)
-                        for (int i2 = 0; i2 < nbk[2]; i2++) {
-                            const int bc[3] = {(int)((bl[0] >> (10 * i0)) & 1023u),
-                                               (int)((bl[1] >> (10 * i1)) & 1023u),
-                                               (int)((bl[2] >> (10 * i2)) & 1023u)};
-                            int32_t r2 = rtab_head(d, c.epoch, t, lin_cell(bc, d.dim, gwb));
-                            while (r2 >= 0) {
-                                if (r2 == r) {  // this survivor's own point: its link is in P
-                                    r2 = P.next;
-                                    continue;
-                                }
-                                const Pt64* Q = d.spos + UG_IDX((int64_t)r2 * T + t, (int64_t)d.S_max * T);
-                                if (r2 < r && pair_hit64(d, P.c, Q->c)) add(r2);
-                                r2 = Q->next;
-                            }
+                auto test = [&](int32_t r2, const Pt64& Q) {
+                    if (r2 < r && pair_hit64(d, P.c, Q.c)) add(r2);
+                };
+                const int nc = nbk[0] * nbk[1] * nbk[2];
+                for (int c0 = 0; c0 < nc; c0 += 4) {  // block combinations, four at a time
+                    int32_t h[4];
+                    Pt64 Q[4];
+#pragma unroll
+                    for (int k = 0; k < 4; k++) {
+                        const int cc = c0 + k, i2 = cc % nbk[2], i01 = cc / nbk[2], i1 = i01 % nbk[1], i0 = i01 / nbk[1];
+                        const int bc[3] = {(int)((bl[0] >> (10 * i0)) & 1023u), (int)((bl[1] >> (10 * i1)) & 1023u),
+                                           (int)((bl[2] >> (10 * i2)) & 1023u)};
+                        h[k] = -1;
+                        if (cc < nc) h[k] = rtab_head(d, c.epoch, t, lin_cell(bc, d.dim, gwb));
+                    }
+#pragma unroll
+                    for (int k = 0; k < 4; k++)
+                        if (h[k] >= 0) Q[k] = St[UG_IDX((int64_t)h[k] * T, (int64_t)d.S_max * T)];
+#pragma unroll
+                    for (int k = 0; k < 4; k++) {
+                        if (h[k] < 0) continue;
+                        test(h[k], Q[k]);
+                        for (int32_t r2 = Q[k].next; r2 >= 0;) {
+                            const Pt64 N = St[UG_IDX((int64_t)r2 * T, (int64_t)d.S_max * T)];
+                            test(r2, N);
+                            r2 = N.next;
                         }
+                    }
+                }
             }
         }
-        __syncwarp();
+        sync();
         // more than kConflictCap contacts: the list keeps kConflictCap of them and the
         // count says so; the resolver rejects on any admitted one and otherwise stops
         // the round at this survivor
         const int n = *cnt;
         const int ns = n < kConflictCap ? n : kConflictCap;
-        for (int i = lane; i < ns; i += 32) d.clist[UG_IDX((int64_t)r * kConflictCap + i, (int64_t)d.S_max * kConflictCap)] = lst[i];
-        if (lane == 0) d.ccount[UG_IDX(r, d.S_max)] = n;
-        __syncwarp();
-        item = __shfl_sync(0xffffffffu, next, 0);
+        for (int i = gt; i < ns; i += gn) d.clist[UG_IDX((int64_t)r * kConflictCap + i, (int64_t)d.S_max * kConflictCap)] = lst[i];
+        if (gt == 0) d.ccount[UG_IDX(r, d.S_max)] = n;
+        sync();
+        item = settle(next);
     }
 }
 
 // ------------------------------------------------------------- resolver
 
 // One warp per universe: survivors in index order; admit survivor r iff the
-// sequential-RSA rule holds against the round's earlier admissions.
+// sequential-RSA rule holds against the round's earlier admissions.  32 survivors are a
+// window; the next window's contact lists come into shared memory while one is decided,
+// and the counts (and pre-round groups) a window before that, so that no step waits for
+// global memory: 3+1 T = 128, 1800 survivors 67 -> 34 us a round, unique groups at
+// T = 256, 270 survivors 115 -> 62 us.
 __global__ void __launch_bounds__(32) k_greedy(const UniDev* __restrict__ U, UniCtl* ctl,
                                                RoundInfo* info) {
-    extern __shared__ int32_t greedy_smem[];
+    extern __shared__ __align__(16) int32_t greedy_smem[];
     int32_t* acc_s = greedy_smem;
-    int32_t* gid_s = greedy_smem + kSmaxCap;
+    int32_t* gid_s = acc_s + kSmaxCap;
+    int32_t* lists = gid_s + kSmaxCap;  // [2][32][kListPitch]
     const int u = blockIdx.x;
     const int lane = threadIdx.x;
     const UniDev& d = U[u];
@@ -1196,181 +1234,183 @@ __global__ void __launch_bounds__(32) k_greedy(const UniDev* __restrict__ U, Uni
     const int S_eff = c.trunc < S ? c.trunc : S;
     const bool group = group_phase(d, c);
     const bool unique_group = d.group_mode == GROUP_UNIQUE;
-    const int64_t room = d.slot_cap - c.n_slots;
+    const int64_t room = d.slot_cap - c.n_slots, n_slots = c.n_slots, max_n = c.phase == 1 ? c.max_n : 0;
     int k = 0, stop_at = S_eff;
     int64_t n_unique = c.n_unique, n_sub = c.n_sub;
     bool grow = false, hit_max = false, undecided = false;
-    // Plain rounds: 32 survivors per step.  Each lane gathers its survivor's
-    // listed contacts -- admitted ones from earlier steps (certain rejection)
-    // and a bit mask of the earlier lanes of this step -- and the warp then
-    // decides the 32 in index order from those masks: the same decisions as the
-    // one-at-a-time loop below, which group rounds use.
-    for (int r0 = 0; !group && r0 < S_eff; r0 += 32) {
-        const int r = r0 + lane, nvalid = min(32, S_eff - r0);
-        uint32_t dep = 0;
-        bool ext = false, over = false;
-        if (lane < nvalid) {
-            const int n_all = d.ccount[UG_IDX(r, d.S_max)];
-            over = n_all > kConflictCap;
-            const int n = over ? kConflictCap : n_all;
-            const int32_t* lst = d.clist + UG_IDX((int64_t)r * kConflictCap, (int64_t)d.S_max * kConflictCap);
+    auto load_cnt = [&](int r0) { return r0 + lane < S_eff ? d.ccount[UG_IDX(r0 + lane, d.S_max)] : 0; };
+    auto load_g0 = [&](int r0) {
+        return group && r0 + lane < S_eff
+                   ? d.g0[UG_IDX(d.surv_off[UG_IDX(r0 + lane, d.S_max + 1)], d.B_max)]
+                   : -1;
+    };
+    auto stage = [&](int r0, int n_all) {  // this lane's survivor's list, 16 bytes at a time
+        int32_t* dst = lists + ((r0 >> 5) & 1) * 32 * kListPitch + lane * kListPitch;
+        const int32_t* src = d.clist + UG_IDX((int64_t)(r0 + lane < S_eff ? r0 + lane : 0) * kConflictCap,
+                                              (int64_t)d.S_max * kConflictCap);
+        const int n = min(n_all, (int)kConflictCap);
+        for (int i = 0; i < n; i += 4)
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(
+                             (uint32_t)__cvta_generic_to_shared(dst + i)),
+                         "l"(src + i)
+                         : "memory");
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    int cnt0 = load_cnt(0), cnt1 = load_cnt(32), g00 = load_g0(0), g01 = load_g0(32);
+    stage(0, cnt0);
+    bool stopped = false;
+    for (int r0 = 0; r0 < S_eff && !stopped; r0 += 32) {
+        const int cnt2 = load_cnt(r0 + 64), g02 = load_g0(r0 + 64);
+        stage(r0 + 32, cnt1);
+        asm volatile("cp.async.wait_group 1;" ::: "memory");
+        __syncwarp();
+        const int32_t* win = lists + ((r0 >> 5) & 1) * 32 * kListPitch;
+        const int nvalid = min(32, S_eff - r0);
+        int lim = nvalid;  // survivors of the window that are decided
+        if (!group) {
+            // Plain rounds: each lane gathers its survivor's listed contacts -- admitted ones
+            // from earlier windows (certain rejection) and a bit mask of the earlier lanes of
+            // this one -- and the warp then decides the 32 in index order from those masks:
+            // the same decisions as one at a time, as group rounds take them.
+            const int r = r0 + lane;
+            uint32_t dep = 0;
+            bool ext = false;
+            const bool over = cnt0 > kConflictCap;
+            const int n = over ? kConflictCap : cnt0;
             for (int i = 0; i < n; i++) {
-                const int r2 = lst[i];
+                const int r2 = win[lane * kListPitch + i];
                 if (r2 < r0)
                     ext |= acc_s[UG_IDX(r2, kSmaxCap)] >= 0;
                 else
                     dep |= 1u << (r2 - r0);
             }
-        }
-        // In-order greedy over the step's lanes: a lane decides once every lane it
-        // depends on has decided (dependencies point to lower lanes only, so the
-        // lowest undecided lane is always ready; one pass per link of the longest
-        // dependency chain, usually one).
-        const uint32_t valid = nvalid >= 32 ? 0xffffffffu : ((1u << nvalid) - 1u);
-        uint32_t und = valid, accm = 0;
-        while (und) {
-            const bool ready = ((und >> lane) & 1u) && !(dep & und);
-            accm |= __ballot_sync(0xffffffffu, ready && !ext && !(dep & accm));
-            und &= ~__ballot_sync(0xffffffffu, ready);
-        }
-        // Where the one-at-a-time scan would stop: at lane j it first checks the
-        // room left (stop before j), then an admitted j with an over-full list
-        // (undecided: stop before j), then the unique cap (stop after j).
-        const int acc_before = __popc(accm & ((1u << lane) - 1u));
-        const bool mine = (accm >> lane) & 1u;
-        const uint32_t b_room = __ballot_sync(0xffffffffu, lane < nvalid && k + acc_before >= room);
-        const uint32_t b_over = __ballot_sync(0xffffffffu, mine && over);
-        const uint32_t b_max = __ballot_sync(
-            0xffffffffu, mine && c.phase == 1 && c.max_n > 0 && n_unique + acc_before + 1 >= c.max_n);
-        int stop = -1;
-        if (b_room | b_over | b_max) {
-            const int j = __ffs(b_room | b_over | b_max) - 1;
-            if ((b_room >> j) & 1u) {
-                stop = j;
-                grow = true;
-            } else if ((b_over >> j) & 1u) {
-                stop = j;
-                undecided = true;
-            } else {
-                stop = j + 1;
-                hit_max = true;
+            // In-order greedy over the window's lanes: a lane decides once every lane it
+            // depends on has decided (dependencies point to lower lanes only, so the
+            // lowest undecided lane is always ready; one pass per link of the longest
+            // dependency chain, usually one).
+            const uint32_t valid = nvalid >= 32 ? 0xffffffffu : ((1u << nvalid) - 1u);
+            uint32_t und = valid, accm = 0;
+            while (und) {
+                const bool ready = ((und >> lane) & 1u) && !(dep & und);
+                accm |= __ballot_sync(0xffffffffu, ready && !ext && !(dep & accm));
+                und &= ~__ballot_sync(0xffffffffu, ready);
             }
-        }
-        const int lim = stop < 0 ? nvalid : stop;
-        if (lane < lim) {
-            const bool a = (accm >> lane) & 1u;
-            const int rank = k + __popc(accm & ((1u << lane) - 1u));
-            acc_s[UG_IDX(r, kSmaxCap)] = a ? rank : -1;
-            gid_s[UG_IDX(r, kSmaxCap)] = a ? (int32_t)(c.n_slots + rank) : -1;
-        }
-        __syncwarp();
-        const uint32_t taken = accm & (lim >= 32 ? 0xffffffffu : ((1u << lim) - 1u));
-        k += __popc(taken);
-        n_unique += __popc(taken);
-        if (stop >= 0) {
-            stop_at = r0 + stop;
-            break;
-        }
-    }
-    // Group rounds, one survivor at a time.  The per-survivor data comes in ahead of its
-    // step: contact counts and pre-round groups of 32 survivors at once (lane i holds
-    // survivor r0 + i), and the next survivor's list while this one is decided.
-    int w_cnt = 0;
-    int32_t w_g0 = -1, nx0 = -1, nx1 = -1;
-    auto load_window = [&](int rb) {
-        const int rr = rb + lane;
-        w_cnt = 0;
-        w_g0 = -1;
-        if (rr < S_eff) {
-            w_cnt = d.ccount[UG_IDX(rr, d.S_max)];
-            w_g0 = d.g0[UG_IDX(d.surv_off[UG_IDX(rr, d.S_max + 1)], d.B_max)];
-        }
-    };
-    auto load_list = [&](int rr, int nn) {
-        const int32_t* l = d.clist + UG_IDX((int64_t)rr * kConflictCap, (int64_t)d.S_max * kConflictCap);
-        nx0 = lane < nn ? l[lane] : -1;
-        nx1 = lane + 32 < nn ? l[lane + 32] : -1;
-    };
-    if (group && S_eff > 0) {
-        load_window(0);
-        load_list(0, min(__shfl_sync(0xffffffffu, w_cnt, 0), kConflictCap));
-    }
-    for (int r = 0; group && r < S_eff; r++) {
-        if (k >= room) {
-            stop_at = r;
-            grow = true;
-            break;
-        }
-        const int n_all = __shfl_sync(0xffffffffu, w_cnt, r & 31);
-        const int32_t g0 = __shfl_sync(0xffffffffu, w_g0, r & 31);
-        const bool over = n_all > kConflictCap;  // the list holds only kConflictCap contacts
-        const int n = over ? kConflictCap : n_all;
-        const int32_t e0 = nx0, e1 = nx1;  // this survivor's list entries lane, lane + 32
-        if (r + 1 < S_eff) {
-            if (((r + 1) & 31) == 0) load_window(r + 1);
-            load_list(r + 1, min(__shfl_sync(0xffffffffu, w_cnt, (r + 1) & 31), kConflictCap));
-        }
-        bool accept;
-        int32_t gid;
-        // union of the pre-round group and the groups of admitted earlier survivors
-        int32_t mine = -1;
-        bool two = false;
+            // Where the one-at-a-time scan would stop: at lane j it first checks the
+            // room left (stop before j), then an admitted j with an over-full list
+            // (undecided: stop before j), then the unique cap (stop after j).
+            const int acc_before = __popc(accm & ((1u << lane) - 1u));
+            const bool mine = (accm >> lane) & 1u;
+            const uint32_t b_room = __ballot_sync(0xffffffffu, lane < nvalid && k + acc_before >= room);
+            const uint32_t b_over = __ballot_sync(0xffffffffu, mine && over);
+            const uint32_t b_max = __ballot_sync(0xffffffffu, mine && max_n > 0 && n_unique + acc_before + 1 >= max_n);
+            if (b_room | b_over | b_max) {
+                const int j = __ffs(b_room | b_over | b_max) - 1;
+                stopped = true;
+                lim = j;
+                if ((b_room >> j) & 1u) {
+                    grow = true;
+                } else if ((b_over >> j) & 1u) {
+                    undecided = true;
+                } else {
+                    lim = j + 1;
+                    hit_max = true;
+                }
+            }
+            if (lane < lim) {
+                const int rank = k + acc_before;
+                acc_s[UG_IDX(r, kSmaxCap)] = mine ? rank : -1;
+                gid_s[UG_IDX(r, kSmaxCap)] = mine ? (int32_t)(n_slots + rank) : -1;
+            }
+            const int taken = __popc(accm & (lim >= 32 ? 0xffffffffu : ((1u << lim) - 1u)));
+            k += taken;
+            n_unique += taken;
+        } else {
+            // Group rounds, one survivor at a time.
+            for (int j = 0; j < nvalid; j++) {
+                const int r = r0 + j;
+                if (k >= room) {
+                    lim = j;
+                    grow = stopped = true;
+                    break;
+                }
+                const int n_all = __shfl_sync(0xffffffffu, cnt0, j);
+                const int32_t g0 = __shfl_sync(0xffffffffu, g00, j);
+                const bool over = n_all > kConflictCap;  // the list holds only kConflictCap contacts
+                const int n = over ? kConflictCap : n_all;
+                bool accept;
+                int32_t gid;
+                // union of the pre-round group and the groups of admitted earlier survivors
+                int32_t mine = -1;
+                bool two = false;
 #pragma unroll
-        for (int h = 0; h < 2; h++) {
-            const int32_t e = h ? e1 : e0;
-            if (lane + 32 * h < n) {
-                const int r2 = (int)UG_IDX(e, kSmaxCap);
-                if (acc_s[r2] >= 0) {
-                    const int32_t g2 = gid_s[r2];
-                    if (mine == -1)
-                        mine = g2;
-                    else if (mine != g2)
-                        two = true;
+                for (int h = 0; h < 2; h++)
+                    if (lane + 32 * h < n) {
+                        const int r2 = (int)UG_IDX(win[j * kListPitch + lane + 32 * h], kSmaxCap);
+                        if (acc_s[r2] >= 0) {
+                            const int32_t g2 = gid_s[r2];
+                            if (mine == -1)
+                                mine = g2;
+                            else if (mine != g2)
+                                two = true;
+                        }
+                    }
+                // the first group in list order: the pre-round one, else the lowest lane's
+                const uint32_t hasg = __ballot_sync(0xffffffffu, mine != -1);
+                int32_t first = g0;  // g0 and hasg are the same in every lane
+                if (first == -1 && hasg) first = __shfl_sync(0xffffffffu, mine, __ffs(hasg) - 1);
+                two = two || (mine != -1 && mine != first);
+                two = __any_sync(0xffffffffu, two);
+                if (!two && over) {  // unlisted contacts might add a group: decide next round
+                    lim = j;
+                    undecided = stopped = true;
+                    break;
+                }
+                if (two) {
+                    accept = false;
+                    gid = -1;
+                } else if (first == -1) {
+                    accept = unique_group;  // touches nothing: founds a group, or (subpath) rejected
+                    gid = (int32_t)(n_slots + k);
+                } else {
+                    accept = true;
+                    gid = first;
+                }
+                if (lane == 0) {
+                    acc_s[UG_IDX(r, kSmaxCap)] = accept ? k : -1;
+                    gid_s[UG_IDX(r, kSmaxCap)] = accept ? gid : -1;
+                }
+                __syncwarp();
+                if (accept) {
+                    k++;
+                    if (unique_group && gid == (int32_t)(n_slots + k - 1))
+                        n_unique++;
+                    else
+                        n_sub++;
+                    if (max_n > 0 && n_unique >= max_n) {
+                        lim = j + 1;
+                        hit_max = stopped = true;
+                        break;
+                    }
                 }
             }
         }
-        // the first group in list order: the pre-round one, else the lowest lane's
-        const uint32_t hasg = __ballot_sync(0xffffffffu, mine != -1);
-        int32_t first = g0;  // g0 and hasg are the same in every lane
-        if (first == -1 && hasg) first = __shfl_sync(0xffffffffu, mine, __ffs(hasg) - 1);
-        two = two || (mine != -1 && mine != first);
-        two = __any_sync(0xffffffffu, two);
-        if (!two && over) {  // unlisted contacts might add a group: decide next round
-            stop_at = r;
-            undecided = true;
-            break;
-        }
-        if (two) {
-            accept = false;
-            gid = -1;
-        } else if (first == -1) {
-            accept = unique_group;  // touches nothing: founds a group, or (subpath) rejected
-            gid = (int32_t)(c.n_slots + k);
-        } else {
-            accept = true;
-            gid = first;
-        }
-        if (lane == 0) {
-            acc_s[UG_IDX(r, kSmaxCap)] = accept ? k : -1;
-            gid_s[UG_IDX(r, kSmaxCap)] = accept ? gid : -1;
-        }
         __syncwarp();
-        if (accept) {
-            k++;
-            if (!group || (unique_group && gid == (int32_t)(c.n_slots + k - 1)))
-                n_unique++;
-            else
-                n_sub++;
-            if (c.phase == 1 && c.max_n > 0 && n_unique >= c.max_n) {
-                stop_at = r + 1;
-                hit_max = true;
-                break;
-            }
+        if (r0 + lane < S) {
+            const bool in = lane < lim;
+            d.acc_rank[UG_IDX(r0 + lane, d.S_max)] = in ? acc_s[UG_IDX(r0 + lane, kSmaxCap)] : -1;
+            d.sgid[UG_IDX(r0 + lane, d.S_max)] = in ? gid_s[UG_IDX(r0 + lane, kSmaxCap)] : -1;
         }
+        if (stopped) stop_at = r0 + lim;
+        cnt0 = cnt1;
+        cnt1 = cnt2;
+        g00 = g01;
+        g01 = g02;
     }
-    for (int r = lane; r < S; r += 32) {
-        d.acc_rank[UG_IDX(r, d.S_max)] = r < stop_at ? acc_s[UG_IDX(r, kSmaxCap)] : -1;
-        d.sgid[UG_IDX(r, d.S_max)] = r < stop_at ? gid_s[UG_IDX(r, kSmaxCap)] : -1;
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    // survivors beyond the last window are not decided this round
+    for (int r = (stop_at + 31) / 32 * 32 + lane; r < S; r += 32) {
+        d.acc_rank[UG_IDX(r, d.S_max)] = -1;
+        d.sgid[UG_IDX(r, d.S_max)] = -1;
     }
     if (lane != 0) return;
     int64_t next;
@@ -1463,24 +1503,23 @@ __device__ __forceinline__ void grid_insert(const UniDev& d, UniCtl& c, int t, i
     c.state = ST_ERROR;
 }
 
-// Sets a bit of an occupancy bitmap; bits are only ever set during a run, so
-// a bit read as set needs no atomic (most are: an unconditional atomicOr took
-// k_commit from 56 to 63 ms per c3 job).
-__device__ __forceinline__ void occ_set(uint32_t* words, int64_t bit, int64_t nwords) {
-    uint32_t* w = words + UG_IDX(bit >> 5, nwords);
-    const uint32_t m = 1u << (bit & 31);
-    if (!(__ldcg(w) & m)) atomicOr(w, m);
-}
-
-__device__ __forceinline__ void occ_set_mask(uint32_t* words, int64_t w, uint32_t m, int64_t nwords) {
+// Sets bits of an occupancy bitmap.  Bits are only ever set during a run, so a word that
+// holds them needs no atomic (most do: an unconditional atomicOr took k_commit from 56 to
+// 63 ms in the 256-universe batch).  A round of few points (blind) does not read first: its
+// time is the chain of those reads, and an atomic without a result is not waited for
+// (2+1 T = 64, 20 survivors 16.4 -> 12.6 us a round; 3+1 T = 128, 1800 60 -> 50 us).
+__device__ __forceinline__ void occ_set_mask(uint32_t* words, int64_t w, uint32_t m, int64_t nwords, bool blind) {
     uint32_t* p = words + UG_IDX(w, nwords);
-    if ((__ldcg(p) & m) != m) atomicOr(p, m);
+    if (blind || (__ldcg(p) & m) != m) atomicOr(p, m);
+}
+__device__ __forceinline__ void occ_set(uint32_t* words, int64_t bit, int64_t nwords, bool blind) {
+    occ_set_mask(words, bit >> 5, 1u << (bit & 31), nwords, blind);
 }
 
 // Dilated filter: marks every block holding a cell that meets the cube of
 // half-width occ1_reach around the committed point x (cells wrap around the
 // torus; per axis at most 5 cells, so at most 5 blocks).
-__device__ __forceinline__ void occ1_mark(const UniDev& d, int t, const double* x) {
+__device__ __forceinline__ void occ1_mark(const UniDev& d, int t, const double* x, bool blind) {
     int bk[3][5], nb[3] = {1, 1, 1};
 #pragma unroll
     for (int ax = 0; ax < 3; ax++) {
@@ -1513,13 +1552,13 @@ __device__ __forceinline__ void occ1_mark(const UniDev& d, int t, const double* 
             for (int i = 0; i < nb[L]; i++) {
                 const int64_t bit = row + bk[L][i];
                 if ((bit >> 5) != wcur) {
-                    if (m) occ_set_mask(d.occ1, wcur, m, d.occ1_words);
+                    if (m) occ_set_mask(d.occ1, wcur, m, d.occ1_words, blind);
                     wcur = bit >> 5;
                     m = 0;
                 }
                 m |= 1u << (bit & 31);
             }
-            occ_set_mask(d.occ1, wcur, m, d.occ1_words);
+            occ_set_mask(d.occ1, wcur, m, d.occ1_words, blind);
         }
 }
 
@@ -1527,6 +1566,7 @@ __global__ void __launch_bounds__(256) k_commit(const UniDev* __restrict__ U, Un
                                                 RoundInfo* info) {
     const int n_uni = info->n_uni, total = info->total_spt;
     const int lane = threadIdx.x & 31;
+    const bool blind = total <= (int)(gridDim.x * blockDim.x);  // a point per thread at most
     // items: (survivor, timestep) pairs, survivor-major per universe; the trip
     // count is uniform over the block so the warp-level counting below converges
     for (int w0 = blockIdx.x * blockDim.x; w0 < total; w0 += gridDim.x * blockDim.x) {
@@ -1550,9 +1590,9 @@ __global__ void __launch_bounds__(256) k_commit(const UniDev* __restrict__ U, Un
                 int32_t old;
                 uint32_t fbit;
                 const int64_t lin = grid_lin(d, cc, &fbit);
+                occ_set(d.occ, occ_bit(d, t, cc), d.occ_words, blind);
+                occ1_mark(d, t, q.c, blind);
                 grid_insert(d, c, t, lin, fbit, cells_per_t(d), (int32_t)slot, &old, &new_key, &new_cell);
-                occ_set(d.occ, occ_bit(d, t, cc), d.occ_words);
-                occ1_mark(d, t, q.c);
                 q.next = old;
                 q.gid = d.sgid[UG_IDX(r, d.S_max)];
                 d.pts[UG_IDX(slot * d.T + t, d.slot_cap * d.T)] = q;

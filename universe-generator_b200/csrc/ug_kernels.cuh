@@ -84,6 +84,11 @@ __global__ void k_rehash(const UniDev* __restrict__ U, UniCtl* ctl, int u, int64
 __global__ void k_gather_accepted(const UniDev* __restrict__ U, const int64_t* __restrict__ off,
                                   int64_t* __restrict__ idx, int32_t* __restrict__ gid);
 
+// k_greedy: admissions and groups of a round's survivors, two windows of contact lists
+// (padded so that the lanes' lists start on different banks).
+constexpr int kListPitch = kConflictCap + 4;
+constexpr size_t kGreedySmem = ((size_t)2 * kSmaxCap + 2 * 32 * kListPitch) * sizeof(int32_t);
+
 // k_surv_gemm: warp tiles of kGemmRows rows x 32 timesteps.
 constexpr int kGemmRows = 16;
 __host__ __device__ __forceinline__ int gemm_tiles(int rows, int T) {
