@@ -184,7 +184,7 @@ struct UniCtl {
     int32_t tile_ns;       // mixed prefilter: slowest tile of the last round (ns), orders the next round's tiles
     int32_t B_min, B_cap;  // round-size adaptation bounds
     int32_t err_code;
-    int32_t pad;
+    int32_t tile_cost;     // mixed prefilter: the last tile_ns that was timed
     // windowed stops (braid_cuda.cu:585-590, 931-943 and the phase-2 new-volume
     // window of :953-1037).  Each window is 32 buckets of q = win_target / 32
     // candidates aligned at the phase start (phase_start); rounds never straddle a

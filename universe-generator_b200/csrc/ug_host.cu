@@ -428,6 +428,19 @@ static int push_unidev(Batch& B) {
 
 // ---------------------------------------------------------- round launch
 
+// The rounds of one replay, and the plan of the round that follows them: a universe that
+// has used its budget is seen as done here (not after R more, empty rounds).
+static int launch_round(Batch& B, bool timed);
+static int launch_rounds(Batch& B, int rounds, bool timed) {
+    for (int r = 0; r < rounds; r++) {
+        const int rc = launch_round(B, timed);
+        if (rc) return rc;
+    }
+    k_plan<<<1, 256, 0, B.st>>>(B.dU, B.dCtl, B.dInfo);
+    CKR(cudaGetLastError());
+    return UG_OK;
+}
+
 static int launch_round(Batch& B, bool timed) {
     B.synced = false;
     auto tb = [&](int k) {
@@ -496,12 +509,9 @@ static int build_graph(Batch& B, int rounds) {
     }
     cudaGraph_t g;
     CKR(cudaStreamBeginCapture(B.st, cudaStreamCaptureModeThreadLocal));
-    for (int r = 0; r < rounds; r++) {
-        int rc = launch_round(B, false);
-        if (rc) {
-            cudaStreamEndCapture(B.st, &g);
-            return rc;
-        }
+    if (int rc = launch_rounds(B, rounds, false)) {
+        cudaStreamEndCapture(B.st, &g);
+        return rc;
     }
     CKR(cudaStreamEndCapture(B.st, &g));
     CKR(cudaGraphInstantiate(&B.gexec, g, 0));
@@ -769,10 +779,9 @@ int ug_batch_run(void* h, int64_t max_rounds) {
             B->synced = false;
             CKR(cudaGraphLaunch(B->gexec, B->st));
         } else {
-            for (int r = 0; r < R; r++)
-                if ((rc = launch_round(*B, B->opts.kernel_timing != 0))) return rc;
+            if ((rc = launch_rounds(*B, R, B->opts.kernel_timing != 0))) return rc;
         }
-        B->launches += (int64_t)R * B->kernels_per_round;
+        B->launches += (int64_t)R * B->kernels_per_round + 1;
         done_rounds += R;
         if ((rc = pull_ctl(*B))) return rc;
         int64_t progress_after = 0;

@@ -65,6 +65,8 @@ __device__ __forceinline__ int block_excl_scan256(int v, int* wsum, int* total) 
     return wpre + incl - v;
 }
 
+// The next round of every universe: the last round's windows closed, phases switched, round
+// sizes and tiles.  Planning a planned round again changes nothing.
 __global__ void k_plan(const UniDev* __restrict__ U, UniCtl* ctl, RoundInfo* info) {
     __shared__ int32_t ntiles[kMaxUni];
     __shared__ int32_t cost[kMaxUni];
@@ -74,9 +76,10 @@ __global__ void k_plan(const UniDev* __restrict__ U, UniCtl* ctl, RoundInfo* inf
         UniCtl& c = ctl[u];
         const UniDev& d = U[u];
         int B = 0;
-        // tile cost: the last round's slowest prefilter tile; before any is timed,
-        // dim * T stands in (all universes start together, so one round uses one kind)
-        cost[u] = c.tile_ns > 0 ? c.tile_ns : d.dim * d.T;
+        // tile cost: the slowest prefilter tile of the last round that timed any; before
+        // that, dim * T stands in (all universes start together, so one round uses one kind)
+        if (c.tile_ns > 0) c.tile_cost = c.tile_ns;
+        cost[u] = c.tile_cost > 0 ? c.tile_cost : d.dim * d.T;
         c.tile_ns = 0;
         // the last round's admissions (k_greedy) and newly occupied cells (k_commit)
         // close the windows' buckets; rounds end on bucket boundaries
@@ -1077,12 +1080,14 @@ __global__ void __launch_bounds__(128) k_conflicts(const UniDev* __restrict__ U,
                                                     RoundInfo* info) {
     __shared__ int32_t s_cnt[4], s_item;
     __shared__ int32_t s_list[4][kConflictCap];
+    __shared__ uint32_t s_seen[4][kSmaxCap / 32];  // earlier survivors already listed
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
     const int n_uni = info->n_uni, total = info->total_surv;
     const bool wide = total <= 2 * (int)gridDim.x;
     const int gt = wide ? threadIdx.x : lane, gn = wide ? 128 : 32;  // thread of the survivor's group
     volatile int32_t* cnt = &s_cnt[wide ? 0 : wib];
     volatile int32_t* lst = s_list[wide ? 0 : wib];
+    uint32_t* seen = s_seen[wide ? 0 : wib];
     auto sync = [&]() {
         if (wide)
             __syncthreads();
@@ -1110,11 +1115,13 @@ __global__ void __launch_bounds__(128) k_conflicts(const UniDev* __restrict__ U,
         UniCtl& c = ctl[u];
         const int T = d.T;
         if (gt == 0) *cnt = 0;
+        for (int i = gt; i <= r >> 5; i += gn) seen[i] = 0u;
         sync();
+        // each earlier survivor once (it is met at many timesteps): with a search of the
+        // list instead, lanes that met it together listed it twice and overfilled the list
         auto add = [&](int32_t r2) {
-            const int n = *cnt < kConflictCap ? *cnt : kConflictCap;
-            for (int i = 0; i < n; i++)
-                if (lst[i] == r2) return;
+            const uint32_t bit = 1u << (r2 & 31);
+            if (atomicOr(&seen[UG_IDX(r2 >> 5, kSmaxCap / 32)], bit) & bit) return;
             const int at = atomicAdd((int32_t*)cnt, 1);
             if (at < kConflictCap) lst[at] = r2;
         };
