@@ -119,7 +119,6 @@ struct UniDev {
     uint32_t* surv_bits;   // [B_max / 32]
     int32_t* g0;           // [B_max]  group mode: single pre-round group touched (-1 none)
     int32_t* surv_off;     // [S_max]  candidate offset within the round
-    int32_t* gray_off;     // [B_max]  FP64 form: offsets of the round's candidates
     Pt64* spos;            // [S_max * T]
     uint64_t* rhead;       // round table [T * rblocks]: epoch<<32 | head survivor rank of
                            // each (timestep, block); entries of other epochs are empty
@@ -171,7 +170,7 @@ struct UniCtl {
     int32_t phase;         // 1 or 2
     int32_t state;         // ST_*
     int32_t epoch;         // round-table epoch
-    int32_t n_gray;        // FP64 form: candidates tested this round
+    int32_t n_gray;        // unused
     int32_t accepted_round;
     int64_t gray_total;    // mixed: FP64 retests over the run
     int64_t rounds;
@@ -457,43 +456,6 @@ __device__ __forceinline__ double eval64(const UniDev& U, const double* alpha, c
         acc = fma(beta[b * stride], __ldg(Cm + (size_t)b * T), acc);
     }
     return torus_wrap(fma(acc, __ldg(U.invsinz + t), a2));
-}
-
-// eval64 of D axes at once (coefficient rows ax * F1 of alpha / beta): each
-// axis accumulates in eval64's order, so every coordinate has eval64's bits;
-// the axes' chains are independent and the basis loads are shared.
-template <int D>
-__device__ __forceinline__ void eval64x(const UniDev& U, const double* alpha, const double* beta, const double* a2,
-                                        int t, double* P) {
-    const int T = U.T, F = U.F, F1 = F + 1;
-    const double* S = U.S + t;
-    const double* Cm = U.Cm + t;
-    double acc[D];
-#pragma unroll
-    for (int ax = 0; ax < D; ax++) acc[ax] = 0.0;
-    int b = 2;
-#pragma unroll 2
-    for (; b + 1 <= F; b += 2) {
-        const double s0 = __ldg(S + (size_t)b * T), c0 = __ldg(Cm + (size_t)b * T);
-        const double s1 = __ldg(S + (size_t)(b + 1) * T);
-#pragma unroll
-        for (int ax = 0; ax < D; ax++) {
-            acc[ax] = fma(alpha[ax * F1 + b], s0, acc[ax]);
-            acc[ax] = fma(beta[ax * F1 + b], c0, acc[ax]);
-            acc[ax] = fma(alpha[ax * F1 + b + 1], s1, acc[ax]);
-        }
-    }
-    if (b <= F) {
-        const double s0 = __ldg(S + (size_t)b * T), c0 = __ldg(Cm + (size_t)b * T);
-#pragma unroll
-        for (int ax = 0; ax < D; ax++) {
-            acc[ax] = fma(alpha[ax * F1 + b], s0, acc[ax]);
-            acc[ax] = fma(beta[ax * F1 + b], c0, acc[ax]);
-        }
-    }
-    const double iz = __ldg(U.invsinz + t);
-#pragma unroll
-    for (int ax = 0; ax < D; ax++) P[ax] = torus_wrap(fma(acc[ax], iz, a2[ax]));
 }
 
 // ------------------------------------------------------------ grid access

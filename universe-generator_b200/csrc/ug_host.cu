@@ -78,6 +78,9 @@ struct Batch {
     UniCtl* dCtl = nullptr;
     std::vector<UniCtl> hCtl;
     RoundInfo* dInfo = nullptr;
+    bool any_fp64 = false;    // some universe takes the FP64 test of every candidate
+    Scratch64 sc64{};
+    int t64_ctas = 0;
     RetestQueue rq{};         // mixed form: undecided candidates of a round
     cudaGraphExec_t gexec = nullptr;
     int graph_rounds = 0;
@@ -373,8 +376,7 @@ static int setup_universe(Batch& B, UniHost& h, int64_t dense_budget, int64_t* d
     if ((rc = alloc_points(h, cap))) return rc;
     // round buffers
     const int Bm = d.B_max, Sm = d.S_max;
-    if ((rc = dalloc(h, &d.surv_bits, Bm / 32, 0)) || (rc = dalloc(h, &d.gray_off, B.opts.precision == UG_PREC_MIXED ? 1 : Bm, 0)) ||
-        (rc = dalloc(h, &d.g0, Bm, 0xff)) || (rc = dalloc(h, &d.surv_off, Sm + 1, 0)) ||
+    if ((rc = dalloc(h, &d.surv_bits, Bm / 32, 0)) ||         (rc = dalloc(h, &d.g0, Bm, 0xff)) || (rc = dalloc(h, &d.surv_off, Sm + 1, 0)) ||
         (rc = dalloc(h, &d.spos, (size_t)Sm * T, 0)) || (rc = dalloc(h, &d.ccount, Sm, 0)) ||
         (rc = dalloc(h, &d.clist, (size_t)Sm * kConflictCap, 0)) ||
         (rc = dalloc(h, &d.sgid, Sm, 0xff)) || (rc = dalloc(h, &d.acc_rank, Sm, 0xff)))
@@ -460,6 +462,11 @@ static int launch_round(Batch& B, bool timed) {
     k_plan<<<1, 256, 0, B.st>>>(B.dU, B.dCtl, B.dInfo);
     te(K_PLAN);
     if (B.opts.precision == UG_PREC_MIXED && B.any_mixed) {
+        if (B.any_fp64) {  // universes that the tensor-core test does not take
+            tb(K_PRE);
+            k_test64<<<B.t64_ctas, kT64Threads, 0, B.st>>>(B.dU, B.dCtl, B.dInfo, B.sc64, 0);
+            te(K_PRE);
+        }
         tb(K_MIXED);
         launch_prefilter_mixed(B.dU, B.dCtl, B.dInfo, B.rq, B.nsm, B.any_group, B.any_euclid, B.st);
         te(K_MIXED);
@@ -467,11 +474,8 @@ static int launch_round(Batch& B, bool timed) {
         k_retest<<<B.nsm * 4, 32 * kSurvWarps, kRetestSmem, B.st>>>(B.dU, B.dCtl, B.dInfo, B.rq);
         te(K_CONFIRM);
     } else {
-        // the FP64 form: every candidate of the round, one warp per candidate
-        // (coefficients in shared memory, lanes over timesteps in endpoint-first order)
         tb(K_PRE);
-        k_all_list<<<B.n, 256, 0, B.st>>>(B.dU, B.dCtl, B.dInfo);
-        k_confirm64w<<<B.nsm * 4, 32 * kSurvWarps, kSurvWarps * kConfSmemPerWarp, B.st>>>(B.dU, B.dCtl, B.dInfo);
+        k_test64<<<B.t64_ctas, kT64Threads, 0, B.st>>>(B.dU, B.dCtl, B.dInfo, B.sc64, 1);
         te(K_PRE);
     }
     tb(K_COMPACT);
@@ -734,10 +738,22 @@ int ug_batch_create(const ug_universe_cfg* cfgs, int32_t n, const ug_run_opts* o
                              (int)(kSurvWarps * kSurvSmemPerWarp)) != cudaSuccess)
         return bail(fail(UG_ECUDA, "smem attribute failed"));
     if (B->any_mixed && (rc = mixed_init_kernels())) return bail(rc);
-    B->kernels_per_round = 10;
-    if (cudaFuncSetAttribute(k_confirm64w, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)(kSurvWarps * kConfSmemPerWarp)) != cudaSuccess)
-        return bail(fail(UG_ECUDA, "smem attribute failed"));
+    for (const UniHost& u : B->U) B->any_fp64 |= !B->any_mixed || !u.d.mx_ok;
+    B->kernels_per_round = 9 + (B->any_mixed ? 1 : 0) + (B->any_mixed && B->any_fp64 ? 1 : 0);
+    if (B->any_fp64) {
+        // per resident CTA: coefficients (and trajectories) of 32 candidates of the widest universe
+        B->t64_ctas = B->nsm * resident_ctas(k_test64, kT64Threads, 0, 4);
+        for (const UniHost& u : B->U)
+            if (!B->any_mixed || !u.d.mx_ok)
+                B->sc64.coef_stride = std::max(B->sc64.coef_stride,
+                                               (size_t)32 * ((size_t)u.d.K * u.d.dim + (u.d.cross1d ? u.d.T : 0)));
+        const size_t n = (size_t)B->t64_ctas;
+        if (cudaMalloc(&B->sc64.coef, n * B->sc64.coef_stride * sizeof(double)) != cudaSuccess ||
+            (B->any_knot && (cudaMalloc(&B->sc64.wgt, n * kKnotStride * sizeof(double)) != cudaSuccess ||
+                             cudaMalloc(&B->sc64.phase, n * kKnotStride * sizeof(double)) != cudaSuccess ||
+                             cudaMalloc(&B->sc64.freq, n * kKnotStride * sizeof(uint16_t)) != cudaSuccess)))
+            return bail(fail(UG_ENOMEM, "FP64 test scratch allocation failed"));
+    }
     if (B->any_mixed) {
         // every candidate of a round may be undecided; masks for an eighth of them
         int64_t cap = 0;
@@ -750,7 +766,7 @@ int ug_batch_create(const ug_universe_cfg* cfgs, int32_t n, const ug_run_opts* o
     }
     // one wave per SM, measured on c3 against 8 / 8 / 16 CTAs per SM: k_surv_gen 27.7 ->
     // 24.5 ms, k_surv_hash 33.5 -> 32.0 ms, k_conflicts 85.5 -> 80.2 ms per job.  k_commit
-    // and k_confirm64w keep 8 and 4 per SM (more than resident): one wave measured slower
+    // and the retest keep 8 and 4 per SM (more than resident): one wave measured slower
     // for them (56.6 -> 60.0 and 38.2 -> 40.6 ms).
     B->res_sgen = resident_ctas(k_surv_gen, 32 * kSurvWarps,
                                 kSurvWarps * (B->any_knot ? kSurvSmemPerWarp : kSurvSmemAxis), 8);
@@ -1231,6 +1247,10 @@ int ug_batch_destroy(void* h) {
         cudaFree(u.d.acc_idx);
         mixed_free(u.mt);
     }
+    cudaFree(B->sc64.coef);
+    cudaFree(B->sc64.wgt);
+    cudaFree(B->sc64.phase);
+    cudaFree(B->sc64.freq);
     cudaFree(B->rq.item);
     cudaFree(B->rq.mask);
     cudaFree(B->dU);

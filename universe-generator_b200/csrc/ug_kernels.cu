@@ -2,9 +2,9 @@
 //
 // One round of every active universe:
 //   k_plan         round sizes, phase transitions, tile decomposition
-//   k_all_list + k_confirm64w
-//                  FP64 form: every candidate, warp per candidate (shared-memory
-//                  coefficients, lanes over timesteps) against the committed packing
+//   k_test64       FP64 form: every candidate against the committed packing, a CTA per
+//                  32 candidates (also the universes of a mixed batch that the tensor-core
+//                  test does not take)
 //   k_prefilter_mixed (ug_mixed.cu) + k_retest
 //                  mixed form: the tensor-core test, then the FP64 test of the
 //                  timesteps that its guard band left undecided
@@ -24,6 +24,7 @@
 #include "ug_kernels.cuh"
 
 #include <algorithm>
+#include <type_traits>
 
 namespace ug {
 
@@ -167,6 +168,7 @@ __global__ void k_plan(const UniDev* __restrict__ U, UniCtl* ctl, RoundInfo* inf
         info->any_active = acc > 0;
         info->total_surv = 0;
         info->total_gray = 0;
+        info->t64_next = 0;
         info->compact_done = 0;
         info->tile_next = 0;
         info->confl_next = 0;
@@ -685,76 +687,6 @@ __global__ void __launch_bounds__(256) k_surv_hash(const UniDev* __restrict__ U,
     }
 }
 
-// The FP64 form's work list: every candidate of the round, per universe, and cleared
-// survivor bits.
-__global__ void __launch_bounds__(256) k_all_list(const UniDev* __restrict__ U, UniCtl* ctl,
-                                                  RoundInfo* info) {
-    __shared__ int32_t wsum[8];
-    __shared__ int32_t s_running;
-    __shared__ bool s_last;
-    const int u = blockIdx.x;
-    const UniDev& d = U[u];
-    UniCtl& c = ctl[u];
-    const int B = c.B;
-    const int nwords = (B + 31) >> 5;
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    if (tid == 0) s_running = 0;
-    __syncthreads();
-    for (int base = 0; base < nwords; base += 256) {
-        const int w = base + tid;
-        uint32_t bits = w < nwords ? 0xffffffffu : 0u;
-        if (w < nwords) d.surv_bits[UG_IDX(w, d.B_max / 32)] = 0u;
-        if (w == nwords - 1 && (B & 31)) bits &= (1u << (B & 31)) - 1u;
-        const int cnt = __popc(bits);
-        int incl = cnt;
-        for (int o = 1; o < 32; o <<= 1) {
-            const int v = __shfl_up_sync(0xffffffffu, incl, o);
-            if (lane >= o) incl += v;
-        }
-        if (lane == 31) wsum[warp] = incl;
-        __syncthreads();
-        int wpre = 0, tot = 0;
-        for (int k = 0; k < 8; k++) {
-            if (k < warp) wpre += wsum[k];
-            tot += wsum[k];
-        }
-        int rank = s_running + wpre + incl - cnt;
-        while (bits) {
-            const int bit = __ffs(bits) - 1;
-            bits &= bits - 1;
-            d.gray_off[UG_IDX(rank, d.B_max)] = w * 32 + bit;
-            rank++;
-        }
-        __syncthreads();
-        if (tid == 0) s_running += tot;
-        __syncthreads();
-    }
-    if (tid == 0) {
-        c.n_gray = s_running;
-        __threadfence();
-        s_last = atomicAdd(&info->gray_done, 1) == info->n_uni - 1;
-    }
-    __syncthreads();
-    if (s_last) {  // the last block: offsets of every universe's candidates
-        __threadfence();
-        const int n = info->n_uni;
-        int acc = 0;
-        for (int b0 = 0; b0 < n; b0 += 256) {
-            const int v = b0 + tid;
-            const int g = v < n ? *(volatile int32_t*)&ctl[v].n_gray : 0;
-            int tot;
-            const int p = block_excl_scan256(g, wsum, &tot);
-            if (v < n) info->gray_pref[v] = acc + p;
-            acc += tot;
-        }
-        if (tid == 0) {
-            info->gray_pref[n] = acc;
-            info->total_gray = acc;
-            info->gray_done = 0;
-        }
-    }
-}
-
 // 1+1D crossing rule in FP64: trajectory P[0..T) against the accepted paths `first`,
 // first + step, ...; stops on *stop (another thread found a contact) outside group rounds.
 // True on rejection; group rounds keep the single touched group in *g.
@@ -790,86 +722,415 @@ __device__ __forceinline__ bool cross64(const UniDev& d, const double* P, int64_
     return false;
 }
 
-__device__ __forceinline__ void eval64_at(const UniDev& d, const double* alpha, const double* beta, const double* a2,
-                                          int t, double* P) {
-    if (d.dim == 3)
-        eval64x<3>(d, alpha, beta, a2, t, P);
-    else if (d.dim == 2)
-        eval64x<2>(d, alpha, beta, a2, t, P);
-    else
-        eval64x<1>(d, alpha, beta, a2, t, P);
-}
+// The FP64 form's test of every candidate of the round (of the universes outside the
+// tensor-core path in a mixed batch), a CTA per tile of 32 candidates:
+//   generation   blocks, logarithms and sines spread over all threads, the normalisation
+//                summed in ascending b by a thread per (candidate, axis); the knot stream is
+//                drawn by a lane per candidate.  Term-ordered coefficient columns in the
+//                CTA's own scratch (L2-resident), a column per (axis, candidate).
+//   evaluation   16 or 32 timesteps at a time in endpoint-first order, as FP64 tensor
+//                products over the live candidates' columns: eval64's bits.
+//   test         the dilated filter for every (candidate, timestep), then the windows of
+//                those it passes, then the chains of the occupied cells, each step over a
+//                queue of the CTA (as in the mixed prefilter's epilogue).
+// Bound by FP64 issue (about 110 FP64 instructions to generate a term) and the chains.  A
+// warp per candidate, lanes over 32 timesteps, summed and (knot stream) drew on one lane;
+// per job: 3+1 L2-ball T = 100, 200 k candidates 6.4 -> 3.9 ms; knot stream 2+1 T = 120,
+// two terms, 200 k 4.9 -> 1.8; T = 65, all terms, 80 k 19.0 -> 1.8.
+template <int D>
+struct Test64 {
+    const UniDev& U;
+    int t;
+    const double* P;
+    int32_t* grp;  // group rounds: the candidate's group (shared by the CTA)
+    int* nvis;
+    Nbhd<D> nb;
+    __device__ __forceinline__ Test64(const UniDev& U_, int t_, const double* P_, const int* c, int32_t* grp_, int* nvis_)
+        : U(U_), t(t_), P(P_), grp(grp_), nvis(nvis_) {
+        int z[D];
+#pragma unroll
+        for (int ax = 0; ax < D; ax++) z[ax] = 0;
+        nbhd_make<D>(U, c, z, z, nb);
+    }
+    __device__ __forceinline__ bool operator()(int32_t p, int32_t& nx) {
+        const Pt64* q = U.pts + UG_IDX((int64_t)p * U.T + t, U.slot_cap * U.T);
+        const Pt64 Q = *q;
+        nx = Q.next;
+        ++*nvis;
+        if (U.gkey_shift > 0) {  // coarse chains: only the points of the 3^D window cells count
+#pragma unroll
+            for (int ax = 0; ax < D; ax++)
+                if (cyc_dist(cell_of(Q.c[ax], U.cell, U.gw), nb.v[ax][0], U.gw) >= nb.n[ax]) return false;
+        }
+        double X[3];
+#pragma unroll
+        for (int ax = 0; ax < D; ax++) X[ax] = P[ax];
+        if (!pair_hit64(U, X, Q.c)) return false;
+        if (!grp) return true;
+        int cur = *(volatile int32_t*)grp;
+        if (cur == -1) cur = atomicCAS(grp, -1, Q.gid);
+        return cur != -1 && cur != Q.gid;
+    }
+};
 
-// The FP64 form's test, one warp per candidate: FP64 regeneration and the exact test
-// against the committed packing, timesteps (1+1D: paths) spread over the lanes.
-// (a register cap instead of launch bounds: with launch bounds alone ptxas keeps 64
-// registers and spills)
-__global__ void __maxnreg__(128) k_confirm64w(const UniDev* __restrict__ U, UniCtl* ctl, RoundInfo* info) {
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    __shared__ int32_t s_hit[kSurvWarps];
-    const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-    unsigned char* my = smem_raw + (size_t)wib * kConfSmemPerWarp;
-    double* alpha = (double*)my;
-    double* beta = alpha + 3 * (kMaxF + 1);
-    double* a2 = beta + 3 * (kMaxF + 1);
-    double* wj = a2 + 3;
-    int32_t* bj = (int32_t*)(wj + kMaxF);
-    double* P1 = (double*)(my + kSurvSmemPerWarpBase);
-    volatile int32_t* vhit = &s_hit[wib];
-    const int n_uni = info->n_uni, total = info->total_gray;
-    const int gwarp = blockIdx.x * kSurvWarps + wib, nwarp = gridDim.x * kSurvWarps;
-    for (int item = gwarp; item < total; item += nwarp) {
-        const int u = find_uni(info->gray_pref, n_uni, item);
-        const UniDev& d = U[u];
-        UniCtl& c = ctl[u];
-        const int off = d.gray_off[UG_IDX(item - info->gray_pref[u], d.B_max)];
-        const uint64_t idx = (uint64_t)(c.round_base + off);
-        const int T = d.T;
-        warp_gen64(d, idx, alpha, beta, a2, bj, wj, lane);
-        if (lane == 0) *vhit = 0;
-        __syncwarp();
-        const bool group = group_phase(d, c);
-        int32_t g = -1;
-        bool hitl = false;
-        int nev = 0, nvis = 0;
-        if (d.dim == 1 && d.cross1d) {
-            for (int t = lane; t < T; t += 32) P1[t] = eval64(d, alpha, beta, 1, a2[0], t);
-            __syncwarp();
-            nev = lane == 0 ? T : 0;
-            hitl = cross64(d, P1, c.n_slots, lane, 32, group, &g, vhit);
-            if (hitl) *vhit = 1;
+// Draws of the knot stream (cuda/braid_knot.cu:111-166 order) by one lane per candidate:
+// per axis the frequencies (perm, low bits) with their sign flips (bit 15), the uniforms of
+// the weights (1 - u) and the phases; a2.  Frequencies are shuffled in shared memory.
+__device__ __forceinline__ void knot_draws(const UniDev& d, uint64_t idx, int cand, uint16_t* perm, const Scratch64& sc,
+                                           size_t cta, double* a2) {
+    Xo r;
+    r.seed(knot_seed(d.seed, idx));
+    const int nw = d.nw;
+    uint16_t* p = perm + cand;  // [j][32]
+    for (int ax = 0; ax < d.dim; ax++) {
+        const size_t o = cta * kKnotStride + (size_t)(ax * 32 + cand);
+        if ((uint32_t)nw == d.modmax) {
+            for (int j = 0; j < nw; j++) p[32 * j] = (uint16_t)(j + 2);
+            for (int j = nw - 1; j > 0; j--) {
+                const int k = (int)r.below((uint32_t)(j + 1));
+                const uint16_t tmp = p[32 * j];
+                p[32 * j] = p[32 * k];
+                p[32 * k] = tmp;
+            }
         } else {
-            const int64_t cpt = cells_per_t(d);
-            for (int oi0 = 0; oi0 < T; oi0 += 32) {
-                const int oi = oi0 + lane;
-                if (oi < T) {
-                    const int t = __ldg(d.order + oi);
-                    double P[3];
-                    eval64_at(d, alpha, beta, a2, t, P);
-                    nev++;
-                    hitl = contacts64(d, t, P, group, &g, cpt, &nvis);
+            for (int j = 0; j < nw; j++) {
+                int b = 0;
+                bool dup = true;
+                for (int guard = 0; dup && guard < 64; guard++) {
+                    b = (int)r.below(d.modmax) + 2;
+                    dup = false;
+                    for (int k = 0; k < j; k++) dup |= p[32 * k] == b;
                 }
-                if (__any_sync(0xffffffffu, hitl)) break;
+                p[32 * j] = (uint16_t)b;
             }
         }
-        // merge the lanes: any rejection, or (group rounds) two distinct groups touched
-        bool rej = __any_sync(0xffffffffu, hitl);
-        int32_t first = -1;
-        for (int o = 0; o < 32; o++) {
-            const int32_t v = __shfl_sync(0xffffffffu, g, o);
-            if (first == -1) first = v;
+        for (int j = 0; j < nw; j++) sc.wgt[o + (size_t)j * 96] = 1.0 - r.f64();
+        for (int j = 0; j < nw; j++) {
+            const int b = p[32 * j];
+            const bool neg = r.flip();
+            if (!(b & 1)) sc.phase[o + (size_t)j * 96] = r.f64() * kPi;
+            sc.freq[o + (size_t)j * 96] = (uint16_t)(b | (neg ? 0x8000 : 0));
         }
-        if (group) rej = rej || __any_sync(0xffffffffu, g != -1 && g != first);
+        a2[ax * 32 + cand] = d.pin ? 0.0 : (r.f64() * 2.0 - 1.0);
+    }
+}
+
+__global__ void __launch_bounds__(kT64Threads, 2) k_test64(const UniDev* __restrict__ U, UniCtl* ctl, RoundInfo* info,
+                                                           Scratch64 sc, int all) {
+    __shared__ double s_P[kT64Pos], s_a2[96], s_sum[96];
+    __shared__ uint2 s_q[kT64Tests];
+    __shared__ __align__(16) uint2 s_cells[kT64Cells];
+    __shared__ int32_t s_t[kMaxF], s_rej[32], s_grp[32], s_slot[32];
+    __shared__ int s_nq, s_nc, s_item;
+    __shared__ uint32_t s_live;
+    static_assert(sizeof(s_cells) >= (size_t)kMaxF * 32 * sizeof(uint16_t), "the frequencies shuffle in the cells' place");
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int gl = lane >> 2, tl = lane & 3;
+    volatile int32_t* vrej = s_rej;
+    double* G = sc.coef + (size_t)blockIdx.x * sc.coef_stride;
+    const int n_uni = info->n_uni, total = info->total_tiles * (kTile / 32);
+    for (;;) {
+        __syncthreads();  // the tile before is done with the shared arrays
+        if (tid == 0) s_item = atomicAdd(&info->t64_next, 1);
+        __syncthreads();
+        const int item = s_item;
+        if (item >= total) break;
+        const int pos = find_uni(info->tile_off, n_uni, item >> 2);
+        const int u = info->tile_uni[pos];
+        const UniDev& d = U[u];
+        UniCtl& c = ctl[u];
+        const int off0 = (item - info->tile_off[pos] * 4) * 32;
+        if ((!all && d.mx_ok) || off0 >= c.B) continue;
+        const int nv = min(32, c.B - off0);
+        const uint64_t idx0 = (uint64_t)(c.round_base + off0);
+        const int dim = d.dim, T = d.T, F = d.F, K = d.K, rows = 32 * dim;
+        const bool group = group_phase(d, c), cross = dim == 1 && d.cross1d;
+        for (int t = tid; t < T; t += kT64Threads) s_t[t] = cross ? t : __ldg(d.order + t);
+        if (tid < 32) {
+            s_rej[tid] = tid < nv ? 0 : 1;
+            s_grp[tid] = -1;
+        }
+        // ---- coefficients: G[k][ax * 32 + candidate]
+        if (d.rng == RNG_KNOT) {
+            const int nw = d.nw;
+            const size_t o = (size_t)blockIdx.x * kKnotStride;
+            if (warp == 0 && lane < nv)
+                knot_draws(d, idx0 + lane, lane, reinterpret_cast<uint16_t*>(s_cells), sc, blockIdx.x, s_a2);
+            const bool full = (uint32_t)nw == d.modmax;  // every frequency once
+            if (!full)
+                for (int e = tid; e < K * rows; e += kT64Threads) G[e] = 0.0;
+            __syncthreads();
+            for (int e = tid; e < nw * rows; e += kT64Threads) {
+                const int row = e % rows, j = e / rows;
+                if ((row & 31) < nv) {
+                    double* w = sc.wgt + o + (size_t)j * 96 + row;
+                    *w = -log(*w);
+                }
+            }
+            __syncthreads();
+            if (tid < rows && (tid & 31) < nv) {
+                const double* w = sc.wgt + o + tid;
+                double sum = 0.0;
+#pragma unroll 4
+                for (int j = 0; j < nw; j++) sum += w[(size_t)j * 96];
+                s_sum[tid] = sum;
+            }
+            __syncthreads();
+            // few terms may list a frequency twice: then a thread per row adds in term order
+            const int nj = full ? nw : 1, step = full ? 1 : nw;
+            for (int e = tid; e < nj * rows; e += kT64Threads) {
+                const int row = e % rows, j0 = e / rows;
+                if ((row & 31) >= nv) continue;
+                for (int j = j0; j < j0 + step; j++) {
+                    const size_t at = o + (size_t)j * 96 + row;
+                    const int fb = sc.freq[at], b = fb & 0x7fff, k = kseq_s(b);
+                    double amp = sc.wgt[at] / s_sum[row] / (double)b;
+                    if (fb & 0x8000) amp = -amp;
+                    double s = amp, co = 0.0;
+                    if (!(b & 1)) {
+                        double sf, cf;
+                        sincos(sc.phase[at], &sf, &cf);
+                        s = amp * cf;
+                        co = amp * sf;
+                    }
+                    double* g = G + (size_t)k * rows + row;
+                    *g = full ? s : *g + s;
+                    if (!(b & 1)) g[rows] = full ? co : g[rows] + co;
+                }
+            }
+        } else {
+            const int np = (F >> 1) + 1;
+            for (int e = tid; e < np * rows; e += kT64Threads) {
+                const int row = e % rows, p = e / rows, ax = row >> 5;
+                const uint4 o = philox_block(d.seed, idx0 + (row & 31), ax, p);
+                if (p == 0) {
+                    s_a2[row] = d.pin ? 0.0 : (double)o.x * (1.0 / 2147483648.0) - 1.0;
+                    continue;
+                }
+                const int be = 2 * p, bo = 2 * p + 1;
+                double* g = G + (size_t)kseq_s(be) * rows + row;
+                const double Ee = -log(((double)o.x + 0.5) * (1.0 / 4294967296.0));
+                g[0] = (o.z & 1u) ? -Ee : Ee;
+                g[rows] = (double)(o.z >> 1) * (1.0 / 2147483648.0) * kPi;  // the phase, until the cosine term
+                if (bo <= F) {
+                    const double Eo = -log(((double)o.y + 0.5) * (1.0 / 4294967296.0));
+                    g[2 * rows] = (o.w & 1u) ? -Eo : Eo;
+                }
+            }
+            __syncthreads();
+            if (tid < rows) {
+                double sum = 0.0;
+#pragma unroll 8
+                for (int b = 2; b <= F; b++) sum += fabs(G[(size_t)kseq_s(b) * rows + tid]);
+                s_sum[tid] = sum;
+            }
+            __syncthreads();
+            for (int e = tid; e < (F - 1) * rows; e += kT64Threads) {
+                const int row = e % rows, b = e / rows + 2;
+                double* g = G + (size_t)kseq_s(b) * rows + row;
+                const double v = *g;
+                double amp = fabs(v) / s_sum[row] / (double)b;
+                if (v < 0.0) amp = -amp;
+                if (b & 1) {
+                    *g = amp;
+                } else {
+                    double sf, cf;
+                    sincos(g[rows], &sf, &cf);
+                    *g = amp * cf;
+                    g[rows] = amp * sf;
+                }
+            }
+        }
+        // ---- timesteps, in stages
+        const int64_t cpt = cells_per_t(d);
+        int nev = 0, nvis = 0;
+        for (int c0 = 0; c0 < T;) {
+            __syncthreads();  // coefficients written; the stage before is tested
+            if (warp == 0) {
+                const uint32_t lv = __ballot_sync(0xffffffffu, s_rej[lane] == 0);
+                if ((lv >> lane) & 1u) s_slot[__popc(lv & ((1u << lane) - 1u))] = lane;
+                if (lane == 0) {
+                    s_live = lv;
+                    s_nq = s_nc = 0;
+                }
+            }
+            __syncthreads();
+            const int nl = __popc(s_live);
+            if (nl == 0) break;
+            const int width = nl > 16 && !cross ? 16 : 32;  // positions: at most 32 x 3 x 16
+            const int nc = min(width, T - c0), nn = (nc + 7) >> 3, L = nl * dim;
+            for (int m0 = warp * 16; m0 < L; m0 += kT64Threads / 32 * 16) {
+                const double *A0, *A1;
+                {
+                    const int i0 = min(m0 + gl, L - 1), i1 = min(m0 + gl + 8, L - 1);
+                    A0 = G + (i0 % dim) * 32 + s_slot[i0 / dim];
+                    A1 = G + (i1 % dim) * 32 + s_slot[i1 / dim];
+                }
+                const double* B[4];
+#pragma unroll
+                for (int j = 0; j < 4; j++) B[j] = d.KT + s_t[min(c0 + 8 * j + gl, T - 1)];
+                struct Step {
+                    double a[4], b[4][2];
+                };
+                auto fetch = [&](int k0, Step& st) {
+#pragma unroll
+                    for (int h = 0; h < 2; h++) {
+                        const int k = k0 + 4 * h + tl;
+                        const bool on = k < K;
+                        st.a[2 * h] = on ? A0[(size_t)k * rows] : 0.0;
+                        st.a[2 * h + 1] = on ? A1[(size_t)k * rows] : 0.0;
+#pragma unroll
+                        for (int j = 0; j < 4; j++)
+                            st.b[j][h] = on && j < nn ? __ldg(B[j] + (size_t)k * d.Tpad) : 0.0;
+                    }
+                };
+                double acc[4][4];
+#pragma unroll
+                for (int j = 0; j < 4; j++)
+#pragma unroll
+                    for (int q = 0; q < 4; q++) acc[j][q] = 0.0;
+                Step st[2];
+                fetch(0, st[0]);
+                for (int k0 = 0; k0 < K; k0 += 16) {
+#pragma unroll
+                    for (int h = 0; h < 2; h++) {
+                        fetch(k0 + 8 * (h + 1), st[h ^ 1]);
+#pragma unroll
+                        for (int j = 0; j < 4; j++)
+                            if (j < nn) dmma_16x8x8(acc[j], st[h].a, st[h].b[j]);
+                    }
+                }
+#pragma unroll
+                for (int q = 0; q < 2; q++) {
+                    const int i = m0 + gl + 8 * q;
+                    if (i >= L) continue;
+                    const double a2 = s_a2[(i % dim) * 32 + s_slot[i / dim]];
+#pragma unroll
+                    for (int j = 0; j < 4; j++)
+#pragma unroll
+                        for (int e = 0; e < 2; e++) {
+                            const int col = 8 * j + 2 * tl + e;
+                            if (col >= nc) continue;
+                            const double X = torus_wrap(fma(acc[j][2 * q + e], __ldg(d.invsinz + s_t[c0 + col]), a2));
+                            if (cross)  // the trajectories, behind the coefficients
+                                G[(size_t)K * 32 + (size_t)s_slot[i] * T + c0 + col] = X;
+                            else
+                                s_P[i * width + col] = X;
+                        }
+                }
+            }
+            __syncthreads();
+            c0 += width;
+            if (cross) continue;
+            const int tb = c0 - width;
+            // the filter
+            for (int i = tid; i < nl * nc; i += kT64Threads) {
+                const int sl = i / nc, j = i - sl * nc;
+                nev++;
+                int cc[3] = {0, 0, 0};
+                int64_t lin = 0;
+#pragma unroll
+                for (int ax = 0; ax < 3; ax++)
+                    if (ax < dim) {
+                        cc[ax] = cell_of(s_P[(sl * dim + ax) * width + j], d.cell, d.gw);
+                        lin = lin * d.occ1_gw + (cc[ax] >> d.occ1_shift);
+                    }
+                const int64_t b = (int64_t)s_t[tb + j] * d.occ1_per_t + lin;
+                if ((__ldg(d.occ1 + UG_IDX(b >> 5, d.occ1_words)) >> (b & 31)) & 1u) {
+                    const int at = atomicAdd(&s_nq, 1);
+                    s_q[UG_IDX(at, kT64Tests)] = make_uint2((uint32_t)(sl << 8 | j), (uint32_t)(cc[0] | cc[1] << 10 | cc[2] << 20));
+                }
+            }
+            __syncthreads();
+            // windows, then chains
+            auto run = [&](auto dc) {
+                constexpr int D = decltype(dc)::value;
+                auto with = [&](int e, auto&& f) {
+                    const uint2 q = s_q[e];
+                    const int sl = q.x >> 8, j = q.x & 255, cand = s_slot[sl];
+                    if (vrej[cand]) return;
+                    double P[D];
+                    int cc[D];
+#pragma unroll
+                    for (int ax = 0; ax < D; ax++) {
+                        P[ax] = s_P[(sl * D + ax) * width + j];
+                        cc[ax] = (q.y >> (10 * ax)) & 1023u;
+                    }
+                    Test64<D> test(d, s_t[tb + j], P, cc, group ? s_grp + cand : nullptr, &nvis);
+                    if (f(test)) vrej[cand] = 1;
+                };
+                const int nq = s_nq;
+                for (int e = tid; e < nq; e += kT64Threads)
+                    with(e, [&](Test64<D>& test) {
+                        if constexpr (D == 1) {
+                            return nbhd_scan<1>(d, test.t, test.nb, cpt, test);
+                        } else {
+                            auto put = [&](int o0, int o1, int o2) {
+                                const int at = atomicAdd(&s_nc, 1);
+                                if (at < kT64Cells) {
+                                    s_cells[at] = make_uint2((uint32_t)e | (uint32_t)o0 << 16, (uint32_t)o1 | (uint32_t)o2 << 16);
+                                    return false;
+                                }
+                                if constexpr (D == 3)
+                                    return brick_cell_visit(d, test.t, test.nb, cpt, o0, o1, o2, test);
+                                else
+                                    return brick_cell_visit2(d, test.t, test.nb, cpt, o0, o1, test);
+                            };
+                            if constexpr (D == 3)
+                                return nbhd_cells3(d, test.t, test.nb, put);
+                            else
+                                return nbhd_cells2(d, test.t, test.nb, [&](int o0, int o1) { return put(o0, o1, 0); });
+                        }
+                    });
+                __syncthreads();
+                if constexpr (D > 1) {
+                    const int ncell = min(s_nc, kT64Cells);
+                    for (int i = tid; i < ncell; i += kT64Threads) {
+                        const uint2 cl = s_cells[i];
+                        with(cl.x & 0xffffu, [&](Test64<D>& test) {
+                            if constexpr (D == 3)
+                                return brick_cell_visit(d, test.t, test.nb, cpt, (int)(cl.x >> 16), (int)(cl.y & 0xffffu),
+                                                        (int)(cl.y >> 16), test);
+                            else
+                                return brick_cell_visit2(d, test.t, test.nb, cpt, (int)(cl.x >> 16), (int)(cl.y & 0xffffu),
+                                                         test);
+                        });
+                    }
+                }
+            };
+            if (dim == 3)
+                run(std::integral_constant<int, 3>{});
+            else if (dim == 2)
+                run(std::integral_constant<int, 2>{});
+            else
+                run(std::integral_constant<int, 1>{});
+        }
+        if (cross) {  // eight threads per candidate over the accepted paths
+            const int cand = tid >> 3, part = tid & 7;
+            __syncthreads();
+            if (cand < nv) {
+                int32_t g = -1;
+                if (part == 0) nev = T;
+                if (cross64(d, G + (size_t)K * 32 + (size_t)cand * T, c.n_slots, part, 8, group, &g, vrej + cand)) vrej[cand] = 1;
+                if (group && g != -1) {
+                    const int32_t old = atomicCAS(&s_grp[cand], -1, g);
+                    if (old != -1 && old != g) vrej[cand] = 1;
+                }
+            }
+        }
         for (int o = 16; o > 0; o >>= 1) nev += __shfl_xor_sync(0xffffffffu, nev, o);
         for (int o = 16; o > 0; o >>= 1) nvis += __shfl_xor_sync(0xffffffffu, nvis, o);
         if (lane == 0) {
             if (nev) atomicAdd((unsigned long long*)&c.evals_fp64, (unsigned long long)nev);
-            if (nev) atomicAdd((unsigned long long*)&c.evals, (unsigned long long)nev);
-            if (nvis) atomicAdd((unsigned long long*)&c.visits, (unsigned long long)nvis);
-            if (!rej) atomicOr(&d.surv_bits[UG_IDX(off >> 5, d.B_max / 32)], 1u << (off & 31));
-            if (d.group_mode != GROUP_NONE) d.g0[UG_IDX(off, d.B_max)] = first;
+            if (all && nev) atomicAdd((unsigned long long*)&c.evals, (unsigned long long)nev);
+            if (all && nvis) atomicAdd((unsigned long long*)&c.visits, (unsigned long long)nvis);
         }
-        __syncwarp();
+        __syncthreads();
+        if (warp == 0) {
+            const uint32_t sb = __ballot_sync(0xffffffffu, s_rej[lane] == 0);
+            if (lane == 0) d.surv_bits[UG_IDX(off0 >> 5, d.B_max / 32)] = sb;
+            if (d.group_mode != GROUP_NONE && lane < nv) d.g0[UG_IDX(off0 + lane, d.B_max)] = s_grp[lane];
+        }
     }
 }
 
@@ -926,8 +1187,8 @@ __device__ __forceinline__ void block_gen64(const UniDev& d, uint64_t idx, doubl
 // The mixed form's retest, one block of four warps per undecided candidate (few per round:
 // one candidate's latency bounds the launch).  Only the timesteps of its mask are
 // evaluated, 32 at a time, eight per warp as FP64 tensor products (the axes are rows), with
-// eval64's bits.  Candidates without a mask (no tensor-core test, the crossing rule, or
-// beyond the masks' room) are tested at all timesteps.  Per round, against a lane per
+// eval64's bits.  Candidates without a mask (the crossing rule, or beyond the
+// masks' room) are tested at all timesteps.  Per round, against a lane per
 // timestep of all T: 2+1 unique groups T = 256 (380 candidates, ~60 timesteps each)
 // 167 -> 108 us, 3+1 T = 128 (310) 50 -> 23 us.
 __global__ void __maxnreg__(128) k_retest(const UniDev* __restrict__ U, UniCtl* ctl, RoundInfo* info,
@@ -935,13 +1196,9 @@ __global__ void __maxnreg__(128) k_retest(const UniDev* __restrict__ U, UniCtl* 
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ int32_t s_hit, s_g, s_nt;
     __shared__ int32_t s_t[kMaxF];
-    __shared__ double s_P[32][3], s_sum[3], s_traj[kMaxF];
-    double* alpha = (double*)smem_raw;
-    double* beta = alpha + 3 * (kMaxF + 1);
-    double* a2 = beta + 3 * (kMaxF + 1);
-    double* wj = a2 + 3;
-    int32_t* bj = (int32_t*)(wj + kMaxF);
-    double* rows = (double*)(smem_raw + kSurvSmemPerWarpBase);
+    __shared__ double s_P[32][3], s_sum[3], a2[3], s_traj[kMaxF];
+    double* rows = (double*)smem_raw;  // [3][kRowK], phases [3][kMaxF]
+    double* phase = rows + 3 * kRowK;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int gl = lane >> 2, tl = lane & 3;
     volatile int32_t* vhit = &s_hit;
@@ -950,24 +1207,11 @@ __global__ void __maxnreg__(128) k_retest(const UniDev* __restrict__ U, UniCtl* 
         const int2 it = rq.item[item];
         const UniDev& d = U[it.x];
         UniCtl& c = ctl[it.x];
-        const int off = it.y, T = d.T, F = d.F, K = d.K, dim = d.dim;
+        const int off = it.y, T = d.T, K = d.K, dim = d.dim;
         const uint64_t idx = (uint64_t)(c.round_base + off);
         const bool group = group_phase(d, c), cross = dim == 1 && d.cross1d;
-        const bool masked = d.mx_ok && !cross && item < rq.mask_cap;
-        if (d.rng == RNG_KNOT) {
-            if (warp == 0) warp_gen64(d, idx, alpha, beta, a2, bj, wj, lane);
-            __syncthreads();
-            for (int e = tid; e < 3 * kRowK; e += blockDim.x) rows[e] = 0.0;
-            __syncthreads();
-            for (int e = tid; e < dim * (F - 1); e += blockDim.x) {
-                const int ax = e / (F - 1), b = e - ax * (F - 1) + 2;
-                double* row = rows + ax * kRowK + kseq_s(b);
-                row[0] = alpha[ax * (F + 1) + b];
-                if (!(b & 1)) row[1] = beta[ax * (F + 1) + b];
-            }
-        } else {
-            block_gen64(d, idx, rows, beta, a2, s_sum);
-        }
+        const bool masked = !cross && item < rq.mask_cap;
+        block_gen64(d, idx, rows, phase, a2, s_sum);
         if (tid == 0) {
             s_hit = 0;
             // masked: the group that the decided timesteps touched

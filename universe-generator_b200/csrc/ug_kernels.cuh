@@ -18,7 +18,7 @@ struct RoundInfo {
     int32_t gemm_next;     // k_surv_gemm: product tiles handed out so far
     int32_t pad1;
     int32_t total_gray;
-    int32_t gray_done;
+    int32_t t64_next;      // k_test64: tiles of 32 candidates handed out so far
     int32_t tile_next;     // mixed prefilter: tiles handed out beyond the first gridDim.x
     int32_t confl_next;    // k_conflicts: survivors handed out so far
     int32_t total_sev;     // k_surv_gemm warp tiles
@@ -27,7 +27,6 @@ struct RoundInfo {
     int32_t tile_uni[kMaxUni];       // the universe at position i of the tile order
     int32_t surv_off[kMaxUni + 1];
     int32_t surv_off_o[kMaxUni + 1];  // survivor offsets of the universes in tile order
-    int32_t gray_pref[kMaxUni + 1];
     int32_t sev_off[kMaxUni + 1];
     int32_t sev_off_o[kMaxUni + 1];   // product tile offsets of the universes in tile order
     int32_t spt_off[kMaxUni + 1];
@@ -62,13 +61,25 @@ struct RetestQueue {
     int32_t mask_cap;
     int32_t cap;
 };
+// k_test64: per CTA, the coefficient columns of its 32 candidates (1+1D crossings: and
+// their trajectories), and for the knot stream its draws.
+constexpr int kT64Threads = 256;
+constexpr int kT64Pos = 32 * 3 * 16;    // positions of a stage
+constexpr int kT64Tests = 32 * 16;      // (candidate, timestep) tests of a stage
+constexpr int kT64Cells = 2048;         // occupied cells of their windows
+constexpr size_t kKnotStride = (size_t)kMaxF * 96;  // [term][axis * 32 + candidate]
+struct Scratch64 {
+    double* coef;
+    size_t coef_stride;
+    double *wgt, *phase;
+    uint16_t* freq;
+};
 constexpr int kMaskWords = kMaxF / 32;
 static_assert(kMaskWords == 8, "a mask is two uint4");
 
 // Kernels (ug_kernels.cu)
 __global__ void k_plan(const UniDev* __restrict__ U, UniCtl* ctl, RoundInfo* info);
-__global__ void k_all_list(const UniDev* __restrict__ U, UniCtl* ctl, RoundInfo* info);
-__global__ void k_confirm64w(const UniDev* __restrict__ U, UniCtl* ctl, RoundInfo* info);
+__global__ void k_test64(const UniDev* __restrict__ U, UniCtl* ctl, RoundInfo* info, Scratch64 sc, int all);
 __global__ void k_retest(const UniDev* __restrict__ U, UniCtl* ctl, RoundInfo* info, RetestQueue rq);
 __global__ void k_compact(const UniDev* __restrict__ U, UniCtl* ctl, RoundInfo* info);
 __global__ void k_surv_gen(const UniDev* __restrict__ U, UniCtl* ctl, RoundInfo* info, int warp_bytes);
@@ -102,10 +113,8 @@ constexpr size_t kSurvSmemPerWarpBase = (size_t)3 * (kMaxF + 1) * 2 * sizeof(dou
 constexpr size_t kSurvSmemPerWarp = kSurvSmemPerWarpBase;
 // k_surv_gen on a batch without knot-stream universes: one axis of alpha / beta
 constexpr size_t kSurvSmemAxis = (size_t)2 * (kMaxF + 1) * sizeof(double);
-// k_confirm64w adds the FP64 trajectory of a 1+1D candidate
-constexpr size_t kConfSmemPerWarp = kSurvSmemPerWarpBase + (size_t)kMaxF * sizeof(double);
-// k_retest adds the candidate's term-ordered coefficient rows
+// k_retest: the candidate's term-ordered coefficient rows and its phases
 constexpr int kRowK = kseq_len_max();
-constexpr size_t kRetestSmem = kSurvSmemPerWarpBase + (size_t)3 * kRowK * sizeof(double);
+constexpr size_t kRetestSmem = (size_t)3 * (kRowK + kMaxF) * sizeof(double);
 
 }  // namespace ug

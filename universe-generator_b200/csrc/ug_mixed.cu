@@ -455,19 +455,7 @@ __global__ void __launch_bounds__(kMxThreads, 1) k_prefilter_mixed(const UniDev*
         }
         const bool valid = off < B;
         const uint64_t idx = (uint64_t)(base + off);
-        if (!d.mx_ok) {  // not eligible for the tensor-core path: everything to the FP64 test
-            if (part == 0 && !dump) {
-                const uint32_t g = __ballot_sync(0xffffffffu, valid);
-                int at = 0;
-                if (lane == 0) {
-                    d.surv_bits[UG_IDX(off >> 5, d.B_max / 32)] = 0u;
-                    at = atomicAdd(&info->total_gray, __popc(g));
-                }
-                at = __shfl_sync(0xffffffffu, at, 0) + __popc(g & ((1u << lane) - 1u));
-                if (valid) rq.item[UG_IDX(at, rq.cap)] = make_int2(u, off);
-            }
-            continue;
-        }
+        if (!d.mx_ok) continue;  // not eligible for the tensor-core path: k_test64 takes the universe
         const int dim = d.dim, T = d.T, nch = d.mx_chunks, tpad = d.mx_tpad, nm = d.mx_nmma;
         const uint32_t bchunk = (uint32_t)tpad * kKC * 2 * 2;  // hi + lo images
         const float r = (float)d.cell, mrg = d.mx_margin, inv_cell = (float)(1.0 / d.cell);
