@@ -660,17 +660,15 @@ void h_comov(const std::vector<double>& a2, const std::vector<double>& a, const 
     *VY = (dd[1] * s - xx[1] * c) / (s * s);
 }
 
+// A call's device buffers: from its batch's cache (kept there for the next call), or its own.
 struct DevBuf {
-    std::vector<void*> p;
-    ~DevBuf() {
-        for (void* q : p) cudaFree(q);
-    }
+    CallBuffers own;
+    CallBuffers& buf;
+    DevBuf() : buf(own) {}
+    explicit DevBuf(CallBuffers& cache) : buf(cache) {}
     template <class T>
     T* get(size_t n) {
-        void* q = nullptr;
-        if (cudaMalloc(&q, std::max<size_t>(n, 1) * sizeof(T)) != cudaSuccess) return nullptr;
-        p.push_back(q);
-        return (T*)q;
+        return (T*)buf.get(std::max<size_t>(n, 1) * sizeof(T));
     }
 };
 
@@ -738,8 +736,8 @@ int check_cfg(const ug_frames_cfg* cfg, ug_frames_out* out, int n) {
 // one only counts and densities do, and no step waits for the host.
 int bake_device(const ug_frames_cfg* cfg, int n, int nw, int bMax, const double* dA2, const double* dA,
                 const double* dB, const double* dF, const std::vector<ObsPath>& obs, ug_frames_out* out,
-                cudaStream_t st) {
-    DevBuf buf;
+                cudaStream_t st, CallBuffers& cache) {
+    DevBuf buf(cache);
     int dev = 0, nsm = 148;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
@@ -770,6 +768,24 @@ int bake_device(const ug_frames_cfg* cfg, int n, int nw, int bMax, const double*
     if (!dS0 || !dC || !dZg || !dChig || !dBasis || !dReach || !dAmp || !dPx || !dPy || !dHits || !dCross || !dCount || (want_density && !dDen))
         return set_error(UG_ENOMEM, "frame_bake: device allocation failed");
     cudaMemsetAsync(dAmp, 0, (size_t)n * 8, st);
+    // without hits no step waits for the host: the densities of finished frames are copied
+    // on a second stream while the next ones are baked, into pages backed meanwhile
+    const bool copies = want_density && !want_hits;
+    const int group = (NF + 63) / 64;  // frames per copy
+    struct Copies {
+        cudaStream_t st = nullptr;
+        std::vector<cudaEvent_t> ev;
+        ~Copies() {
+            for (cudaEvent_t e : ev) cudaEventDestroy(e);
+            if (st) cudaStreamDestroy(st);
+        }
+    } cp;
+    PagesAhead pages;
+    if (copies) {
+        if (cudaStreamCreateWithFlags(&cp.st, cudaStreamNonBlocking) != cudaSuccess)
+            return set_error(UG_ECUDA, "frame_bake: stream creation failed");
+        pages.add(out->density, bins2 * NF * NO * 4);
+    }
     if (horner) cudaMemsetAsync(dC, 0, (size_t)n * 2 * (bMax + 1) * sizeof(double2), st);
     k_fb_prep<<<(int)std::min<int64_t>(((int64_t)n * 2 + 3) / 4, nsm * 64), 128, 0, st>>>(n, nw, bMax, horner, dA, dB,
                                                                                         dF, dS0, dC, dAmp);
@@ -894,7 +910,24 @@ int bake_device(const ug_frames_cfg* cfg, int n, int nw, int bMax, const double*
                 written += (int64_t)nh;
             }
         }
+        if (copies && ((fi + 1) % group == 0 || fi + 1 == NF)) {
+            cudaEvent_t ev = nullptr;
+            if (cudaEventCreateWithFlags(&ev, cudaEventDisableTiming) != cudaSuccess)
+                return set_error(UG_ECUDA, "frame_bake: event creation failed");
+            cp.ev.push_back(ev);
+            cudaEventRecord(ev, st);
+        }
     }
+    pages.wait();
+    for (size_t k = 0; k < cp.ev.size(); k++) {
+        const size_t all = bins2 * NO * NF, part = bins2 * NO * group, at = part * k;
+        if (cudaStreamWaitEvent(cp.st, cp.ev[k], 0) != cudaSuccess ||
+            cudaMemcpyAsync(out->density + at, dDen + at, std::min(part, all - at) * 4, cudaMemcpyDeviceToHost, cp.st) !=
+                cudaSuccess)
+            return set_error(UG_ECUDA, "frame_bake: density copy failed");
+    }
+    if (copies && cudaStreamSynchronize(cp.st) != cudaSuccess)
+        return set_error(UG_ECUDA, "frame_bake: density copy failed");
     const cudaError_t e = cudaStreamSynchronize(st);
     if (e != cudaSuccess) {
         std::string m = std::string("frame_bake: ") + cudaGetErrorString(e);
@@ -910,10 +943,6 @@ int bake_device(const ug_frames_cfg* cfg, int n, int nw, int bMax, const double*
             if (out->hit_count) out->hit_count[i] = (int64_t)counts[i];
             out->hits_total += (int64_t)counts[i];
         }
-        if (want_density && (cudaMemcpyAsync(out->density, dDen, bins2 * NF * NO * 4, cudaMemcpyDeviceToHost, st) !=
-                                 cudaSuccess ||
-                             cudaStreamSynchronize(st) != cudaSuccess))
-            return set_error(UG_ECUDA, "frame_bake: density copy failed");
     }
     if (want_hits && out->hits_total > out->hit_cap) return set_error(UG_ECAP, "frame_bake: hit buffer too small");
     return UG_OK;
@@ -929,9 +958,9 @@ __global__ void k_fb_maxb(int64_t m, const int32_t* b, int* out) {
 }
 
 // Largest frequency of device-resident dump parameters.
-int max_b_device(const int32_t* b, int64_t m, int* out, cudaStream_t st) {
-    int* d = nullptr;
-    if (cudaMalloc(&d, 4) != cudaSuccess) return set_error(UG_ENOMEM, "frame_bake: device allocation failed");
+int max_b_device(const int32_t* b, int64_t m, int* out, cudaStream_t st, CallBuffers& buf) {
+    int* d = (int*)buf.get(4);
+    if (!d) return set_error(UG_ENOMEM, "frame_bake: device allocation failed");
     int dev = 0, nsm = 148;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
@@ -939,17 +968,16 @@ int max_b_device(const int32_t* b, int64_t m, int* out, cudaStream_t st) {
     k_fb_maxb<<<nsm * 4, 256, 0, st>>>(m, b, d);
     cudaError_t e = cudaMemcpyAsync(out, d, 4, cudaMemcpyDeviceToHost, st);
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-    cudaFree(d);
     return e == cudaSuccess ? UG_OK : set_error(UG_ECUDA, "frame_bake: reduction failed");
 }
 
 // Frames of the accepted paths of a packer universe, straight from the device
 // (the dump -> frame_bake pipeline without a CSV or host round trip).
 int frames_from_params(const ug_frames_cfg* cfg, int n, int nw, int bMax, const double* dA2, const double* dA,
-                       const int32_t* dBi, const double* dF, ug_frames_out* out, cudaStream_t st) {
+                       const int32_t* dBi, const double* dF, ug_frames_out* out, cudaStream_t st, CallBuffers& cache) {
     int rc = check_cfg(cfg, out, n);
     if (rc) return rc;
-    DevBuf buf;
+    DevBuf buf(cache);
     double* dB = buf.get<double>((size_t)n * 2 * nw);
     if (!dB) return set_error(UG_ENOMEM, "frame_bake: device allocation failed");
     int dev = 0, nsm = 148;
@@ -974,7 +1002,7 @@ int frames_from_params(const ug_frames_cfg* cfg, int n, int nw, int bMax, const 
             return set_error(UG_ECUDA, "frame_bake: observer copy failed");
         for (int j = 0; j < 2 * nw; j++) q.b[j] = bi[j];
     }
-    return bake_device(cfg, n, nw, bMax, dA2, dA, dB, dF, obs, out, st);
+    return bake_device(cfg, n, nw, bMax, dA2, dA, dB, dF, obs, out, st, cache);
 }
 
 }  // namespace ug
@@ -1016,7 +1044,7 @@ extern "C" int ug_frame_bake(const ug_frames_cfg* cfg, int32_t n, int32_t nw, co
         obs[o].b.assign(b + p * 2 * nw, b + (p + 1) * 2 * nw);
         obs[o].f.assign(f + p * 2 * nw, f + (p + 1) * 2 * nw);
     }
-    return bake_device(cfg, n, nw, bMax, dA2, dA, dB, dF, obs, out, st);
+    return bake_device(cfg, n, nw, bMax, dA2, dA, dB, dF, obs, out, st, buf.buf);
 }
 
 // ------------------------------------------------------- observer view remap

@@ -17,6 +17,7 @@
 #include <vector>
 
 #include "../../include/ug.h"
+#include "ug_buffers.cuh"
 #include "ug_frames.cuh"
 #include "ug_kernels.cuh"
 #include "ug_mixed.cuh"
@@ -59,14 +60,16 @@ static const char* kKernelNames[12] = {"k_plan",      "k_prefilter64w", "k_prefi
 struct UniHost {
     ug_universe_cfg cfg;
     UniDev d;
-    std::vector<void*> owned;  // fixed-size allocations
     int64_t dense_bytes = 0;
     int64_t hcap = 0;
+    bool points_fixed = false, hash_fixed = false;  // in the arena: as large as they can get
     int64_t occ_words = 0, occ1_words = 0;
     MixedTables mt;            // tensor-core operand tables (mixed precision)
 };
 
 struct Batch {
+    Arena arena;         // fixed buffers
+    CallBuffers call;    // buffers of read-back and frame calls
     int dev = 0;
     cudaStream_t st = nullptr;
     bool own_stream = false;
@@ -84,6 +87,7 @@ struct Batch {
     RetestQueue rq{};         // mixed form: undecided candidates of a round
     cudaGraphExec_t gexec = nullptr;
     int graph_rounds = 0;
+    int64_t replays = 0;
     cudaEvent_t ev[2 * K_NK]{};
     double kms[K_NK]{};
     int64_t klaunch[K_NK]{};
@@ -125,12 +129,11 @@ static int64_t pow2_at_least(int64_t v) {
 }
 
 template <class T>
-static int dalloc(UniHost& h, T** p, size_t n, int fill = -2) {
+static int dalloc(Batch& B, T** p, size_t n, int fill = -2) {
     void* q = nullptr;
     if (n == 0) n = 1;
-    CKR(cudaMalloc(&q, n * sizeof(T)));
+    CKR(B.arena.take(n * sizeof(T), &q));
     if (fill != -2) CKR(cudaMemset(q, fill, n * sizeof(T)));
-    h.owned.push_back(q);
     *p = (T*)q;
     return UG_OK;
 }
@@ -183,30 +186,58 @@ static void host_tables(const ug_universe_cfg& c, std::vector<double>& S, std::v
     });
 }
 
-static int alloc_points(UniHost& h, int64_t cap) {
+// Admissions a universe can reach at most: one per candidate.
+static int64_t total_budget(const ug_universe_cfg& c) {
+    return c.attempts + (c.group_mode == UG_GROUP_SUBPATH ? (c.sub_attempts ? c.sub_attempts : c.attempts) : 0);
+}
+// Capacities that `rounds` more rounds may need: accepted paths, and hash keys.
+static int64_t slots_ahead(const UniHost& h, int64_t n_slots, int rounds) {
+    const int64_t more = std::max<int64_t>(h.d.S_max, (int64_t)rounds * h.d.S_max / 4);
+    return std::min(n_slots + more, total_budget(h.cfg) + 1);
+}
+static int64_t keys_ahead(const UniHost& h, int64_t n_slots, int64_t used, int rounds) {
+    const int64_t more = std::min<int64_t>((int64_t)rounds * h.d.S_max, std::max<int64_t>(0, total_budget(h.cfg) - n_slots));
+    return used + more * h.cfg.T;
+}
+
+// Buffers that may grow are allocated on their own; one that holds all a universe can
+// reach comes from the batch's arena.
+static int alloc_points(Batch& B, UniHost& h, int64_t cap) {
     const int T = h.cfg.T;
-    Pt64* p = nullptr;
-    Pt32* f = nullptr;
-    int64_t* ai = nullptr;
-    CKR(cudaMalloc(&p, (size_t)cap * T * sizeof(Pt64)));
-    CKR(cudaMalloc(&f, (size_t)cap * T * sizeof(Pt32)));
-    CKR(cudaMalloc(&ai, (size_t)cap * sizeof(int64_t)));
-    h.d.pts = p;
-    h.d.ptf = f;
-    h.d.acc_idx = ai;
+    const bool fixed = cap > total_budget(h.cfg);
+    void *p = nullptr, *f = nullptr, *ai = nullptr;
+    auto take = [&](size_t n, void** q) { return fixed ? B.arena.take(n, q) : cudaMalloc(q, n); };
+    CKR(take((size_t)cap * T * sizeof(Pt64), &p));
+    CKR(take((size_t)cap * T * sizeof(Pt32), &f));
+    CKR(take((size_t)cap * sizeof(int64_t), &ai));
+    h.d.pts = (Pt64*)p;
+    h.d.ptf = (Pt32*)f;
+    h.d.acc_idx = (int64_t*)ai;
     h.d.slot_cap = cap;
+    h.points_fixed = fixed;
     return UG_OK;
+}
+static void free_points(const UniHost& h) {
+    if (h.points_fixed) return;
+    cudaFree(h.d.pts);
+    cudaFree(h.d.ptf);
+    cudaFree(h.d.acc_idx);
 }
 
 // Hash grid of cap slots, all empty (key and head all ones: no key, head -1).
-static int alloc_hash(UniHost& h, int64_t cap) {
-    ulonglong2* s = nullptr;
-    CKR(cudaMalloc(&s, (size_t)cap * sizeof(ulonglong2)));
-    CKR(cudaMemset(s, 0xff, (size_t)cap * sizeof(ulonglong2)));
-    h.d.hslot = s;
+static int alloc_hash(Batch& B, UniHost& h, int64_t cap) {
+    const bool fixed = keys_ahead(h, 0, 0, INT32_MAX / kSmaxCap) * 2 <= cap;
+    void* q = nullptr;
+    CKR(fixed ? B.arena.take((size_t)cap * sizeof(ulonglong2), &q) : cudaMalloc(&q, (size_t)cap * sizeof(ulonglong2)));
+    CKR(cudaMemset(q, 0xff, (size_t)cap * sizeof(ulonglong2)));
+    h.d.hslot = (ulonglong2*)q;
     h.d.hmask = (uint64_t)(cap - 1);
     h.hcap = cap;
+    h.hash_fixed = fixed;
     return UG_OK;
+}
+static void free_hash(const UniHost& h) {
+    if (h.d.grid_kind == GRID_HASH && !h.hash_fixed) cudaFree(h.d.hslot);
 }
 
 static int setup_universe(Batch& B, UniHost& h, int64_t dense_budget, int64_t* dense_used) {
@@ -266,8 +297,8 @@ static int setup_universe(Batch& B, UniHost& h, int64_t dense_budget, int64_t* d
     double *dS, *dC, *dI;
     int32_t* dO;
     int rc;
-    if ((rc = dalloc(h, &dS, S.size())) || (rc = dalloc(h, &dC, Cm.size())) ||
-        (rc = dalloc(h, &dI, inv.size())) || (rc = dalloc(h, &dO, order.size())))
+    if ((rc = dalloc(B, &dS, S.size())) || (rc = dalloc(B, &dC, Cm.size())) ||
+        (rc = dalloc(B, &dI, inv.size())) || (rc = dalloc(B, &dO, order.size())))
         return rc;
     CKR(cudaMemcpy(dS, S.data(), S.size() * 8, cudaMemcpyHostToDevice));
     CKR(cudaMemcpy(dC, Cm.data(), Cm.size() * 8, cudaMemcpyHostToDevice));
@@ -293,8 +324,8 @@ static int setup_universe(Batch& B, UniHost& h, int64_t dense_budget, int64_t* d
             }
         }
         double* dK;
-        if ((rc = dalloc(h, &dK, kt.size())) || (rc = dalloc(h, &d.coef, (size_t)d.K * d.Rpad, 0)) ||
-            (rc = dalloc(h, &d.a2row, (size_t)d.Rpad, 0)))
+        if ((rc = dalloc(B, &dK, kt.size())) || (rc = dalloc(B, &d.coef, (size_t)d.K * d.Rpad, 0)) ||
+            (rc = dalloc(B, &d.a2row, (size_t)d.Rpad, 0)))
             return rc;
         CKR(cudaMemcpy(dK, kt.data(), kt.size() * 8, cudaMemcpyHostToDevice));
         d.KT = dK;
@@ -305,14 +336,15 @@ static int setup_universe(Batch& B, UniHost& h, int64_t dense_budget, int64_t* d
     const int64_t dense = (int64_t)T * cpt * 4;
     if (!B.opts.force_hash && dense <= (int64_t)4 << 30 && *dense_used + dense <= dense_budget) {
         d.grid_kind = GRID_DENSE;
-        if ((rc = dalloc(h, &d.heads, (size_t)T * cpt, 0xff))) return rc;
+        if ((rc = dalloc(B, &d.heads, (size_t)T * cpt, 0xff))) return rc;
         d.dense_cells = (int64_t)T * cpt;
         h.dense_bytes = dense;
         *dense_used += dense;
     } else {
         d.grid_kind = GRID_HASH;
-        if ((rc = alloc_hash(h, pow2_at_least(std::max<int64_t>(1 << 16, 4LL * d.S_max * T)))))
-            return rc;
+        // what the first replay may fill, at a load of 1/4 (grown at 1/2)
+        const int64_t keys = std::max<int64_t>(1 << 14, keys_ahead(h, 0, 0, B.opts.rounds_per_sync));
+        if ((rc = alloc_hash(B, h, pow2_at_least(4 * keys)))) return rc;
     }
     // occupancy bitmap, coarsened until it is at most 512 MiB (T <= 256 in 3D
     // keeps 2 cells per coarse cell per axis or finer)
@@ -349,7 +381,7 @@ static int setup_universe(Batch& B, UniHost& h, int64_t dense_budget, int64_t* d
         // keys the coarse cells too (one probe per occupied coarse cell instead of
         // one per window cell in it), with the cells' occupancy mask in the slot.
         d.gkey_shift = (d.grid_kind == GRID_HASH && c.dim >= 2 && sh * c.dim <= 5) ? sh : 0;
-        if ((rc = dalloc(h, &d.occ, (size_t)h.occ_words, 0))) return rc;
+        if ((rc = dalloc(B, &d.occ, (size_t)h.occ_words, 0))) return rc;
         // the finest blocks within 16 MiB (2^27 bits): commits mark it at random and
         // every test reads it, so a small map that stays in L2 pays more than fine
         // blocks (c3 job: 2^27 bits 513 ms, 2^29 515 ms, 2^32 541 ms).  The FP64
@@ -366,20 +398,19 @@ static int setup_universe(Batch& B, UniHost& h, int64_t dense_budget, int64_t* d
         d.occ1_per_t = per1;
         h.occ1_words = ((int64_t)T * per1 + 31) / 32;
         d.occ1_words = h.occ1_words;
-        if ((rc = dalloc(h, &d.occ1, (size_t)h.occ1_words, 0))) return rc;
+        if ((rc = dalloc(B, &d.occ1, (size_t)h.occ1_words, 0))) return rc;
     }
     // accepted points
-    const int64_t total_budget =
-        c.attempts + (c.group_mode == UG_GROUP_SUBPATH ? (c.sub_attempts ? c.sub_attempts : c.attempts) : 0);
-    int64_t cap = B.opts.slot_hint > 0 ? B.opts.slot_hint : 8192;
-    cap = std::max<int64_t>(std::min<int64_t>(cap, total_budget + 1), 1024);
-    if ((rc = alloc_points(h, cap))) return rc;
+    int64_t cap = B.opts.slot_hint > 0 ? B.opts.slot_hint
+                                       : std::max<int64_t>(8192, slots_ahead(h, 0, B.opts.rounds_per_sync));
+    cap = std::max<int64_t>(std::min<int64_t>(cap, total_budget(c) + 1), 1024);
+    if ((rc = alloc_points(B, h, cap))) return rc;
     // round buffers
     const int Bm = d.B_max, Sm = d.S_max;
-    if ((rc = dalloc(h, &d.surv_bits, Bm / 32, 0)) ||         (rc = dalloc(h, &d.g0, Bm, 0xff)) || (rc = dalloc(h, &d.surv_off, Sm + 1, 0)) ||
-        (rc = dalloc(h, &d.spos, (size_t)Sm * T, 0)) || (rc = dalloc(h, &d.ccount, Sm, 0)) ||
-        (rc = dalloc(h, &d.clist, (size_t)Sm * kConflictCap, 0)) ||
-        (rc = dalloc(h, &d.sgid, Sm, 0xff)) || (rc = dalloc(h, &d.acc_rank, Sm, 0xff)))
+    if ((rc = dalloc(B, &d.surv_bits, Bm / 32, 0)) ||         (rc = dalloc(B, &d.g0, Bm, 0xff)) || (rc = dalloc(B, &d.surv_off, Sm + 1, 0)) ||
+        (rc = dalloc(B, &d.spos, (size_t)Sm * T, 0)) || (rc = dalloc(B, &d.ccount, Sm, 0)) ||
+        (rc = dalloc(B, &d.clist, (size_t)Sm * kConflictCap, 0)) ||
+        (rc = dalloc(B, &d.sgid, Sm, 0xff)) || (rc = dalloc(B, &d.acc_rank, Sm, 0xff)))
         return rc;
     // Round table: one 8-byte head per (timestep, block), at most 2^25 entries (the
     // block grows past the cost model's choice if needed).
@@ -389,7 +420,7 @@ static int setup_universe(Batch& B, UniHost& h, int64_t dense_budget, int64_t* d
         for (int ax = 0; ax < c.dim; ax++) d.rblocks *= g;
         if ((int64_t)T * d.rblocks <= ((int64_t)1 << 25) || d.rblock_shift >= 6) break;
     }
-    if ((rc = dalloc(h, &d.rhead, (size_t)T * d.rblocks, 0xff))) return rc;
+    if ((rc = dalloc(B, &d.rhead, (size_t)T * d.rblocks, 0xff))) return rc;
     return UG_OK;
 }
 
@@ -550,23 +581,19 @@ static int ensure_capacity(Batch& B, int rounds) {
         UniCtl& k = B.hCtl[i];
         if (k.state == ST_ERROR) return fail(UG_ECAP, "universe %d: device error %d", i, k.err_code);
         if (k.state == ST_DONE) continue;
-        const int64_t need = k.n_slots + std::max<int64_t>(h.d.S_max, (int64_t)rounds * h.d.S_max / 4);
+        const int64_t need = slots_ahead(h, k.n_slots, rounds);
         if (need > h.d.slot_cap || k.state == ST_GROW) {
             int64_t ncap = std::max<int64_t>(h.d.slot_cap * 2, need);
             const int T = h.cfg.T;
-            Pt64* op = h.d.pts;
-            Pt32* of = h.d.ptf;
-            int64_t* oi = h.d.acc_idx;
+            const UniHost old = h;
             const int64_t n = k.n_slots;
-            int rc = alloc_points(h, ncap);
+            int rc = alloc_points(B, h, ncap);
             if (rc) return rc;
-            CKR(cudaMemcpyAsync(h.d.pts, op, (size_t)n * T * sizeof(Pt64), cudaMemcpyDeviceToDevice, B.st));
-            CKR(cudaMemcpyAsync(h.d.ptf, of, (size_t)n * T * sizeof(Pt32), cudaMemcpyDeviceToDevice, B.st));
-            CKR(cudaMemcpyAsync(h.d.acc_idx, oi, (size_t)n * sizeof(int64_t), cudaMemcpyDeviceToDevice, B.st));
+            CKR(cudaMemcpyAsync(h.d.pts, old.d.pts, (size_t)n * T * sizeof(Pt64), cudaMemcpyDeviceToDevice, B.st));
+            CKR(cudaMemcpyAsync(h.d.ptf, old.d.ptf, (size_t)n * T * sizeof(Pt32), cudaMemcpyDeviceToDevice, B.st));
+            CKR(cudaMemcpyAsync(h.d.acc_idx, old.d.acc_idx, (size_t)n * sizeof(int64_t), cudaMemcpyDeviceToDevice, B.st));
             CKR(cudaStreamSynchronize(B.st));
-            cudaFree(op);
-            cudaFree(of);
-            cudaFree(oi);
+            free_points(old);
             if (k.state == ST_GROW) {
                 k.state = ST_ACTIVE;
                 CKR(cudaMemcpyAsync(&B.dCtl[i].state, &k.state, sizeof(int32_t), cudaMemcpyHostToDevice, B.st));
@@ -574,12 +601,12 @@ static int ensure_capacity(Batch& B, int rounds) {
             changed = true;
         }
         if (h.d.grid_kind == GRID_HASH) {
-            const int64_t need_keys = k.hash_used + (int64_t)rounds * h.d.S_max * h.cfg.T;
+            const int64_t need_keys = keys_ahead(h, k.n_slots, k.hash_used, rounds);
             if (need_keys * 2 > h.hcap) {
-                ulonglong2* os = h.d.hslot;
-                int rc = alloc_hash(h, pow2_at_least(need_keys * 4));
+                const UniHost old = h;
+                int rc = alloc_hash(B, h, pow2_at_least(need_keys * 4));
                 if (rc) return rc;
-                cudaFree(os);
+                free_hash(old);
                 int64_t zero = 0;
                 k.hash_used = 0;
                 CKR(cudaMemcpyAsync(&B.dCtl[i].hash_used, &zero, sizeof zero, cudaMemcpyHostToDevice, B.st));
@@ -717,9 +744,7 @@ int ug_batch_create(const ug_universe_cfg* cfgs, int32_t n, const ug_run_opts* o
         if (cfgs[i].euclid) B->any_euclid = true;
         if (cfgs[i].rng == UG_RNG_KNOT) B->any_knot = true;
     }
-    if (cudaMalloc(&B->dU, sizeof(UniDev) * n) != cudaSuccess ||
-        cudaMalloc(&B->dCtl, sizeof(UniCtl) * n) != cudaSuccess ||
-        cudaMalloc(&B->dInfo, sizeof(RoundInfo)) != cudaSuccess)
+    if (dalloc(*B, &B->dU, n) || dalloc(*B, &B->dCtl, n) || dalloc(*B, &B->dInfo, 1))
         return bail(fail(UG_ENOMEM, "control block allocation failed"));
     B->hCtl.resize(n);
     for (int i = 0; i < n; i++) init_ctl(cfgs[i], B->U[i].d, B->hCtl[i]);
@@ -748,10 +773,9 @@ int ug_batch_create(const ug_universe_cfg* cfgs, int32_t n, const ug_run_opts* o
                 B->sc64.coef_stride = std::max(B->sc64.coef_stride,
                                                (size_t)32 * ((size_t)u.d.K * u.d.dim + (u.d.cross1d ? u.d.T : 0)));
         const size_t n = (size_t)B->t64_ctas;
-        if (cudaMalloc(&B->sc64.coef, n * B->sc64.coef_stride * sizeof(double)) != cudaSuccess ||
-            (B->any_knot && (cudaMalloc(&B->sc64.wgt, n * kKnotStride * sizeof(double)) != cudaSuccess ||
-                             cudaMalloc(&B->sc64.phase, n * kKnotStride * sizeof(double)) != cudaSuccess ||
-                             cudaMalloc(&B->sc64.freq, n * kKnotStride * sizeof(uint16_t)) != cudaSuccess)))
+        if (dalloc(*B, &B->sc64.coef, n * B->sc64.coef_stride) ||
+            (B->any_knot && (dalloc(*B, &B->sc64.wgt, n * kKnotStride) || dalloc(*B, &B->sc64.phase, n * kKnotStride) ||
+                             dalloc(*B, &B->sc64.freq, n * kKnotStride))))
             return bail(fail(UG_ENOMEM, "FP64 test scratch allocation failed"));
     }
     if (B->any_mixed) {
@@ -760,8 +784,7 @@ int ug_batch_create(const ug_universe_cfg* cfgs, int32_t n, const ug_run_opts* o
         for (const UniHost& u : B->U) cap += u.d.B_max;
         B->rq.cap = (int32_t)std::min<int64_t>(cap, INT32_MAX);
         B->rq.mask_cap = (int32_t)std::min<int64_t>(cap / 8 + 1, INT32_MAX);
-        if (cudaMalloc(&B->rq.item, sizeof(int2) * (size_t)B->rq.cap) != cudaSuccess ||
-            cudaMalloc(&B->rq.mask, 2 * sizeof(uint4) * (size_t)B->rq.mask_cap) != cudaSuccess)
+        if (dalloc(*B, &B->rq.item, (size_t)B->rq.cap) || dalloc(*B, &B->rq.mask, 2 * (size_t)B->rq.mask_cap))
             return bail(fail(UG_ENOMEM, "retest queue allocation failed"));
     }
     // one wave per SM, measured on c3 against 8 / 8 / 16 CTAs per SM: k_surv_gen 27.7 ->
@@ -772,7 +795,8 @@ int ug_batch_create(const ug_universe_cfg* cfgs, int32_t n, const ug_run_opts* o
                                 kSurvWarps * (B->any_knot ? kSurvSmemPerWarp : kSurvSmemAxis), 8);
     B->res_shash = resident_ctas(k_surv_hash, 256, 0, 8);
     B->res_confl = resident_ctas(k_conflicts, 128, 0, 16);
-    for (int k = 0; k < 2 * K_NK; k++) cudaEventCreate(&B->ev[k]);
+    if (B->opts.kernel_timing)
+        for (int k = 0; k < 2 * K_NK; k++) cudaEventCreate(&B->ev[k]);
     *out = B;
     return UG_OK;
 }
@@ -790,7 +814,9 @@ int ug_batch_run(void* h, int64_t max_rounds) {
         for (const UniCtl& k : B->hCtl) progress_before += k.next_cand + k.n_slots;
         if (max_rounds > 0 && done_rounds >= max_rounds) return UG_OK;
         if ((rc = ensure_capacity(*B, R))) return rc;
-        if (B->opts.use_graph && !B->opts.kernel_timing) {
+        // the graph is built at the second replay: a job that ends with the first would pay
+        // 1.3 ms for 80 launches of 2 us
+        if (B->opts.use_graph && !B->opts.kernel_timing && B->replays++ > 0) {
             if (!B->gexec && (rc = build_graph(*B, R))) return rc;
             B->synced = false;
             CKR(cudaGraphLaunch(B->gexec, B->st));
@@ -955,22 +981,24 @@ int ug_batch_params(void* h, int32_t u, double* a2, double* a, int32_t* b, doubl
     if (N == 0) return UG_OK;
     const UniDev& d = B->U[u].d;
     const int nw = d.nw, D = d.dim;
-    double *da2, *da, *df;
-    int32_t* db;
-    CKR(cudaMalloc(&da2, (size_t)N * D * 8));
-    CKR(cudaMalloc(&da, (size_t)N * D * nw * 8));
-    CKR(cudaMalloc(&df, (size_t)N * D * nw * 8));
-    CKR(cudaMalloc(&db, (size_t)N * D * nw * 4));
+    const size_t nt = (size_t)N * D * nw;
+    PagesAhead pages;
+    pages.add(a, nt * 8);
+    pages.add(f, nt * 8);
+    pages.add(b, nt * 4);
+    CallScope scope{B->call};
+    double* da2 = (double*)B->call.get((size_t)N * D * 8);
+    double* da = (double*)B->call.get(nt * 8);
+    double* df = (double*)B->call.get(nt * 8);
+    int32_t* db = (int32_t*)B->call.get(nt * 4);
+    if (!da2 || !da || !df || !db) return fail(UG_ENOMEM, "params: device allocation failed");
     launch_params(B->dU, u, B->U[u].d.rng, B->U[u].d.dim, N, da2, da, db, df, B->st);
     cudaError_t e = cudaStreamSynchronize(B->st);
+    pages.wait();
     if (e == cudaSuccess && a2) e = cudaMemcpy(a2, da2, (size_t)N * D * 8, cudaMemcpyDeviceToHost);
     if (e == cudaSuccess && a) e = cudaMemcpy(a, da, (size_t)N * D * nw * 8, cudaMemcpyDeviceToHost);
     if (e == cudaSuccess && f) e = cudaMemcpy(f, df, (size_t)N * D * nw * 8, cudaMemcpyDeviceToHost);
     if (e == cudaSuccess && b) e = cudaMemcpy(b, db, (size_t)N * D * nw * 4, cudaMemcpyDeviceToHost);
-    cudaFree(da2);
-    cudaFree(da);
-    cudaFree(df);
-    cudaFree(db);
     if (e != cudaSuccess) return fail(UG_ECUDA, "params: %s", cudaGetErrorString(e));
     return UG_OK;
 }
@@ -985,28 +1013,16 @@ int ug_batch_frames(void* h, int32_t u, const ug_frames_cfg* cfg, ug_frames_out*
     if (N < 1) return fail(UG_EINVAL, "frames: the universe has no accepted paths");
     if (N > INT32_MAX / 2) return fail(UG_ECAP, "frames: too many paths");
     const int nw = B->U[u].d.nw;
-    double *da2 = nullptr, *da = nullptr, *df = nullptr;
-    int32_t* db = nullptr;
-    auto release = [&]() {
-        cudaFree(da2);
-        cudaFree(da);
-        cudaFree(df);
-        cudaFree(db);
-    };
-    if (cudaMalloc(&da2, (size_t)N * 2 * 8) != cudaSuccess || cudaMalloc(&da, (size_t)N * 2 * nw * 8) != cudaSuccess ||
-        cudaMalloc(&df, (size_t)N * 2 * nw * 8) != cudaSuccess || cudaMalloc(&db, (size_t)N * 2 * nw * 4) != cudaSuccess) {
-        release();
-        return fail(UG_ENOMEM, "frames: device allocation failed");
-    }
+    CallScope scope{B->call};
+    double* da2 = (double*)B->call.get((size_t)N * 2 * 8);
+    double* da = (double*)B->call.get((size_t)N * 2 * nw * 8);
+    double* df = (double*)B->call.get((size_t)N * 2 * nw * 8);
+    int32_t* db = (int32_t*)B->call.get((size_t)N * 2 * nw * 4);
+    if (!da2 || !da || !df || !db) return fail(UG_ENOMEM, "frames: device allocation failed");
     launch_params(B->dU, u, B->U[u].d.rng, B->U[u].d.dim, N, da2, da, db, df, B->st);
     int bMax = 2;
-    if (cudaStreamSynchronize(B->st) != cudaSuccess || (rc = max_b_device(db, N * 2 * nw, &bMax, B->st))) {
-        release();
-        return rc ? rc : fail(UG_ECUDA, "frames: parameter kernel failed");
-    }
-    rc = frames_from_params(cfg, (int)N, nw, bMax, da2, da, db, df, out, B->st);
-    release();
-    return rc;
+    if ((rc = max_b_device(db, N * 2 * nw, &bMax, B->st, B->call))) return rc;
+    return frames_from_params(cfg, (int)N, nw, bMax, da2, da, db, df, out, B->st, B->call);
 }
 
 int ug_batch_probe(void* h, int32_t u, uint64_t seed, int64_t n, int32_t bins, int64_t* proposed,
@@ -1107,8 +1123,8 @@ int ug_batch_restore(void* h, int32_t u, int64_t n, const int64_t* idx, const in
         const int64_t need = std::max<int64_t>(1 << 16, pow2_at_least((n * T + (int64_t)d.S_max * T) * 4));
         if (need > U.hcap) {
             CKR(cudaStreamSynchronize(B->st));
-            cudaFree(d.hslot);
-            if ((rc = alloc_hash(U, need))) return rc;
+            free_hash(U);
+            if ((rc = alloc_hash(*B, U, need))) return rc;
         } else {
             CKR(cudaMemsetAsync(d.hslot, 0xff, (size_t)U.hcap * sizeof(ulonglong2), B->st));
         }
@@ -1119,10 +1135,8 @@ int ug_batch_restore(void* h, int32_t u, int64_t n, const int64_t* idx, const in
     // room for the admissions and the next rounds
     if (n + (int64_t)d.S_max * 2 > d.slot_cap) {
         CKR(cudaStreamSynchronize(B->st));
-        cudaFree(d.pts);
-        cudaFree(d.ptf);
-        cudaFree(d.acc_idx);
-        if ((rc = alloc_points(U, n + (int64_t)d.S_max * 2))) return rc;
+        free_points(U);
+        if ((rc = alloc_points(*B, U, n + (int64_t)d.S_max * 2))) return rc;
     }
     if ((rc = push_unidev(*B))) return rc;
     // rebuild control block: k_commit reads these and accumulates hash keys and cells
@@ -1240,25 +1254,13 @@ int ug_batch_destroy(void* h) {
     if (B->st) cudaStreamSynchronize(B->st);
     if (B->gexec) cudaGraphExecDestroy(B->gexec);
     for (UniHost& u : B->U) {
-        for (void* p : u.owned) cudaFree(p);
-        if (u.d.grid_kind == GRID_HASH) cudaFree(u.d.hslot);
-        cudaFree(u.d.pts);
-        cudaFree(u.d.ptf);
-        cudaFree(u.d.acc_idx);
+        free_hash(u);
+        free_points(u);
         mixed_free(u.mt);
     }
-    cudaFree(B->sc64.coef);
-    cudaFree(B->sc64.wgt);
-    cudaFree(B->sc64.phase);
-    cudaFree(B->sc64.freq);
-    cudaFree(B->rq.item);
-    cudaFree(B->rq.mask);
-    cudaFree(B->dU);
-    cudaFree(B->dCtl);
     cudaFree(B->d_gather_idx);
     cudaFree(B->d_gather_gid);
     cudaFree(B->d_gather_off);
-    cudaFree(B->dInfo);
     for (int k = 0; k < 2 * K_NK; k++)
         if (B->ev[k]) cudaEventDestroy(B->ev[k]);
     if (B->own_stream && B->st) cudaStreamDestroy(B->st);
