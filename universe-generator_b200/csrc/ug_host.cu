@@ -963,11 +963,18 @@ int ug_batch_positions(void* h, int32_t u, double* pos, int64_t cap_paths) {
     const int64_t N = B->hCtl[u].n_slots;
     if (cap_paths < N) return fail(UG_ECAP, "positions buffer too small");
     const UniDev& d = B->U[u].d;
-    std::vector<Pt64> tmp((size_t)N * d.T);
-    if (N) CKR(cudaMemcpy(tmp.data(), d.pts, tmp.size() * sizeof(Pt64), cudaMemcpyDeviceToHost));
-    for (int64_t i = 0; i < N; i++)
-        for (int ax = 0; ax < d.dim; ax++)
-            for (int t = 0; t < d.T; t++) pos[(i * d.dim + ax) * d.T + t] = tmp[(size_t)i * d.T + t].c[ax];
+    if (N == 0) return UG_OK;
+    const size_t m = (size_t)N * d.dim * d.T;
+    PagesAhead pages;
+    pages.add(pos, m * sizeof(double));
+    CallScope scope{B->call};
+    double* dp = (double*)B->call.get(m * sizeof(double));
+    if (!dp) return fail(UG_ENOMEM, "positions: device allocation failed");
+    k_positions<<<(int)std::min<int64_t>((N * d.T + 255) / 256, (int64_t)B->nsm * 16), 256, 0, B->st>>>(B->dU, u, N, dp);
+    CKR(cudaGetLastError());
+    pages.wait();
+    CKR(cudaMemcpyAsync(pos, dp, m * sizeof(double), cudaMemcpyDeviceToHost, B->st));
+    CKR(cudaStreamSynchronize(B->st));
     return UG_OK;
 }
 

@@ -92,6 +92,7 @@ __global__ void k_conflicts(const UniDev* __restrict__ U, UniCtl* ctl, RoundInfo
 __global__ void k_greedy(const UniDev* __restrict__ U, UniCtl* ctl, RoundInfo* info);
 __global__ void k_commit(const UniDev* __restrict__ U, UniCtl* ctl, RoundInfo* info);
 __global__ void k_rehash(const UniDev* __restrict__ U, UniCtl* ctl, int u, int64_t n_slots);
+__global__ void k_positions(const UniDev* __restrict__ U, int u, int64_t n, double* __restrict__ out);
 __global__ void k_gather_accepted(const UniDev* __restrict__ U, const int64_t* __restrict__ off,
                                   int64_t* __restrict__ idx, int32_t* __restrict__ gid);
 
