@@ -12,13 +12,16 @@ namespace ug {
 
 // A batch's fixed buffers, carved from chunks: a cudaMalloc and its cudaFree take 0.3 to
 // 0.6 ms together and a universe has about thirty buffers (creating, running and releasing
-// a 20 k candidate job: 6.3 -> 3.7 ms).  Chunks double from 4 to 64 MiB, so that a small
-// universe does not map what it does not need.  Freed with the batch.
+// a 20 k candidate job: 6.3 -> 3.7 ms).  The first chunk is about what the universes
+// take (2 to 64 MiB: a small universe does not map what it does not need), later ones
+// double.  Freed with the batch.
 class Arena {
 public:
     ~Arena() {
         for (void* c : chunks_) cudaFree(c);
     }
+    // Size of the first chunk: about what will be taken.
+    void expect(size_t bytes) { next_ = std::min(kMost, std::max<size_t>((size_t)2 << 20, bytes)); }
     cudaError_t take(size_t bytes, void** out) {
         bytes = (std::max<size_t>(bytes, 1) + 255) / 256 * 256;
         if (bytes > kMost / 4) return chunk(bytes, out);

@@ -403,6 +403,7 @@ static int setup_universe(Batch& B, UniHost& h, int64_t dense_budget, int64_t* d
     // accepted points
     int64_t cap = B.opts.slot_hint > 0 ? B.opts.slot_hint
                                        : std::max<int64_t>(8192, slots_ahead(h, 0, B.opts.rounds_per_sync));
+    if (B.opts.slot_hint <= 0 && total_budget(c) < 2 * cap) cap = total_budget(c) + 1;  // all it can reach
     cap = std::max<int64_t>(std::min<int64_t>(cap, total_budget(c) + 1), 1024);
     if ((rc = alloc_points(B, h, cap))) return rc;
     // round buffers
@@ -732,6 +733,15 @@ int ug_batch_create(const ug_universe_cfg* cfgs, int32_t n, const ug_run_opts* o
     cudaMemGetInfo(&freeb, &totalb);
     const int64_t dense_budget = (int64_t)(freeb * 0.35);
     int64_t dense_used = 0;
+    {  // about what the fixed buffers take: survivors' points, coefficients and lists
+        size_t est = 0;
+        for (int i = 0; i < n; i++) {
+            const size_t sm = std::min<size_t>(cfgs[i].surv_cap ? cfgs[i].surv_cap : cfgs[i].dim == 1 ? 256 : (1 << 20) / cfgs[i].T,
+                                               std::min<size_t>(kSmaxCap, cfgs[i].round_size ? cfgs[i].round_size : 65536));
+            est += sm * ((size_t)cfgs[i].T * (sizeof(Pt64) + 12 * cfgs[i].dim) + 4 * kConflictCap);
+        }
+        B->arena.expect(2 * est);
+    }
     for (int i = 0; i < n; i++) {
         B->U[i].cfg = cfgs[i];
         B->max_T = std::max(B->max_T, cfgs[i].T);
@@ -768,14 +778,18 @@ int ug_batch_create(const ug_universe_cfg* cfgs, int32_t n, const ug_run_opts* o
     if (B->any_fp64) {
         // per resident CTA: coefficients (and trajectories) of 32 candidates of the widest universe
         B->t64_ctas = B->nsm * resident_ctas(k_test64, kT64Threads, 0, 4);
-        for (const UniHost& u : B->U)
+        for (const UniHost& u : B->U) {
+            if (u.d.rng == UG_RNG_KNOT)
+                B->sc64.knot_stride = std::max(B->sc64.knot_stride, (size_t)u.d.nw * 32 * u.d.dim);
             if (!B->any_mixed || !u.d.mx_ok)
                 B->sc64.coef_stride = std::max(B->sc64.coef_stride,
                                                (size_t)32 * ((size_t)u.d.K * u.d.dim + (u.d.cross1d ? u.d.T : 0)));
+        }
         const size_t n = (size_t)B->t64_ctas;
         if (dalloc(*B, &B->sc64.coef, n * B->sc64.coef_stride) ||
-            (B->any_knot && (dalloc(*B, &B->sc64.wgt, n * kKnotStride) || dalloc(*B, &B->sc64.phase, n * kKnotStride) ||
-                             dalloc(*B, &B->sc64.freq, n * kKnotStride))))
+            (B->any_knot && (dalloc(*B, &B->sc64.wgt, n * B->sc64.knot_stride) ||
+                             dalloc(*B, &B->sc64.phase, n * B->sc64.knot_stride) ||
+                             dalloc(*B, &B->sc64.freq, n * B->sc64.knot_stride))))
             return bail(fail(UG_ENOMEM, "FP64 test scratch allocation failed"));
     }
     if (B->any_mixed) {

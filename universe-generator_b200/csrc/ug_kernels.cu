@@ -780,10 +780,10 @@ __device__ __forceinline__ void knot_draws(const UniDev& d, uint64_t idx, int ca
                                            size_t cta, double* a2) {
     Xo r;
     r.seed(knot_seed(d.seed, idx));
-    const int nw = d.nw;
+    const int nw = d.nw, rows = 32 * d.dim;
     uint16_t* p = perm + cand;  // [j][32]
     for (int ax = 0; ax < d.dim; ax++) {
-        const size_t o = cta * kKnotStride + (size_t)(ax * 32 + cand);
+        const size_t o = cta * sc.knot_stride + (size_t)(ax * 32 + cand);
         if ((uint32_t)nw == d.modmax) {
             for (int j = 0; j < nw; j++) p[32 * j] = (uint16_t)(j + 2);
             for (int j = nw - 1; j > 0; j--) {
@@ -804,12 +804,12 @@ __device__ __forceinline__ void knot_draws(const UniDev& d, uint64_t idx, int ca
                 p[32 * j] = (uint16_t)b;
             }
         }
-        for (int j = 0; j < nw; j++) sc.wgt[o + (size_t)j * 96] = 1.0 - r.f64();
+        for (int j = 0; j < nw; j++) sc.wgt[o + (size_t)j * rows] = 1.0 - r.f64();
         for (int j = 0; j < nw; j++) {
             const int b = p[32 * j];
             const bool neg = r.flip();
-            if (!(b & 1)) sc.phase[o + (size_t)j * 96] = r.f64() * kPi;
-            sc.freq[o + (size_t)j * 96] = (uint16_t)(b | (neg ? 0x8000 : 0));
+            if (!(b & 1)) sc.phase[o + (size_t)j * rows] = r.f64() * kPi;
+            sc.freq[o + (size_t)j * rows] = (uint16_t)(b | (neg ? 0x8000 : 0));
         }
         a2[ax * 32 + cand] = d.pin ? 0.0 : (r.f64() * 2.0 - 1.0);
     }
@@ -853,7 +853,7 @@ __global__ void __launch_bounds__(kT64Threads, 2) k_test64(const UniDev* __restr
         // ---- coefficients: G[k][ax * 32 + candidate]
         if (d.rng == RNG_KNOT) {
             const int nw = d.nw;
-            const size_t o = (size_t)blockIdx.x * kKnotStride;
+            const size_t o = (size_t)blockIdx.x * sc.knot_stride;
             if (warp == 0 && lane < nv)
                 knot_draws(d, idx0 + lane, lane, reinterpret_cast<uint16_t*>(s_cells), sc, blockIdx.x, s_a2);
             const bool full = (uint32_t)nw == d.modmax;  // every frequency once
@@ -861,9 +861,8 @@ __global__ void __launch_bounds__(kT64Threads, 2) k_test64(const UniDev* __restr
                 for (int e = tid; e < K * rows; e += kT64Threads) G[e] = 0.0;
             __syncthreads();
             for (int e = tid; e < nw * rows; e += kT64Threads) {
-                const int row = e % rows, j = e / rows;
-                if ((row & 31) < nv) {
-                    double* w = sc.wgt + o + (size_t)j * 96 + row;
+                if ((e % rows & 31) < nv) {
+                    double* w = sc.wgt + o + e;
                     *w = -log(*w);
                 }
             }
@@ -872,7 +871,7 @@ __global__ void __launch_bounds__(kT64Threads, 2) k_test64(const UniDev* __restr
                 const double* w = sc.wgt + o + tid;
                 double sum = 0.0;
 #pragma unroll 4
-                for (int j = 0; j < nw; j++) sum += w[(size_t)j * 96];
+                for (int j = 0; j < nw; j++) sum += w[(size_t)j * rows];
                 s_sum[tid] = sum;
             }
             __syncthreads();
@@ -882,7 +881,7 @@ __global__ void __launch_bounds__(kT64Threads, 2) k_test64(const UniDev* __restr
                 const int row = e % rows, j0 = e / rows;
                 if ((row & 31) >= nv) continue;
                 for (int j = j0; j < j0 + step; j++) {
-                    const size_t at = o + (size_t)j * 96 + row;
+                    const size_t at = o + (size_t)j * rows + row;
                     const int fb = sc.freq[at], b = fb & 0x7fff, k = kseq_s(b);
                     double amp = sc.wgt[at] / s_sum[row] / (double)b;
                     if (fb & 0x8000) amp = -amp;

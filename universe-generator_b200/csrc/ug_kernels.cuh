@@ -67,12 +67,12 @@ constexpr int kT64Threads = 256;
 constexpr int kT64Pos = 32 * 3 * 16;    // positions of a stage
 constexpr int kT64Tests = 32 * 16;      // (candidate, timestep) tests of a stage
 constexpr int kT64Cells = 2048;         // occupied cells of their windows
-constexpr size_t kKnotStride = (size_t)kMaxF * 96;  // [term][axis * 32 + candidate]
 struct Scratch64 {
     double* coef;
     size_t coef_stride;
-    double *wgt, *phase;
+    double *wgt, *phase;  // [term][axis * 32 + candidate]
     uint16_t* freq;
+    size_t knot_stride;
 };
 constexpr int kMaskWords = kMaxF / 32;
 static_assert(kMaskWords == 8, "a mask is two uint4");
