@@ -180,7 +180,7 @@ struct UniCtl {
     int64_t visits;        // prefilter: accepted points examined by the neighbour tests
     int64_t evals_fp64;    // of which evaluated in FP64 (plain path / guard-band retest)
     int32_t stop_at;       // survivors [0, stop_at) resolved this round
-    int32_t tile_ns;       // mixed prefilter: slowest tile of the last round (ns), orders the next round's tiles
+    int32_t tile_ns;       // mixed prefilter: slowest tile of the last round (ns, as a full tile), orders the next round's tiles
     int32_t B_min, B_cap;  // round-size adaptation bounds
     int32_t err_code;
     int32_t tile_cost;     // mixed prefilter: the last tile_ns that was timed

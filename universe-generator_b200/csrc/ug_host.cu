@@ -470,7 +470,7 @@ static int launch_rounds(Batch& B, int rounds, bool timed) {
         const int rc = launch_round(B, timed);
         if (rc) return rc;
     }
-    k_plan<<<1, 256, 0, B.st>>>(B.dU, B.dCtl, B.dInfo);
+    k_plan<<<1, 256, 0, B.st>>>(B.dU, B.dCtl, B.dInfo, B.nsm);
     CKR(cudaGetLastError());
     return UG_OK;
 }
@@ -491,7 +491,7 @@ static int launch_round(Batch& B, bool timed) {
         }
     };
     tb(K_PLAN);
-    k_plan<<<1, 256, 0, B.st>>>(B.dU, B.dCtl, B.dInfo);
+    k_plan<<<1, 256, 0, B.st>>>(B.dU, B.dCtl, B.dInfo, B.nsm);
     te(K_PLAN);
     if (B.opts.precision == UG_PREC_MIXED && B.any_mixed) {
         if (B.any_fp64) {  // universes that the tensor-core test does not take

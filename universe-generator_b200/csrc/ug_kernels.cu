@@ -68,10 +68,17 @@ __device__ __forceinline__ int block_excl_scan256(int v, int* wsum, int* total) 
 
 // The next round of every universe: the last round's windows closed, phases switched, round
 // sizes and tiles.  Planning a planned round again changes nothing.
-__global__ void k_plan(const UniDev* __restrict__ U, UniCtl* ctl, RoundInfo* info) {
+__global__ void k_plan(const UniDev* __restrict__ U, UniCtl* ctl, RoundInfo* info, int nsm) {
     __shared__ int32_t ntiles[kMaxUni];
     __shared__ int32_t cost[kMaxUni];
     __shared__ int32_t order[kMaxUni];
+    __shared__ unsigned long long s_work;
+    __shared__ int32_t s_busy;
+    if (threadIdx.x == 0) {
+        s_work = 0;
+        s_busy = 0;
+    }
+    __syncthreads();
     const int n = info->n_uni;
     for (int u = threadIdx.x; u < n; u += blockDim.x) {
         UniCtl& c = ctl[u];
@@ -135,6 +142,36 @@ __global__ void k_plan(const UniDev* __restrict__ U, UniCtl* ctl, RoundInfo* inf
         c.n_gray = 0;
         if (B > 0) c.epoch = (c.epoch + 1) & 0xFFFFFF;
         ntiles[u] = (B + kTile - 1) / kTile;
+        if (B > 0) {
+            atomicAdd(&s_work, (unsigned long long)cost[u] * ntiles[u]);
+            atomicAdd(&s_busy, 1);
+        }
+    }
+    __syncthreads();
+    // Tiles of the tensor-core test take kTile candidates.  Where one such tile is long
+    // against the round's work per SM, its universe's tiles are cut to 64 or 32: a tile of
+    // 64 takes about two thirds of the time (generation and products do not shrink, the
+    // tests do), one of 32 half, but two to four times the SMs share them.  A universe
+    // alone also cuts the tiles of its last, partial wave.  Per job: four 3+1 universes of
+    // T = 113 to 253 (40 tiles a round on 148 SMs) 18.3 -> 15.0 ms of prefilter, one of
+    // T = 128 (up to 512 tiles) 37.3 -> 35.3 ms.
+    const unsigned long long per_sm = s_work / nsm;
+    for (int u = threadIdx.x; u < n; u += blockDim.x) {
+        const int nt = ntiles[u];
+        int full = nt, rows = kTile;
+        if (nt > 0 && U[u].mx_ok) {
+            if ((unsigned long long)cost[u] >= 2 * per_sm) {
+                full = 0;
+                rows = (unsigned long long)cost[u] >= 4 * per_sm ? 32 : 64;
+            } else if (s_busy == 1 && nt > nsm) {
+                const int rest = nt % nsm;
+                rows = rest * 4 <= nsm ? 32 : (rest * 2 <= nsm ? 64 : kTile);
+                full = rows < kTile ? nt - rest : nt;
+            }
+            if (rows < kTile) ntiles[u] = full + (ctl[u].B - full * kTile + rows - 1) / rows;
+        }
+        info->tile_full[u] = full;
+        info->tile_rows[u] = rows;
     }
     __syncthreads();
     // Tiles are handed out costliest universe first, so the long tiles start in

@@ -25,6 +25,8 @@ struct RoundInfo {
     int32_t total_spt;     // survivor timesteps (k_surv_hash / k_commit items)
     int32_t tile_off[kMaxUni + 1];   // prefilter tiles: first tile of the i-th universe in tile order
     int32_t tile_uni[kMaxUni];       // the universe at position i of the tile order
+    int32_t tile_full[kMaxUni];      // universe u: tiles of kTile candidates, then ...
+    int32_t tile_rows[kMaxUni];      // ... tiles of this many (32, 64 or kTile)
     int32_t surv_off[kMaxUni + 1];
     int32_t surv_off_o[kMaxUni + 1];  // survivor offsets of the universes in tile order
     int32_t sev_off[kMaxUni + 1];
@@ -78,7 +80,7 @@ constexpr int kMaskWords = kMaxF / 32;
 static_assert(kMaskWords == 8, "a mask is two uint4");
 
 // Kernels (ug_kernels.cu)
-__global__ void k_plan(const UniDev* __restrict__ U, UniCtl* ctl, RoundInfo* info);
+__global__ void k_plan(const UniDev* __restrict__ U, UniCtl* ctl, RoundInfo* info, int nsm);
 __global__ void k_test64(const UniDev* __restrict__ U, UniCtl* ctl, RoundInfo* info, Scratch64 sc, int all);
 __global__ void k_retest(const UniDev* __restrict__ U, UniCtl* ctl, RoundInfo* info, RetestQueue rq);
 __global__ void k_compact(const UniDev* __restrict__ U, UniCtl* ctl, RoundInfo* info);

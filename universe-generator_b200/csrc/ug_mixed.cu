@@ -443,7 +443,9 @@ __global__ void __launch_bounds__(kMxThreads, 1) k_prefilter_mixed(const UniDev*
         const UniDev& d = U[u];
         const int lt = dump ? tile : tile - s_toff[pos];
         const uint64_t tile_t0 = tid == 0 ? globaltimer() : 0;
-        const int off = lt * kTile + row;
+        const int full = dump ? INT32_MAX : info->tile_full[u];
+        const int rows = lt < full ? kTile : info->tile_rows[u];  // candidates of this tile
+        const int off = lt < full ? lt * kTile + row : full * kTile + (lt - full) * rows + row;
         int64_t base;
         int B;
         if (dump) {
@@ -453,7 +455,7 @@ __global__ void __launch_bounds__(kMxThreads, 1) k_prefilter_mixed(const UniDev*
             base = ctl[u].round_base;
             B = ctl[u].B;
         }
-        const bool valid = off < B;
+        const bool valid = off < B && row < rows;
         const uint64_t idx = (uint64_t)(base + off);
         if (!d.mx_ok) continue;  // not eligible for the tensor-core path: k_test64 takes the universe
         const int dim = d.dim, T = d.T, nch = d.mx_chunks, tpad = d.mx_tpad, nm = d.mx_nmma;
@@ -978,7 +980,7 @@ __global__ void __launch_bounds__(kMxThreads, 1) k_prefilter_mixed(const UniDev*
             for (int o = 16; o > 0; o >>= 1) nvis += __shfl_xor_sync(0xffffffffu, nvis, o);
             if (lane == 0 && nev) atomicAdd((unsigned long long*)&ctl[u].evals, (unsigned long long)nev);
             if (lane == 0 && nvis) atomicAdd((unsigned long long*)&ctl[u].visits, (unsigned long long)nvis);
-            if (part == 0) {
+            if (part == 0 && (warp & 3) * 32 < rows) {  // a warp per word
                 const bool rej = vrej[row] != 0, gry = vgray[row] != 0;
                 const bool surv = valid && !rej && !gry && !timeout;
                 const bool gr = valid && !rej && (gry || timeout);
@@ -1006,7 +1008,8 @@ __global__ void __launch_bounds__(kMxThreads, 1) k_prefilter_mixed(const UniDev*
             }
             fence_proxy_async();  // the next tile's operand loads follow this tile's queue in shared memory
             if (tid == 0) {  // this tile's time orders the next round's tiles
-                const uint64_t dt = globaltimer() - tile_t0;
+                uint64_t dt = globaltimer() - tile_t0;
+                dt = rows == kTile ? dt : (rows == 64 ? dt * 3 / 2 : dt * 2);  // as a full tile
                 atomicMax(&ctl[u].tile_ns, (int)(dt < 0x7fffffffull ? dt : 0x7fffffffull));
             }
             __syncthreads();
