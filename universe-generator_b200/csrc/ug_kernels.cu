@@ -1504,8 +1504,8 @@ __global__ void __launch_bounds__(128) k_conflicts(const UniDev* __restrict__ U,
 // sequential-RSA rule holds against the round's earlier admissions.  32 survivors are a
 // window; the next window's contact lists come into shared memory while one is decided,
 // and the counts (and pre-round groups) a window before that, so that no step waits for
-// global memory: 3+1 T = 128, 1800 survivors 67 -> 34 us a round, unique groups at
-// T = 256, 270 survivors 115 -> 62 us.
+// global memory: 3+1 T = 128, 1800 survivors 67 -> 34 us a round; unique groups at T = 256,
+// 270 survivors 115 -> 62 us, 51 us since they are decided from registers.
 __global__ void __launch_bounds__(32) k_greedy(const UniDev* __restrict__ U, UniCtl* ctl,
                                                RoundInfo* info) {
     extern __shared__ __align__(16) int32_t greedy_smem[];
@@ -1612,64 +1612,62 @@ __global__ void __launch_bounds__(32) k_greedy(const UniDev* __restrict__ U, Uni
             k += taken;
             n_unique += taken;
         } else {
-            // Group rounds, one survivor at a time.
+            // Group rounds: each lane first gathers what its survivor's list says of earlier
+            // windows -- the one group its contacts (and the pre-round test) name, or that
+            // there are two -- and the mask of earlier lanes it touches.  The 32 are then
+            // decided in index order from registers (a lane's contacts within the window by
+            // its mask), some 70 cycles each instead of a list walk of 450.
+            const int r = r0 + lane;
+            const bool over = cnt0 > kConflictCap;  // the list holds only kConflictCap contacts
+            const int n = over ? kConflictCap : cnt0;
+            int32_t eg = g00, my_acc = -1, my_gid = -1;
+            bool two = false;
+            uint32_t dep = 0;
+            const int4* list = reinterpret_cast<const int4*>(win + lane * kListPitch);
+            for (int i = 0; i < n; i += 4) {
+                const int4 l4 = list[i >> 2];
+                const int r4[4] = {l4.x, l4.y, l4.z, l4.w};
+                int32_t g4[4];
+#pragma unroll
+                for (int q = 0; q < 4; q++)  // a rejected survivor's group is -1
+                    g4[q] = i + q < n && r4[q] < r0 ? gid_s[UG_IDX(r4[q], kSmaxCap)] : -1;
+#pragma unroll
+                for (int q = 0; q < 4; q++) {
+                    if (i + q < n && r4[q] >= r0) dep |= 1u << (r4[q] - r0);
+                    if (g4[q] == -1) continue;
+                    two |= eg != -1 && g4[q] != eg;
+                    if (eg == -1) eg = g4[q];
+                }
+            }
+            const uint32_t m_two = __ballot_sync(0xffffffffu, two), m_over = __ballot_sync(0xffffffffu, over);
             for (int j = 0; j < nvalid; j++) {
-                const int r = r0 + j;
                 if (k >= room) {
                     lim = j;
                     grow = stopped = true;
                     break;
                 }
-                const int n_all = __shfl_sync(0xffffffffu, cnt0, j);
-                const int32_t g0 = __shfl_sync(0xffffffffu, g00, j);
-                const bool over = n_all > kConflictCap;  // the list holds only kConflictCap contacts
-                const int n = over ? kConflictCap : n_all;
-                bool accept;
-                int32_t gid;
-                // union of the pre-round group and the groups of admitted earlier survivors
-                int32_t mine = -1;
-                bool two = false;
-#pragma unroll
-                for (int h = 0; h < 2; h++)
-                    if (lane + 32 * h < n) {
-                        const int r2 = (int)UG_IDX(win[j * kListPitch + lane + 32 * h], kSmaxCap);
-                        if (acc_s[r2] >= 0) {
-                            const int32_t g2 = gid_s[r2];
-                            if (mine == -1)
-                                mine = g2;
-                            else if (mine != g2)
-                                two = true;
-                        }
-                    }
-                // the first group in list order: the pre-round one, else the lowest lane's
-                const uint32_t hasg = __ballot_sync(0xffffffffu, mine != -1);
-                int32_t first = g0;  // g0 and hasg are the same in every lane
-                if (first == -1 && hasg) first = __shfl_sync(0xffffffffu, mine, __ffs(hasg) - 1);
-                two = two || (mine != -1 && mine != first);
-                two = __any_sync(0xffffffffu, two);
-                if (!two && over) {  // unlisted contacts might add a group: decide next round
+                // union of the lane's group and those of admitted contacts in the window
+                const uint32_t dj = __shfl_sync(0xffffffffu, dep, j);
+                int32_t first = __shfl_sync(0xffffffffu, eg, j);
+                const int32_t mine = ((dj >> lane) & 1u) && my_acc >= 0 ? my_gid : -1;
+                const uint32_t has = __ballot_sync(0xffffffffu, mine != -1);
+                if (first == -1 && has) first = __shfl_sync(0xffffffffu, mine, __ffs(has) - 1);
+                const bool both = ((m_two >> j) & 1u) || (has && __any_sync(0xffffffffu, mine != -1 && mine != first));
+                if (!both && ((m_over >> j) & 1u)) {  // unlisted contacts might add a group: decide next round
                     lim = j;
                     undecided = stopped = true;
                     break;
                 }
-                if (two) {
-                    accept = false;
-                    gid = -1;
-                } else if (first == -1) {
-                    accept = unique_group;  // touches nothing: founds a group, or (subpath) rejected
-                    gid = (int32_t)(n_slots + k);
-                } else {
-                    accept = true;
-                    gid = first;
+                // two groups touched: rejected; none: founds one, or (subpath) rejected
+                const bool founds = !both && first == -1;
+                const bool accept = !both && (first != -1 || unique_group);
+                if (lane == j && accept) {
+                    my_acc = k;
+                    my_gid = founds ? (int32_t)(n_slots + k) : first;
                 }
-                if (lane == 0) {
-                    acc_s[UG_IDX(r, kSmaxCap)] = accept ? k : -1;
-                    gid_s[UG_IDX(r, kSmaxCap)] = accept ? gid : -1;
-                }
-                __syncwarp();
                 if (accept) {
                     k++;
-                    if (unique_group && gid == (int32_t)(n_slots + k - 1))
+                    if (founds)
                         n_unique++;
                     else
                         n_sub++;
@@ -1679,6 +1677,10 @@ __global__ void __launch_bounds__(32) k_greedy(const UniDev* __restrict__ U, Uni
                         break;
                     }
                 }
+            }
+            if (lane < lim) {
+                acc_s[UG_IDX(r, kSmaxCap)] = my_acc;
+                gid_s[UG_IDX(r, kSmaxCap)] = my_gid;
             }
         }
         __syncwarp();
