@@ -772,8 +772,8 @@ __device__ __forceinline__ bool cross64(const UniDev& d, const double* P, int64_
 //                queue of the CTA (as in the mixed prefilter's epilogue).
 // Bound by FP64 issue (about 110 FP64 instructions to generate a term) and the chains.  A
 // warp per candidate, lanes over 32 timesteps, summed and (knot stream) drew on one lane;
-// per job: 3+1 L2-ball T = 100, 200 k candidates 6.4 -> 3.9 ms; knot stream 2+1 T = 120,
-// two terms, 200 k 4.9 -> 1.8; T = 65, all terms, 80 k 19.0 -> 1.8.
+// per job: 3+1 L2-ball T = 100, 200 k candidates 6.4 -> 3.45 ms; knot stream 2+1 T = 120,
+// two terms, 200 k 4.9 -> 1.4; T = 65, all terms, 80 k 19.0 -> 1.7.
 template <int D>
 struct Test64 {
     const UniDev& U;
@@ -995,18 +995,22 @@ __global__ void __launch_bounds__(kT64Threads, 2) k_test64(const UniDev* __restr
             if (nl == 0) break;
             const int width = nl > 16 && !cross ? 16 : 32;  // positions: at most 32 x 3 x 16
             const int nc = min(width, T - c0), nn = (nc + 7) >> 3, L = nl * dim;
-            for (int m0 = warp * 16; m0 < L; m0 += kT64Threads / 32 * 16) {
-                const double *A0, *A1;
-                {
-                    const int i0 = min(m0 + gl, L - 1), i1 = min(m0 + gl + 8, L - 1);
-                    A0 = G + (i0 % dim) * 32 + s_slot[i0 / dim];
-                    A1 = G + (i1 % dim) * 32 + s_slot[i1 / dim];
-                }
-                const double* B[4];
+            // A warp per 16 rows x 8 or 16 timesteps: 16 once 8 would be more jobs than warps.  The
+            // operands come from L2, 32 terms ahead with 8 timesteps, 16 with 16: with all timesteps
+            // of a stage in one warp, eight terms ahead, a step of eight terms took 1700 cycles and
+            // warps without rows idled (two-term knots 1.84 -> 1.43 ms per job, 3+1 L2-ball 3.9 ->
+            // 3.45; 8 timesteps throughout: 1.44 and 3.96).
+            auto product = [&](auto pair, int job) {
+                constexpr int kN = decltype(pair)::value;
+                const int nj = (nn + kN - 1) / kN, m0 = job / nj * 16, n0 = job % nj * 8 * kN;
+                const int i0 = min(m0 + gl, L - 1), i1 = min(m0 + gl + 8, L - 1);
+                const double* A0 = G + (i0 % dim) * 32 + s_slot[i0 / dim];
+                const double* A1 = G + (i1 % dim) * 32 + s_slot[i1 / dim];
+                const double* B[kN];
 #pragma unroll
-                for (int j = 0; j < 4; j++) B[j] = d.KT + s_t[min(c0 + 8 * j + gl, T - 1)];
+                for (int n = 0; n < kN; n++) B[n] = d.KT + s_t[min(c0 + n0 + 8 * n + gl, T - 1)];
                 struct Step {
-                    double a[4], b[4][2];
+                    double a[4], b[kN][2];
                 };
                 auto fetch = [&](int k0, Step& st) {
 #pragma unroll
@@ -1016,24 +1020,20 @@ __global__ void __launch_bounds__(kT64Threads, 2) k_test64(const UniDev* __restr
                         st.a[2 * h] = on ? A0[(size_t)k * rows] : 0.0;
                         st.a[2 * h + 1] = on ? A1[(size_t)k * rows] : 0.0;
 #pragma unroll
-                        for (int j = 0; j < 4; j++)
-                            st.b[j][h] = on && j < nn ? __ldg(B[j] + (size_t)k * d.Tpad) : 0.0;
+                        for (int n = 0; n < kN; n++) st.b[n][h] = on ? __ldg(B[n] + (size_t)k * d.Tpad) : 0.0;
                     }
                 };
-                double acc[4][4];
+                constexpr int kAhead = 4 / kN;
+                double acc[kN][4] = {};
+                Step st[kAhead];
 #pragma unroll
-                for (int j = 0; j < 4; j++)
+                for (int h = 0; h < kAhead; h++) fetch(8 * h, st[h]);
+                for (int k0 = 0; k0 < K; k0 += 8 * kAhead) {
 #pragma unroll
-                    for (int q = 0; q < 4; q++) acc[j][q] = 0.0;
-                Step st[2];
-                fetch(0, st[0]);
-                for (int k0 = 0; k0 < K; k0 += 16) {
+                    for (int h = 0; h < kAhead; h++) {
 #pragma unroll
-                    for (int h = 0; h < 2; h++) {
-                        fetch(k0 + 8 * (h + 1), st[h ^ 1]);
-#pragma unroll
-                        for (int j = 0; j < 4; j++)
-                            if (j < nn) dmma_16x8x8(acc[j], st[h].a, st[h].b[j]);
+                        for (int n = 0; n < kN; n++) dmma_16x8x8(acc[n], st[h].a, st[h].b[n]);
+                        fetch(k0 + 8 * (kAhead + h), st[h]);
                     }
                 }
 #pragma unroll
@@ -1042,19 +1042,24 @@ __global__ void __launch_bounds__(kT64Threads, 2) k_test64(const UniDev* __restr
                     if (i >= L) continue;
                     const double a2 = s_a2[(i % dim) * 32 + s_slot[i / dim]];
 #pragma unroll
-                    for (int j = 0; j < 4; j++)
+                    for (int n = 0; n < kN; n++)
 #pragma unroll
                         for (int e = 0; e < 2; e++) {
-                            const int col = 8 * j + 2 * tl + e;
+                            const int col = n0 + 8 * n + 2 * tl + e;
                             if (col >= nc) continue;
-                            const double X = torus_wrap(fma(acc[j][2 * q + e], __ldg(d.invsinz + s_t[c0 + col]), a2));
+                            const double X = torus_wrap(fma(acc[n][2 * q + e], __ldg(d.invsinz + s_t[c0 + col]), a2));
                             if (cross)  // the trajectories, behind the coefficients
                                 G[(size_t)K * 32 + (size_t)s_slot[i] * T + c0 + col] = X;
                             else
                                 s_P[i * width + col] = X;
                         }
                 }
-            }
+            };
+            const int mt = (L + 15) / 16;
+            if (mt * nn <= kT64Threads / 32)
+                for (int job = warp; job < mt * nn; job += kT64Threads / 32) product(std::integral_constant<int, 1>{}, job);
+            else
+                for (int job = warp; job < mt * ((nn + 1) / 2); job += kT64Threads / 32) product(std::integral_constant<int, 2>{}, job);
             __syncthreads();
             c0 += width;
             if (cross) continue;
