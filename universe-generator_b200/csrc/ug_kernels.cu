@@ -460,13 +460,87 @@ __device__ __forceinline__ void warp_gen64_axis(const UniDev& d, uint64_t idx, i
     __syncwarp();
 }
 
-// All axes of candidate idx by one warp (the knot stream is sequential: lane 0
-// replays it).
-__device__ __forceinline__ void warp_gen64(const UniDev& d, uint64_t idx, double* alpha, double* beta,
-                                       double* a2, int32_t* bj, double* wj, int lane) {
-    if (d.rng == RNG_KNOT) {
-        if (lane == 0) gen_knot64(d, idx, alpha, beta, a2, bj, wj, 1);
+// The knot stream's coefficients (gen_knot64's draws and operations) by one warp: lane 0
+// draws and sums in list order, the lanes take the logarithms, sines and divisions, whose
+// FP64 chains were most of a lane's work: T = 65, all 64 terms of 3 axes, 122 -> 67 us a round.
+// ph: nw phases.
+__device__ __forceinline__ void warp_knot64(const UniDev& d, uint64_t idx, double* alpha, double* beta, double* a2,
+                                            int32_t* bj, double* wj, double* ph, int lane) {
+    Xo r;
+    if (lane == 0) r.seed(knot_seed(d.seed, idx));
+    const int nw = d.nw, F1 = d.F + 1;
+    const bool full = (uint32_t)nw == d.modmax;  // every frequency once
+    for (int ax = 0; ax < d.dim; ax++) {
+        double* al = alpha + ax * F1;
+        double* bt = beta + ax * F1;
+        for (int b = lane; b < F1; b += 32) al[b] = bt[b] = 0.0;
+        if (full)
+            for (int j = lane; j < nw; j += 32) bj[j] = j + 2;
         __syncwarp();
+        if (lane == 0) {
+            if (full) {
+                for (int j = nw - 1; j > 0; j--) {
+                    const int k = (int)r.below((uint32_t)(j + 1));
+                    const int32_t tmp = bj[j];
+                    bj[j] = bj[k];
+                    bj[k] = tmp;
+                }
+            } else {
+                for (int j = 0; j < nw; j++) {
+                    int b = 0;
+                    bool dup = true;
+                    for (int guard = 0; dup && guard < 64; guard++) {
+                        b = (int)r.below(d.modmax) + 2;
+                        dup = false;
+                        for (int k = 0; k < j; k++) dup |= bj[k] == b;
+                    }
+                    bj[j] = b;
+                }
+            }
+            for (int j = 0; j < nw; j++) wj[j] = 1.0 - r.f64();
+            for (int j = 0; j < nw; j++) {
+                const int b = bj[j];
+                if (r.flip()) bj[j] = -b;
+                if (!(b & 1)) ph[j] = r.f64() * kPi;
+            }
+            a2[ax] = d.pin ? 0.0 : (r.f64() * 2.0 - 1.0);
+        }
+        __syncwarp();
+        for (int j = lane; j < nw; j += 32) wj[j] = -log(wj[j]);
+        __syncwarp();
+        double sum = 0.0;
+        if (lane == 0)
+            for (int j = 0; j < nw; j++) sum += wj[j];
+        sum = __shfl_sync(0xffffffffu, sum, 0);
+        for (int j = lane; j < nw; j += 32) {
+            const int b = abs(bj[j]);
+            double amp = wj[j] / sum / (double)b;
+            if (bj[j] < 0) amp = -amp;
+            if (b & 1) {
+                wj[j] = amp;
+            } else {
+                double sf, cf;
+                sincos(ph[j], &sf, &cf);
+                wj[j] = amp * cf;
+                ph[j] = amp * sf;
+            }
+        }
+        __syncwarp();
+        // few terms may list a frequency twice: then one lane adds in term order
+        for (int j = full || lane == 0 ? lane : nw; j < nw; j += full ? 32 : 1) {
+            const int b = abs(bj[j]);
+            al[b] += wj[j];
+            if (!(b & 1)) bt[b] += ph[j];
+        }
+        __syncwarp();
+    }
+}
+
+// All axes of candidate idx by one warp.
+__device__ __forceinline__ void warp_gen64(const UniDev& d, uint64_t idx, double* alpha, double* beta,
+                                       double* a2, int32_t* bj, double* wj, double* ph, int lane) {
+    if (d.rng == RNG_KNOT) {
+        warp_knot64(d, idx, alpha, beta, a2, bj, wj, ph, lane);
     } else {
         for (int ax = 0; ax < d.dim; ax++) warp_gen64_axis(d, idx, ax, alpha, beta, a2, lane);
     }
@@ -505,7 +579,8 @@ __global__ void __launch_bounds__(32 * kSurvWarps) k_surv_gen(const UniDev* __re
     double* beta = alpha + 3 * (kMaxF + 1);
     double* a2 = beta + 3 * (kMaxF + 1);
     double* wj = a2 + 3;
-    int32_t* bj = (int32_t*)(wj + kMaxF);
+    double* ph = wj + kMaxF;
+    int32_t* bj = (int32_t*)(ph + kMaxF);
     const int n_uni = info->n_uni, total = info->total_surv;
     const int gwarp = blockIdx.x * kSurvWarps + wib, nwarps = gridDim.x * kSurvWarps;
     for (int item = gwarp; item < total; item += nwarps) {
@@ -561,7 +636,7 @@ __global__ void __launch_bounds__(32 * kSurvWarps) k_surv_gen(const UniDev* __re
             }
             continue;
         }
-        warp_gen64(d, idx, alpha, beta, a2, bj, wj, lane);
+        warp_gen64(d, idx, alpha, beta, a2, bj, wj, ph, lane);
         store_coef_rows(d, r, alpha, beta, a2, lane);
         __syncwarp();
     }
@@ -578,11 +653,12 @@ __global__ void __launch_bounds__(32 * kSurvWarps) k_restore_gen(const UniDev* _
     double* beta = alpha + 3 * (kMaxF + 1);
     double* a2 = beta + 3 * (kMaxF + 1);
     double* wj = a2 + 3;
-    int32_t* bj = (int32_t*)(wj + kMaxF);
+    double* ph = wj + kMaxF;
+    int32_t* bj = (int32_t*)(ph + kMaxF);
     const UniDev& d = U[u];
     const int gwarp = blockIdx.x * kSurvWarps + wib, nwarps = gridDim.x * kSurvWarps;
     for (int r = gwarp; r < m; r += nwarps) {
-        warp_gen64(d, (uint64_t)idx[r], alpha, beta, a2, bj, wj, lane);
+        warp_gen64(d, (uint64_t)idx[r], alpha, beta, a2, bj, wj, ph, lane);
         store_coef_rows(d, r, alpha, beta, a2, lane);
         __syncwarp();
     }

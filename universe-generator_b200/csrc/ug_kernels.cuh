@@ -111,9 +111,8 @@ __host__ __device__ __forceinline__ int gemm_tiles(int rows, int T) {
 
 // Shared memory of k_surv_gen per warp (bytes), for F <= kMaxF.
 constexpr int kSurvWarps = 4;
-constexpr size_t kSurvSmemPerWarpBase = (size_t)3 * (kMaxF + 1) * 2 * sizeof(double) + 3 * sizeof(double) +
-                                    (size_t)kMaxF * (sizeof(int32_t) + sizeof(double));
-constexpr size_t kSurvSmemPerWarp = kSurvSmemPerWarpBase;
+constexpr size_t kSurvSmemPerWarp = (size_t)3 * (kMaxF + 1) * 2 * sizeof(double) + 3 * sizeof(double) +
+                                    (size_t)kMaxF * (sizeof(int32_t) + 2 * sizeof(double));
 // k_surv_gen on a batch without knot-stream universes: one axis of alpha / beta
 constexpr size_t kSurvSmemAxis = (size_t)2 * (kMaxF + 1) * sizeof(double);
 // k_retest: the candidate's term-ordered coefficient rows and its phases
