@@ -380,62 +380,99 @@ constexpr int kNodes = 16;
 constexpr double kSure = 1e-12;   // |g| above this: the interpolant's sign is the path's
 constexpr double kWide = 5e-13;   // largest error of an interpolated position
 
-// Wiggles of both axes at kQ instants: wiggle_horner's operations for each, as
-// independent chains that share every coefficient load.
-template <int kQ>
-__device__ __forceinline__ void wiggles(const FPaths& P, int p, const double* z, double (*w)[kQ]) {
+// Wiggles of both axes of a few-term dump's path.
+__device__ __forceinline__ void wiggles(const FPaths& P, int p, double z, double (*w)[1]) {
     const size_t o = (size_t)p * 2;
-    if (P.horner) {
-        const double2* c0 = P.coef + o * (P.bmax + 1);
-        const double2* c1 = c0 + (P.bmax + 1);
-        double sz[kQ], cz[kQ], pr[2][kQ], pi[2][kQ];
 #pragma unroll
-        for (int q = 0; q < kQ; q++) {
-            sincos(z[q], &sz[q], &cz[q]);
-            pr[0][q] = c0[P.bmax].x;
-            pi[0][q] = c0[P.bmax].y;
-            pr[1][q] = c1[P.bmax].x;
-            pi[1][q] = c1[P.bmax].y;
-        }
-#pragma unroll 4
-        for (int k = P.bmax - 1; k >= 0; k--) {
-            const double2 ck[2] = {__ldg(c0 + k), __ldg(c1 + k)};
+    for (int ax = 0; ax < 2; ax++)
+        w[ax][0] = wiggle_direct(P.a + (o + ax) * P.nw, P.b + (o + ax) * P.nw, P.f + (o + ax) * P.nw, P.nw, z);
+}
+
+// Terms of a path that its eight lanes stage at a time, a buffer being read, one coming in.
+constexpr int kFbTerms = 16;
+struct FbStage {
+    double2 c[2][2][kFbTerms];  // [buffer][axis][terms k, descending from b_max]
+    double2 pad;                // a warp's four paths in different banks
+};
+
+// Wiggles of a path (wiggle_horner's operations) by the eight lanes (mask oct, lane j) that
+// hold it: of both axes at the lane's own kQ instants (kAx = 2), or of axis j & 1 (kAx = 1).  The terms come in by cp.async,
+// so their way from memory runs behind the products.
+template <int kQ, int kAx>
+__device__ __forceinline__ void oct_wiggles(const FPaths& P, int p, const double* z, double (*w)[kQ], FbStage& S,
+                                            uint32_t oct, int j) {
+    const int nt = P.bmax + 1, nst = (nt + kFbTerms - 1) / kFbTerms;
+    const double2* src = P.coef + (size_t)p * 2 * nt;
+    auto stage = [&](int ch) {
+        if (ch < nst)
 #pragma unroll
-            for (int ax = 0; ax < 2; ax++)
+            for (int h = 0; h < 2 * kFbTerms / 8; h++) {
+                const int e = j + 8 * h, ax = e / kFbTerms, q = e % kFbTerms, k = P.bmax - (ch * kFbTerms + q);
+                const uint32_t dst = (uint32_t)__cvta_generic_to_shared(&S.c[ch & 1][ax][q]);
+                asm volatile("cp.async.ca.shared.global [%0], [%1], 16, %2;" ::"r"(dst),
+                             "l"(src + (size_t)ax * nt + max(k, 0)), "r"(k >= 0 ? 16 : 0)
+                             : "memory");
+            }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    double sz[kQ], cz[kQ], pr[kAx][kQ], pi[kAx][kQ];
+    __syncwarp(oct);  // the buffers' last readers
+    stage(0);
+#pragma unroll
+    for (int q = 0; q < kQ; q++) {
+        sincos(z[q], &sz[q], &cz[q]);
+#pragma unroll
+        for (int ax = 0; ax < kAx; ax++) pr[ax][q] = pi[ax][q] = 0.0;
+    }
+    for (int ch = 0; ch < nst; ch++) {
+        stage(ch + 1);
+        asm volatile("cp.async.wait_group 1;" ::: "memory");
+        __syncwarp(oct);  // chunk ch has landed
+        const double2(*cs)[kFbTerms] = S.c[ch & 1];
+        const int n = min(kFbTerms, nt - ch * kFbTerms);
+        auto term = [&](int e) {
+#pragma unroll
+            for (int ax = 0; ax < kAx; ax++) {
+                const double2 ck = cs[kAx == 2 ? ax : j & 1][e];
 #pragma unroll
                 for (int q = 0; q < kQ; q++) {
-                    const double nr = fma(pr[ax][q], cz[q], fma(-pi[ax][q], sz[q], ck[ax].x));
-                    const double ni = fma(pr[ax][q], sz[q], fma(pi[ax][q], cz[q], ck[ax].y));
+                    const double nr = fma(pr[ax][q], cz[q], fma(-pi[ax][q], sz[q], ck.x));
+                    const double ni = fma(pr[ax][q], sz[q], fma(pi[ax][q], cz[q], ck.y));
                     pr[ax][q] = nr;
                     pi[ax][q] = ni;
                 }
+            }
+        };
+        if (n == kFbTerms) {
+#pragma unroll 4
+            for (int e = 0; e < kFbTerms; e++) term(e);
+        } else {
+            for (int e = 0; e < n; e++) term(e);
         }
-#pragma unroll
-        for (int q = 0; q < kQ; q++) {
-            w[0][q] = pi[0][q];
-            w[1][q] = pi[1][q];
-        }
-    } else {
-#pragma unroll
-        for (int ax = 0; ax < 2; ax++)
-#pragma unroll
-            for (int q = 0; q < kQ; q++)
-                w[ax][q] = wiggle_direct(P.a + (o + ax) * P.nw, P.b + (o + ax) * P.nw, P.f + (o + ax) * P.nw, P.nw, z[q]);
+        __syncwarp(oct);  // before chunk ch + 2 replaces it
     }
+#pragma unroll
+    for (int ax = 0; ax < kAx; ax++)
+#pragma unroll
+        for (int q = 0; q < kQ; q++) w[ax][q] = pi[ax][q];
 }
 
-// Four lanes per crossing; a pass takes three bisection steps: the seven midpoints they
-// can reach (two per lane) are evaluated, then the steps follow from the signs -- the same
-// midpoints, from the same operations, as one step at a time.  Bound by FP64 issue: 0.24 ms
-// for 18 k crossings at b_max 256.  One thread per crossing, with 25 evaluations of its path
-// 8 KB from its neighbours', took 2.06 ms; four lanes with 9 of them 0.74 ms.
-__global__ void __launch_bounds__(128) k_fb_refine(FPaths P, FFront F, double ox, double oy, const double* zg,
+// Eight lanes per crossing; a pass takes three bisection steps: the seven midpoints they
+// can reach (one per lane) are evaluated, then the steps follow from the signs -- the same
+// midpoints, from the same operations, as one step at a time.  Bound by FP64
+// issue (40 % of it busy) and a last wave that is not full: 0.20 ms for 26 k crossings at b_max
+// 256, 80 registers and six blocks an SM (eight with 64 registers: the same).  Four lanes, two
+// points each and the terms loaded where they are used took 162 registers, and 15 % of the
+// warps waited for memory: 0.31 ms; one thread per crossing 2.06 ms for 18 k.
+constexpr int kFbThreads = 128;
+__global__ void __launch_bounds__(kFbThreads, 6) k_fb_refine(FPaths P, FFront F, double ox, double oy, const double* zg,
                                                    const double* chig, const FCross* cross,
                                                    const unsigned long long* count, unsigned long long cap,
                                                    ug_hit* hits) {
     static_assert(kBisect % 3 == 0, "three bisection steps a pass");
-    __shared__ double s_cos[kNodes][kNodes];       // cos(k theta_i) / 8 (row 0: 1 / 16)
-    __shared__ double s_w[32][2][kNodes + 1];      // samples, then coefficients, of each crossing
+    __shared__ double s_cos[kNodes][kNodes + 1];               // cos(k theta_i) / 8 (row 0: 1 / 16)
+    __shared__ double s_w[kFbThreads / 8][2][kNodes + 1];      // samples, then coefficients, of each crossing
+    __shared__ __align__(16) FbStage s_st[kFbThreads / 8];
     const unsigned long long c = *count;
     const int64_t n = (int64_t)(c < cap ? c : cap);
     for (int e = threadIdx.x; e < kNodes * kNodes; e += blockDim.x) {
@@ -443,12 +480,13 @@ __global__ void __launch_bounds__(128) k_fb_refine(FPaths P, FFront F, double ox
         s_cos[k][i] = k == 0 ? 1.0 / kNodes : cospi((double)(k * (2 * i + 1)) / (2 * kNodes)) * (2.0 / kNodes);
     }
     __syncthreads();
-    const int j = threadIdx.x & 3;                       // lane of the crossing's four
-    const int sh = threadIdx.x & 28;                     // its first lane of the warp
-    double(*ws)[kNodes + 1] = s_w[threadIdx.x >> 2];
-    const uint32_t quad = 0xfu << sh;  // the four lanes share all of their crossing's branches
-    const int64_t stride = (int64_t)gridDim.x * blockDim.x >> 2;
-    for (int64_t k = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 2; k < n; k += stride) {
+    const int j = threadIdx.x & 7;                       // lane of the crossing's eight
+    const int sh = threadIdx.x & 24;                     // its first lane of the warp
+    double(*ws)[kNodes + 1] = s_w[threadIdx.x >> 3];
+    FbStage& S = s_st[threadIdx.x >> 3];
+    const uint32_t oct = 0xffu << sh;  // the eight lanes share all of their crossing's branches
+    const int64_t stride = (int64_t)gridDim.x * blockDim.x >> 3;
+    for (int64_t k = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 3; k < n; k += stride) {
         const FCross x = cross[k];
         const int p = x.p, i = x.i;
         const bool inside = x.inside != 0;
@@ -469,99 +507,84 @@ __global__ void __launch_bounds__(128) k_fb_refine(FPaths P, FFront F, double ox
             smooth = P.amp[p] * (4.0 / 2.0922789888e13 * u + 1e-15 * P.bmax) < kWide * fmin(sin(zc - zh), sin(zc + zh));
         }
         if (smooth) {
-            double z[4], w[2][4];
+            double z[2], w[2][2];
 #pragma unroll
-            for (int q = 0; q < 4; q++) z[q] = fma(zh, cospi((2 * (4 * j + q) + 1) / (2.0 * kNodes)), zc);
-            wiggles<4>(P, p, z, w);
+            for (int q = 0; q < 2; q++) z[q] = fma(zh, cospi((2 * (2 * j + q) + 1) / (2.0 * kNodes)), zc);
+            oct_wiggles<2, 2>(P, p, z, w, S, oct, j);
 #pragma unroll
-            for (int q = 0; q < 4; q++) {
-                ws[0][4 * j + q] = w[0][q];
-                ws[1][4 * j + q] = w[1][q];
+            for (int q = 0; q < 2; q++) {
+                ws[0][2 * j + q] = w[0][q];
+                ws[1][2 * j + q] = w[1][q];
             }
-            __syncwarp(quad);
+            __syncwarp(oct);
 #pragma unroll
-            for (int q = 0; q < 4; q++) w[0][q] = w[1][q] = 0.0;
+            for (int q = 0; q < 2; q++) w[0][q] = w[1][q] = 0.0;
             for (int e = 0; e < kNodes; e++)
 #pragma unroll
-                for (int q = 0; q < 4; q++) {
-                    w[0][q] = fma(s_cos[4 * j + q][e], ws[0][e], w[0][q]);
-                    w[1][q] = fma(s_cos[4 * j + q][e], ws[1][e], w[1][q]);
+                for (int q = 0; q < 2; q++) {
+                    w[0][q] = fma(s_cos[2 * j + q][e], ws[0][e], w[0][q]);
+                    w[1][q] = fma(s_cos[2 * j + q][e], ws[1][e], w[1][q]);
                 }
-            __syncwarp(quad);
+            __syncwarp(oct);
 #pragma unroll
-            for (int q = 0; q < 4; q++) {
-                ws[0][4 * j + q] = w[0][q];
-                ws[1][4 * j + q] = w[1][q];
+            for (int q = 0; q < 2; q++) {
+                ws[0][2 * j + q] = w[0][q];
+                ws[1][2 * j + q] = w[1][q];
             }
-            __syncwarp(quad);
+            __syncwarp(oct);
         }
         const double izh = 1.0 / zh;
         for (int it = 0; it < kBisect; it += 3) {
             // nodes of the pass's tree: 1 the midpoint, 2 and 3 those of its halves, 4..7
-            // of its quarters; lane j evaluates 4 + j and (j > 0) j
-            double m[2], z[2], w[2][2];
-#pragma unroll
-            for (int q = 0; q < 2; q++) {
-                const int node = q == 0 ? 4 + j : max(j, 1);
-                double l = lo, h = hi;
-                m[q] = (l + h) / 2.0;
-                for (int lev = node >= 4 ? 1 : (node >= 2 ? 0 : -1); lev >= 0; lev--) {
-                    if ((node >> lev) & 1)
-                        l = m[q];
-                    else
-                        h = m[q];
-                    m[q] = (l + h) / 2.0;
-                }
-                z[q] = F.budget ? m[q] : 2.0 * atan(exp(F.etaObs - m[q] / F.spd));
+            // of its quarters; lane j evaluates node j (lane 0 node 1 as well)
+            const int mine = max(j, 1);
+            double l = lo, h = hi, m = (l + h) / 2.0;
+            for (int lev = mine >= 4 ? 1 : (mine >= 2 ? 0 : -1); lev >= 0; lev--) {
+                if ((mine >> lev) & 1)
+                    l = m;
+                else
+                    h = m;
+                m = (l + h) / 2.0;
             }
-            if (smooth) {  // Clenshaw, both axes and points together
-                double t2[2], b1[2][2] = {{0.0, 0.0}, {0.0, 0.0}}, b2[2][2] = {{0.0, 0.0}, {0.0, 0.0}};
+            const double z = F.budget ? m : 2.0 * atan(exp(F.etaObs - m / F.spd));
+            double w[2][1];
+            if (smooth) {  // Clenshaw, both axes together
+                const double t2 = 2.0 * (z - zc) * izh;
+                double b1[2] = {0.0, 0.0}, b2[2] = {0.0, 0.0};
+                for (int e = kNodes - 1; e > 0; e--)
 #pragma unroll
-                for (int q = 0; q < 2; q++) t2[q] = 2.0 * (z[q] - zc) * izh;
-                for (int e = kNodes - 1; e > 0; e--) {
-                    const double cc[2] = {ws[0][e], ws[1][e]};
+                    for (int ax = 0; ax < 2; ax++) {
+                        const double b0 = fma(t2, b1[ax], ws[ax][e] - b2[ax]);
+                        b2[ax] = b1[ax];
+                        b1[ax] = b0;
+                    }
 #pragma unroll
-                    for (int ax = 0; ax < 2; ax++)
-#pragma unroll
-                        for (int q = 0; q < 2; q++) {
-                            const double b0 = fma(t2[q], b1[ax][q], cc[ax] - b2[ax][q]);
-                            b2[ax][q] = b1[ax][q];
-                            b1[ax][q] = b0;
-                        }
-                }
-#pragma unroll
-                for (int ax = 0; ax < 2; ax++)
-#pragma unroll
-                    for (int q = 0; q < 2; q++) w[ax][q] = fma(0.5 * t2[q], b1[ax][q], ws[ax][0] - b2[ax][q]);
+                for (int ax = 0; ax < 2; ax++) w[ax][0] = fma(0.5 * t2, b1[ax], ws[ax][0] - b2[ax]);
+            } else if (P.horner) {
+                oct_wiggles<1, 2>(P, p, &z, w, S, oct, j);
             } else {
-                wiggles<2>(P, p, z, w);
+                wiggles(P, p, z, w);
             }
-            uint32_t up = 0, sure = 0;  // bit of each node: the crossing lies above its midpoint
-            double front[2];
-#pragma unroll
-            for (int q = 0; q < 2; q++) {
-                const double s = sin(z[q]);
-                front[q] = F.budget ? reach_tab(F, m[q]) : m[q];
-                const double gm =
-                    metric((a2x * s + w[0][q] - s0x) / s + bx, (a2y * s + w[1][q] - s0y) / s + by, F.cheb) - front[q];
-                const uint32_t b = (__ballot_sync(quad, (gm < 0.0) == inside) >> sh) & 0xfu;
-                const uint32_t f = (__ballot_sync(quad, !smooth || fabs(gm) > kSure) >> sh) & 0xfu;
-                up |= q == 0 ? b << 4 : b & 0xeu;
-                sure |= q == 0 ? f << 4 : f & 0xeu;
-            }
+            const double s = sin(z);
+            const double gm = metric((a2x * s + w[0][0] - s0x) / s + bx, (a2y * s + w[1][0] - s0y) / s + by, F.cheb) -
+                              (F.budget ? reach_tab(F, m) : m);
+            // bit of each node: the crossing lies above its midpoint; its sign is certain
+            const uint32_t up = __ballot_sync(oct, (gm < 0.0) == inside) >> sh;
+            const uint32_t sure = __ballot_sync(oct, !smooth || fabs(gm) > kSure) >> sh;
             int node = 1;
 #pragma unroll
             for (int lev = 0; lev < 3; lev++) {
                 const double mid = (lo + hi) / 2.0;
                 int u = (up >> node) & 1;
                 if (!((sure >> node) & 1)) {  // the path itself
-                    double z1[1] = {F.budget ? mid : 2.0 * atan(exp(F.etaObs - mid / F.spd))}, w1[2][1];
-                    wiggles<1>(P, p, z1, w1);
-                    const double s = sin(z1[0]);
-                    const double gm =
-                        metric((a2x * s + w1[0][0] - s0x) / s + bx, (a2y * s + w1[1][0] - s0y) / s + by, F.cheb) -
+                    const double z1 = F.budget ? mid : 2.0 * atan(exp(F.etaObs - mid / F.spd));
+                    double w1[2][1];
+                    oct_wiggles<1, 2>(P, p, &z1, w1, S, oct, j);
+                    const double s1 = sin(z1);
+                    const double g1 =
+                        metric((a2x * s1 + w1[0][0] - s0x) / s1 + bx, (a2y * s1 + w1[1][0] - s0y) / s1 + by, F.cheb) -
                         (F.budget ? reach_tab(F, mid) : mid);
-                    u = (gm < 0.0) == inside;
+                    u = (g1 < 0.0) == inside;
                 }
                 if (u)
                     lo = mid;
@@ -570,24 +593,30 @@ __global__ void __launch_bounds__(128) k_fb_refine(FPaths P, FFront F, double ox
                 node = 2 * node + u;
             }
         }
-        __syncwarp(quad);  // the next crossing's samples replace the coefficients
-        if (j != 0) continue;
-        double chi, z1[1], w1[2][1];
+        double chi, z1;
         if (F.budget) {
-            z1[0] = (lo + hi) / 2.0;
-            chi = reach_tab(F, z1[0]);
+            z1 = (lo + hi) / 2.0;
+            chi = reach_tab(F, z1);
         } else {
             chi = (lo + hi) / 2.0;
-            z1[0] = 2.0 * atan(exp(F.etaObs - chi / F.spd));
+            z1 = 2.0 * atan(exp(F.etaObs - chi / F.spd));
         }
-        wiggles<1>(P, p, z1, w1);
-        const double s = sin(z1[0]);
+        double w[2][1];
+        if (P.horner) {  // lane 0 the first axis, lane 1 the second
+            oct_wiggles<1, 1>(P, p, &z1, w, S, oct, j);
+            w[1][0] = __shfl_sync(oct, w[0][0], sh + 1);
+        } else {
+            wiggles(P, p, z1, w);
+        }
+        __syncwarp(oct);  // the next crossing's samples replace the coefficients
+        if (j != 0) continue;
+        const double s = sin(z1);
         ug_hit h;
         h.src = (uint32_t)p;
-        h.dx = (float)((a2x * s + w1[0][0] - s0x) / s + bx);
-        h.dy = (float)((a2y * s + w1[1][0] - s0y) / s + by);
+        h.dx = (float)((a2x * s + w[0][0] - s0x) / s + bx);
+        h.dy = (float)((a2y * s + w[1][0] - s0y) / s + by);
         h.chi = (float)chi;
-        h.z_emit = (float)z1[0];
+        h.z_emit = (float)z1;
         hits[k] = h;
     }
 }
@@ -876,7 +905,7 @@ int bake_device(const ug_frames_cfg* cfg, int n, int nw, int bMax, const double*
             unsigned long long* cnt = dCount + (size_t)fi * NO + o;
             k_fb_cross<<<std::min((n + 3) / 4, nsm * 64), 128, 0, st>>>(
                 P, F, ox, oy, K, cfg->obs_type[o] == 0 ? cfg->obs_path[o] : -1, chig, dPx, dPy, dCross, cnt, hitCap);
-            k_fb_refine<<<nsm * 8, 128, 0, st>>>(P, F, ox, oy, zg, chig, dCross, cnt, hitCap, dHits);
+            k_fb_refine<<<nsm * 8, kFbThreads, 0, st>>>(P, F, ox, oy, zg, chig, dCross, cnt, hitCap, dHits);
             if (!want_hits) {
                 if (want_density)
                     launch_density(dHits, 0, cnt, hitCap, F.chiMax, cfg->density_bins,
