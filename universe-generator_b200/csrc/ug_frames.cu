@@ -14,9 +14,10 @@
 //
 // Evaluation: X(z) = [a2 sin z + sum_j a_j (sin(b_j z + f_j) - sin f_j)] / sin z
 // (frame_bake.cu:201-212).  Full-band dumps evaluate sum_j a_j sin(b_j z + f_j)
-// as Im P(e^{iz}) with P(w) = sum_b (a_b e^{i f_b}) w^b by complex Horner --
-// one sincos per evaluation instead of one per term; few-term dumps sum the
-// terms directly.
+// on the rewind grid as an FP64 tensor product over sin, cos(b z), and at single
+// instants as Im P(e^{iz}) with P(w) = sum_b (a_b e^{i f_b}) w^b by complex
+// Horner -- one sincos per evaluation instead of one per term; few-term dumps
+// sum the terms directly.
 #include <cuda_runtime.h>
 
 #include <algorithm>

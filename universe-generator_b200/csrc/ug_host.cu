@@ -2,8 +2,8 @@
 //
 // One handle = one batch of independent universes on one GPU.  The host
 // allocates every universe's tables, grid, point store and round buffers,
-// then replays the round pipeline (ug_kernels.cu) -- optionally captured as
-// a CUDA graph of `rounds_per_sync` rounds -- and reads back the small
+// then replays the round pipeline (ug_kernels.cu), `rounds_per_sync` rounds at a
+// time -- optionally as a CUDA graph from the second time on -- and reads back the small
 // control blocks between replays to grow capacities and detect completion.
 // Nothing per candidate crosses PCIe.
 #include <cuda_runtime.h>
@@ -52,6 +52,7 @@ enum KernelId {
     K_PLAN, K_PRE, K_MIXED, K_CONFIRM, K_COMPACT, K_SGEN, K_CONFL, K_GREEDY, K_COMMIT, K_SGEMM, K_SHASH,
     K_NK
 };
+// names of the timed stages: k_prefilter64w is k_test64's, k_confirm64w is k_retest's
 static const char* kKernelNames[12] = {"k_plan",      "k_prefilter64w", "k_prefilter_mixed",
                                        "k_confirm64w", "k_compact",     "k_surv_gen",
                                        "k_conflicts", "k_greedy",      "k_commit",

@@ -10,7 +10,7 @@
 //                  timesteps that its guard band left undecided
 //   k_compact      survivors in candidate-index order (deterministic)
 //   k_surv_gen     FP64 coefficients of the survivors (term-ordered rows)
-//   k_surv_gemm    their FP64 trajectories as a register-tiled product
+//   k_surv_gemm    their FP64 trajectories as an FP64 tensor product
 //   k_surv_hash    round-table insert of every survivor timestep
 //   k_conflicts    each survivor's contacts with EARLIER survivors of the round
 //   k_greedy       in-order resolution: survivor i is admitted iff it touches

@@ -16,11 +16,13 @@
 // between marks the timestep for the FP64 retest (k_retest), so every
 // decision equals the FP64 one.
 //
-// Pipeline per CTA (128 threads, one candidate per thread, persistent over
-// tiles): shared memory holds two stages of {A_hi, A_lo, B_hi, B_lo}.  All
-// threads generate stage s while the tensor core consumes stage s^1; one
-// thread issues cp.async.bulk for the B chunk (completion on an mbarrier)
-// and the MMAs (completion via tcgen05.commit on an mbarrier).  Every wait is
+// Pipeline per CTA (512 threads, tiles of 128, 64 or 32 candidates, persistent
+// over tiles): shared memory holds two stages of {A_hi, A_lo, B_hi, B_lo}.
+// All threads generate stage s while the tensor core consumes stage s^1; one
+// thread issues cp.async.bulk for the B chunk (completion on an mbarrier) and
+// the warps take turns issuing a chunk's MMAs once all have written it
+// (completion via tcgen05.commit on an mbarrier).  The epilogue tests columns
+// in stages, its exact tests spread over the CTA by a queue.  Every wait is
 // bounded; on timeout the kernel records UG_ETIMEDOUT in the control block,
 // frees its tensor memory and returns.
 #include <cuda_bf16.h>
@@ -720,9 +722,13 @@ __global__ void __launch_bounds__(kMxThreads, 1) k_prefilter_mixed(const UniDev*
             // first-level loads of all of them together (the dilated occupancy bit of each
             // position's own cell block; a clear bit proves the neighbourhood empty).  The
             // positions with a set bit go to one queue of the CTA, from which all 512 threads
-            // take the exact guard-band tests, windows first, then chains.  These are chains of dependent loads: a lane
+            // take the exact guard-band tests, windows first, then chains: dependent loads, so a lane
             // that tested its own row's columns one after another (8 at a time, all parts at
             // once) held its tile for up to 64 of them and tested 32 columns of every row.
+            // Per job: 3+1 T = 128 46.2 -> 35.3 ms, unique groups T = 256 65.8 -> 27.9, 2+1 T = 64
+            // alone 2.97 -> 2.85; a batch of 97 2+1 universes of T = 16 to 256, whose tests mostly end
+            // at the first-level bit, 37.7 -> 44.2 (the stages' barriers; stages twice as wide
+            // 44.5, only where T <= 64 46.1), the 256-universe batch with it 156.6 -> 163.4.
             float4* queue = reinterpret_cast<float4*>(sm);  // the operand stages are idle
             uint2* cells = reinterpret_cast<uint2*>(queue + kQueue);
             if (part == 0) s_rho[row] = rho;
