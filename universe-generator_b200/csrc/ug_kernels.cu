@@ -164,9 +164,11 @@ __global__ void k_plan(const UniDev* __restrict__ U, UniCtl* ctl, RoundInfo* inf
                 full = 0;
                 rows = (unsigned long long)cost[u] >= 4 * per_sm ? 32 : 64;
             } else if (s_busy == 1 && nt > nsm) {
-                const int rest = nt % nsm;
-                rows = rest * 4 <= nsm ? 32 : (rest * 2 <= nsm ? 64 : kTile);
-                full = rows < kTile ? nt - rest : nt;
+                const int rest = nt % nsm;  // whole waves alone have no last wave to share
+                if (rest > 0 && rest * 2 <= nsm) {
+                    rows = rest * 4 <= nsm ? 32 : 64;
+                    full = nt - rest;
+                }
             }
             if (rows < kTile) ntiles[u] = full + (ctl[u].B - full * kTile + rows - 1) / rows;
         }
