@@ -684,6 +684,7 @@ __global__ void __launch_bounds__(kMxThreads, 1) k_prefilter_mixed(const UniDev*
                     if (sl == slo || sl == shi) continue;
                     walk(sl);
                 }
+                fence_proxy_async();  // as at the end of the other epilogue
                 __syncthreads();
                 continue;  // single pass for dim 1
             }
@@ -978,6 +979,8 @@ __global__ void __launch_bounds__(kMxThreads, 1) k_prefilter_mixed(const UniDev*
                     for (int i = tid; i < ncell; i += kMxThreads) chain(dc, ec, i);
                 });
             }
+            // the next pass's (or tile's) operand copies take the place of this pass's queue
+            fence_proxy_async();
             tc_fence_before();
             __syncthreads();
         }
@@ -1012,7 +1015,6 @@ __global__ void __launch_bounds__(kMxThreads, 1) k_prefilter_mixed(const UniDev*
                     }
                 }
             }
-            fence_proxy_async();  // the next tile's operand loads follow this tile's queue in shared memory
             if (tid == 0) {  // this tile's time orders the next round's tiles
                 uint64_t dt = globaltimer() - tile_t0;
                 dt = rows == kTile ? dt : (rows == 64 ? dt * 3 / 2 : dt * 2);  // as a full tile
