@@ -53,3 +53,19 @@ def test_tiles_of_every_kind(ug, dim, T, mode, euclid, plan):
     assert np.array_equal(idx, ref)
     if mode:
         assert np.array_equal(gid, rgid)
+
+
+def test_waits_after_one_that_gave_up_do_not_wait(ug):
+    """A stuck pipeline is reported after one wait's limit, however many waits follow."""
+    import ctypes as C
+    import time
+
+    from ugb200 import _lib
+
+    st, took = C.c_int32(-1), []
+    for _ in range(2):  # the first call may load the kernel
+        t0 = time.perf_counter()
+        assert _lib.load().ug_selftest_bounded_wait(200_000_000, C.byref(st)) == 0
+        took.append(time.perf_counter() - t0)
+        assert st.value == _lib.UG_ETIMEDOUT
+    assert 0.2 <= took[1] < 0.4  # the kernel makes sixteen waits

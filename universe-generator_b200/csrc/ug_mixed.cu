@@ -66,19 +66,18 @@ __device__ __forceinline__ uint64_t globaltimer() {
     asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
     return t;
 }
-// Bounded wait: gives up after limit_ns of device time (or 2^26 polls).
-__device__ __forceinline__ bool mbar_wait_ns(uint64_t* bar, uint32_t parity, uint64_t limit_ns) {
+// Bounded wait: gives up after limit_ns of device time (or 2^26 polls), or at once where
+// another wait of the CTA has given up (*gave_up, which a wait that gives up sets).
+__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volatile int* gave_up,
+                                          uint64_t limit_ns = 1000000000ull) {
     if (mbar_try(bar, parity)) return true;
     const uint64_t t0 = globaltimer();
-    for (uint32_t it = 0; it < (1u << 26); it++) {
+    for (uint32_t it = 0; it < (1u << 26) && !*gave_up; it++) {
         if (mbar_try(bar, parity)) return true;
         if ((it & 255) == 0 && globaltimer() - t0 > limit_ns) break;
     }
+    *gave_up = 1;
     return false;
-}
-// The prefilter's waits: ~1 s.
-__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity) {
-    return mbar_wait_ns(bar, parity, 1000000000ull);
 }
 __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
@@ -487,7 +486,7 @@ __global__ void __launch_bounds__(kMxThreads, 1) k_prefilter_mixed(const UniDev*
         int nev = 0, nvis = 0, stage = 0;
         for (int pass = 0; pass < d.mx_npass && !timeout; pass++) {
             if (pass > 0 && __syncthreads_count(vrej[row] == 0) == 0) break;
-            for (int ax = 0; ax < dim; ax++) {
+            for (int ax = 0; ax < dim && !timeout; ax++) {
                 double sumE = 0.0, sumEb = 0.0;
                 if (pass == 0 && valid) {
                     const uint4 o = philox_block(d.seed, idx, ax, 0);
@@ -501,9 +500,13 @@ __global__ void __launch_bounds__(kMxThreads, 1) k_prefilter_mixed(const UniDev*
                     uint8_t* a_hi = sm + st * stage_bytes;
                     uint8_t* a_lo = a_hi + kAImgBytes;
                     if ((busy >> st) & 1) {  // one lane per warp polls for the stage
-                        if (lane == 0 && !mbar_wait(&bar_m[st], (ph_m >> st) & 1)) *vto = 1;
+                        const int ok = lane == 0 ? mbar_wait(&bar_m[st], (ph_m >> st) & 1, vto) : 0;
+                        if (!__shfl_sync(0xffffffffu, ok, 0)) {  // the stage stays busy
+                            timeout = true;
+                            break;
+                        }
                         ph_m ^= 1u << st;
-                        __syncwarp();
+                        busy &= ~(1u << st);
                     }
                     if (tid == 0) {
                         mbar_expect_tx(&bar_b[st], bchunk);
@@ -523,10 +526,10 @@ __global__ void __launch_bounds__(kMxThreads, 1) k_prefilter_mixed(const UniDev*
                         tc_fence_before();
                         mbar_arrive(&bar_a[st]);
                         if (warp == (seq & (kMxThreads / 32 - 1))) {
-                            if (!mbar_wait(&bar_a[st], (ph_b >> st) & 1)) *vto = 1;
+                            bool ok = mbar_wait(&bar_a[st], (ph_b >> st) & 1, vto);
                             tc_fence_after();
-                            if (!mbar_wait(&bar_b[st], (ph_b >> st) & 1)) *vto = 1;
-                            if (!*vto) {
+                            ok = ok && mbar_wait(&bar_b[st], (ph_b >> st) & 1, vto);
+                            if (ok) {
                                 const uint32_t idesc = idesc_bf16(128, nm);
                                 const uint32_t ah = smem_u32(a_hi), al = ah + kAImgBytes;
                                 const uint32_t bh = ah + 2 * kAImgBytes + (uint32_t)(pass * nm * 16);
@@ -557,17 +560,15 @@ __global__ void __launch_bounds__(kMxThreads, 1) k_prefilter_mixed(const UniDev*
                 }
             }
             // the pass's products: earlier chunks of a stage were waited for at its next use
-#pragma unroll
-            for (int st = 0; st < 2; st++)
-                if ((busy >> st) & 1) {
-                    if (tid == 0 && !mbar_wait(&bar_m[st], (ph_m >> st) & 1)) *vto = 1;
-                    ph_m ^= 1u << st;
-                }
-            busy = 0;
-            if (__syncthreads_or(*vto != 0)) {
+            if (tid == 0)
+                for (int st = 0; st < 2; st++)
+                    if ((busy >> st) & 1) mbar_wait(&bar_m[st], (ph_m >> st) & 1, vto);
+            if (__syncthreads_or(timeout || *vto)) {
                 timeout = true;
                 break;
             }
+            ph_m ^= busy;
+            busy = 0;
             if (pass == 0) {  // combine the four partial sums of the row in a fixed order
 #pragma unroll
                 for (int ax = 0; ax < 3; ax++)
@@ -1029,27 +1030,40 @@ __global__ void __launch_bounds__(kMxThreads, 1) k_prefilter_mixed(const UniDev*
             ctl[v].state = ST_ERROR;
         }
     }
-    // after a timeout: products in flight must land before tensor memory is freed
-#pragma unroll
-    for (int st = 0; st < 2; st++)
-        if (((busy >> st) & 1) && tid == 0) mbar_wait(&bar_m[st], (ph_m >> st) & 1);
+    // After a timeout: the operand copies and products of the stages still busy must land
+    // (warp 0 has passed every chunk whose products were issued) before shared and tensor
+    // memory are given back; bounded once more.
+    if (tid == 0)
+        for (int st = 0; st < 2; st++)
+            if ((busy >> st) & 1) {
+                int late = 0;
+                mbar_wait(&bar_b[st], ((ph_b >> st) & 1) ^ 1, &late);
+                mbar_wait(&bar_m[st], (ph_m >> st) & 1, &late);
+            }
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
     if (warp == 0) tmem_dealloc(tmem, L.ncols);
 }
 
-// Self-test of the bounded wait: one thread waits on an mbarrier that nothing
-// arrives on.  The wait gives up after limit_ns and the kernel records
-// UG_ETIMEDOUT in *status and returns, as the prefilter does on a stuck pipeline.
+// Self-test of the bounded wait: one thread waits again and again on an mbarrier that
+// nothing arrives on.  The first wait gives up after limit_ns and the others at once, and
+// the kernel records UG_ETIMEDOUT in *status and returns, as the prefilter does on a stuck
+// pipeline.
 __global__ void k_wait_selftest(uint64_t limit_ns, int32_t* status) {
     __shared__ uint64_t bar;
+    __shared__ int s_to;
     if (threadIdx.x == 0) {
         mbar_init(&bar, 1);
         fence_mbar_init();
+        s_to = 0;
     }
     __syncthreads();
-    if (threadIdx.x == 0) *status = mbar_wait_ns(&bar, 0, limit_ns) ? UG_OK : UG_ETIMEDOUT;
+    if (threadIdx.x == 0) {
+        int landed = 0;
+        for (int k = 0; k < 16; k++) landed += mbar_wait(&bar, 0, &s_to, limit_ns);
+        *status = landed ? UG_OK : UG_ETIMEDOUT;
+    }
 }
 
 int wait_selftest(int64_t limit_ns, int32_t* status) {
