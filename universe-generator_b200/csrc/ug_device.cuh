@@ -376,6 +376,15 @@ __device__ __forceinline__ double gen_philox64(const UniDev& U, uint64_t idx, in
     return a2;
 }
 
+// Adds an even frequency's term of the knot stream to its coefficients.  Few-term lists may
+// name a frequency twice (the redraws are bounded), so the operations are spelt out: every
+// kernel that sums a candidate's terms gives the same bits, the sine's coefficient fused, the
+// product of the cosine's rounded first (the bits that stored trajectories have had).
+__device__ __forceinline__ void add_even_term(double& al, double& bt, double amp, double sf, double cf) {
+    al = fma(amp, cf, al);
+    bt = __dadd_rn(bt, __dmul_rn(amp, sf));
+}
+
 // Knot stream (reference draw order, cuda/braid_knot.cu:111-166) for ALL axes.
 // bj/aj/fj: scratch [nw] per axis (stride applies), coefficients accumulated
 // into alpha/beta [dim][F+1] (row pitch F+1, stride applies).
@@ -423,8 +432,7 @@ __device__ inline void gen_knot64(const UniDev& U, uint64_t idx, double* alpha, 
                 const double f = r.f64() * kPi;
                 double sf, cf;
                 sincos(f, &sf, &cf);
-                al[b * stride] += amp * cf;
-                bt[b * stride] += amp * sf;
+                add_even_term(al[b * stride], bt[b * stride], amp, sf, cf);
             } else {
                 al[b * stride] += amp;
             }

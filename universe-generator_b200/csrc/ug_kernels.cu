@@ -514,25 +514,28 @@ __device__ __forceinline__ void warp_knot64(const UniDev& d, uint64_t idx, doubl
         if (lane == 0)
             for (int j = 0; j < nw; j++) sum += wj[j];
         sum = __shfl_sync(0xffffffffu, sum, 0);
-        for (int j = lane; j < nw; j += 32) {
-            const int b = abs(bj[j]);
-            double amp = wj[j] / sum / (double)b;
-            if (bj[j] < 0) amp = -amp;
-            if (b & 1) {
-                wj[j] = amp;
-            } else {
-                double sf, cf;
-                sincos(ph[j], &sf, &cf);
-                wj[j] = amp * cf;
-                ph[j] = amp * sf;
+        for (int j0 = 0; j0 < nw; j0 += 32) {
+            const int j = j0 + lane, b = j < nw ? abs(bj[j]) : 1;
+            double amp = 0.0, sf = 0.0, cf = 0.0;
+            if (j < nw) {
+                amp = wj[j] / sum / (double)b;
+                if (bj[j] < 0) amp = -amp;
+                if (!(b & 1)) sincos(ph[j], &sf, &cf);
             }
-        }
-        __syncwarp();
-        // few terms may list a frequency twice: then one lane adds in term order
-        for (int j = full || lane == 0 ? lane : nw; j < nw; j += full ? 32 : 1) {
-            const int b = abs(bj[j]);
-            al[b] += wj[j];
-            if (!(b & 1)) bt[b] += ph[j];
+            auto add = [&]() {
+                if (b & 1)
+                    al[b] += amp;
+                else
+                    add_even_term(al[b], bt[b], amp, sf, cf);
+            };
+            if (full) {
+                if (j < nw) add();
+            } else {  // few terms may list a frequency twice: added in term order
+                for (int q = 0; q < min(32, nw - j0); q++) {
+                    if (lane == q) add();
+                    __syncwarp();
+                }
+            }
         }
         __syncwarp();
     }
@@ -1000,16 +1003,16 @@ __global__ void __launch_bounds__(kT64Threads, 2) k_test64(const UniDev* __restr
                     const int fb = sc.freq[at], b = fb & 0x7fff, k = kseq_s(b);
                     double amp = sc.wgt[at] / s_sum[row] / (double)b;
                     if (fb & 0x8000) amp = -amp;
-                    double s = amp, co = 0.0;
-                    if (!(b & 1)) {
+                    double* g = G + (size_t)k * rows + row;
+                    if (full) *g = 0.0;
+                    if (b & 1) {
+                        *g += amp;
+                    } else {
                         double sf, cf;
                         sincos(sc.phase[at], &sf, &cf);
-                        s = amp * cf;
-                        co = amp * sf;
+                        if (full) g[rows] = 0.0;
+                        add_even_term(*g, g[rows], amp, sf, cf);
                     }
-                    double* g = G + (size_t)k * rows + row;
-                    *g = full ? s : *g + s;
-                    if (!(b & 1)) g[rows] = full ? co : g[rows] + co;
                 }
             }
         } else {
