@@ -41,3 +41,17 @@ def test_a_last_round_of_whole_waves_tests_every_candidate(ug):
             assert at[-1] in _steps(p)[-2:]  # the last round starts there
             idx = p.accepted(0)[0]
         assert np.array_equal(idx, ref[ref < at[-1] + last - n]), n
+
+
+def test_windows_count_the_round_that_ran_out_of_slots(ug):
+    """A round cut short for lack of slots (the host then grows the buffers) counts in the
+    windows like any other: the stop does not depend on the buffers' first size.  The
+    threshold is just below the rate of the first window, so one admission lost from it
+    would stop the run there; the window after it has lost the first, crowded bucket."""
+    kw = dict(dim=3, T=64, zgrid=1, excl=1, seed=2, round_size=65536)
+    window = 20_000_000
+    n = ug.pack(ug.Universe(attempts=window, **kw), precision=ug.PREC_MIXED, slot_hint=300_000)[0].n
+    for hint in (300_000, 1):
+        u = ug.Universe(attempts=3 * window, accept_rate=(n - 1) / window, **kw)
+        s = ug.pack(u, precision=ug.PREC_MIXED, slot_hint=hint)[0]
+        assert s.attempts == window + window // 32, hint

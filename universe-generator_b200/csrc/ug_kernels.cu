@@ -66,8 +66,9 @@ __device__ __forceinline__ int block_excl_scan256(int v, int* wsum, int* total) 
     return wpre + incl - v;
 }
 
-// The next round of every universe: the last round's windows closed, phases switched, round
-// sizes and tiles.  Planning a planned round again changes nothing.
+// The next round of every universe: the last round's windows closed (also of a universe that
+// waits for the host to grow its buffers), phases switched, round sizes and tiles.  Planning
+// a planned round again changes nothing but the epoch of a round table not yet written.
 __global__ void k_plan(const UniDev* __restrict__ U, UniCtl* ctl, RoundInfo* info, int nsm) {
     __shared__ int32_t ntiles[kMaxUni];
     __shared__ int32_t cost[kMaxUni];
@@ -95,7 +96,7 @@ __global__ void k_plan(const UniDev* __restrict__ U, UniCtl* ctl, RoundInfo* inf
             const int64_t nc = c.round_new;
             c.round_new = 0;
             c.filled += nc;
-            if (c.last_used > 0 && c.state == ST_ACTIVE) {
+            if (c.last_used > 0 && (c.state == ST_ACTIVE || c.state == ST_GROW)) {
                 const int64_t in_phase = c.next_cand - c.phase_start;
                 c.win_cur += c.accepted_round;
                 c.fwin_cur += nc;
