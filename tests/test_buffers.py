@@ -1,0 +1,95 @@
+"""Device memory of batches and calls (ug_buffers.cuh) on a stand-in for the CUDA runtime:
+host memory with a limit, which counts allocations and checks that blocks are whole."""
+
+import os
+import subprocess
+
+import pytest
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+CSRC = os.path.join(ROOT, "universe-generator_b200", "csrc")
+
+RUNTIME = r"""
+#pragma once
+#include <cstddef>
+#include <cstdint>
+#include <cstdlib>
+#include <map>
+#include <mutex>
+enum cudaError_t { cudaSuccess = 0, cudaErrorMemoryAllocation = 2 };
+inline std::mutex g_mu;
+inline std::map<void*, size_t> g_live;
+inline size_t g_used = 0, g_limit = SIZE_MAX, g_mallocs = 0, g_frees = 0;
+inline cudaError_t cudaMalloc(void** p, size_t n) {
+    std::lock_guard<std::mutex> lock(g_mu);
+    if (n > g_limit - g_used) return cudaErrorMemoryAllocation;
+    *p = malloc(16);  // never touched: sizes are what counts
+    g_live[*p] = n;
+    g_used += n;
+    g_mallocs++;
+    return cudaSuccess;
+}
+inline cudaError_t cudaFree(void* p) {
+    if (!p) return cudaSuccess;
+    std::lock_guard<std::mutex> lock(g_mu);
+    if (!g_live.count(p)) abort();  // not allocated, or freed twice
+    g_used -= g_live[p];
+    g_live.erase(p);
+    free(p);
+    g_frees++;
+    return cudaSuccess;
+}
+inline cudaError_t cudaGetLastError() { return cudaSuccess; }
+"""
+
+PROLOGUE = r"""
+#include <cstdio>
+#include <cstdlib>
+#include <set>
+#include "ug_buffers.cuh"
+using namespace ug;
+#define CHECK(x) do { if (!(x)) { printf("line %d: %s\n", __LINE__, #x); exit(1); } } while (0)
+constexpr size_t MB = (size_t)1 << 20;
+"""
+
+PROGRAMS = {
+    # calls of several threads on one batch never hold the same block
+    "threads": r"""
+int main() {
+    {
+        CallBuffers cache;
+        std::mutex mu;
+        std::set<void*> held;
+        auto work = [&](unsigned seed) {
+            for (int i = 0; i < 3000; i++) {
+                CallScope s(&cache);
+                char* p[3];
+                for (auto& q : p) {
+                    q = s.get<char>((1 + rand_r(&seed) % 5) * MB);
+                    CHECK(q);
+                    std::lock_guard<std::mutex> lock(mu);
+                    CHECK(held.insert(q).second);
+                }
+                std::lock_guard<std::mutex> lock(mu);
+                for (auto q : p) held.erase(q);
+            }
+        };
+        std::vector<std::thread> t;
+        for (unsigned k = 0; k < 8; k++) t.emplace_back(work, k);
+        for (auto& x : t) x.join();
+    }
+    CHECK(g_live.empty());
+}
+""",
+}
+
+
+@pytest.mark.parametrize("name", PROGRAMS)
+def test_program(name, tmp_path):
+    (tmp_path / "cuda_runtime.h").write_text(RUNTIME)
+    src = tmp_path / (name + ".cpp")
+    src.write_text(PROLOGUE + PROGRAMS[name])
+    subprocess.run(["g++", "-std=c++17", "-O1", "-pthread", "-I", str(tmp_path), "-I", CSRC, "-o", tmp_path / name, src],
+                   check=True)
+    r = subprocess.run([tmp_path / name], capture_output=True, text=True, timeout=120)
+    assert r.returncode == 0, r.stdout + r.stderr

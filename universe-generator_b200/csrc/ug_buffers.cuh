@@ -5,6 +5,7 @@
 
 #include <algorithm>
 #include <cstdint>
+#include <mutex>
 #include <thread>
 #include <vector>
 
@@ -52,58 +53,73 @@ private:
     size_t left_ = 0, next_ = (size_t)4 << 20;
 };
 
-// Device buffers of a read-back or frame call, kept by its batch for the next call on it
-// (which runs on the same stream).  A call's buffers are taken with get(); end() keeps them
-// and frees what the call did not use, so the cache never holds more than one call needs.
+// Device buffers of a batch's finished read-back and frame calls, kept for its next ones
+// (which run on the same stream).  A block belongs to one call at a time, so calls of
+// several threads on one batch are as independent as with buffers of their own.
 class CallBuffers {
 public:
-    ~CallBuffers() {
-        for (Block& b : blocks_) cudaFree(b.p);
-    }
-    void* get(size_t bytes) {
-        bytes = std::max<size_t>(bytes, 1);
-        Block* best = nullptr;
-        for (Block& b : blocks_)
-            if (!b.used && b.n >= bytes && b.n <= 2 * bytes + (1 << 16) && (!best || b.n < best->n)) best = &b;
-        if (!best) {
-            void* p = nullptr;
-            if (cudaMalloc(&p, bytes) != cudaSuccess) {  // make room: drop what this call does not hold
-                cudaGetLastError();
-                drop();
-                if (cudaMalloc(&p, bytes) != cudaSuccess) return nullptr;
-            }
-            blocks_.push_back(Block{p, bytes, false});
-            best = &blocks_.back();
-        }
-        best->used = true;
-        return best->p;
-    }
-    void end() {
-        drop();
-        for (Block& b : blocks_) b.used = false;
-    }
-
-private:
     struct Block {
         void* p;
         size_t n;
-        bool used;
     };
-    void drop() {
-        size_t k = 0;
-        for (Block& b : blocks_) {
-            if (b.used)
-                blocks_[k++] = b;
-            else
-                cudaFree(b.p);
+    ~CallBuffers() { drop(); }
+    // A kept block of about this size, or a new one; p is null when there is no memory.
+    Block take(size_t bytes) {
+        {
+            std::lock_guard<std::mutex> lock(mu_);
+            auto best = kept_.end();
+            for (auto b = kept_.begin(); b != kept_.end(); ++b)
+                if (b->n >= bytes && b->n <= 2 * bytes + (1 << 16) && (best == kept_.end() || b->n < best->n)) best = b;
+            if (best != kept_.end()) {
+                const Block r = *best;
+                kept_.erase(best);
+                return r;
+            }
         }
-        blocks_.resize(k);
+        Block r{nullptr, bytes};
+        if (cudaMalloc(&r.p, bytes) != cudaSuccess) {  // make room
+            cudaGetLastError();
+            drop();
+            if (cudaMalloc(&r.p, bytes) != cudaSuccess) r.p = nullptr;
+        }
+        return r;
     }
-    std::vector<Block> blocks_;
+    // The blocks of a finished call; what it did not use goes.
+    void give(std::vector<Block>& blocks) {
+        std::lock_guard<std::mutex> lock(mu_);
+        kept_.swap(blocks);
+        for (Block& b : blocks) cudaFree(b.p);
+        blocks.clear();
+    }
+    void drop() {
+        std::lock_guard<std::mutex> lock(mu_);
+        for (Block& b : kept_) cudaFree(b.p);
+        kept_.clear();
+    }
+
+private:
+    std::mutex mu_;
+    std::vector<Block> kept_;
 };
-struct CallScope {
-    CallBuffers& b;
-    ~CallScope() { b.end(); }
+
+// The buffers of one call: taken from its batch's kept ones and given back at the end, or
+// (no cache) the call's own.
+class CallScope {
+public:
+    explicit CallScope(CallBuffers* cache) : cache_(cache ? cache : &own_) {}
+    CallScope(const CallScope&) = delete;
+    ~CallScope() { cache_->give(blocks_); }
+    template <class T>
+    T* get(size_t n) {
+        const CallBuffers::Block b = cache_->take(std::max<size_t>(n, 1) * sizeof(T));
+        if (b.p) blocks_.push_back(b);
+        return (T*)b.p;
+    }
+
+private:
+    CallBuffers own_;
+    CallBuffers* cache_;
+    std::vector<CallBuffers::Block> blocks_;
 };
 
 // Backs the pages of a host result with memory while the GPU computes it: a copy into fresh

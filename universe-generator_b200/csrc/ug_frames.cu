@@ -690,18 +690,6 @@ void h_comov(const std::vector<double>& a2, const std::vector<double>& a, const 
     *VY = (dd[1] * s - xx[1] * c) / (s * s);
 }
 
-// A call's device buffers: from its batch's cache (kept there for the next call), or its own.
-struct DevBuf {
-    CallBuffers own;
-    CallBuffers& buf;
-    DevBuf() : buf(own) {}
-    explicit DevBuf(CallBuffers& cache) : buf(cache) {}
-    template <class T>
-    T* get(size_t n) {
-        return (T*)buf.get(std::max<size_t>(n, 1) * sizeof(T));
-    }
-};
-
 // Per (path, axis): s0 = sum_j a_j sin f_j, summed in term order, and the polynomial's
 // coefficients a_b e^{i f_b} (coef zeroed by the caller; a frequency listed twice adds up).
 // One warp per (path, axis): coalesced reads and the sines spread over the lanes (18 k
@@ -766,8 +754,7 @@ int check_cfg(const ug_frames_cfg* cfg, ug_frames_out* out, int n) {
 // one only counts and densities do, and no step waits for the host.
 int bake_device(const ug_frames_cfg* cfg, int n, int nw, int bMax, const double* dA2, const double* dA,
                 const double* dB, const double* dF, const std::vector<ObsPath>& obs, ug_frames_out* out,
-                cudaStream_t st, CallBuffers& cache) {
-    DevBuf buf(cache);
+                cudaStream_t st, CallScope& buf) {
     int dev = 0, nsm = 148;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
@@ -806,6 +793,7 @@ int bake_device(const ug_frames_cfg* cfg, int n, int nw, int bMax, const double*
         cudaStream_t st = nullptr;
         std::vector<cudaEvent_t> ev;
         ~Copies() {
+            if (st) cudaStreamSynchronize(st);  // an early return: none may outlive the call's buffers
             for (cudaEvent_t e : ev) cudaEventDestroy(e);
             if (st) cudaStreamDestroy(st);
         }
@@ -988,8 +976,8 @@ __global__ void k_fb_maxb(int64_t m, const int32_t* b, int* out) {
 }
 
 // Largest frequency of device-resident dump parameters.
-int max_b_device(const int32_t* b, int64_t m, int* out, cudaStream_t st, CallBuffers& buf) {
-    int* d = (int*)buf.get(4);
+int max_b_device(const int32_t* b, int64_t m, int* out, cudaStream_t st, CallScope& buf) {
+    int* d = buf.get<int>(1);
     if (!d) return set_error(UG_ENOMEM, "frame_bake: device allocation failed");
     int dev = 0, nsm = 148;
     cudaGetDevice(&dev);
@@ -1004,10 +992,9 @@ int max_b_device(const int32_t* b, int64_t m, int* out, cudaStream_t st, CallBuf
 // Frames of the accepted paths of a packer universe, straight from the device
 // (the dump -> frame_bake pipeline without a CSV or host round trip).
 int frames_from_params(const ug_frames_cfg* cfg, int n, int nw, int bMax, const double* dA2, const double* dA,
-                       const int32_t* dBi, const double* dF, ug_frames_out* out, cudaStream_t st, CallBuffers& cache) {
+                       const int32_t* dBi, const double* dF, ug_frames_out* out, cudaStream_t st, CallScope& buf) {
     int rc = check_cfg(cfg, out, n);
     if (rc) return rc;
-    DevBuf buf(cache);
     double* dB = buf.get<double>((size_t)n * 2 * nw);
     if (!dB) return set_error(UG_ENOMEM, "frame_bake: device allocation failed");
     int dev = 0, nsm = 148;
@@ -1032,7 +1019,7 @@ int frames_from_params(const ug_frames_cfg* cfg, int n, int nw, int bMax, const 
             return set_error(UG_ECUDA, "frame_bake: observer copy failed");
         for (int j = 0; j < 2 * nw; j++) q.b[j] = bi[j];
     }
-    return bake_device(cfg, n, nw, bMax, dA2, dA, dB, dF, obs, out, st, cache);
+    return bake_device(cfg, n, nw, bMax, dA2, dA, dB, dF, obs, out, st, buf);
 }
 
 }  // namespace ug
@@ -1046,7 +1033,7 @@ extern "C" int ug_frame_bake(const ug_frames_cfg* cfg, int32_t n, int32_t nw, co
     if (rc) return rc;
     int bMax = 2;
     for (size_t i = 0; i < (size_t)n * 2 * nw; i++) bMax = std::max(bMax, (int)b[i]);
-    DevBuf buf;
+    CallScope buf(nullptr);
     const size_t m = (size_t)n * 2 * nw;
     double* dA2 = buf.get<double>((size_t)n * 2);
     double* dA = buf.get<double>(m);
@@ -1074,7 +1061,7 @@ extern "C" int ug_frame_bake(const ug_frames_cfg* cfg, int32_t n, int32_t nw, co
         obs[o].b.assign(b + p * 2 * nw, b + (p + 1) * 2 * nw);
         obs[o].f.assign(f + p * 2 * nw, f + (p + 1) * 2 * nw);
     }
-    return bake_device(cfg, n, nw, bMax, dA2, dA, dB, dF, obs, out, st, buf.buf);
+    return bake_device(cfg, n, nw, bMax, dA2, dA, dB, dF, obs, out, st, buf);
 }
 
 // ------------------------------------------------------- observer view remap
@@ -1180,7 +1167,7 @@ extern "C" int ug_apparent_positions(const ug_hit* hits, int64_t n, double beta_
     int rc = check_view(n, mode);
     if (rc || n == 0) return rc;
     if (!hits || !ax || !ay || !ln_dopp) return set_error(UG_EINVAL, "apparent_positions: null buffer");
-    DevBuf buf;
+    CallScope buf(nullptr);
     ug_hit* dH = buf.get<ug_hit>((size_t)n);
     double* dO = buf.get<double>((size_t)n * 3);
     if (!dH || !dO) return set_error(UG_ENOMEM, "apparent_positions: device allocation failed");

@@ -982,8 +982,8 @@ int ug_batch_positions(void* h, int32_t u, double* pos, int64_t cap_paths) {
     const size_t m = (size_t)N * d.dim * d.T;
     PagesAhead pages;
     pages.add(pos, m * sizeof(double));
-    CallScope scope{B->call};
-    double* dp = (double*)B->call.get(m * sizeof(double));
+    CallScope buf(&B->call);
+    double* dp = buf.get<double>(m);
     if (!dp) return fail(UG_ENOMEM, "positions: device allocation failed");
     k_positions<<<(int)std::min<int64_t>((N * d.T + 255) / 256, (int64_t)B->nsm * 16), 256, 0, B->st>>>(B->dU, u, N, dp);
     CKR(cudaGetLastError());
@@ -1008,11 +1008,11 @@ int ug_batch_params(void* h, int32_t u, double* a2, double* a, int32_t* b, doubl
     pages.add(a, nt * 8);
     pages.add(f, nt * 8);
     pages.add(b, nt * 4);
-    CallScope scope{B->call};
-    double* da2 = (double*)B->call.get((size_t)N * D * 8);
-    double* da = (double*)B->call.get(nt * 8);
-    double* df = (double*)B->call.get(nt * 8);
-    int32_t* db = (int32_t*)B->call.get(nt * 4);
+    CallScope buf(&B->call);
+    double* da2 = buf.get<double>((size_t)N * D);
+    double* da = buf.get<double>(nt);
+    double* df = buf.get<double>(nt);
+    int32_t* db = buf.get<int32_t>(nt);
     if (!da2 || !da || !df || !db) return fail(UG_ENOMEM, "params: device allocation failed");
     launch_params(B->dU, u, B->U[u].d.rng, B->U[u].d.dim, N, da2, da, db, df, B->st);
     cudaError_t e = cudaStreamSynchronize(B->st);
@@ -1035,16 +1035,16 @@ int ug_batch_frames(void* h, int32_t u, const ug_frames_cfg* cfg, ug_frames_out*
     if (N < 1) return fail(UG_EINVAL, "frames: the universe has no accepted paths");
     if (N > INT32_MAX / 2) return fail(UG_ECAP, "frames: too many paths");
     const int nw = B->U[u].d.nw;
-    CallScope scope{B->call};
-    double* da2 = (double*)B->call.get((size_t)N * 2 * 8);
-    double* da = (double*)B->call.get((size_t)N * 2 * nw * 8);
-    double* df = (double*)B->call.get((size_t)N * 2 * nw * 8);
-    int32_t* db = (int32_t*)B->call.get((size_t)N * 2 * nw * 4);
+    CallScope buf(&B->call);
+    double* da2 = buf.get<double>((size_t)N * 2);
+    double* da = buf.get<double>((size_t)N * 2 * nw);
+    double* df = buf.get<double>((size_t)N * 2 * nw);
+    int32_t* db = buf.get<int32_t>((size_t)N * 2 * nw);
     if (!da2 || !da || !df || !db) return fail(UG_ENOMEM, "frames: device allocation failed");
     launch_params(B->dU, u, B->U[u].d.rng, B->U[u].d.dim, N, da2, da, db, df, B->st);
     int bMax = 2;
-    if ((rc = max_b_device(db, N * 2 * nw, &bMax, B->st, B->call))) return rc;
-    return frames_from_params(cfg, (int)N, nw, bMax, da2, da, db, df, out, B->st, B->call);
+    if ((rc = max_b_device(db, N * 2 * nw, &bMax, B->st, buf))) return rc;
+    return frames_from_params(cfg, (int)N, nw, bMax, da2, da, db, df, out, B->st, buf);
 }
 
 int ug_batch_probe(void* h, int32_t u, uint64_t seed, int64_t n, int32_t bins, int64_t* proposed,
