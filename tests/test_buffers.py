@@ -81,6 +81,27 @@ int main() {
     CHECK(g_live.empty());
 }
 """,
+    # calls of different kinds in turn allocate nothing once each has run; what is kept is bounded
+    "in_turn": r"""
+int main() {
+    {
+        CallBuffers cache;
+        auto params = [&] { CallScope s(&cache); s.get<char>(MB); s.get<char>(24 * MB); s.get<char>(24 * MB); s.get<char>(12 * MB); };
+        auto positions = [&] { CallScope s(&cache); s.get<char>(100 * MB); };
+        params(), positions();
+        const size_t n = g_mallocs;
+        for (int i = 0; i < 4; i++) params(), positions();
+        CHECK(g_mallocs == n && g_frees == 0);
+        for (size_t k = 1; k < 40; k++) {
+            { CallScope s(&cache); s.get<char>(k * 7 * MB); s.get<char>(k * 3 * MB); }
+            CHECK(g_used <= CallBuffers::kKeep);
+        }
+        { CallScope s(&cache); s.get<char>(CallBuffers::kKeep + 1); }
+        CHECK(g_used <= CallBuffers::kKeep && g_used > 0);
+    }
+    CHECK(g_live.empty());
+}
+""",
 }
 
 

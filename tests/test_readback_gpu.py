@@ -10,7 +10,7 @@ pytestmark = pytest.mark.gpu
 
 @pytest.fixture(scope="module")
 def packed(ug):
-    with ug.Packer([ug.Universe(dim=2, T=64, zgrid=1, excl=1, seed=s, attempts=30_000, round_size=4096)
+    with ug.Packer([ug.Universe(dim=3, T=48, zgrid=1, excl=1, seed=s, attempts=40_000, round_size=4096)
                     for s in (1, 2)]) as p:
         p.run()
         yield p
@@ -32,3 +32,14 @@ def test_threads_read_one_batch(packed):
     for t in threads:
         t.join()
     assert not bad
+
+
+def test_reading_in_turn_allocates_nothing_after_the_first_pass(packed):
+    import torch
+
+    free = []
+    for _ in range(4):
+        for read in (packed.params, packed.positions):
+            read(0)
+            free.append(torch.cuda.mem_get_info()[0])
+    assert len(set(free[2:])) == 1

@@ -55,7 +55,10 @@ private:
 
 // Device buffers of a batch's finished read-back and frame calls, kept for its next ones
 // (which run on the same stream).  A block belongs to one call at a time, so calls of
-// several threads on one batch are as independent as with buffers of their own.
+// several threads on one batch are as independent as with buffers of their own.  At most
+// kKeep bytes are kept, the longest unused go first: a job that reads parameters and
+// trajectories in turn allocates nothing from its second pass on, and larger blocks (the
+// densities of many frames) go back at once as they did before any were kept.
 class CallBuffers {
 public:
     struct Block {
@@ -73,6 +76,7 @@ public:
             if (best != kept_.end()) {
                 const Block r = *best;
                 kept_.erase(best);
+                bytes_ -= r.n;
                 return r;
             }
         }
@@ -84,22 +88,37 @@ public:
         }
         return r;
     }
-    // The blocks of a finished call; what it did not use goes.
+    // The blocks of a finished call.
     void give(std::vector<Block>& blocks) {
         std::lock_guard<std::mutex> lock(mu_);
-        kept_.swap(blocks);
-        for (Block& b : blocks) cudaFree(b.p);
+        for (const Block& b : blocks) {
+            if (b.n > kKeep) {
+                cudaFree(b.p);
+                continue;
+            }
+            kept_.push_back(b);
+            bytes_ += b.n;
+        }
         blocks.clear();
+        size_t k = 0;
+        for (; bytes_ > kKeep; k++) {
+            bytes_ -= kept_[k].n;
+            cudaFree(kept_[k].p);
+        }
+        kept_.erase(kept_.begin(), kept_.begin() + k);
     }
     void drop() {
         std::lock_guard<std::mutex> lock(mu_);
         for (Block& b : kept_) cudaFree(b.p);
         kept_.clear();
+        bytes_ = 0;
     }
+    static constexpr size_t kKeep = (size_t)256 << 20;
 
 private:
     std::mutex mu_;
-    std::vector<Block> kept_;
+    std::vector<Block> kept_;  // the longest unused first
+    size_t bytes_ = 0;
 };
 
 // The buffers of one call: taken from its batch's kept ones and given back at the end, or
