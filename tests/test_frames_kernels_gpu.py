@@ -94,3 +94,31 @@ def test_dumped_parameters_equal_the_oracle(ug, oracle, dim, T, pin):
         assert np.array_equal(par["b"][k], c["b"])
         for q in ("a", "f", "a2"):  # an ulp of the two libms' logarithms
             np.testing.assert_allclose(par[q][k], c[q], rtol=1e-14, atol=1e-300)
+
+
+@pytest.mark.parametrize("hits", [True, False])
+def test_more_hits_than_the_first_room(ug, hits):
+    """Paths that waver about the observer cross the young front some twenty times each: more
+    hits than the room first made for them; the same as those of the paths in small groups."""
+    from ugb200.frames import bake
+
+    n, part = 6000, 1000
+    r = np.random.default_rng(8)
+    b = np.full((n, 2, 1), 100.0)
+    a = np.full((n, 2, 1), 0.3)
+    f = r.uniform(0, math.pi, (n, 2, 1))
+    a2 = np.array([0.13, -0.29]) + 0.3 * np.sin(f[..., 0]) / math.sin(0.3 * math.pi) + r.uniform(-0.05, 0.05, (n, 2))
+    kw = dict(observers=[("point", 0.13, -0.29)], from_pi=0.35, to_pi=0.45, frames=2, zmin_pi=0.05, front="fit",
+              metric="square", density_bins=32, hits=hits)
+    whole = bake(a2, a, b, f, **kw)
+    parts = [bake(a2[k:k + part], a[k:k + part], b[k:k + part], f[k:k + part], **kw) for k in range(0, n, part)]
+    assert whole.counts.min() > 1 << 17 and max(p.counts.max() for p in parts) < 1 << 16
+    assert np.array_equal(whole.counts, sum(p.counts for p in parts))
+    assert np.array_equal(whole.density, sum(p.density for p in parts))
+    if hits:
+        for fi in range(2):
+            h = whole.hits[fi][0]
+            want = np.concatenate([p.hits[fi][0] for p in parts])
+            want["src"] += np.repeat(np.arange(0, n, part), [len(p.hits[fi][0]) for p in parts]).astype(np.uint32)
+            key = ("src", "chi", "dx", "dy", "z_emit")
+            assert np.array_equal(np.sort(h, order=key), np.sort(want, order=key))

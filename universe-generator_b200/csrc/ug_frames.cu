@@ -779,10 +779,8 @@ int bake_device(const ug_frames_cfg* cfg, int n, int nw, int bMax, const double*
     // all of them on the device otherwise (one copy at the end)
     uint32_t* dDen = want_density ? buf.get<uint32_t>(want_hits ? bins2 : bins2 * NF * NO) : nullptr;
     const unsigned long long hitCap = 1ull << 24;  // per (frame, observer) launch, frame_bake.cu:515
-    ug_hit* dHits = buf.get<ug_hit>(hitCap);
-    FCross* dCross = buf.get<FCross>(hitCap);
     unsigned long long* dCount = buf.get<unsigned long long>((size_t)NF * NO);
-    if (!dS0 || !dC || !dZg || !dChig || !dBasis || !dReach || !dAmp || !dPx || !dPy || !dHits || !dCross || !dCount || (want_density && !dDen))
+    if (!dS0 || !dC || !dZg || !dChig || !dBasis || !dReach || !dAmp || !dPx || !dPy || !dCount || (want_density && !dDen))
         return set_error(UG_ENOMEM, "frame_bake: device allocation failed");
     cudaMemsetAsync(dAmp, 0, (size_t)n * 8, st);
     // without hits no step waits for the host: the densities of finished frames are copied
@@ -853,9 +851,27 @@ int bake_device(const ug_frames_cfg* cfg, int n, int nw, int bMax, const double*
     }
     cudaMemcpyAsync(dZg, zgAll.data(), zgAll.size() * 8, cudaMemcpyHostToDevice, st);
     cudaMemcpyAsync(dChig, chigAll.data(), chigAll.size() * 8, cudaMemcpyHostToDevice, st);
+    // Room for the hits of a launch.  A path slower than the front meets it once per image, about
+    // chi_max^2 times over the torus: four times that, and the search is repeated with the
+    // room it needs where fast or wavering paths meet it more often.  (Room for hitCap
+    // in every call is 600 MB.)
+    double chiTop = 0.0;
+    for (const FFront& F : fronts) chiTop = std::max(chiTop, F.chiMax);
+    unsigned long long room = 0;
+    ug_hit* dHits = nullptr;
+    FCross* dCross = nullptr;
+    auto make_room = [&](double want) {
+        room = (unsigned long long)std::min<double>((double)hitCap, std::max<double>({1 << 16, 2.0 * room, want}));
+        dHits = buf.get<ug_hit>(room);
+        dCross = buf.get<FCross>(room);
+        return dHits && dCross ? UG_OK : set_error(UG_ENOMEM, "frame_bake: device allocation failed");
+    };
+    if (const int rc = make_room(4.0 * n * (1.0 + chiTop) * (1.0 + chiTop))) return rc;
     int64_t written = 0;
     out->hits_total = 0;
     std::vector<ug_hit> hh;
+    std::vector<unsigned long long> counts((size_t)NF * NO);
+search_again:  // (without hits: with more room)
     for (int fi = 0; fi < NF; fi++) {
         const FFront& F = fronts[fi];
         const int K = Ks[fi];
@@ -892,25 +908,34 @@ int bake_device(const ug_frames_cfg* cfg, int n, int nw, int bMax, const double*
                 m[3] = byv;
             }
             unsigned long long* cnt = dCount + (size_t)fi * NO + o;
-            k_fb_cross<<<std::min((n + 3) / 4, nsm * 64), 128, 0, st>>>(
-                P, F, ox, oy, K, cfg->obs_type[o] == 0 ? cfg->obs_path[o] : -1, chig, dPx, dPy, dCross, cnt, hitCap);
-            k_fb_refine<<<nsm * 8, kFbThreads, 0, st>>>(P, F, ox, oy, zg, chig, dCross, cnt, hitCap, dHits);
+            auto search = [&]() {
+                k_fb_cross<<<std::min((n + 3) / 4, nsm * 64), 128, 0, st>>>(
+                    P, F, ox, oy, K, cfg->obs_type[o] == 0 ? cfg->obs_path[o] : -1, chig, dPx, dPy, dCross, cnt, room);
+                k_fb_refine<<<nsm * 8, kFbThreads, 0, st>>>(P, F, ox, oy, zg, chig, dCross, cnt, room, dHits);
+            };
+            search();
             if (!want_hits) {
                 if (want_density)
-                    launch_density(dHits, 0, cnt, hitCap, F.chiMax, cfg->density_bins,
+                    launch_density(dHits, 0, cnt, room, F.chiMax, cfg->density_bins,
                                    dDen + ((size_t)fi * NO + o) * bins2, st);
                 continue;
             }
             unsigned long long nh = 0;
-            cudaError_t e = cudaMemcpyAsync(&nh, cnt, 8, cudaMemcpyDeviceToHost, st);
-            if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-            if (e != cudaSuccess) {
-                std::string m = std::string("frame_bake: ") + cudaGetErrorString(e);
-                return set_error(UG_ECUDA, m.c_str());
+            for (;;) {
+                cudaError_t e = cudaMemcpyAsync(&nh, cnt, 8, cudaMemcpyDeviceToHost, st);
+                if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+                if (e != cudaSuccess) {
+                    std::string m = std::string("frame_bake: ") + cudaGetErrorString(e);
+                    return set_error(UG_ECUDA, m.c_str());
+                }
+                if (nh <= room || nh > hitCap) break;
+                if (const int rc = make_room((double)nh)) return rc;
+                cudaMemsetAsync(cnt, 0, 8, st);
+                search();
             }
             if (nh > hitCap) return set_error(UG_ECAP, "frame_bake: hit cap overflow (lower the wraps)");
             if (want_density) {
-                launch_density(dHits, (int64_t)nh, nullptr, hitCap, F.chiMax, cfg->density_bins, dDen, st);
+                launch_density(dHits, (int64_t)nh, nullptr, room, F.chiMax, cfg->density_bins, dDen, st);
                 cudaMemcpyAsync(out->density + ((size_t)fi * NO + o) * bins2, dDen, bins2 * 4, cudaMemcpyDeviceToHost,
                                 st);
             }
@@ -952,12 +977,19 @@ int bake_device(const ug_frames_cfg* cfg, int n, int nw, int bMax, const double*
         return set_error(UG_ECUDA, m.c_str());
     }
     if (!want_hits) {
-        std::vector<unsigned long long> counts((size_t)NF * NO);
         if (cudaMemcpyAsync(counts.data(), dCount, counts.size() * 8, cudaMemcpyDeviceToHost, st) != cudaSuccess ||
             cudaStreamSynchronize(st) != cudaSuccess)
             return set_error(UG_ECUDA, "frame_bake: count copy failed");
+        const unsigned long long most = *std::max_element(counts.begin(), counts.end());
+        if (most > hitCap) return set_error(UG_ECAP, "frame_bake: hit cap overflow (lower the wraps)");
+        if (most > room) {
+            if (const int rc = make_room((double)most)) return rc;
+            cudaMemsetAsync(dCount, 0, counts.size() * 8, st);
+            for (cudaEvent_t ev : cp.ev) cudaEventDestroy(ev);
+            cp.ev.clear();
+            goto search_again;
+        }
         for (size_t i = 0; i < counts.size(); i++) {
-            if (counts[i] > hitCap) return set_error(UG_ECAP, "frame_bake: hit cap overflow (lower the wraps)");
             if (out->hit_count) out->hit_count[i] = (int64_t)counts[i];
             out->hits_total += (int64_t)counts[i];
         }
