@@ -102,6 +102,49 @@ int main() {
     CHECK(g_live.empty());
 }
 """,
+    # what other batches keep makes room for an allocation that would fail; what calls hold does not
+    "room": r"""
+int main() {
+    {
+        CallBuffers a, b;
+        g_limit = 300 * MB;
+        { CallScope s(&a); s.get<char>(100 * MB); }
+        CallScope held(&b);
+        CHECK(held.get<char>(80 * MB));
+        { CallScope s(&b); s.get<char>(60 * MB); }
+        CHECK(g_used == 240 * MB);
+        int64_t* p = nullptr;
+        CHECK(dev_malloc(&p, 200 * MB) == cudaSuccess && g_used == 280 * MB);
+        Arena arena;
+        void* q = nullptr;
+        CHECK(arena.take(100 * MB, &q) != cudaSuccess && !held.get<char>(100 * MB));
+        cudaFree(p);
+        { CallScope s(&a); s.get<char>(200 * MB); }
+        CHECK(arena.take(100 * MB, &q) == cudaSuccess && g_used == 180 * MB);
+    }
+    CHECK(g_live.empty());
+}
+""",
+    # a scarce device: several threads' calls make room for one another and never lock up
+    "room_threads": r"""
+int main() {
+    {
+        CallBuffers cache[4];
+        g_limit = 4 * 12 * MB;
+        auto work = [&](unsigned seed) {
+            for (int i = 0; i < 2000; i++) {
+                CallScope s(&cache[rand_r(&seed) % 4]);
+                s.get<char>((1 + rand_r(&seed) % 6) * MB);
+                s.get<char>((1 + rand_r(&seed) % 6) * MB);
+            }
+        };
+        std::vector<std::thread> t;
+        for (unsigned k = 0; k < 4; k++) t.emplace_back(work, k);
+        for (auto& x : t) x.join();
+    }
+    CHECK(g_live.empty());
+}
+""",
 }
 
 

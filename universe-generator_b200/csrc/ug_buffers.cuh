@@ -11,6 +11,110 @@
 
 namespace ug {
 
+// cudaMalloc of the library's own buffers: where there is no memory, the blocks that batches
+// keep from finished calls are given back, and it is tried once more.
+inline cudaError_t dev_malloc(void** p, size_t bytes);
+template <class T>
+cudaError_t dev_malloc(T** p, size_t bytes) {
+    return dev_malloc((void**)p, bytes);
+}
+
+// Device buffers of a batch's finished read-back and frame calls, kept for its next ones
+// (which run on the same stream).  A block belongs to one call at a time, so calls of
+// several threads on one batch are as independent as with buffers of their own.  At most
+// kKeep bytes are kept, the longest unused go first: a job that reads parameters and
+// trajectories in turn allocates nothing from its second pass on, and larger blocks (the
+// densities of many frames) go back at once as they did before any were kept.
+class CallBuffers {
+public:
+    struct Block {
+        void* p;
+        size_t n;
+    };
+    CallBuffers() {
+        std::lock_guard<std::mutex> lock(all_mu());
+        all().push_back(this);
+    }
+    ~CallBuffers() {
+        {
+            std::lock_guard<std::mutex> lock(all_mu());
+            all().erase(std::find(all().begin(), all().end(), this));
+        }
+        drop();
+    }
+    CallBuffers(const CallBuffers&) = delete;
+    // A kept block of about this size, or a new one; p is null when there is no memory.
+    Block take(size_t bytes) {
+        {
+            std::lock_guard<std::mutex> lock(mu_);
+            auto best = kept_.end();
+            for (auto b = kept_.begin(); b != kept_.end(); ++b)
+                if (b->n >= bytes && b->n <= 2 * bytes + (1 << 16) && (best == kept_.end() || b->n < best->n)) best = b;
+            if (best != kept_.end()) {
+                const Block r = *best;
+                kept_.erase(best);
+                bytes_ -= r.n;
+                return r;
+            }
+        }
+        Block r{nullptr, bytes};
+        if (dev_malloc(&r.p, bytes) != cudaSuccess) r.p = nullptr;
+        return r;
+    }
+    // The blocks of a finished call.
+    void give(std::vector<Block>& blocks) {
+        std::lock_guard<std::mutex> lock(mu_);
+        for (const Block& b : blocks) {
+            if (b.n > kKeep) {
+                cudaFree(b.p);
+                continue;
+            }
+            kept_.push_back(b);
+            bytes_ += b.n;
+        }
+        blocks.clear();
+        size_t k = 0;
+        for (; bytes_ > kKeep; k++) {
+            bytes_ -= kept_[k].n;
+            cudaFree(kept_[k].p);
+        }
+        kept_.erase(kept_.begin(), kept_.begin() + k);
+    }
+    void drop() {
+        std::lock_guard<std::mutex> lock(mu_);
+        for (Block& b : kept_) cudaFree(b.p);
+        kept_.clear();
+        bytes_ = 0;
+    }
+    static void drop_all() {
+        std::lock_guard<std::mutex> lock(all_mu());
+        for (CallBuffers* c : all()) c->drop();
+    }
+    static constexpr size_t kKeep = (size_t)256 << 20;
+
+private:
+    // every cache of the process (never destroyed: a batch may outlive static objects)
+    static std::mutex& all_mu() {
+        static std::mutex* m = new std::mutex;
+        return *m;
+    }
+    static std::vector<CallBuffers*>& all() {
+        static std::vector<CallBuffers*>* v = new std::vector<CallBuffers*>;
+        return *v;
+    }
+    std::mutex mu_;
+    std::vector<Block> kept_;  // the longest unused first
+    size_t bytes_ = 0;
+};
+
+inline cudaError_t dev_malloc(void** p, size_t bytes) {
+    cudaError_t e = cudaMalloc(p, bytes);
+    if (e != cudaErrorMemoryAllocation) return e;
+    cudaGetLastError();
+    CallBuffers::drop_all();
+    return cudaMalloc(p, bytes);
+}
+
 // A batch's fixed buffers, carved from chunks: a cudaMalloc and its cudaFree take 0.3 to
 // 0.6 ms together and a universe has about thirty buffers (creating, running and releasing
 // a 20 k candidate job: 6.3 -> 3.7 ms).  The first chunk is about what the universes
@@ -44,81 +148,13 @@ public:
 private:
     static constexpr size_t kMost = (size_t)64 << 20;
     cudaError_t chunk(size_t bytes, void** out) {
-        const cudaError_t e = cudaMalloc(out, bytes);
+        const cudaError_t e = dev_malloc(out, bytes);
         if (e == cudaSuccess) chunks_.push_back(*out);
         return e;
     }
     std::vector<void*> chunks_;
     char* cur_ = nullptr;
     size_t left_ = 0, next_ = (size_t)4 << 20;
-};
-
-// Device buffers of a batch's finished read-back and frame calls, kept for its next ones
-// (which run on the same stream).  A block belongs to one call at a time, so calls of
-// several threads on one batch are as independent as with buffers of their own.  At most
-// kKeep bytes are kept, the longest unused go first: a job that reads parameters and
-// trajectories in turn allocates nothing from its second pass on, and larger blocks (the
-// densities of many frames) go back at once as they did before any were kept.
-class CallBuffers {
-public:
-    struct Block {
-        void* p;
-        size_t n;
-    };
-    ~CallBuffers() { drop(); }
-    // A kept block of about this size, or a new one; p is null when there is no memory.
-    Block take(size_t bytes) {
-        {
-            std::lock_guard<std::mutex> lock(mu_);
-            auto best = kept_.end();
-            for (auto b = kept_.begin(); b != kept_.end(); ++b)
-                if (b->n >= bytes && b->n <= 2 * bytes + (1 << 16) && (best == kept_.end() || b->n < best->n)) best = b;
-            if (best != kept_.end()) {
-                const Block r = *best;
-                kept_.erase(best);
-                bytes_ -= r.n;
-                return r;
-            }
-        }
-        Block r{nullptr, bytes};
-        if (cudaMalloc(&r.p, bytes) != cudaSuccess) {  // make room
-            cudaGetLastError();
-            drop();
-            if (cudaMalloc(&r.p, bytes) != cudaSuccess) r.p = nullptr;
-        }
-        return r;
-    }
-    // The blocks of a finished call.
-    void give(std::vector<Block>& blocks) {
-        std::lock_guard<std::mutex> lock(mu_);
-        for (const Block& b : blocks) {
-            if (b.n > kKeep) {
-                cudaFree(b.p);
-                continue;
-            }
-            kept_.push_back(b);
-            bytes_ += b.n;
-        }
-        blocks.clear();
-        size_t k = 0;
-        for (; bytes_ > kKeep; k++) {
-            bytes_ -= kept_[k].n;
-            cudaFree(kept_[k].p);
-        }
-        kept_.erase(kept_.begin(), kept_.begin() + k);
-    }
-    void drop() {
-        std::lock_guard<std::mutex> lock(mu_);
-        for (Block& b : kept_) cudaFree(b.p);
-        kept_.clear();
-        bytes_ = 0;
-    }
-    static constexpr size_t kKeep = (size_t)256 << 20;
-
-private:
-    std::mutex mu_;
-    std::vector<Block> kept_;  // the longest unused first
-    size_t bytes_ = 0;
 };
 
 // The buffers of one call: taken from its batch's kept ones and given back at the end, or

@@ -207,7 +207,7 @@ static int alloc_points(Batch& B, UniHost& h, int64_t cap) {
     const int T = h.cfg.T;
     const bool fixed = cap > total_budget(h.cfg);
     void *p = nullptr, *f = nullptr, *ai = nullptr;
-    auto take = [&](size_t n, void** q) { return fixed ? B.arena.take(n, q) : cudaMalloc(q, n); };
+    auto take = [&](size_t n, void** q) { return fixed ? B.arena.take(n, q) : dev_malloc(q, n); };
     CKR(take((size_t)cap * T * sizeof(Pt64), &p));
     CKR(take((size_t)cap * T * sizeof(Pt32), &f));
     CKR(take((size_t)cap * sizeof(int64_t), &ai));
@@ -229,7 +229,7 @@ static void free_points(const UniHost& h) {
 static int alloc_hash(Batch& B, UniHost& h, int64_t cap) {
     const bool fixed = keys_ahead(h, 0, 0, INT32_MAX / kSmaxCap) * 2 <= cap;
     void* q = nullptr;
-    CKR(fixed ? B.arena.take((size_t)cap * sizeof(ulonglong2), &q) : cudaMalloc(&q, (size_t)cap * sizeof(ulonglong2)));
+    CKR(fixed ? B.arena.take((size_t)cap * sizeof(ulonglong2), &q) : dev_malloc(&q, (size_t)cap * sizeof(ulonglong2)));
     CKR(cudaMemset(q, 0xff, (size_t)cap * sizeof(ulonglong2)));
     h.d.hslot = (ulonglong2*)q;
     h.d.hmask = (uint64_t)(cap - 1);
@@ -948,11 +948,11 @@ int ug_batch_accepted_all(void* h, int64_t* idx, int32_t* gid, int64_t cap, int6
         B->d_gather_idx = nullptr;
         B->d_gather_gid = nullptr;
         const int64_t c = pow2_at_least(total);
-        CKR(cudaMalloc(&B->d_gather_idx, (size_t)c * sizeof(int64_t)));
-        CKR(cudaMalloc(&B->d_gather_gid, (size_t)c * sizeof(int32_t)));
+        CKR(dev_malloc(&B->d_gather_idx, (size_t)c * sizeof(int64_t)));
+        CKR(dev_malloc(&B->d_gather_gid, (size_t)c * sizeof(int32_t)));
         B->gather_cap = c;
     }
-    if (!B->d_gather_off) CKR(cudaMalloc(&B->d_gather_off, (size_t)(kMaxUni + 1) * sizeof(int64_t)));
+    if (!B->d_gather_off) CKR(dev_malloc(&B->d_gather_off, (size_t)(kMaxUni + 1) * sizeof(int64_t)));
     CKR(cudaMemcpyAsync(B->d_gather_off, off.data(), off.size() * sizeof(int64_t), cudaMemcpyHostToDevice, B->st));
     B->h2d += off.size() * sizeof(int64_t);
     k_gather_accepted<<<B->n, 256, 0, B->st>>>(B->dU, B->d_gather_off, B->d_gather_idx, B->d_gather_gid);
@@ -1055,7 +1055,7 @@ int ug_batch_probe(void* h, int32_t u, uint64_t seed, int64_t n, int32_t bins, i
     int rc = pull_ctl(*B);
     if (rc) return rc;
     unsigned long long* dh = nullptr;
-    CKR(cudaMalloc(&dh, sizeof(unsigned long long) * 2 * bins));
+    CKR(dev_malloc(&dh, sizeof(unsigned long long) * 2 * bins));
     cudaError_t e = cudaMemsetAsync(dh, 0, sizeof(unsigned long long) * 2 * bins, B->st);
     if (e == cudaSuccess && n > 0) {
         const int blocks = (int)std::min<int64_t>((n + kTile - 1) / kTile, (int64_t)B->nsm * 16);
@@ -1171,7 +1171,7 @@ int ug_batch_restore(void* h, int32_t u, int64_t n, const int64_t* idx, const in
     std::vector<int32_t> iota(d.S_max), zero(d.S_max + 1, 0);
     for (int i = 0; i < d.S_max; i++) iota[i] = i;
     int64_t* dIdx = nullptr;
-    CKR(cudaMalloc(&dIdx, (size_t)d.S_max * sizeof(int64_t)));
+    CKR(dev_malloc(&dIdx, (size_t)d.S_max * sizeof(int64_t)));
     RoundInfo* ri = new RoundInfo();
     int64_t done = 0;
     while (done < n && rc == UG_OK) {

@@ -34,6 +34,7 @@
 #include <type_traits>
 #include <vector>
 
+#include "ug_buffers.cuh"
 #include "ug_mixed.cuh"
 
 namespace ug {
@@ -1068,7 +1069,7 @@ __global__ void k_wait_selftest(uint64_t limit_ns, int32_t* status) {
 
 int wait_selftest(int64_t limit_ns, int32_t* status) {
     int32_t* d = nullptr;
-    if (cudaMalloc(&d, sizeof(int32_t)) != cudaSuccess) return UG_ENOMEM;
+    if (dev_malloc(&d, sizeof(int32_t)) != cudaSuccess) return UG_ENOMEM;
     cudaMemset(d, 0xff, sizeof(int32_t));
     k_wait_selftest<<<1, 32>>>((uint64_t)limit_ns, d);
     cudaError_t e = cudaGetLastError();
@@ -1204,7 +1205,7 @@ int mixed_setup(const ug_universe_cfg& cfg, UniDev& d, MixedTables& mt) {
         }
     }
     void* dimg = nullptr;
-    if (cudaMalloc(&dimg, host.size() * 2) != cudaSuccess) return UG_ENOMEM;
+    if (dev_malloc(&dimg, host.size() * 2) != cudaSuccess) return UG_ENOMEM;
     if (cudaMemcpy(dimg, host.data(), host.size() * 2, cudaMemcpyHostToDevice) != cudaSuccess) return UG_ECUDA;
     mt.bhi = dimg;
     d.mx_bimg = (const uint8_t*)dimg;
@@ -1279,8 +1280,8 @@ int mixed_error(const UniDev* dU, int u, const UniDev& d, const MixedTables& mt,
     const size_t n = nm * d.dim;
     float *d32 = nullptr, *dm = nullptr;
     double* d64 = nullptr;
-    if (cudaMalloc(&d32, n * 4) != cudaSuccess || cudaMalloc(&dm, nm * 4) != cudaSuccess ||
-        cudaMalloc(&d64, n * 8) != cudaSuccess) {
+    if (dev_malloc(&d32, n * 4) != cudaSuccess || dev_malloc(&dm, nm * 4) != cudaSuccess ||
+        dev_malloc(&d64, n * 8) != cudaSuccess) {
         cudaFree(d32);
         cudaFree(dm);
         return UG_ENOMEM;
