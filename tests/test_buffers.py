@@ -125,6 +125,22 @@ int main() {
     CHECK(g_live.empty());
 }
 """,
+    # memory for what is asked but not for a whole chunk
+    "chunk": r"""
+int main() {
+    {
+        Arena arena;
+        arena.expect(32 * MB);
+        g_limit = 50 * MB;
+        void* p = nullptr;
+        CHECK(arena.take(10 * MB, &p) == cudaSuccess && g_used == 32 * MB);
+        for (int i = 0; i < 3; i++) CHECK(arena.take(10 * MB, &p) == cudaSuccess);
+        CHECK(g_used == 42 * MB && arena.take(10 * MB, &p) == cudaErrorMemoryAllocation);
+        CHECK(arena.take(8 * MB, &p) == cudaSuccess);
+    }
+    CHECK(g_live.empty());
+}
+""",
     # a scarce device: several threads' calls make room for one another and never lock up
     "room_threads": r"""
 int main() {

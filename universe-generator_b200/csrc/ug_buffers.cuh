@@ -112,7 +112,9 @@ inline cudaError_t dev_malloc(void** p, size_t bytes) {
     if (e != cudaErrorMemoryAllocation) return e;
     cudaGetLastError();
     CallBuffers::drop_all();
-    return cudaMalloc(p, bytes);
+    e = cudaMalloc(p, bytes);
+    if (e == cudaErrorMemoryAllocation) cudaGetLastError();  // reported here, not at a later launch
+    return e;
 }
 
 // A batch's fixed buffers, carved from chunks: a cudaMalloc and its cudaFree take 0.3 to
@@ -131,9 +133,11 @@ public:
         bytes = (std::max<size_t>(bytes, 1) + 255) / 256 * 256;
         if (bytes > kMost / 4) return chunk(bytes, out);
         if (bytes > left_) {
-            const size_t n = std::max(next_, bytes);
+            size_t n = std::max(next_, bytes);
             void* c = nullptr;
-            const cudaError_t e = chunk(n, &c);
+            cudaError_t e = chunk(n, &c);
+            if (e == cudaErrorMemoryAllocation && n > bytes)  // less than a chunk is left: what is asked
+                e = chunk(n = bytes, &c);
             if (e != cudaSuccess) return e;
             cur_ = (char*)c;
             left_ = n;
