@@ -63,7 +63,8 @@ struct UniHost {
     UniDev d;
     int64_t dense_bytes = 0;
     int64_t hcap = 0;
-    bool points_fixed = false, hash_fixed = false;  // in the arena: as large as they can get
+    int64_t budget = 0;        // admissions it can reach at most
+    bool points_fixed = false, hash_fixed = false;  // in the arena
     int64_t occ_words = 0, occ1_words = 0;
     MixedTables mt;            // tensor-core operand tables (mixed precision)
 };
@@ -187,27 +188,30 @@ static void host_tables(const ug_universe_cfg& c, std::vector<double>& S, std::v
     });
 }
 
-// Admissions a universe can reach at most: one per candidate.
+// Admissions a universe can reach at most: one per candidate (a budget without end is cut).
 static int64_t total_budget(const ug_universe_cfg& c) {
-    return c.attempts + (c.group_mode == UG_GROUP_SUBPATH ? (c.sub_attempts ? c.sub_attempts : c.attempts) : 0);
+    const int64_t most = (int64_t)1 << 60;
+    const int64_t sub = c.group_mode == UG_GROUP_SUBPATH ? (c.sub_attempts ? c.sub_attempts : c.attempts) : 0;
+    return std::min(c.attempts, most) + std::min(sub, most);
 }
 // Capacities that `rounds` more rounds may need: accepted paths, and hash keys.
 static int64_t slots_ahead(const UniHost& h, int64_t n_slots, int rounds) {
     const int64_t more = std::max<int64_t>(h.d.S_max, (int64_t)rounds * h.d.S_max / 4);
-    return std::min(n_slots + more, total_budget(h.cfg) + 1);
+    return std::min(n_slots + more, h.budget + 1);
 }
 static int64_t keys_ahead(const UniHost& h, int64_t n_slots, int64_t used, int rounds) {
-    const int64_t more = std::min<int64_t>((int64_t)rounds * h.d.S_max, std::max<int64_t>(0, total_budget(h.cfg) - n_slots));
+    const int64_t more = std::min<int64_t>((int64_t)rounds * h.d.S_max, std::max<int64_t>(0, h.budget - n_slots));
     return used + more * h.cfg.T;
 }
 
-// Buffers that may grow are allocated on their own; one that holds all a universe can
-// reach comes from the batch's arena.
-static int alloc_points(Batch& B, UniHost& h, int64_t cap) {
+// Buffers that may grow are allocated on their own.  A first one (arena) that holds all the
+// universe can reach comes from the batch's arena; a later one never does, whose place
+// would be free again only with the batch.
+static int alloc_points(UniHost& h, int64_t cap, Arena* arena = nullptr) {
     const int T = h.cfg.T;
-    const bool fixed = cap > total_budget(h.cfg);
+    const bool fixed = arena && cap > h.budget;
     void *p = nullptr, *f = nullptr, *ai = nullptr;
-    auto take = [&](size_t n, void** q) { return fixed ? B.arena.take(n, q) : dev_malloc(q, n); };
+    auto take = [&](size_t n, void** q) { return fixed ? arena->take(n, q) : dev_malloc(q, n); };
     CKR(take((size_t)cap * T * sizeof(Pt64), &p));
     CKR(take((size_t)cap * T * sizeof(Pt32), &f));
     CKR(take((size_t)cap * sizeof(int64_t), &ai));
@@ -226,10 +230,10 @@ static void free_points(const UniHost& h) {
 }
 
 // Hash grid of cap slots, all empty (key and head all ones: no key, head -1).
-static int alloc_hash(Batch& B, UniHost& h, int64_t cap) {
-    const bool fixed = keys_ahead(h, 0, 0, INT32_MAX / kSmaxCap) * 2 <= cap;
+static int alloc_hash(UniHost& h, int64_t cap, Arena* arena = nullptr) {
+    const bool fixed = arena && keys_ahead(h, 0, 0, INT32_MAX / kSmaxCap) * 2 <= cap;
     void* q = nullptr;
-    CKR(fixed ? B.arena.take((size_t)cap * sizeof(ulonglong2), &q) : dev_malloc(&q, (size_t)cap * sizeof(ulonglong2)));
+    CKR(fixed ? arena->take((size_t)cap * sizeof(ulonglong2), &q) : dev_malloc(&q, (size_t)cap * sizeof(ulonglong2)));
     CKR(cudaMemset(q, 0xff, (size_t)cap * sizeof(ulonglong2)));
     h.d.hslot = (ulonglong2*)q;
     h.d.hmask = (uint64_t)(cap - 1);
@@ -245,6 +249,7 @@ static int setup_universe(Batch& B, UniHost& h, int64_t dense_budget, int64_t* d
     const ug_universe_cfg& c = h.cfg;
     UniDev& d = h.d;
     memset(&d, 0, sizeof d);
+    h.budget = total_budget(c);
     d.dim = c.dim;
     d.T = c.T;
     d.F = c.T;
@@ -345,7 +350,7 @@ static int setup_universe(Batch& B, UniHost& h, int64_t dense_budget, int64_t* d
         d.grid_kind = GRID_HASH;
         // what the first replay may fill, at a load of 1/4 (grown at 1/2)
         const int64_t keys = std::max<int64_t>(1 << 14, keys_ahead(h, 0, 0, B.opts.rounds_per_sync));
-        if ((rc = alloc_hash(B, h, pow2_at_least(4 * keys)))) return rc;
+        if ((rc = alloc_hash(h, pow2_at_least(4 * keys), &B.arena))) return rc;
     }
     // occupancy bitmap, coarsened until it is at most 512 MiB (T <= 256 in 3D
     // keeps 2 cells per coarse cell per axis or finer)
@@ -404,9 +409,9 @@ static int setup_universe(Batch& B, UniHost& h, int64_t dense_budget, int64_t* d
     // accepted points
     int64_t cap = B.opts.slot_hint > 0 ? B.opts.slot_hint
                                        : std::max<int64_t>(8192, slots_ahead(h, 0, B.opts.rounds_per_sync));
-    if (B.opts.slot_hint <= 0 && total_budget(c) < 2 * cap) cap = total_budget(c) + 1;  // all it can reach
-    cap = std::max<int64_t>(std::min<int64_t>(cap, total_budget(c) + 1), 1024);
-    if ((rc = alloc_points(B, h, cap))) return rc;
+    if (B.opts.slot_hint <= 0 && h.budget < 2 * cap) cap = h.budget + 1;  // all it can reach
+    cap = std::max<int64_t>(std::min<int64_t>(cap, h.budget + 1), 1024);
+    if ((rc = alloc_points(h, cap, &B.arena))) return rc;
     // round buffers
     const int Bm = d.B_max, Sm = d.S_max;
     if ((rc = dalloc(B, &d.surv_bits, Bm / 32, 0)) ||         (rc = dalloc(B, &d.g0, Bm, 0xff)) || (rc = dalloc(B, &d.surv_off, Sm + 1, 0)) ||
@@ -589,7 +594,7 @@ static int ensure_capacity(Batch& B, int rounds) {
             const int T = h.cfg.T;
             const UniHost old = h;
             const int64_t n = k.n_slots;
-            int rc = alloc_points(B, h, ncap);
+            int rc = alloc_points(h, ncap);
             if (rc) return rc;
             CKR(cudaMemcpyAsync(h.d.pts, old.d.pts, (size_t)n * T * sizeof(Pt64), cudaMemcpyDeviceToDevice, B.st));
             CKR(cudaMemcpyAsync(h.d.ptf, old.d.ptf, (size_t)n * T * sizeof(Pt32), cudaMemcpyDeviceToDevice, B.st));
@@ -606,7 +611,7 @@ static int ensure_capacity(Batch& B, int rounds) {
             const int64_t need_keys = keys_ahead(h, k.n_slots, k.hash_used, rounds);
             if (need_keys * 2 > h.hcap) {
                 const UniHost old = h;
-                int rc = alloc_hash(B, h, pow2_at_least(need_keys * 4));
+                int rc = alloc_hash(h, pow2_at_least(need_keys * 4));
                 if (rc) return rc;
                 free_hash(old);
                 int64_t zero = 0;
@@ -1136,17 +1141,19 @@ int ug_batch_restore(void* h, int32_t u, int64_t n, const int64_t* idx, const in
     if (rc) return rc;
     UniDev& d = U.d;
     const int T = U.cfg.T;
+    // the state runs on to its own budgets, which may be above this batch's
+    U.budget = std::max({U.budget, total_budget(hd.cfg), n});
     // clear the universe's grid, bitmaps and round table
     if (d.grid_kind == GRID_DENSE) {
         int64_t cpt = 1;
         for (int ax = 0; ax < d.dim; ax++) cpt *= d.gw;
         CKR(cudaMemsetAsync(d.heads, 0xff, (size_t)T * cpt * sizeof(int32_t), B->st));
     } else {
-        const int64_t need = std::max<int64_t>(1 << 16, pow2_at_least((n * T + (int64_t)d.S_max * T) * 4));
-        if (need > U.hcap) {
+        const int64_t keys = keys_ahead(U, n, n * T, 1);
+        if (keys * 2 > U.hcap) {
             CKR(cudaStreamSynchronize(B->st));
             free_hash(U);
-            if ((rc = alloc_hash(*B, U, need))) return rc;
+            if ((rc = alloc_hash(U, pow2_at_least(keys * 4)))) return rc;
         } else {
             CKR(cudaMemsetAsync(d.hslot, 0xff, (size_t)U.hcap * sizeof(ulonglong2), B->st));
         }
@@ -1155,10 +1162,11 @@ int ug_batch_restore(void* h, int32_t u, int64_t n, const int64_t* idx, const in
     CKR(cudaMemsetAsync(d.occ1, 0, (size_t)U.occ1_words * sizeof(uint32_t), B->st));
     CKR(cudaMemsetAsync(d.rhead, 0xff, (size_t)T * d.rblocks * sizeof(uint64_t), B->st));
     // room for the admissions and the next rounds
-    if (n + (int64_t)d.S_max * 2 > d.slot_cap) {
+    const int64_t slots = slots_ahead(U, n, 8);
+    if (slots > d.slot_cap) {
         CKR(cudaStreamSynchronize(B->st));
         free_points(U);
-        if ((rc = alloc_points(*B, U, n + (int64_t)d.S_max * 2))) return rc;
+        if ((rc = alloc_points(U, slots))) return rc;
     }
     if ((rc = push_unidev(*B))) return rc;
     // rebuild control block: k_commit reads these and accumulates hash keys and cells
