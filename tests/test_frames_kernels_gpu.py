@@ -122,3 +122,47 @@ def test_more_hits_than_the_first_room(ug, hits):
             want["src"] += np.repeat(np.arange(0, n, part), [len(p.hits[fi][0]) for p in parts]).astype(np.uint32)
             key = ("src", "chi", "dx", "dy", "z_emit")
             assert np.array_equal(np.sort(h, order=key), np.sort(want, order=key))
+
+
+@pytest.mark.parametrize("n,K,speed,metric", [
+    (1, 16, 14.0, "square"), (3, 15, 11.0, "square"), (2, 36, 25.0, "square"), (2, 40, 0.33, "square"),
+    (2, 17, 9.0, "euclid"), (5, 3, 2.0, "euclid"), (40, 2, 0.4, "euclid"),
+])
+def test_hits_over_many_images(ug, n, K, speed, metric):
+    """Images beyond 32 a side, and more of them than the front reaches."""
+    from ugb200.frames import bake
+
+    a2, a, b, f = _dump(n, 6, 8, 7 * n + K)
+    at, z_min, z_obs = (0.13, -0.29), 0.05 * math.pi, 0.4 * math.pi
+    bk = bake(a2, a, b, f, observers=[("point", *at)], from_pi=0.4, to_pi=0.4, zmin_pi=0.05, front="speed",
+              metric=metric, speed=speed, wraps=K)
+    eta = lambda z: np.log(np.tan(z / 2))  # noqa: E731
+    chi = speed * (eta(z_obs) - eta(z_min)) * np.arange(421) / 420
+    x = _x(a2, a, b, f, 2 * np.arctan(np.exp(eta(z_obs) - chi / speed)))
+    want = np.zeros(n, int)
+    for nx in range(-K, K + 1):
+        for ny in range(-K, K + 1):
+            dmin = max(0.0, 2.0 * max(abs(nx), abs(ny)) - 4.0)
+            if dmin >= chi[-1]:
+                continue
+            i0 = max(1, math.ceil(dmin * 420 / chi[-1]))
+            d = x + np.array([2 * nx - at[0], 2 * ny - at[1]])[:, None]
+            g = (np.abs(d).max(1) if metric == "square" else np.hypot(d[:, 0], d[:, 1])) - chi
+            want += ((g[:, i0 - 1:-1] < 0) != (g[:, i0:] < 0)).sum(1)
+    assert np.array_equal(np.bincount(bk.hits[0][0]["src"], minlength=n), want)
+
+
+def test_images_out_of_reach_cost_nothing(ug):
+    """One path, a front of radius one and 301 images a side: milliseconds (a thread per image
+    took 3, a warp that walked them all 840)."""
+    import time
+
+    from ugb200.frames import bake
+
+    took = []
+    for _ in range(4):
+        t0 = time.perf_counter()
+        bake(*_dump(1, 6, 8, 1), observers=[("point", 0.13, -0.29)], from_pi=0.3, to_pi=0.4, frames=4,
+             zmin_pi=0.05, front="fit", metric="square", wraps=150, hits=False)
+        took.append(time.perf_counter() - t0)
+    assert min(took) < 0.1

@@ -286,25 +286,35 @@ __device__ __forceinline__ int first_row(const FFront& F, int s) {
     return F.budget ? 1 : max(1, (int)ceil(dmin * F.M / F.chiMax));
 }
 
-// One warp per path.  A lane holds a rewind row (chunks of 32 rows, the first of which is
-// the last of the chunk before), a ballot the signs of dist(image) - chi_front at all of
-// them; neighbouring bits that differ are the crossings, which k_fb_refine bisects.
-// The square metric is separable: max(|dx|, |dy|) < chi is |dx| < chi and |dy| < chi, so
-// 2 (2K + 1) ballots serve the (2K + 1)^2 images and the lanes combine one image each.
-// Bound by issue: 0.11 ms for 18 k paths (one thread per (path, image) walking the 421
-// rows: 0.36 ms).
+// Nearest |n| to zero of n0 .. n0 + w - 1.
+__device__ __forceinline__ int nearest_ring(int n0, int w) { return n0 > 0 ? n0 : (n0 + w > 0 ? 0 : 1 - n0 - w); }
+
+// One warp per path and 32 x 32 of its (2K + 1)^2 torus images.  A lane holds a rewind row
+// (chunks of 32 rows, the first of which is the last of the chunk before), a ballot the
+// signs of dist(image) - chi_front at all of them; neighbouring bits that differ are the
+// crossings, which k_fb_refine bisects.  The square metric is separable: max(|dx|, |dy|) <
+// chi is |dx| < chi and |dy| < chi, so 2 x 32 ballots serve the 32 x 32 images and the
+// lanes combine one image each.  Chunks before the front reaches an image are left out.
+// Bound by issue: 0.11 ms for 18 k paths of 49 images (one thread per (path, image)
+// walking the 421 rows: 0.36 ms).  A warp for all images of a path, with a ballot each
+// beyond 32 a side, left a view of few paths and many images to few warps (one path, 301
+// images a side: 840 ms).
 __global__ void __launch_bounds__(128) k_fb_cross(FPaths P, FFront F, double ox, double oy, int K, int obsIdx,
                                                   const double* __restrict__ chig, const double* __restrict__ px,
                                                   const double* __restrict__ py, FCross* cross,
                                                   unsigned long long* count, unsigned long long cap) {
     const int lane = threadIdx.x & 31;
     const int warps = gridDim.x * (blockDim.x >> 5);
-    const int R = F.M + 1, side = 2 * K + 1;
-    const bool split = F.cheb && side <= 32;
-    for (int p = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); p < P.n; p += warps) {
+    const int R = F.M + 1, side = (2 * K + 32) / 32, tiles = side * side;  // tiles a side, in all
+    const int64_t items = (int64_t)P.n * tiles;
+    for (int64_t item = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); item < items; item += warps) {
+        const int p = (int)(item / tiles), tile = (int)(item % tiles);
+        const int x0 = tile % side * 32 - K, y0 = tile / side * 32 - K;
+        const int wx = min(32, K + 1 - x0), wy = min(32, K + 1 - y0), images = wx * wy;
+        const int first = first_row(F, max(nearest_ring(x0, wx), nearest_ring(y0, wy)));
         const double* X = px + (int64_t)p * R;
         const double* Y = py + (int64_t)p * R;
-        for (int c0 = 0; c0 + 1 < R; c0 += 31) {
+        for (int c0 = (first - 1) / 31 * 31; c0 + 1 < R; c0 += 31) {
             const int i = c0 + lane;
             const double x = i < R ? X[i] : 0.0, y = i < R ? Y[i] : 0.0, chi = i < R ? chig[i] : 0.0;
             // rows that a crossing may end at: all of the chunk's but its first
@@ -313,23 +323,29 @@ __global__ void __launch_bounds__(128) k_fb_cross(FPaths P, FFront F, double ox,
             const bool own = p == obsIdx && c0 == 0 && fabs(metric(x + (0.0 - ox), y + (0.0 - oy), F.cheb) - chi) < 1e-9;
             const bool own0 = __shfl_sync(0xffffffffu, (int)own, 0) != 0;
             uint32_t mx = 0, my = 0;
-            if (split)
-                for (int k = 0; k < side; k++) {
-                    const double b = 2.0 * (k - K);
-                    const uint32_t bx = __ballot_sync(0xffffffffu, i < R && fabs(x + (b - ox)) < chi);
-                    const uint32_t by = __ballot_sync(0xffffffffu, i < R && fabs(y + (b - oy)) < chi);
-                    if (lane == k) mx = bx, my = by;
+            if (F.cheb) {
+                for (int k = 0; k < wx; k++) {
+                    const uint32_t b = __ballot_sync(0xffffffffu, i < R && fabs(x + (2.0 * (x0 + k) - ox)) < chi);
+                    if (lane == k) mx = b;
                 }
-            for (int m0 = 0; m0 < side * side; m0 += 32) {
-                // this lane's image and the signs of its rows
+                for (int k = 0; k < wy; k++) {
+                    const uint32_t b = __ballot_sync(0xffffffffu, i < R && fabs(y + (2.0 * (y0 + k) - oy)) < chi);
+                    if (lane == k) my = b;
+                }
+            }
+            for (int m0 = 0; m0 < images; m0 += 32) {
+                // this lane's image and the signs of its rows, from the first that counts on
                 const int m = m0 + lane;
-                const int nx = m % side - K, ny = m / side - K;
+                const int xi = m % wx, yi = m / wx, nx = x0 + xi, ny = y0 + yi;
+                const int i0 = m < images ? first_row(F, max(abs(nx), abs(ny))) : R;
+                const uint32_t on = __ballot_sync(0xffffffffu, i0 < c0 + 32 && i0 < R);
+                if (!on) continue;
                 uint32_t sg = 0;
-                if (split) {
-                    sg = __shfl_sync(0xffffffffu, mx, (nx + K) & 31) & __shfl_sync(0xffffffffu, my, (ny + K) & 31);
+                if (F.cheb) {
+                    sg = __shfl_sync(0xffffffffu, mx, xi) & __shfl_sync(0xffffffffu, my, yi & 31);
                 } else {
-                    for (int q = 0; q < 32 && m0 + q < side * side; q++) {
-                        const int qx = (m0 + q) % side - K, qy = (m0 + q) / side - K;
+                    for (uint32_t w = on; w; w &= w - 1) {
+                        const int q = __ffs(w) - 1, qx = x0 + (m0 + q) % wx, qy = y0 + (m0 + q) / wx;
                         const uint32_t b = __ballot_sync(
                             0xffffffffu,
                             i < R && metric(x + (2.0 * qx - ox), y + (2.0 * qy - oy), F.cheb) - chi < 0.0);
@@ -337,11 +353,10 @@ __global__ void __launch_bounds__(128) k_fb_cross(FPaths P, FFront F, double ox,
                     }
                 }
                 uint32_t cr = 0;
-                if (m < side * side) {
-                    if (own0 && nx == 0 && ny == 0 && first_row(F, 0) == 1) sg |= 1u;
-                    const int i0 = first_row(F, max(abs(nx), abs(ny)));
+                if ((on >> lane) & 1u) {
+                    if (own0 && nx == 0 && ny == 0 && i0 == 1) sg |= 1u;
                     cr = (sg ^ (sg << 1)) & rows;
-                    if (i0 > c0) cr &= i0 - c0 < 32 ? ~((1u << (i0 - c0)) - 1u) : 0u;  // rows from i0 on
+                    if (i0 > c0) cr &= ~((1u << (i0 - c0)) - 1u);  // rows from i0 on
                 }
                 const uint32_t any = __ballot_sync(0xffffffffu, cr != 0u);
                 if (!any) continue;
@@ -874,7 +889,10 @@ int bake_device(const ug_frames_cfg* cfg, int n, int nw, int bMax, const double*
 search_again:  // (without hits: with more room)
     for (int fi = 0; fi < NF; fi++) {
         const FFront& F = fronts[fi];
-        const int K = Ks[fi];
+        // rings of images that the front reaches (as first_row says; further ones hold no hit)
+        int K = std::min(Ks[fi], (int)std::min(32767.0, std::max(2.0, ceil(0.5 * F.chiMax + 2.0))));
+        while (K > 2 && 2.0 * K - 4.0 >= F.chiMax) K--;
+        const int tiles = ((2 * K + 32) / 32) * ((2 * K + 32) / 32);
         const double* zg = dZg + (size_t)fi * (Mmax + 1);
         const double* chig = dChig + (size_t)fi * (Mmax + 1);
         if (F.budget) k_fb_reach<<<(bMax + 127) / 128, 128, 0, st>>>(bMax, F.zObs, dReach);
@@ -909,7 +927,7 @@ search_again:  // (without hits: with more room)
             }
             unsigned long long* cnt = dCount + (size_t)fi * NO + o;
             auto search = [&]() {
-                k_fb_cross<<<std::min((n + 3) / 4, nsm * 64), 128, 0, st>>>(
+                k_fb_cross<<<(int)std::min<int64_t>(((int64_t)n * tiles + 3) / 4, nsm * 64), 128, 0, st>>>(
                     P, F, ox, oy, K, cfg->obs_type[o] == 0 ? cfg->obs_path[o] : -1, chig, dPx, dPy, dCross, cnt, room);
                 k_fb_refine<<<nsm * 8, kFbThreads, 0, st>>>(P, F, ox, oy, zg, chig, dCross, cnt, room, dHits);
             };
