@@ -166,3 +166,30 @@ def test_images_out_of_reach_cost_nothing(ug):
              zmin_pi=0.05, front="fit", metric="square", wraps=150, hits=False)
         took.append(time.perf_counter() - t0)
     assert min(took) < 0.1
+
+
+def test_a_frequency_listed_many_times_adds_up_the_same_way(ug):
+    """Coefficients of repeated frequencies, within a warp's 32 terms and across them: the
+    hits of a dump equal those of the dump with each frequency's terms added up, and two
+    bakes are equal bit for bit."""
+    from ugb200.frames import bake
+
+    n, nw = 64, 70
+    r = np.random.default_rng(12)
+    b = r.integers(2, 34, (n, 2, nw)).astype(float)
+    a = r.dirichlet(np.ones(nw), (n, 2)) / b * r.choice([-1.0, 1.0], (n, 2, nw))
+    f = np.where(b % 2 == 0, r.uniform(0, math.pi, b.shape), 0.0)
+    a2 = r.uniform(-1, 1, (n, 2))
+    c = np.zeros((n, 2, 34), complex)
+    for j in range(nw):
+        np.add.at(c, (*np.indices((n, 2)), b[..., j].astype(int)), a[..., j] * np.exp(1j * f[..., j]))
+    sums = np.broadcast_to(np.arange(2.0, 34.0), (n, 2, 32))
+    kw = dict(observers=[("point", 0.1, 0.2)], from_pi=0.4, to_pi=0.4, zmin_pi=0.05, front="fit", metric="square")
+    one, two = (bake(a2, a, b, f, **kw).hits[0][0] for _ in range(2))
+    key = ("src", "chi", "dx", "dy", "z_emit")
+    assert len(one) > n // 2 and np.array_equal(np.sort(one, order=key), np.sort(two, order=key))
+    ref = bake(a2, np.abs(c[..., 2:]), sums, np.angle(c[..., 2:]), **kw).hits[0][0]
+    assert np.array_equal(np.bincount(one["src"], minlength=n), np.bincount(ref["src"], minlength=n))
+    x, y = np.sort(one, order=("src", "chi")), np.sort(ref, order=("src", "chi"))
+    for k in ("dx", "dy", "chi", "z_emit"):
+        np.testing.assert_allclose(x[k], y[k], atol=TOL)

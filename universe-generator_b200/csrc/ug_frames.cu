@@ -706,7 +706,8 @@ void h_comov(const std::vector<double>& a2, const std::vector<double>& a, const 
 }
 
 // Per (path, axis): s0 = sum_j a_j sin f_j, summed in term order, and the polynomial's
-// coefficients a_b e^{i f_b} (coef zeroed by the caller; a frequency listed twice adds up).
+// coefficients a_b e^{i f_b} (coef zeroed by the caller; a frequency listed more than once
+// adds up in term order).
 // One warp per (path, axis): coalesced reads and the sines spread over the lanes (18 k
 // paths of 255 terms: 0.55 -> 0.14 ms against a thread each).
 __global__ void __launch_bounds__(128) k_fb_prep(int n, int nw, int bmax, int horner, const double* __restrict__ a,
@@ -718,17 +719,27 @@ __global__ void __launch_bounds__(128) k_fb_prep(int n, int nw, int bmax, int ho
         double acc = 0.0, aa = 0.0;
         for (int j0 = 0; j0 < nw; j0 += 32) {
             const int j = j0 + lane;
-            double term = 0.0;
+            double term = 0.0, re = 0.0;
+            int fb = -1 - lane;  // no term: unlike any other lane's
             if (j < nw) {
                 const int64_t o = i * nw + j;
                 double sf, cf;
                 sincos(f[o], &sf, &cf);
                 aa += fabs(a[o]);
                 term = __dmul_rn(a[o], sf);
-                if (horner) {
-                    double2* c = coef + i * (bmax + 1) + (int)b[o];
-                    atomicAdd(&c->x, a[o] * cf);
-                    atomicAdd(&c->y, term);
+                re = __dmul_rn(a[o], cf);
+                fb = (int)b[o];
+            }
+            if (horner) {  // the lanes of one frequency take turns: one turn where all differ
+                const uint32_t same = __match_any_sync(0xffffffffu, fb);
+                const int rank = __popc(same & ((1u << lane) - 1u));
+                for (int turn = 0; __any_sync(0xffffffffu, rank >= turn); turn++) {
+                    if (rank == turn && j < nw) {
+                        double2* c = coef + i * (bmax + 1) + fb;
+                        c->x += re;
+                        c->y += term;
+                    }
+                    __syncwarp();
                 }
             }
             const int m = min(32, nw - j0);
