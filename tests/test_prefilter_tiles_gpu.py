@@ -1,6 +1,7 @@
-"""The prefilter on every kind of tile that the round plan makes -- full ones, ones of 64
-candidates, and full ones with a last wave of 64 or 32 -- against the FP64 form, which
-shares none of its kernels."""
+"""The prefilter on every kind of tile that the round plan makes -- full ones (up to 128 live
+rows: the epilogue's narrowest stages), ones of 64 candidates, and full ones with a last
+wave of 64 or 32 -- against the FP64 form, which shares none of its kernels.  Small rounds
+of a universe alone take tiles of 32 only."""
 
 import functools
 
@@ -37,6 +38,9 @@ def _universe(ug, dim, T, mode, euclid, rs):
 
 
 @pytest.mark.parametrize("dim,T,mode,euclid", [
+    (1, 4, 0, 0), (1, 33, 0, 0), (2, 4, 0, 0), (2, 9, 0, 0), (2, 17, 0, 0), (2, 31, 1, 0), (2, 40, 0, 1),
+    (2, 65, 2, 0), (2, 129, 2, 0), (2, 255, 0, 0), (2, 256, 2, 0), (3, 5, 0, 0), (3, 16, 0, 0), (3, 33, 0, 0), (3, 47, 2, 1),
+    (3, 128, 0, 0), (3, 170, 0, 0),
     (3, 171, 0, 0), (3, 193, 0, 1), (3, 176, 2, 0),  # two passes of the columns
 ])
 @pytest.mark.parametrize("plan", ["full", "64", "full+64", "full+32"])
