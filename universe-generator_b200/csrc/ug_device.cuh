@@ -170,7 +170,7 @@ struct UniCtl {
     int32_t phase;         // 1 or 2
     int32_t state;         // ST_*
     int32_t epoch;         // round-table epoch
-    int32_t n_gray;        // unused
+    int32_t n_gray;        // 0; keeps the layout of saved states
     int32_t accepted_round;
     int64_t gray_total;    // mixed: FP64 retests over the run
     int64_t rounds;

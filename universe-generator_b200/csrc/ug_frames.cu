@@ -27,6 +27,7 @@
 #include <string>
 #include <vector>
 
+#include "ug_dmma.cuh"
 #include "ug_frames.cuh"
 
 namespace ug {
@@ -165,16 +166,6 @@ __global__ void k_fb_basis(int bmax, int R, int Rp, const double* __restrict__ z
         basis[(int64_t)(2 * b) * Rp + c] = s;
         basis[(int64_t)(2 * b + 1) * Rp + c] = co;
     }
-}
-
-// FP64 tensor product D += A B, 16 x 8 x 8.  Lane (g, t) = (lane / 4, lane % 4) holds
-// A(g, t), A(g + 8, t), A(g, t + 4), A(g + 8, t + 4); B(t, g), B(t + 4, g); and
-// D(g, 2t), D(g, 2t + 1), D(g + 8, 2t), D(g + 8, 2t + 1).
-__device__ __forceinline__ void dmma_16x8x8(double* d, const double* a, const double* b) {
-    asm volatile(
-        "mma.sync.aligned.m16n8k8.row.col.f64.f64.f64.f64 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-        : "+d"(d[0]), "+d"(d[1]), "+d"(d[2]), "+d"(d[3])
-        : "d"(a[0]), "d"(a[1]), "d"(a[2]), "d"(a[3]), "d"(b[0]), "d"(b[1]));
 }
 
 // One CTA per 64 x 72 tile, a warp per 16 rows (9 products of 16 x 8 a step of four

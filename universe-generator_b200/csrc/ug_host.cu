@@ -52,7 +52,8 @@ enum KernelId {
     K_PLAN, K_PRE, K_MIXED, K_CONFIRM, K_COMPACT, K_SGEN, K_CONFL, K_GREEDY, K_COMMIT, K_SGEMM, K_SHASH,
     K_NK
 };
-// names of the timed stages: k_prefilter64w is k_test64's, k_confirm64w is k_retest's
+// names of the timed stages, part of the interface: k_prefilter64w is k_test64's, k_confirm64w
+// is k_retest's
 static const char* kKernelNames[12] = {"k_plan",      "k_prefilter64w", "k_prefilter_mixed",
                                        "k_confirm64w", "k_compact",     "k_surv_gen",
                                        "k_conflicts", "k_greedy",      "k_commit",
@@ -414,8 +415,8 @@ static int setup_universe(Batch& B, UniHost& h, int64_t dense_budget, int64_t* d
     if ((rc = alloc_points(h, cap, &B.arena))) return rc;
     // round buffers
     const int Bm = d.B_max, Sm = d.S_max;
-    if ((rc = dalloc(B, &d.surv_bits, Bm / 32, 0)) ||         (rc = dalloc(B, &d.g0, Bm, 0xff)) || (rc = dalloc(B, &d.surv_off, Sm + 1, 0)) ||
-        (rc = dalloc(B, &d.spos, (size_t)Sm * T, 0)) || (rc = dalloc(B, &d.ccount, Sm, 0)) ||
+    if ((rc = dalloc(B, &d.surv_bits, Bm / 32, 0)) || (rc = dalloc(B, &d.g0, Bm, 0xff)) ||
+        (rc = dalloc(B, &d.surv_off, Sm + 1, 0)) || (rc = dalloc(B, &d.spos, (size_t)Sm * T, 0)) || (rc = dalloc(B, &d.ccount, Sm, 0)) ||
         (rc = dalloc(B, &d.clist, (size_t)Sm * kConflictCap, 0)) ||
         (rc = dalloc(B, &d.sgid, Sm, 0xff)) || (rc = dalloc(B, &d.acc_rank, Sm, 0xff)))
         return rc;

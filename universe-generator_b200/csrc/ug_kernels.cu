@@ -21,6 +21,7 @@
 // order against the round's earlier admissions.  The accepted set is
 // therefore exactly sequential RSA over the candidate stream -- the
 // exact-index admission of cuda/braid_knot.cu:433-462, made device-resident.
+#include "ug_dmma.cuh"
 #include "ug_kernels.cuh"
 
 #include <algorithm>
@@ -140,7 +141,6 @@ __global__ void k_plan(const UniDev* __restrict__ U, UniCtl* ctl, RoundInfo* inf
         c.B = B;
         c.round_base = c.next_cand;
         c.S = c.S_raw = c.trunc = c.stop_at = 0;
-        c.n_gray = 0;
         if (B > 0) c.epoch = (c.epoch + 1) & 0xFFFFFF;
         ntiles[u] = (B + kTile - 1) / kTile;
         if (B > 0) {
@@ -299,7 +299,6 @@ __device__ __forceinline__ bool group_phase(const UniDev& d, const UniCtl& c) {
 }
 
 // --------------------------------------------------------------- compact
-
 
 __global__ void __launch_bounds__(256) k_compact(const UniDev* __restrict__ U, UniCtl* ctl,
                                                  RoundInfo* info) {
@@ -668,23 +667,6 @@ __global__ void __launch_bounds__(32 * kSurvWarps) k_restore_gen(const UniDev* _
         store_coef_rows(d, r, alpha, beta, a2, lane);
         __syncwarp();
     }
-}
-
-// FP64 tensor products D += A B.  8 x 8 x 4: lane (g, t) = (lane / 4, lane % 4) holds A(g, t),
-// B(t, g) and D(g, 2t), D(g, 2t + 1).  16 x 8 x 8: A(g, t), A(g + 8, t), A(g, t + 4),
-// A(g + 8, t + 4); B(t, g), B(t + 4, g); D(g, 2t), D(g, 2t + 1), D(g + 8, 2t), D(g + 8, 2t + 1).
-// Each element accumulates its products in ascending order, one rounding each: the same
-// bits as a chain of fused multiply-adds.
-__device__ __forceinline__ void dmma_8x8x4(double* d, double a, double b) {
-    asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};"
-                 : "+d"(d[0]), "+d"(d[1])
-                 : "d"(a), "d"(b));
-}
-__device__ __forceinline__ void dmma_16x8x8(double* d, const double* a, const double* b) {
-    asm volatile(
-        "mma.sync.aligned.m16n8k8.row.col.f64.f64.f64.f64 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-        : "+d"(d[0]), "+d"(d[1]), "+d"(d[2]), "+d"(d[3])
-        : "d"(a[0]), "d"(a[1]), "d"(a[2]), "d"(a[3]), "d"(b[0]), "d"(b[1]));
 }
 
 // k_surv_gemm: X[row][t] = wrap(a2 + invsinz_t * sum_k coef[k][row] KT[k][t]), one warp per
