@@ -92,11 +92,13 @@ int main() {
         const size_t n = g_mallocs;
         for (int i = 0; i < 4; i++) params(), positions();
         CHECK(g_mallocs == n && g_frees == 0);
-        for (size_t k = 1; k < 40; k++) {
-            { CallScope s(&cache); s.get<char>(k * 7 * MB); s.get<char>(k * 3 * MB); }
+        CallBuffers other;
+        for (size_t k = 1; k < 160; k++) {
+            { CallScope s(k % 3 ? &cache : &other); s.get<char>(k * 7 * MB); s.get<char>(k * 3 * MB); }
             CHECK(g_used <= CallBuffers::kKeep);
         }
         { CallScope s(&cache); s.get<char>(CallBuffers::kKeep + 1); }
+        { CallScope s(&other); s.get<char>(CallBuffers::kKeep / 2); }
         CHECK(g_used <= CallBuffers::kKeep && g_used > 0);
     }
     CHECK(g_live.empty());
