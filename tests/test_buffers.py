@@ -11,6 +11,7 @@ CSRC = os.path.join(ROOT, "universe-generator_b200", "csrc")
 
 RUNTIME = r"""
 #pragma once
+#include <atomic>
 #include <cstddef>
 #include <cstdint>
 #include <cstdlib>
@@ -40,6 +41,11 @@ inline cudaError_t cudaFree(void* p) {
     return cudaSuccess;
 }
 inline cudaError_t cudaGetLastError() { return cudaSuccess; }
+using cudaStream_t = struct Stream*;
+inline int g_device = 0;
+inline std::atomic<size_t> g_waits{0};
+inline cudaError_t cudaGetDevice(int* d) { *d = g_device; return cudaSuccess; }
+inline cudaError_t cudaStreamSynchronize(cudaStream_t) { g_waits++; return cudaSuccess; }
 """
 
 PROLOGUE = r"""
@@ -53,16 +59,16 @@ constexpr size_t MB = (size_t)1 << 20;
 """
 
 PROGRAMS = {
-    # calls of several threads on one batch never hold the same block
+    # calls of several threads and batches never hold the same block
     "threads": r"""
 int main() {
     {
-        CallBuffers cache;
+        CallBuffers::User batch[2];
         std::mutex mu;
         std::set<void*> held;
         auto work = [&](unsigned seed) {
             for (int i = 0; i < 3000; i++) {
-                CallScope s(&cache);
+                CallScope s((cudaStream_t) nullptr);
                 char* p[3];
                 for (auto& q : p) {
                     q = s.get<char>((1 + rand_r(&seed) % 5) * MB);
@@ -82,46 +88,64 @@ int main() {
 }
 """,
     # calls of different kinds in turn allocate nothing once each has run; what is kept is bounded
+    # and goes with the last batch; a call's stream is waited for before its blocks come back
     "in_turn": r"""
 int main() {
+    auto params = [&] { CallScope s((cudaStream_t) nullptr); s.get<char>(MB); s.get<char>(24 * MB); s.get<char>(24 * MB); s.get<char>(12 * MB); };
+    auto positions = [&] { CallScope s((cudaStream_t) nullptr); s.get<char>(100 * MB); };
+    params();
+    CHECK(g_live.empty());  // no batch
     {
-        CallBuffers cache;
-        auto params = [&] { CallScope s(&cache); s.get<char>(MB); s.get<char>(24 * MB); s.get<char>(24 * MB); s.get<char>(12 * MB); };
-        auto positions = [&] { CallScope s(&cache); s.get<char>(100 * MB); };
-        params(), positions();
-        const size_t n = g_mallocs;
-        for (int i = 0; i < 4; i++) params(), positions();
-        CHECK(g_mallocs == n && g_frees == 0);
-        CallBuffers other;
+        CallBuffers::User batch;
+        {
+            CallBuffers::User other;
+            params(), positions();
+            const size_t n = g_mallocs, f = g_frees, w = g_waits;
+            for (int i = 0; i < 4; i++) params(), positions();
+            CHECK(g_mallocs == n && g_frees == f && g_waits == w + 8);
+        }
+        CHECK(g_used == 161 * MB);
         for (size_t k = 1; k < 160; k++) {
-            { CallScope s(k % 3 ? &cache : &other); s.get<char>(k * 7 * MB); s.get<char>(k * 3 * MB); }
+            { CallScope s((cudaStream_t) nullptr); s.get<char>(k * 7 * MB); s.get<char>(k * 3 * MB); }
             CHECK(g_used <= CallBuffers::kKeep);
         }
-        { CallScope s(&cache); s.get<char>(CallBuffers::kKeep + 1); }
-        { CallScope s(&other); s.get<char>(CallBuffers::kKeep / 2); }
+        { CallScope s((cudaStream_t) nullptr); s.get<char>(CallBuffers::kKeep + 1); }
         CHECK(g_used <= CallBuffers::kKeep && g_used > 0);
+        { CallScope own; CHECK(own.get<char>(MB)); }
     }
     CHECK(g_live.empty());
 }
 """,
-    # what other batches keep makes room for an allocation that would fail; what calls hold does not
+    # a block stays on its device
+    "devices": r"""
+int main() {
+    CallBuffers::User batch;
+    { CallScope s((cudaStream_t) nullptr); s.get<char>(8 * MB); }
+    g_device = 1;
+    { CallScope s((cudaStream_t) nullptr); s.get<char>(8 * MB); }
+    CHECK(g_mallocs == 2);
+    g_device = 0;
+    { CallScope s((cudaStream_t) nullptr); s.get<char>(8 * MB); }
+    CHECK(g_mallocs == 2);
+}
+""",
+    # what is kept makes room for an allocation that would fail; what calls hold does not
     "room": r"""
 int main() {
     {
-        CallBuffers a, b;
+        CallBuffers::User batch;
         g_limit = 300 * MB;
-        { CallScope s(&a); s.get<char>(100 * MB); }
-        CallScope held(&b);
+        CallScope held((cudaStream_t) nullptr);
         CHECK(held.get<char>(80 * MB));
-        { CallScope s(&b); s.get<char>(60 * MB); }
-        CHECK(g_used == 240 * MB);
+        { CallScope s((cudaStream_t) nullptr); s.get<char>(100 * MB); s.get<char>(40 * MB); }
+        CHECK(g_used == 220 * MB);
         int64_t* p = nullptr;
         CHECK(dev_malloc(&p, 200 * MB) == cudaSuccess && g_used == 280 * MB);
         Arena arena;
         void* q = nullptr;
         CHECK(arena.take(100 * MB, &q) != cudaSuccess && !held.get<char>(100 * MB));
         cudaFree(p);
-        { CallScope s(&a); s.get<char>(200 * MB); }
+        { CallScope s((cudaStream_t) nullptr); s.get<char>(200 * MB); }
         CHECK(arena.take(100 * MB, &q) == cudaSuccess && g_used == 180 * MB);
     }
     CHECK(g_live.empty());
@@ -147,11 +171,11 @@ int main() {
     "room_threads": r"""
 int main() {
     {
-        CallBuffers cache[4];
+        CallBuffers::User batch;
         g_limit = 4 * 12 * MB;
         auto work = [&](unsigned seed) {
             for (int i = 0; i < 2000; i++) {
-                CallScope s(&cache[rand_r(&seed) % 4]);
+                CallScope s((cudaStream_t) nullptr);
                 s.get<char>((1 + rand_r(&seed) % 6) * MB);
                 s.get<char>((1 + rand_r(&seed) % 6) * MB);
             }

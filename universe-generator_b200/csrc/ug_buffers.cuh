@@ -4,7 +4,6 @@
 #include <sys/mman.h>
 
 #include <algorithm>
-#include <atomic>
 #include <cstdint>
 #include <mutex>
 #include <thread>
@@ -12,116 +11,111 @@
 
 namespace ug {
 
-// cudaMalloc of the library's own buffers: where there is no memory, the blocks that batches
-// keep from finished calls are given back, and it is tried once more.
-inline cudaError_t dev_malloc(void** p, size_t bytes);
-template <class T>
-cudaError_t dev_malloc(T** p, size_t bytes) {
-    return dev_malloc((void**)p, bytes);
-}
-
-// Device buffers of a batch's finished read-back and frame calls, kept for its next ones
-// (which run on the same stream).  A block belongs to one call at a time, so calls of
-// several threads on one batch are as independent as with buffers of their own.  A job that
-// reads parameters and trajectories in turn allocates nothing from its second pass on.  All
-// batches together keep at most kKeep bytes; beyond that a batch gives its longest unused
-// blocks back.  The densities of 32 frames of 1024 x 1024 and two observers of 25 k paths
-// need 0.9 GB (64.9 ms a call; 71.6 with a bound of 256 MB, which most of it exceeds).
+// Device blocks of finished read-back and frame calls, kept for the next ones of any batch of
+// the process while there is a batch.  A block belongs to one call at a time and comes back
+// when that call's work has ended, so calls of several threads, batches and streams are as
+// independent as with buffers of their own.  A job that reads parameters and trajectories in
+// turn allocates nothing from its second pass on.  At most kKeep bytes are kept, the longest
+// unused go first; all go where an allocation of the library finds no memory, and with the
+// last batch.  The densities of 32 frames of 1024 x 1024 and two observers of 25 k paths need
+// 0.9 GB (64.9 ms a call; 71.6 with a bound of 256 MB, which most of it exceeds).
 class CallBuffers {
 public:
     struct Block {
         void* p;
         size_t n;
+        int dev;
     };
-    CallBuffers() {
-        std::lock_guard<std::mutex> lock(all_mu());
-        all().push_back(this);
+    static constexpr size_t kKeep = (size_t)1 << 30;
+
+    static CallBuffers& get() {  // never destroyed: a batch may outlive static objects
+        static CallBuffers* b = new CallBuffers;
+        return *b;
     }
-    ~CallBuffers() {
-        {
-            std::lock_guard<std::mutex> lock(all_mu());
-            all().erase(std::find(all().begin(), all().end(), this));
-        }
-        drop();
-    }
-    CallBuffers(const CallBuffers&) = delete;
     // A kept block of about this size, or a new one; p is null when there is no memory.
-    Block take(size_t bytes) {
-        {
-            std::lock_guard<std::mutex> lock(mu_);
-            auto best = kept_.end();
-            for (auto b = kept_.begin(); b != kept_.end(); ++b)
-                if (b->n >= bytes && b->n <= 2 * bytes + (1 << 16) && (best == kept_.end() || b->n < best->n)) best = b;
-            if (best != kept_.end()) {
-                const Block r = *best;
-                kept_.erase(best);
-                total() -= r.n;
-                return r;
-            }
-        }
-        Block r{nullptr, bytes};
-        if (dev_malloc(&r.p, bytes) != cudaSuccess) r.p = nullptr;
-        return r;
-    }
+    Block take(size_t bytes);
     // The blocks of a finished call.
     void give(std::vector<Block>& blocks) {
         std::lock_guard<std::mutex> lock(mu_);
         for (const Block& b : blocks) {
-            if (b.n > kKeep) {
+            if (users_ == 0 || b.n > kKeep) {
                 cudaFree(b.p);
                 continue;
             }
             kept_.push_back(b);
-            total() += b.n;
+            bytes_ += b.n;
         }
         blocks.clear();
         size_t k = 0;
-        for (; k < kept_.size() && total() > kKeep; k++) {
-            total() -= kept_[k].n;
+        for (; bytes_ > kKeep; k++) {
+            bytes_ -= kept_[k].n;
             cudaFree(kept_[k].p);
         }
         kept_.erase(kept_.begin(), kept_.begin() + k);
     }
     void drop() {
         std::lock_guard<std::mutex> lock(mu_);
-        for (Block& b : kept_) {
-            total() -= b.n;
-            cudaFree(b.p);
+        free_all();
+    }
+    // A batch: while there is one, blocks are kept.
+    struct User {
+        User() {
+            std::lock_guard<std::mutex> lock(get().mu_);
+            get().users_++;
         }
-        kept_.clear();
-    }
-    static void drop_all() {
-        std::lock_guard<std::mutex> lock(all_mu());
-        for (CallBuffers* c : all()) c->drop();
-    }
-    static constexpr size_t kKeep = (size_t)1 << 30;
+        ~User() {
+            std::lock_guard<std::mutex> lock(get().mu_);
+            if (--get().users_ == 0) get().free_all();
+        }
+        User(const User&) = delete;
+    };
 
 private:
-    // every cache of the process (never destroyed: a batch may outlive static objects)
-    static std::mutex& all_mu() {
-        static std::mutex* m = new std::mutex;
-        return *m;
-    }
-    static std::vector<CallBuffers*>& all() {
-        static std::vector<CallBuffers*>* v = new std::vector<CallBuffers*>;
-        return *v;
-    }
-    static std::atomic<size_t>& total() {  // kept by all of them
-        static std::atomic<size_t> n{0};
-        return n;
+    void free_all() {
+        for (Block& b : kept_) cudaFree(b.p);
+        kept_.clear();
+        bytes_ = 0;
     }
     std::mutex mu_;
     std::vector<Block> kept_;  // the longest unused first
+    size_t bytes_ = 0;
+    int users_ = 0;
 };
 
+// cudaMalloc of the library's own buffers: where there is no memory, the blocks kept from
+// finished calls are given back, and it is tried once more.
 inline cudaError_t dev_malloc(void** p, size_t bytes) {
     cudaError_t e = cudaMalloc(p, bytes);
     if (e != cudaErrorMemoryAllocation) return e;
     cudaGetLastError();
-    CallBuffers::drop_all();
+    CallBuffers::get().drop();
     e = cudaMalloc(p, bytes);
     if (e == cudaErrorMemoryAllocation) cudaGetLastError();  // reported here, not at a later launch
     return e;
+}
+template <class T>
+cudaError_t dev_malloc(T** p, size_t bytes) {
+    return dev_malloc((void**)p, bytes);
+}
+
+inline CallBuffers::Block CallBuffers::take(size_t bytes) {
+    Block r{nullptr, bytes, 0};
+    cudaGetDevice(&r.dev);
+    {
+        std::lock_guard<std::mutex> lock(mu_);
+        auto best = kept_.end();
+        for (auto b = kept_.begin(); b != kept_.end(); ++b)
+            if (b->dev == r.dev && b->n >= bytes && b->n <= 2 * bytes + (1 << 16) && (best == kept_.end() || b->n < best->n))
+                best = b;
+        if (best != kept_.end()) {
+            r = *best;
+            kept_.erase(best);
+            bytes_ -= r.n;
+            return r;
+        }
+    }
+    if (dev_malloc(&r.p, bytes) != cudaSuccess) r.p = nullptr;
+    return r;
 }
 
 // A batch's fixed buffers, carved from chunks: a cudaMalloc and its cudaFree take 0.3 to
@@ -168,23 +162,38 @@ private:
     size_t left_ = 0, next_ = (size_t)4 << 20;
 };
 
-// The buffers of one call: taken from its batch's kept ones and given back at the end, or
-// (no cache) the call's own.
+// The buffers of one call.  A batch's call (on the batch's stream) takes them from the kept ones
+// and gives them back at its end, after the stream's work (an early return may leave some); a
+// call without a batch has its own.
 class CallScope {
 public:
-    explicit CallScope(CallBuffers* cache) : cache_(cache ? cache : &own_) {}
+    CallScope() = default;
+    explicit CallScope(cudaStream_t st) : kept_(true), st_(st) {}
     CallScope(const CallScope&) = delete;
-    ~CallScope() { cache_->give(blocks_); }
+    ~CallScope() {
+        if (blocks_.empty()) return;
+        if (kept_) {
+            cudaStreamSynchronize(st_);
+            CallBuffers::get().give(blocks_);
+        } else {
+            for (CallBuffers::Block& b : blocks_) cudaFree(b.p);
+        }
+    }
     template <class T>
     T* get(size_t n) {
-        const CallBuffers::Block b = cache_->take(std::max<size_t>(n, 1) * sizeof(T));
+        const size_t bytes = std::max<size_t>(n, 1) * sizeof(T);
+        CallBuffers::Block b{nullptr, bytes, 0};
+        if (kept_)
+            b = CallBuffers::get().take(bytes);
+        else if (dev_malloc(&b.p, bytes) != cudaSuccess)
+            b.p = nullptr;
         if (b.p) blocks_.push_back(b);
         return (T*)b.p;
     }
 
 private:
-    CallBuffers own_;
-    CallBuffers* cache_;
+    bool kept_ = false;
+    cudaStream_t st_ = nullptr;
     std::vector<CallBuffers::Block> blocks_;
 };
 

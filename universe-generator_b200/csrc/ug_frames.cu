@@ -1085,7 +1085,7 @@ extern "C" int ug_frame_bake(const ug_frames_cfg* cfg, int32_t n, int32_t nw, co
     if (rc) return rc;
     int bMax = 2;
     for (size_t i = 0; i < (size_t)n * 2 * nw; i++) bMax = std::max(bMax, (int)b[i]);
-    CallScope buf(nullptr);
+    CallScope buf;
     const size_t m = (size_t)n * 2 * nw;
     double* dA2 = buf.get<double>((size_t)n * 2);
     double* dA = buf.get<double>(m);
@@ -1219,7 +1219,7 @@ extern "C" int ug_apparent_positions(const ug_hit* hits, int64_t n, double beta_
     int rc = check_view(n, mode);
     if (rc || n == 0) return rc;
     if (!hits || !ax || !ay || !ln_dopp) return set_error(UG_EINVAL, "apparent_positions: null buffer");
-    CallScope buf(nullptr);
+    CallScope buf;
     ug_hit* dH = buf.get<ug_hit>((size_t)n);
     double* dO = buf.get<double>((size_t)n * 3);
     if (!dH || !dO) return set_error(UG_ENOMEM, "apparent_positions: device allocation failed");

@@ -72,7 +72,7 @@ struct UniHost {
 
 struct Batch {
     Arena arena;         // fixed buffers
-    CallBuffers call;    // buffers of read-back and frame calls
+    CallBuffers::User calls;  // keeps the buffers of read-back and frame calls
     int dev = 0;
     cudaStream_t st = nullptr;
     bool own_stream = false;
@@ -988,7 +988,7 @@ int ug_batch_positions(void* h, int32_t u, double* pos, int64_t cap_paths) {
     const size_t m = (size_t)N * d.dim * d.T;
     PagesAhead pages;
     pages.add(pos, m * sizeof(double));
-    CallScope buf(&B->call);
+    CallScope buf(B->st);
     double* dp = buf.get<double>(m);
     if (!dp) return fail(UG_ENOMEM, "positions: device allocation failed");
     k_positions<<<(int)std::min<int64_t>((N * d.T + 255) / 256, (int64_t)B->nsm * 16), 256, 0, B->st>>>(B->dU, u, N, dp);
@@ -1014,7 +1014,7 @@ int ug_batch_params(void* h, int32_t u, double* a2, double* a, int32_t* b, doubl
     pages.add(a, nt * 8);
     pages.add(f, nt * 8);
     pages.add(b, nt * 4);
-    CallScope buf(&B->call);
+    CallScope buf(B->st);
     double* da2 = buf.get<double>((size_t)N * D);
     double* da = buf.get<double>(nt);
     double* df = buf.get<double>(nt);
@@ -1041,7 +1041,7 @@ int ug_batch_frames(void* h, int32_t u, const ug_frames_cfg* cfg, ug_frames_out*
     if (N < 1) return fail(UG_EINVAL, "frames: the universe has no accepted paths");
     if (N > INT32_MAX / 2) return fail(UG_ECAP, "frames: too many paths");
     const int nw = B->U[u].d.nw;
-    CallScope buf(&B->call);
+    CallScope buf(B->st);
     double* da2 = buf.get<double>((size_t)N * 2);
     double* da = buf.get<double>((size_t)N * 2 * nw);
     double* df = buf.get<double>((size_t)N * 2 * nw);
